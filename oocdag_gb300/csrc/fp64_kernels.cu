@@ -43,14 +43,14 @@ __device__ __forceinline__ void dmma884(double& c0, double& c1, double a, double
 
 // Loads rows [r0, r0+BMX) x columns [k0, k0+16) of the column-major operand M (rows
 // valid below `rows`, columns below `kmax`) into S[k][r] (row length BMX + PAD).
-template <bool VEC, int BMX = BM>
+template <bool VEC, int BMX = BM, int BKX = BK>
 __device__ __forceinline__ void load_slab(double* S, const double* M, i64 ld, int r0, int rows,
                                           int k0, int kmax) {
   constexpr int L = BMX + PAD;
   const int t = threadIdx.x;
   if (VEC) {
 #pragma unroll
-    for (int it = 0; it < (BMX * BK / 2) / GEMM_THREADS; it++) {
+    for (int it = 0; it < (BMX * BKX / 2) / GEMM_THREADS; it++) {
       int idx = t + it * GEMM_THREADS;
       int kc = idx / (BMX / 2);
       int r = (idx % (BMX / 2)) * 2;
@@ -61,7 +61,7 @@ __device__ __forceinline__ void load_slab(double* S, const double* M, i64 ld, in
       cp_async16(S + kc * L + r, src, nvalid * 8);
     }
   } else {
-    for (int idx = t; idx < BMX * BK; idx += GEMM_THREADS) {
+    for (int idx = t; idx < BMX * BKX; idx += GEMM_THREADS) {
       int kc = idx / BMX;
       int r = idx % BMX;
       int gr = r0 + r, gk = k0 + kc;
@@ -81,10 +81,11 @@ __device__ __forceinline__ void gemm_block(const double* __restrict__ A, i64 lda
                                            double* __restrict__ C, i64 ldc, int m, int n, int k,
                                            int m0, int n0, int lower, double alpha) {
   constexpr int L = BMX + PAD;
+  constexpr int BKX = BMX == 16 ? 64 : BK;  // a 16 x 16 block takes K <= 64 in one slab: one round trip
   constexpr int TI = BMX / 16;  // DMMA tiles per warp dimension
   constexpr int WT = BMX / 2;   // warp tile
-  __shared__ __align__(16) double As[2][BK * L];
-  __shared__ __align__(16) double Bs[2][BK * L];
+  __shared__ __align__(16) double As[2][BKX * L];
+  __shared__ __align__(16) double Bs[2][BKX * L];
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
   const int wm = warp & 1, wn = warp >> 1;
@@ -96,17 +97,17 @@ __device__ __forceinline__ void gemm_block(const double* __restrict__ A, i64 lda
 #pragma unroll
     for (int j = 0; j < TI; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
 
-  const int nslab = (k + BK - 1) / BK;
+  const int nslab = (k + BKX - 1) / BKX;
   if (nslab > 0) {
-    load_slab<VEC, BMX>(As[0], A, lda, m0, m, 0, k);
-    load_slab<VEC, BMX>(Bs[0], B, ldb, n0, n, 0, k);
+    load_slab<VEC, BMX, BKX>(As[0], A, lda, m0, m, 0, k);
+    load_slab<VEC, BMX, BKX>(Bs[0], B, ldb, n0, n, 0, k);
     if (VEC) cp_async_commit();
   }
   for (int s = 0; s < nslab; s++) {
     const int cur = s & 1;
     if (s + 1 < nslab) {
-      load_slab<VEC, BMX>(As[cur ^ 1], A, lda, m0, m, (s + 1) * BK, k);
-      load_slab<VEC, BMX>(Bs[cur ^ 1], B, ldb, n0, n, (s + 1) * BK, k);
+      load_slab<VEC, BMX, BKX>(As[cur ^ 1], A, lda, m0, m, (s + 1) * BKX, k);
+      load_slab<VEC, BMX, BKX>(Bs[cur ^ 1], B, ldb, n0, n, (s + 1) * BKX, k);
       if (VEC) { cp_async_commit(); cp_async_wait<1>(); }
     } else {
       if (VEC) cp_async_wait<0>();
@@ -114,8 +115,8 @@ __device__ __forceinline__ void gemm_block(const double* __restrict__ A, i64 lda
     __syncthreads();
     const double* as = As[cur];
     const double* bs = Bs[cur];
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
+#pragma unroll 4
+    for (int kk = 0; kk < BKX; kk += 4) {
       double a[TI], b[TI];
 #pragma unroll
       for (int i = 0; i < TI; i++) a[i] = as[(kk + tig) * L + wm * WT + i * 8 + g];
@@ -210,143 +211,221 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm_batched(GemmBatch gb, con
 }
 
 // ---------------------------------------------------------------------------------
-// Unblocked lower Cholesky of an n x n block (n <= 64) in shared memory, right-looking.
-// LAPACK convention: a pivot that is not > 0 (or is NaN) stops the factorization and
-// reports info = col0 + j + 1.
+// Lower Cholesky of an n x n block (n <= 64) in shared memory, by four warps in column
+// blocks of 16.  A warp-wide FP64 instruction occupies its SM sub-partition for 64 clocks
+// whatever its active lanes, and an SM issues one per 19 clocks, so both the number of FP64
+// instructions and the dependent chain per column count:
+//   * inside a block the columns stay unscaled (a(r,j), not l(r,j)): thread (row r, half h)
+//     holds every second column of its row in registers, and column j's step is
+//     u = a(r,j) / d, a(r,c) -= u a(c,j), with the quotient from an FP32 reciprocal seed
+//     refined by one cubic Newton step (e = 1 - d r0, a r0 (1 + e + e^2): error e^3 <
+//     2^-66), four dependent FP64 instructions where a square root and a division took
+//     twenty; one barrier per column;
+//   * the 16 square roots and their reciprocals are taken side by side at the block's end;
+//   * the columns to the right take the block as one rank-16 update on the FP64 MMA.
+// Measured on a 64 x 64 block: 90 us with a square root and a division per column on the
+// barrier-to-barrier path, 50 us now.
+// LAPACK convention: a pivot that is not > 0 (or is NaN) stops the factorization and reports
+// info = col0 + j + 1; the columns before it are written back.
 // ---------------------------------------------------------------------------------
 constexpr int SB = 64;
+constexpr int PB = 16;               // columns per block
+constexpr int PT_THREADS = 128;
+constexpr int SP = SB + 1;           // column pitch in shared memory
 
-__global__ void __launch_bounds__(256) k_potrf_small(double* A, i64 ld, int n, i64 col0, int* status) {
+// r0 ~ 1 / d to 23 bits, from the FP32 reciprocal of the mantissa, for a d well inside the
+// exponent range (recip_ok).
+__device__ __forceinline__ bool recip_ok(double d) {
+  return (unsigned)((__double2hiint(d) >> 20) - 23) <= 2000u;  // 2^-1000 <= d < 2^1001
+}
+__device__ __forceinline__ double recip_seed(double d) {
+  const int hi = __double2hiint(d), lo = __double2loint(d);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(0x3F800000u | ((uint32_t)(hi & 0xFFFFF) << 3) | ((uint32_t)lo >> 29))));
+  const uint32_t rb = __float_as_uint(r);  // in [1/2, 1]
+  const int e = (int)(rb >> 23) - 127 - ((hi >> 20) - 1023) + 1023;
+  return __hiloint2double((e << 20) | (int)((rb & 0x7FFFFFu) >> 3), (int)(rb << 29));
+}
+__device__ __noinline__ double slow_div(double a, double d) { return a / d; }
+__device__ __forceinline__ bool positive(double d) {  // d > 0 (false for NaN), off the FP64 pipe
+  return (unsigned long long)__double_as_longlong(d) - 1ull < 0x7FF0000000000000ull;
+}
+
+__global__ void __launch_bounds__(PT_THREADS) k_potrf_small(double* A, i64 ld, int n, i64 col0, int* status) {
   if (*(volatile int*)status) return;
-  __shared__ double S[SB][SB + 1];  // S[col][row]
-  __shared__ int failed;
-  __shared__ double s_inv;
-  const int t = threadIdx.x;
-  {  // 64 rows x 4 column groups: 16 loads in flight per thread
+  __shared__ double S[SB * SP];       // S[c * SP + r]
+  __shared__ double sq[PB], rs[PB];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  {  // 64 rows x 2 column groups; beyond n the identity
     const int r = t & (SB - 1), cg = t >> 6;
-#pragma unroll
-    for (int i = 0; i < SB / 4; i++) {
-      const int c = cg + 4 * i;
-      if (r < n && c < n && r >= c) S[c][r] = A[r + (i64)c * ld];
+#pragma unroll 16
+    for (int i = 0; i < SB / 2; i++) {
+      const int c = cg + 2 * i;
+      S[c * SP + r] = (r < n && c < n) ? (r >= c ? A[r + (i64)c * ld] : 0.0) : (r == c ? 1.0 : 0.0);
     }
-  }
-  // Column j's pivot (one FP64 square root and one division, by thread 0).  Thread 0 also
-  // owns element (j+1, j+1) in column j's trailing update (row j + 1 + 0, first column
-  // group), so it takes the next pivot as soon as that element is final, while the other
-  // threads are still updating: two barriers per column, and the serial pivot mostly off
-  // the barrier-to-barrier path.
-  auto pivot = [&](int j) {
-    const double d = S[j][j];
-    if (!(d > 0.0)) {
-      failed = 1;
-      atomicCAS(status, 0, (int)(col0 + j + 1));
-    } else {
-      const double sq = sqrt(d);
-      S[j][j] = sq;
-      s_inv = 1.0 / sq;
-    }
-  };
-  if (t == 0) {
-    failed = 0;
-    if (n > 0) pivot(0);
   }
   __syncthreads();
-  for (int j = 0; j < n; j++) {
-    if (failed) break;
-    const double inv = s_inv;  // read before the barrier below; thread 0 rewrites it after
-    for (int r = j + 1 + t; r < n; r += blockDim.x) S[j][r] *= inv;
-    __syncthreads();
-    // trailing lower triangle: thread t takes row j + 1 + (t mod 64) and every fourth
-    // column from j + 1 + (t / 64) up to that row (independent updates, no index division)
-    {
-      const int r = j + 1 + (t & (SB - 1));
-      if (r < n) {
-        const double lr = S[j][r];
-#pragma unroll 4
-        for (int c = j + 1 + (t >> 6); c <= r; c += 4) S[c][r] -= lr * S[j][c];
+  const int r = t >> 1, h = t & 1;
+  const int g = lane >> 2, tig = lane & 3;
+  int fail = -1;
+  for (int k = 0; k < n && fail < 0; k += PB) {
+    const bool act = r >= k;  // whole warps: warp w holds rows 16 w .. 16 w + 15
+    double x[PB / 2];         // columns k + 2 i + h of row r
+#pragma unroll
+    for (int i = 0; i < PB / 2; i++) x[i] = S[(k + 2 * i + h) * SP + r];
+    int nfin = PB;
+#pragma unroll
+    for (int j = 0; j < PB; j++) {
+      double* cb = S + (k + j) * SP;
+      if (act && h == (j & 1)) cb[r] = x[j >> 1];
+      __syncthreads();
+      if (nfin == PB) {
+        const double d = cb[k + j];
+        if (!positive(d)) {
+          nfin = j;
+        } else if (act) {
+          double u = cb[r];
+          if (recip_ok(d)) {
+            const double r0 = recip_seed(d), e = fma(-d, r0, 1.0), w = u * r0;
+            u = fma(w, fma(e, e, e), w);
+          } else {
+            u = slow_div(u, d);
+          }
+          const double* cc = cb + k + h;
+          if ((j & 1) == 0 && h == 1) x[j >> 1] = fma(-u, cc[j], x[j >> 1]);
+#pragma unroll
+          for (int i = (j >> 1) + 1; i < PB / 2; i++) x[i] = fma(-u, cc[2 * i], x[i]);
+        }
       }
     }
-    if (t == 0 && j + 1 < n) pivot(j + 1);
+    __syncthreads();
+    if (lane < PB && warp < 2) {  // the block's square roots and their reciprocals, a warp each
+      const double d = S[(k + lane) * SP + k + lane];
+      if (warp == 0) sq[lane] = lane < nfin ? sqrt(d) : 1.0;
+      else rs[lane] = lane < nfin ? rsqrt(d) : 1.0;
+    }
+    __syncthreads();
+    if (act) {
+#pragma unroll
+      for (int i = 0; i < PB / 2; i++) {
+        const int c = 2 * i + h;
+        double* e = S + (k + c) * SP + r;
+        if (r == k + c && c < nfin) *e = sq[c];
+        else if (r > k + c) *e *= rs[c];
+      }
+    }
+    __syncthreads();
+    if (nfin < PB) {
+      fail = k + nfin;
+      if (t == 0) atomicCAS(status, 0, (int)(col0 + fail + 1));
+      break;
+    }
+    // rank-16 update of the lower triangle to the right, an 8 x 8 MMA tile per warp and turn
+    const int o = k + PB, nt = (SB - o) / 8;
+    for (int b = warp; b < nt * (nt + 1) / 2; b += PT_THREADS / 32) {
+      int I = (int)((sqrtf(8.f * (float)b + 1.f) - 1.f) * 0.5f);
+      if ((I + 1) * (I + 2) / 2 <= b) I++;
+      if (I * (I + 1) / 2 > b) I--;
+      const int J = b - I * (I + 1) / 2;
+      const int row = o + 8 * I + g, col = o + 8 * J;
+      double c0 = S[(col + 2 * tig) * SP + row], c1 = S[(col + 2 * tig + 1) * SP + row];
+#pragma unroll
+      for (int q = 0; q < PB; q += 4)
+        dmma884(c0, c1, -S[(k + q + tig) * SP + row], S[(k + q + tig) * SP + col + g]);
+      S[(col + 2 * tig) * SP + row] = c0;
+      S[(col + 2 * tig + 1) * SP + row] = c1;
+    }
     __syncthreads();
   }
-  // Columns factored before a failure are written back as well (LAPACK leaves the
-  // leading part of the factor in place).
-  for (int idx = t; idx < n * n; idx += blockDim.x) {
-    int c = idx / n, r = idx % n;
-    if (r >= c) A[r + (i64)c * ld] = S[c][r];
+  {
+    const int rr = t & (SB - 1), cg = t >> 6;
+#pragma unroll 16
+    for (int i = 0; i < SB / 2; i++) {
+      const int c = cg + 2 * i;
+      if (rr < n && c <= rr) A[rr + (i64)c * ld] = S[c * SP + rr];
+    }
   }
 }
 
 // ---------------------------------------------------------------------------------
 // B := B L^-T for a block of up to 64 columns: L is n x n lower (n <= 64), B rows are
-// independent.  Four lanes per row, each holding every fourth column in registers, 32 rows
-// per CTA of 128 threads; z = blockIdx.y walks a batch of row panels (tiles) with stride
-// sB, the last of which has m_last rows.  FP64 issues from each SM sub-partition at about
-// one FMA per two clocks, so a row group must spread over the sub-partitions: one thread
-// per row left three of them idle and took ~100 us per 64-column step.  Right-looking:
-// once x_c is final (computed by its owner lane and passed to the row's other lanes by a
-// shuffle), every later column takes its FMA with it, in increasing c, as a substitution
-// does.  L sits in shared memory, padded to 64 with the identity, and is read by broadcast;
-// x_c = v * (1 / L(c,c)).
+// independent.  R rows per CTA of 128 threads, 128 / R lanes per row, each holding every
+// (128/R)-th column in registers.  FP64 issues from each SM sub-partition at about one FMA
+// per two clocks, so a row group must spread over the sub-partitions, and a launch with few
+// rows over as many SMs as there are: R = 4 solves its rows in 12.5 us,
+// R = 32 in 31 us (31 us for any row count with 32 rows a CTA only).  Right-looking: once x_c is final (computed by its owner lane and passed to the
+// row's other lanes by a shuffle), every later column takes its FMA with it, in increasing c,
+// as a substitution does; the same operations whatever R.  L sits in shared memory, padded
+// to 64 with the identity, and is read by broadcast; x_c = v * (1 / L(c,c)).
+// Row i of the m rows sits at B + ((org + i) / nb) * sB + (org + i) % nb (a column of tiles of
+// nb rows).  z = blockIdx.y walks a batch of independent systems: L + z sL, B + z sZ, the last
+// of which has n_last columns.
 // ---------------------------------------------------------------------------------
-constexpr int TS_ROWS = 32;                  // rows per CTA
-constexpr int TS_LPR = 4;                    // lanes per row
-constexpr int TS_THREADS = TS_ROWS * TS_LPR;
-constexpr int TS_C = SB / TS_LPR;            // columns per lane
+constexpr int TS_THREADS = 128;
 
-__global__ void __launch_bounds__(TS_THREADS) k_trsm_small(const double* L, i64 ldl, double* B, i64 ldb, i64 sB,
-                                                           int m, int m_last, int batch, int n,
-                                                           const int* status) {
+struct TrsmArgs {
+  const double* L;
+  i64 ldl, sL;
+  double* B;
+  i64 ldb, sB, sZ;
+  int nb;
+  i64 org;
+  int m, n, n_last;
+};
+
+template <int R>
+__global__ void __launch_bounds__(TS_THREADS) k_trsm_small(const TrsmArgs a, const int* status) {
+  constexpr int LPR = TS_THREADS / R;  // lanes per row
+  constexpr int TC = SB / LPR;         // columns per lane
   if (status && *(volatile const int*)status) return;
   __shared__ __align__(16) double Ls[SB * SB];  // Ls[c * SB + r] = L(r, c)
   __shared__ double Rinv[SB];
   const int t = threadIdx.x, lane = t & 31;
-  const int s = t & (TS_LPR - 1);   // this lane holds columns s, s + 4, ...
+  const int s = t & (LPR - 1);   // this lane holds columns s, s + LPR, ...
   const int z = blockIdx.y;
-  const int mz = (z == batch - 1) ? m_last : m;
-  const int r0 = blockIdx.x * TS_ROWS;
-  if (r0 >= mz) return;
-  double* Bz = B + (i64)z * sB;
-  {  // L column by column, threads down the rows (two columns per pass), 8 loads in flight
+  const int n = (z == (int)gridDim.y - 1) ? a.n_last : a.n;
+  const int r0 = blockIdx.x * R;
+  if (r0 >= a.m || n <= 0) return;
+  const double* L = a.L + (i64)z * a.sL;
+  const int row = r0 + t / LPR;
+  const int nl = (row < a.m) ? n : 0;  // columns this row loads and stores
+  const i64 gr = a.org + (row < a.m ? row : 0);
+  double* p = a.B + (i64)z * a.sZ + (gr / a.nb) * a.sB + gr % a.nb;
+  double x[TC];
+#pragma unroll
+  for (int j = 0; j < TC; j++) {
+    const int q = LPR * j + s;
+    x[j] = (q < nl) ? p[(i64)q * a.ldb] : 0.0;
+  }
+  {  // L column by column, threads down the rows (two columns per pass), 16 loads in flight
     const int r = t & (SB - 1), cg = t / SB;
-#pragma unroll 8
+#pragma unroll 16
     for (int c = cg; c < SB; c += TS_THREADS / SB) {
       double v = (r == c) ? 1.0 : 0.0;
-      if (r < n && c < n && r >= c) v = L[r + (i64)c * ldl];
+      if (r < n && c < n && r >= c) v = L[r + (i64)c * a.ldl];
       Ls[c * SB + r] = v;
     }
   }
   __syncthreads();
   if (t < SB) Rinv[t] = 1.0 / Ls[t * SB + t];
-  const int row = r0 + t / TS_LPR;
-  const int nl = (row < mz) ? n : 0;  // columns this row loads and stores
-  double* p = Bz + (row < mz ? row : 0);
-  double x[TS_C];
-#pragma unroll
-  for (int j = 0; j < TS_C; j++) {
-    const int q = TS_LPR * j + s;
-    x[j] = (q < nl) ? p[(i64)q * ldb] : 0.0;
-  }
   __syncthreads();
-  const int zero = n >> 30;  // n <= 64: 0 at run time, opaque to the compiler
-  const int base = lane & ~(TS_LPR - 1);
+  const int base = lane & ~(LPR - 1);
 #pragma unroll
-  for (int c = 0; c < SB; c++) {
-    const int i = c / TS_LPR, sc = c % TS_LPR;
-    const double xc = __shfl_sync(0xffffffffu, x[i] * Rinv[c], base | sc);  // the owner's x_c
-    if (s == sc) x[i] = xc;
-    // column c's loads of L wait for x_c (not all hoisted into registers)
-    const double* lc = Ls + c * SB + (zero & __double2hiint(xc));
+  for (int i = 0; i < TC; i++) {
+#pragma unroll (R == 4 ? 8 : LPR)
+    for (int sc = 0; sc < LPR; sc++) {  // column c = LPR i + sc, held by lane sc of the row
+      const double* lc = Ls + (LPR * i + sc) * SB + s;
+      const double xc = __shfl_sync(0xffffffffu, x[i] * Rinv[LPR * i + sc], base | sc);  // the owner's x_c
+      if (s == sc) x[i] = xc;
+      if (s > sc) x[i] = fma(-xc, lc[LPR * i], x[i]);
 #pragma unroll
-    for (int j = 0; j < TS_C; j++) {
-      const int q = TS_LPR * j + s;
-      if (q > c) x[j] = fma(-xc, lc[q], x[j]);
+      for (int j = i + 1; j < TC; j++) x[j] = fma(-xc, lc[LPR * j], x[j]);
     }
   }
 #pragma unroll
-  for (int j = 0; j < TS_C; j++) {
-    const int q = TS_LPR * j + s;
-    if (q < nl) p[(i64)q * ldb] = x[j];
+  for (int j = 0; j < TC; j++) {
+    const int q = LPR * j + s;
+    if (q < nl) p[(i64)q * a.ldb] = x[j];
   }
 }
 
@@ -374,6 +453,16 @@ int launch_panel_update(const TileCol& X, const TileMap& C, int Ht, int Kt, i64 
   return OOC_OK;
 }
 
+static int sm_count() {
+  static int nsm = [] {
+    int d = 0, v = 0;
+    cudaGetDevice(&d);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d);
+    return v > 0 ? v : 1;
+  }();
+  return nsm;
+}
+
 static int launch_gemm_batched(const GemmBatch& gb, const int* status, cudaStream_t s) {
   if (gb.batch <= 0 || gb.n <= 0 || (gb.m <= 0 && gb.m_last <= 0)) return OOC_OK;
   if (gb.batch > 65535) return OOC_ERR_INTERNAL;
@@ -383,15 +472,16 @@ static int launch_gemm_batched(const GemmBatch& gb, const int* status, cudaStrea
   bool vec = aligned16(gb.A) && aligned16(gb.B) && aligned16(gb.C) && gb.lda % 2 == 0 &&
              gb.ldb % 2 == 0 && gb.sA % 2 == 0 && gb.sB % 2 == 0;
   if (gb.k <= 0) return OOC_OK;
-  // Fewer 64 x 64 blocks than two per SM: 32 x 32 blocks, four times as many CTAs (the
-  // FP64 pipe of an SM does ~2 FMAs per clock, so a 64 x 64 x 64 block alone takes ~75 us)
-  static int nsm = [] {
-    int d = 0, v = 0;
-    cudaGetDevice(&d);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, d);
-    return v > 0 ? v : 1;
-  }();
-  if ((i64)mb * nbk * gb.batch < 2LL * nsm && (i64)gb.batch <= 65535) {
+  // An SM does ~1.75 FP64 FMAs per clock, so a 64 x 64 x 64 block alone takes ~75 us, a 32 x 32
+  // one ~20 and a 16 x 16 one ~5: the blocks are as small as it takes to fill the GPU (up
+  // to four 16 x 16 blocks per SM, which then take about as long as one 32 x 32 block).
+  const i64 b64 = (i64)mb * nbk * gb.batch;
+  if (8 * b64 < 2LL * sm_count()) {
+    const int mb16 = (max(gb.m, gb.m_last) + 15) / 16, nb16 = (gb.n + 15) / 16;
+    dim3 g16(mb16 * nb16, gb.batch);
+    if (vec) k_gemm_batched<true, 16><<<g16, GEMM_THREADS, 0, s>>>(gb, status);
+    else k_gemm_batched<false, 16><<<g16, GEMM_THREADS, 0, s>>>(gb, status);
+  } else if (b64 < 2LL * sm_count()) {
     const int mb32 = (max(gb.m, gb.m_last) + 31) / 32, nb32 = (gb.n + 31) / 32;
     dim3 g32(mb32 * nb32, gb.batch);
     if (vec) k_gemm_batched<true, 32><<<g32, GEMM_THREADS, 0, s>>>(gb, status);
@@ -417,12 +507,29 @@ int launch_gemm_nt_trib(const double* A, i64 lda, const double* B, i64 ldb, doub
   return launch_gemm_batched(gb, status, s);
 }
 
+// Rows per CTA: as few as fill the GPU (4 rows a CTA up to one wave, then 8, 16, 32).
+static int launch_trsm(const TrsmArgs& a, int batch, const int* status, cudaStream_t s) {
+  if (batch <= 0 || a.m <= 0 || (a.n <= 0 && a.n_last <= 0)) return OOC_OK;
+  if (a.n > SB || a.n_last > SB || batch > 65535) return OOC_ERR_INTERNAL;
+  const i64 rows = (i64)a.m * batch;
+  if (rows <= 4LL * sm_count()) k_trsm_small<4><<<dim3((a.m + 3) / 4, batch), TS_THREADS, 0, s>>>(a, status);
+  else if (rows <= 8LL * sm_count()) k_trsm_small<8><<<dim3((a.m + 7) / 8, batch), TS_THREADS, 0, s>>>(a, status);
+  else if (rows <= 16LL * sm_count()) k_trsm_small<16><<<dim3((a.m + 15) / 16, batch), TS_THREADS, 0, s>>>(a, status);
+  else k_trsm_small<32><<<dim3((a.m + 31) / 32, batch), TS_THREADS, 0, s>>>(a, status);
+  OOC_CUDA_TRY(cudaGetLastError());
+  return OOC_OK;
+}
+
 static int launch_trsm_small(const double* L, i64 ldl, double* B, i64 ldb, i64 sB, int m, int m_last,
                              int batch, int n, const int* status, cudaStream_t s) {
   if (batch <= 0 || n <= 0) return OOC_OK;
+  return launch_trsm(TrsmArgs{L, ldl, 0, B, ldb, sB, 0, m > 0 ? m : 1, 0, (batch - 1) * m + m_last, n, n}, 1, status, s);
+}
+
+static int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStream_t s) {
+  if (n <= 0) return OOC_OK;
   if (n > SB) return OOC_ERR_INTERNAL;
-  dim3 grid((max(m, m_last) + TS_ROWS - 1) / TS_ROWS, batch);
-  k_trsm_small<<<grid, TS_THREADS, 0, s>>>(L, ldl, B, ldb, sB, m, m_last, batch, n, status);
+  k_potrf_small<<<1, PT_THREADS, 0, s>>>(A, ld, n, col0, status);
   OOC_CUDA_TRY(cudaGetLastError());
   return OOC_OK;
 }
@@ -431,12 +538,12 @@ int launch_potrf_tile(double* A, i64 ld, int n, i64 col0, int* status, cudaStrea
   for (int k = 0; k < n; k += SB) {
     const int kb = min(SB, n - k);
     double* Akk = A + k + (i64)k * ld;
-    k_potrf_small<<<1, 256, 0, s>>>(Akk, ld, kb, col0 + k, status);
-    OOC_CUDA_TRY(cudaGetLastError());
+    int rc = launch_potrf_block(Akk, ld, kb, col0 + k, status, s);
+    if (rc) return rc;
     const int rest = n - k - kb;
     if (rest > 0) {
       double* Bp = A + (k + kb) + (i64)k * ld;  // rows below the block, columns k..k+kb
-      int rc = launch_trsm_small(Akk, ld, Bp, ld, 0, rest, rest, 1, kb, status, s);
+      rc = launch_trsm_small(Akk, ld, Bp, ld, 0, rest, rest, 1, kb, status, s);
       if (rc) return rc;
       double* Ct = A + (k + kb) + (i64)(k + kb) * ld;
       rc = launch_gemm_nt(Bp, ld, Bp, ld, Ct, ld, rest, rest, kb, 1, -1.0, status, s);
