@@ -85,6 +85,18 @@ int launch_potrf_tile(double* A, i64 ld, int n, i64 col0, int* status, cudaStrea
 int launch_trsm_col(const double* L, i64 ldl, const TileCol& B, int ntiles, int nb, int m_last,
                     int n, const int* status, cudaStream_t s);
 
+// The same for one block of n <= 64 columns.
+int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStream_t s);
+
+// Row i of a tile column, i = 0 .. m-1, sits at B + ((org + i) / nb) * stride + (org + i) % nb.
+// B := B L^-T for its first n <= 64 columns (L: n x n lower).
+int launch_trsm_rows(const double* L, i64 ldl, double* B, i64 ldb, i64 stride, int nb, i64 org, i64 m, int n,
+                     const int* status, cudaStream_t s);
+// C(i, c) -= X(i) X(c)^T, c < w <= 64, i >= c, with X (K columns) and C (w columns) addressed by the
+// same rows; 32 divides nb and org.
+int launch_half_update(const double* X, double* C, i64 ld, i64 stride, int nb, i64 org, i64 m, int w, int K,
+                       const int* status, cudaStream_t s);
+
 // ---------------------------------------------------------------------------------
 // Handle accessors shared between translation units (ooc_driver.cu).
 // ---------------------------------------------------------------------------------

@@ -429,6 +429,24 @@ __global__ void __launch_bounds__(TS_THREADS) k_trsm_small(const TrsmArgs a, con
   }
 }
 
+// ---------------------------------------------------------------------------------
+// C(r, c) -= X(r) X(c)^T for the rows r >= c of a tile column and `w` <= 64 of its columns: the
+// step between the two 64-column halves of a 128-column run.  Row i (counted from org, the
+// run's second half) is addressed as in k_trsm_small; 16 divides nb and org.
+// ---------------------------------------------------------------------------------
+template <bool VEC, int BMX>
+__global__ void __launch_bounds__(GEMM_THREADS)
+k_half_update(const double* X, double* C, i64 ld, i64 stride, int nb, i64 org, int m, int w, int K, const int* status) {
+  if (status && *(volatile const int*)status) return;
+  const int cblocks = (w + BMX - 1) / BMX;
+  const int rb = blockIdx.x / cblocks, cb = blockIdx.x % cblocks;
+  if (cb > rb) return;
+  const i64 gr = org + (i64)rb * BMX, gc = org + (i64)cb * BMX;
+  const i64 ro = (gr / nb) * stride + gr % nb, co = (gc / nb) * stride + gc % nb;
+  gemm_block<VEC, BMX>(X + ro, ld, X + co, ld, C + ro + (i64)cb * BMX * ld, ld, min(BMX, m - rb * BMX),
+                       min(BMX, w - cb * BMX), K, 0, 0, cb == rb, -1.0);
+}
+
 inline bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
@@ -526,10 +544,37 @@ static int launch_trsm_small(const double* L, i64 ldl, double* B, i64 ldb, i64 s
   return launch_trsm(TrsmArgs{L, ldl, 0, B, ldb, sB, 0, m > 0 ? m : 1, 0, (batch - 1) * m + m_last, n, n}, 1, status, s);
 }
 
-static int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStream_t s) {
+int launch_trsm_rows(const double* L, i64 ldl, double* B, i64 ldb, i64 stride, int nb, i64 org, i64 m, int n,
+                     const int* status, cudaStream_t s) {
+  if (m <= 0 || n <= 0) return OOC_OK;
+  if (m > (1 << 30)) return OOC_ERR_INTERNAL;
+  return launch_trsm(TrsmArgs{L, ldl, 0, B, ldb, stride, 0, nb, org, (int)m, n, n}, 1, status, s);
+}
+
+int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStream_t s) {
   if (n <= 0) return OOC_OK;
   if (n > SB) return OOC_ERR_INTERNAL;
   k_potrf_small<<<1, PT_THREADS, 0, s>>>(A, ld, n, col0, status);
+  OOC_CUDA_TRY(cudaGetLastError());
+  return OOC_OK;
+}
+
+// 16 x 16 blocks up to about two per SM, then 32 x 32.
+int launch_half_update(const double* X, double* C, i64 ld, i64 stride, int nb, i64 org, i64 m, int w, int K,
+                       const int* status, cudaStream_t s) {
+  if (m <= 0 || w <= 0 || K <= 0) return OOC_OK;
+  if (w > SB || m > (1 << 30) || nb % 32 || org % 32) return OOC_ERR_INTERNAL;
+  const bool vec = aligned16(X) && aligned16(C) && ld % 2 == 0 && stride % 2 == 0;
+  const bool small = ((m + 15) / 16) * ((w + 15) / 16) <= 2LL * sm_count();
+  const int bx = small ? 16 : 32;
+  const unsigned grid = (unsigned)(((m + bx - 1) / bx) * ((w + bx - 1) / bx));
+  if (small) {
+    if (vec) k_half_update<true, 16><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
+    else k_half_update<false, 16><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
+  } else {
+    if (vec) k_half_update<true, 32><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
+    else k_half_update<false, 32><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
+  }
   OOC_CUDA_TRY(cudaGetLastError());
   return OOC_OK;
 }

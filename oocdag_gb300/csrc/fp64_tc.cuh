@@ -1,0 +1,34 @@
+// FP64 updates on the tensor cores by exact digit products (fp64_tc.cu).
+#pragma once
+
+#include "common.cuh"
+
+constexpr int DIGIT_K = 128;    // columns of X per run (one exponent per row and run)
+constexpr int DIGIT_RUNS = 4;   // most runs an update sums before it rounds into C
+
+// Runs of at most DIGIT_K columns of a column of tiles: element (r, k), r = org .. org + rows - 1,
+// k < K, of run q sits at X + (r / nb) * stride + r % nb + (q DIGIT_K + k) * ldx (stride = nb for a plain
+// column-major panel); its digits at planes + q * slot.
+struct DigitRuns {
+  const double* X;
+  i64 ldx, stride;
+  int nb;
+  i64 org, rows;
+  int K;                 // columns in all; every run but the last has DIGIT_K
+  void* planes;
+  size_t slot;           // bytes between the runs' planes, >= digit_plane_bytes of each
+  i64 org_of[DIGIT_RUNS];  // row each run's planes start at (org, or a multiple of 128 rows above it)
+};
+
+// Bytes of the digit planes and row exponents of `rows` rows of K columns.
+size_t digit_plane_bytes(i64 rows, int K);
+
+// The planes of every run of X for rows org.. (sets org_of).
+int launch_digits(DigitRuns& X, const int* status, cudaStream_t s);
+
+// C(org + r, org + c) -= sum over the runs of X(r) X(c)^T, for r < rows, c in [c_lo, c_hi), r >= c, after
+// launch_digits: one rounding into C per call.  64 divides C.nb, org and c_lo; columns are
+// updated in whole groups of 64, so c_hi is a multiple of 64 or the last row.  X is read
+// where a row holds an infinity or NaN.
+int launch_digit_update(const DigitRuns& X, const TileMap& C, i64 c_lo, i64 c_hi, const int* status, cudaStream_t s,
+                        int reserve_sms = 0);

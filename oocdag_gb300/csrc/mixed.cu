@@ -30,6 +30,7 @@
 
 #include "common.cuh"
 #include "devpool.cuh"
+#include "fp64_tc.cuh"
 
 namespace {
 
@@ -3253,7 +3254,17 @@ extern "C" int ooc_dsyrk_ln(ooc_handle* h, int prec, int n, int k, const double*
   cudaMemsetAsync(status, 0, sizeof(int), s);
   DevBuf work;
   int rc;
-  if (prec == OOC_PREC_FP64) {
+  const size_t slot = (digit_plane_bytes(n, std::min(k, DIGIT_K)) + 255) / 256 * 256;
+  if (prec == OOC_PREC_FP64 && n > 64 && k >= 16 && !work.ensure(slot * std::min(DIGIT_RUNS, (k + DIGIT_K - 1) / DIGIT_K))) {
+    // digit products on the tensor cores (from one block and half a stage on: fp64_tc.cu)
+    const int nb = (n + 63) / 64 * 64;  // one tile
+    rc = OOC_OK;
+    for (int k0 = 0; k0 < k && !rc; k0 += DIGIT_RUNS * DIGIT_K) {
+      DigitRuns D{A + (i64)k0 * lda, lda, nb, nb, 0, n, std::min(DIGIT_RUNS * DIGIT_K, k - k0), work.p, slot, {}};
+      rc = launch_digits(D, status, s);
+      if (!rc) rc = launch_digit_update(D, TileMap{C, ldc, 0, 1, nb}, 0, n, status, s);
+    }
+  } else if (prec == OOC_PREC_FP64) {
     rc = launch_gemm_nt(A, lda, A, lda, C, ldc, n, n, k, 1, -1.0, status, s);
   } else {
     rc = syrk_lowprec(prec, A, lda, C, ldc, n, k, status, s, work);

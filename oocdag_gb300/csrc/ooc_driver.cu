@@ -37,6 +37,7 @@
 
 #include "common.cuh"
 #include "devpool.cuh"
+#include "fp64_tc.cuh"
 
 // ---------------------------------------------------------------------------------
 // Error reporting
@@ -76,6 +77,7 @@ struct ooc_handle {
   std::shared_ptr<DevPool> pool;  // device buffers of the handle's factor objects
   GrowBuf batch_ws;               // launch tables of the batched solvers
   GrowBuf solve_ws;               // panels and vectors of ooc_dpotrs_L
+  GrowBuf digit_ws;               // digit planes of the tensor-core FP64 updates (two runs of 128 columns)
   int last_info = 0;
   std::vector<cudaEvent_t> ev_pool;  // reusable timing-free events
   size_t ev_next = 0;
@@ -197,6 +199,7 @@ extern "C" int ooc_destroy(ooc_handle* h) {
     if (h->d_buf) cudaFree(h->d_buf);
     h->batch_ws.release();
     h->solve_ws.release();
+    h->digit_ws.release();
     if (h->d_status) cudaFree(h->d_status);
     if (h->h_status) cudaFreeHost(h->h_status);
     if (h->s_h2d) cudaStreamDestroy(h->s_h2d);
@@ -340,6 +343,8 @@ struct Run {
   ooc_stats st{};
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> upd_ev, fac_ev;
   std::vector<double> upd_flops;
+  void* planes[2] = {nullptr, nullptr};  // digit planes, two sets (null: FP64-pipe updates)
+  size_t slot = 0;                       // bytes of one run's planes
 };
 
 double pair_flops(int Ht, int Kt, i64 H, i64 Kc, int nb, int K) {
@@ -409,6 +414,163 @@ int copy_d2h(Run& R, double* dst, i64 lda, const double* src, i64 ldt, i64 rows,
   return OOC_OK;
 }
 
+// Marks a span of work on a stream for the profile option (out[0], out[1]: its events).
+int prof_mark(Run& R, cudaStream_t s, cudaEvent_t* ev) {
+  if (!R.h->profile) return OOC_OK;
+  if (next_prof_event(R.h, ev) != cudaSuccess) return OOC_ERR_CUDA;
+  OOC_CUDA_TRY(cudaEventRecord(*ev, s));
+  return OOC_OK;
+}
+
+// C(r, c) -= X(r) X(c)^T over columns [c_lo, c_hi) of the runs' rows (their digits are ready).
+int digit_update(Run& R, const DigitRuns& X, const TileMap& C, i64 c_lo, i64 c_hi, int reserve, cudaStream_t s) {
+  ooc_handle* h = R.h;
+  cudaEvent_t e0 = nullptr, e1 = nullptr;
+  int rc = prof_mark(R, s, &e0);
+  if (!rc) rc = launch_digit_update(X, C, c_lo, c_hi, h->d_status, s, reserve);
+  if (!rc) rc = prof_mark(R, s, &e1);
+  if (rc) return rc;
+  R.st.kernel_launches++;
+  if (h->profile) {
+    const double w = (double)(c_hi - c_lo);
+    R.upd_ev.push_back({e0, e1});
+    R.upd_flops.push_back(w * (2.0 * (double)(X.rows - c_lo) - w + 1.0) * X.K);
+  }
+  return OOC_OK;
+}
+
+// Columns of X per update: up to DIGIT_RUNS runs, which share a row grid of 128 and so have to
+// start at multiples of 128 inside the tile column; one run at a time where 128 does not divide nb.
+int group_cols(int nb) { return nb % DIGIT_K == 0 ? DIGIT_RUNS * DIGIT_K : DIGIT_K; }
+
+// Left-looking update of a panel (YM rows, YN columns) by one earlier tile column X.
+int digit_update_column(Run& R, const TileCol& X, const TileMap& P, i64 YM, i64 YN) {
+  ooc_handle* h = R.h;
+  const int gc = group_cols(P.nb);
+  for (int c0 = 0; c0 < P.nb; c0 += gc) {
+    DigitRuns D{X.base + (i64)c0 * X.ld, X.ld, X.stride, P.nb, 0, YM, std::min(gc, P.nb - c0), R.planes[0], R.slot, {}};
+    int rc = launch_digits(D, h->d_status, h->s_comp);
+    if (!rc) rc = digit_update(R, D, P, 0, YN, 0, h->s_comp);
+    if (rc) return rc;
+    R.st.kernel_launches++;
+  }
+  return OOC_OK;
+}
+
+// In-panel factorization with tensor-core updates (64 divides nb), right-looking over groups
+// of at most group_cols columns of a tile column, and inside a group over runs of DIGIT_K.
+//   s1, one run: 64-column diagonal blocks, their row solve over every row of the panel
+//       below, the update of the run's second half by its first, the run's digits, the
+//       update of the group's later columns by the run; after a group's last run, the
+//       update of the next group's first run by the whole group (one rounding into C per
+//       group, as a tile column's update by FP64 FMAs had).  The chain stays on one
+//       stream: an event between two streams costs it ~6 us.
+//   s0: the rest of the next group's columns (evT), then everything to their right (evU),
+//       beside the next group's runs.
+// Every element takes the same updates in the same order wherever its panel starts: groups
+// and runs are cut inside tile columns, and the choice of kernel for the second half depends
+// on the rows below alone.
+//   kHalfRows: below it the half update runs on the FP64 pipe (16 x 16 or 32 x 32 blocks,
+//              8 to 23 us up to 2048 rows), above it as digit planes and an update (23 us).
+//   kChainSMs: SMs the bulk update leaves to the chain's kernels.
+constexpr i64 kHalfRows = 2048;
+constexpr int kChainSMs = 16;
+
+int factor_panel_tc(Run& R, const TileMap& P, int Ym, i64 YM, i64 YN, i64 col0, double* hostA, i64 lda) {
+  ooc_handle* h = R.h;
+  const int nb = P.nb;
+  const i64 tstride = P.packed ? (i64)nb * nb : (i64)nb;
+  cudaStream_t s0 = h->s_comp, s1 = h->s_h2d;
+  cudaEvent_t evA, evP, evT = nullptr, evU = nullptr;  // A: the panel is ready; P: a run is done
+  OOC_CUDA_TRY(next_event(h, &evA));
+  OOC_CUDA_TRY(cudaEventRecord(evA, s0));
+  OOC_CUDA_TRY(cudaStreamWaitEvent(s1, evA, 0));
+  // end of the group that starts at column g (a multiple of group_cols inside its tile column)
+  auto group_end = [&](i64 g) { return std::min(std::min(g + group_cols(nb), (g / nb + 1) * nb), YN); };
+  int set = 0;
+  for (i64 g0 = 0; g0 < YN; g0 = group_end(g0), set ^= 1) {
+    const i64 g1 = group_end(g0);
+    const int j = (int)(g0 / nb);
+    // element (r, g0 + k) of the panel: cb + (r / nb) * tstride + r % nb + k * ld
+    double* cb = P.base + (P.packed ? ((i64)j * P.Ym - ((i64)j * (j + 1)) / 2) * nb * nb : (i64)j * nb * P.ld) +
+                 (g0 - (i64)j * nb) * P.ld;
+    auto at = [&](i64 r, i64 k) { return cb + (r / nb) * tstride + r % nb + k * P.ld; };
+    DigitRuns G{cb, P.ld, tstride, nb, g1, YM - g1, (int)(g1 - g0), R.planes[set], R.slot, {}};
+    int rc;
+    for (i64 p0 = g0; p0 < g1; p0 += DIGIT_K) {
+      const int w = (int)std::min<i64>(DIGIT_K, g1 - p0);
+      const int run = (int)((p0 - g0) / DIGIT_K);
+      const i64 p1 = p0 + w, rest = YM - p1;
+      char* planes = (char*)R.planes[set] + (size_t)run * R.slot;
+      cudaEvent_t f0 = nullptr, f1 = nullptr;
+      if ((rc = prof_mark(R, s1, &f0))) return rc;
+      for (int k = 0; k < w; k += 64) {
+        const int kb = std::min(64, w - k);
+        const i64 d = p0 + k, m = YM - d - kb, kg = d - g0;  // kg: the block's column in the group
+        if ((rc = launch_potrf_block(at(d, kg), P.ld, kb, col0 + d, h->d_status, s1))) return rc;
+        if ((rc = launch_trsm_rows(at(d, kg), P.ld, cb + kg * P.ld, P.ld, tstride, nb, d + kb, m, kb, h->d_status, s1)))
+          return rc;
+        R.st.kernel_launches += 2;
+        if (k + 64 >= w) break;
+        if (m >= kHalfRows) {
+          DigitRuns D{cb + kg * P.ld, P.ld, tstride, nb, d + 64, m, 64, planes, R.slot, {}};
+          if ((rc = launch_digits(D, h->d_status, s1)) || (rc = launch_digit_update(D, P, 0, w - 64, h->d_status, s1)))
+            return rc;
+          R.st.kernel_launches += 2;
+        } else {
+          rc = launch_half_update(cb + kg * P.ld, cb + (kg + 64) * P.ld, P.ld, tstride, nb, d + 64, m, w - 64, 64,
+                                  h->d_status, s1);
+          if (rc) return rc;
+          R.st.kernel_launches++;
+        }
+      }
+      DigitRuns D{cb + (p0 - g0) * P.ld, P.ld, tstride, nb, p1, rest, w, planes, R.slot, {}};
+      if (p1 < YN) {
+        if ((rc = launch_digits(D, h->d_status, s1))) return rc;
+        G.org_of[run] = p1;
+        R.st.kernel_launches++;
+      }
+      if ((rc = prof_mark(R, s1, &f1))) return rc;
+      if (h->profile) R.fac_ev.push_back({f0, f1});
+      if (p1 < g1) {  // the group's later columns
+        if (evT) OOC_CUDA_TRY(cudaStreamWaitEvent(s1, evT, 0));
+        evT = nullptr;
+        if ((rc = digit_update(R, D, P, 0, g1 - p1, 0, s1))) return rc;
+      }
+    }
+    OOC_CUDA_TRY(next_event(h, &evP));
+    OOC_CUDA_TRY(cudaEventRecord(evP, s1));
+    OOC_CUDA_TRY(cudaStreamWaitEvent(s0, evP, 0));
+    if (hostA && (g1 % nb == 0 || g1 == YN)) {
+      // Tile column j is final: copy it back while the trailing update proceeds
+      // (oocquark.cpp:394,409).
+      const i64 LN = g1 - (i64)j * nb;
+      OOC_CUDA_TRY(cudaStreamWaitEvent(h->s_d2h, evP, 0));
+      for (int i = j; i < Ym; i++) {
+        const i64 LM = std::min<i64>(nb, YM - (i64)i * nb);
+        rc = copy_d2h(R, hostA + (i64)i * nb + (i64)j * nb * lda, lda, tile_ptr(P, i, j), P.ld, LM, LN, h->s_d2h);
+        if (rc) return rc;
+      }
+    }
+    if (g1 < YN) {
+      const i64 g2 = group_end(g1), gn = std::min<i64>(g1 + DIGIT_K, g2);  // next group, end of its first run
+      // the next group has taken every earlier bulk update; with that done, the other set of
+      // planes is free as well
+      if (evU) OOC_CUDA_TRY(cudaStreamWaitEvent(s1, evU, 0));
+      if ((rc = digit_update(R, G, P, 0, gn - g1, 0, s1))) return rc;
+      if (gn < g2) {
+        if ((rc = digit_update(R, G, P, gn - g1, g2 - g1, kChainSMs, s0))) return rc;
+        OOC_CUDA_TRY(next_event(h, &evT));
+        OOC_CUDA_TRY(cudaEventRecord(evT, s0));
+      }
+      if (g2 < YN && (rc = digit_update(R, G, P, g2 - g1, YN - g1, kChainSMs, s0))) return rc;
+      OOC_CUDA_TRY(next_event(h, &evU));
+      OOC_CUDA_TRY(cudaEventRecord(evU, s0));
+    }
+  }
+  return OOC_OK;
+}
+
 // In-panel factorization (oocquark.cpp:389-419).  P maps the panel's tiles; YM / YN are
 // its element extents; col0 its first global column; hostA (may be null) the host
 // address of the panel's tile (0,0) with leading dimension lda.
@@ -418,6 +580,7 @@ int copy_d2h(Run& R, double* dst, i64 lda, const double* src, i64 ldt, i64 rows,
 // s_comp, which first updates tile column j+1 alone and signals s1.  Every tile still
 // receives the same updates, from the same kernels, in the same order.
 int factor_panel(Run& R, const TileMap& P, int Ym, int Yn, i64 YM, i64 YN, i64 col0, double* hostA, i64 lda) {
+  if (R.planes[0]) return factor_panel_tc(R, P, Ym, YM, YN, col0, hostA, lda);
   ooc_handle* h = R.h;
   const int nb = P.nb;
   const i64 tstride = P.packed ? (i64)nb * nb : (i64)nb;
@@ -608,7 +771,7 @@ int dpotrf_host(Run& R, double* A, i64 n, i64 lda, int nb, size_t budget) {
       OOC_CUDA_TRY(cudaEventRecord(ev_x, h->s_h2d));
       OOC_CUDA_TRY(cudaStreamWaitEvent(h->s_comp, ev_x, 0));
       TileCol Xc{X, nb, tile_elems};
-      rc = timed_update(R, Xc, P, Ym, Yn, YM, YN, nb);
+      rc = R.planes[0] ? digit_update_column(R, Xc, P, YM, YN) : timed_update(R, Xc, P, Ym, Yn, YM, YN, nb);
       if (rc) return rc;
       cudaEvent_t ev_f;
       OOC_CUDA_TRY(next_event(h, &ev_f));
@@ -685,6 +848,17 @@ extern "C" int ooc_dpotrf_L(ooc_handle* h, double* A, int64_t n, int64_t lda, in
   }
   *h->h_status = 0;
   if (!rc) rc = ooc_wait_stream(h, h->s_comp);
+  // Tensor-core updates where 64 divides nb (their blocks are 64 columns wide) and there is a
+  // trailing matrix; other tile sizes, and a device without room for the planes (28 bytes per
+  // row and column of a group), keep the FP64-pipe updates.
+  if (!rc && nb % 64 == 0 && n > 64) {
+    R.slot = (digit_plane_bytes(n, std::min(nb, DIGIT_K)) + 255) / 256 * 256;
+    const size_t bytes = R.slot * ((std::min(group_cols(nb), nb) + DIGIT_K - 1) / DIGIT_K);
+    if (h->digit_ws.ensure(2 * bytes) == OOC_OK) {
+      R.planes[0] = h->digit_ws.p;
+      R.planes[1] = (char*)h->digit_ws.p + bytes;
+    }
+  }
   auto t0 = std::chrono::steady_clock::now();
   if (!rc) rc = on_device ? dpotrf_device(R, A, n, lda, nb) : dpotrf_host(R, A, n, lda, nb, dev_budget);
   int rc2 = sync_all(h);
