@@ -880,9 +880,8 @@ def refine_launches(iters, npanels):
     kernels and a column maximum), the maximum of B, X0 (two conversions and a triangular
     solve), per residual evaluation (iters + 1 of them) an initialisation, three pass
     kernels and two column maxima, and per correction two conversions and a solve.  A
-    solve is two kernels per panel and sweep, less the one copy per sweep that replaces
-    the last panel's product."""
-    solve = 4 * npanels - 2
+    solve is one kernel, whatever the number of panels."""
+    solve = 1
     return 4 + 1 + (2 + solve) + 6 * (iters + 1) + iters * (2 + solve)
 
 

@@ -92,6 +92,9 @@ int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStre
 // B := B L^-T for its first n <= 64 columns (L: n x n lower).
 int launch_trsm_rows(const double* L, i64 ldl, double* B, i64 ldb, i64 stride, int nb, i64 org, i64 m, int n,
                      const int* status, cudaStream_t s);
+// The inverses L_bb^{-T} of the 64 x 64 diagonal blocks of L (n x n lower), one after another
+// (64 x 64 each, column-major; the last may hold fewer columns).
+int launch_diag_inverses(const double* L, i64 ldl, i64 n, double* Dinv, cudaStream_t s);
 // C(i, c) -= X(i) X(c)^T, c < w <= 64, i >= c, with X (K columns) and C (w columns) addressed by the
 // same rows; 32 divides nb and org.
 int launch_half_update(const double* X, double* C, i64 ld, i64 stride, int nb, i64 org, i64 m, int w, int K,

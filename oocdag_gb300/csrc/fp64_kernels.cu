@@ -371,6 +371,7 @@ struct TrsmArgs {
   int nb;
   i64 org;
   int m, n, n_last;
+  int identity;  // B starts as the identity and is not read
 };
 
 template <int R>
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(TS_THREADS) k_trsm_small(const TrsmArgs a, con
 #pragma unroll
   for (int j = 0; j < TC; j++) {
     const int q = LPR * j + s;
-    x[j] = (q < nl) ? p[(i64)q * a.ldb] : 0.0;
+    x[j] = a.identity ? (q == row && q < nl ? 1.0 : 0.0) : (q < nl) ? p[(i64)q * a.ldb] : 0.0;
   }
   {  // L column by column, threads down the rows (two columns per pass), 16 loads in flight
     const int r = t & (SB - 1), cg = t / SB;
@@ -541,14 +542,26 @@ static int launch_trsm(const TrsmArgs& a, int batch, const int* status, cudaStre
 static int launch_trsm_small(const double* L, i64 ldl, double* B, i64 ldb, i64 sB, int m, int m_last,
                              int batch, int n, const int* status, cudaStream_t s) {
   if (batch <= 0 || n <= 0) return OOC_OK;
-  return launch_trsm(TrsmArgs{L, ldl, 0, B, ldb, sB, 0, m > 0 ? m : 1, 0, (batch - 1) * m + m_last, n, n}, 1, status, s);
+  return launch_trsm(TrsmArgs{L, ldl, 0, B, ldb, sB, 0, m > 0 ? m : 1, 0, (batch - 1) * m + m_last, n, n, 0}, 1, status, s);
 }
 
 int launch_trsm_rows(const double* L, i64 ldl, double* B, i64 ldb, i64 stride, int nb, i64 org, i64 m, int n,
                      const int* status, cudaStream_t s) {
   if (m <= 0 || n <= 0) return OOC_OK;
   if (m > (1 << 30)) return OOC_ERR_INTERNAL;
-  return launch_trsm(TrsmArgs{L, ldl, 0, B, ldb, stride, 0, nb, org, (int)m, n, n}, 1, status, s);
+  return launch_trsm(TrsmArgs{L, ldl, 0, B, ldb, stride, 0, nb, org, (int)m, n, n, 0}, 1, status, s);
+}
+
+int launch_diag_inverses(const double* L, i64 ldl, i64 n, double* Dinv, cudaStream_t s) {
+  const i64 nblk = (n + SB - 1) / SB;
+  for (i64 z = 0; z < nblk; z += 65535) {
+    const int batch = (int)min(nblk - z, (i64)65535);
+    const int last = z + batch == nblk ? (int)(n - (nblk - 1) * SB) : SB;
+    int rc = launch_trsm(TrsmArgs{L + z * SB * (ldl + 1), ldl, SB * (ldl + 1), Dinv + z * SB * SB, SB, 0, SB * SB, SB, 0, SB, SB,
+                                  last, 1}, batch, nullptr, s);
+    if (rc) return rc;
+  }
+  return OOC_OK;
 }
 
 int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStream_t s) {

@@ -13,7 +13,7 @@
 //                    products (hi*hi + hi*lo + lo*hi) accumulated in FP32 in TMEM and added
 //                    into the FP32 trailing matrix by TMA reductions (k_syrk2_bf16x3).
 // Split-BF16 factors use nb/2-wide panels for the last OOC_OPT_TAIL_ORDER orders.
-// Solves use the kept inverses of the diagonal tiles (solve_with).  The refinement
+// Solves use the kept inverses of the diagonal tiles (trsolve.cu).  The refinement
 // computes residuals in FP64 against the FP64 matrix (device, or the lower triangle of a
 // host matrix copied once), and corrects with the FP32 factor until the normwise backward
 // error ||b - A x||_inf / (||A||_inf ||x||_inf + ||b||_inf) reaches the tolerance.
@@ -31,6 +31,7 @@
 #include "common.cuh"
 #include "devpool.cuh"
 #include "fp64_tc.cuh"
+#include "trsolve.cuh"
 
 namespace {
 
@@ -859,22 +860,10 @@ __global__ void k_to_f32(const double* __restrict__ X, i64 ldx, float* __restric
 constexpr int RMAX = 16;
 constexpr int NN_KCHUNK = 256;
 
-// Optional copy done by the first CTA of a small product: dst(0:n, 0:r) := src (the
-// block a triangular-solve step has just finished, moved into place without a launch).
-template <typename TC>
-struct CopyOut {
-  const TC* src = nullptr;
-  i64 lds = 0;
-  TC* dst = nullptr;
-  i64 ldd = 0;
-  int n = 0;
-};
-
 template <typename TA, typename TC, int R>
 __global__ void __launch_bounds__(256) k_gemm_nn_small(const TA* __restrict__ A, i64 lda, const TC* __restrict__ B,
                                                        i64 ldb, TC* __restrict__ C, i64 ldc, int m, int k, int r,
-                                                       int kslice, TC* __restrict__ P, TC alpha, TC beta,
-                                                       CopyOut<TC> co) {
+                                                       int kslice, TC* __restrict__ P, TC alpha, TC beta) {
   // CTA: 32 rows x 8 warps; warp w sums its eighth of the CTA's k slice for the 32 rows
   // (lane = row, so each load is 32 consecutive rows of one column); the eight partial
   // sums are then added in warp order.
@@ -883,11 +872,6 @@ __global__ void __launch_bounds__(256) k_gemm_nn_small(const TA* __restrict__ A,
   const i64 row = (i64)blockIdx.x * 32 + lane;
   const int k0 = blockIdx.y * kslice;
   const int k1 = min(k, k0 + kslice);
-  if (co.n > 0 && blockIdx.x == 0 && blockIdx.y == 0)
-    for (int idx = threadIdx.x; idx < co.n * r; idx += blockDim.x) {
-      const int q = idx / co.n, i = idx % co.n;
-      co.dst[i + (i64)q * co.ldd] = co.src[i + (i64)q * co.lds];
-    }
   TC acc[R];
 #pragma unroll
   for (int q = 0; q < R; q++) acc[q] = 0;
@@ -964,14 +948,9 @@ __global__ void k_reduce_slices(const TC* __restrict__ P, int nslice, TC* __rest
 template <typename TA, typename TC, int R>
 __global__ void __launch_bounds__(256) k_gemm_tn_small(const TA* __restrict__ A, i64 lda, const TC* __restrict__ B,
                                                        i64 ldb, TC* __restrict__ C, i64 ldc, int m, int k, int r,
-                                                       TC alpha, TC beta, CopyOut<TC> co) {
+                                                       TC alpha, TC beta) {
   __shared__ TC Bs[NN_KCHUNK * R];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (co.n > 0 && blockIdx.x == 0)
-    for (int idx = threadIdx.x; idx < co.n * r; idx += blockDim.x) {
-      const int q = idx / co.n, i = idx % co.n;
-      co.dst[i + (i64)q * co.ldd] = co.src[i + (i64)q * co.lds];
-    }
   const i64 row = (i64)blockIdx.x * (blockDim.x / 32) + warp;
   TC acc[R];
 #pragma unroll
@@ -1024,72 +1003,6 @@ __global__ void __launch_bounds__(256) k_gemm_tn_small(const TA* __restrict__ A,
     if (q >= r) break;
     TC* c = C + row + (i64)q * ldc;
     *c = (beta != TC(0)) ? fma(alpha, acc[q], *c) : alpha * acc[q];
-  }
-}
-
-// One right-hand side through a diagonal block's inverse: x = U^T b (TRANS) or x = U b,
-// U = Dinv_J = L_JJ^{-T} (LN x LN, ld ldu, upper triangular), so output i takes only
-// k <= i (TRANS) or k >= i.  CTA = 32 outputs x 16 warps, warp w takes k in [32w, 32w+32):
-// all of a thread's loads are issued before its first FMA (one round trip instead of a
-// walk), the 16 warp sums added in warp order.  TRANS: lane = k, 32 outputs per lane, then
-// a transposing butterfly leaves lane l with its warp's sum for output l; otherwise lane =
-// output row, b(k) passed along the warp by shuffles.  LN <= 512.
-constexpr int DMV_WARPS = 16;
-// a[0..S) := the lane's kept half plus the partner's passed half (partner = lane ^ S)
-template <typename T, int S>
-__device__ __forceinline__ void dmv_fold(T (&a)[32], int lane) {
-  const bool hi = (lane & S) != 0;
-#pragma unroll
-  for (int j = 0; j < S; j++) {
-    const T send = hi ? a[j] : a[j + S];
-    const T keep = hi ? a[j + S] : a[j];
-    a[j] = keep + __shfl_xor_sync(0xffffffffu, send, S);
-  }
-}
-
-template <typename T, bool TRANS>
-__global__ void __launch_bounds__(DMV_WARPS * 32) k_dinv_mv(const T* __restrict__ U, i64 ldu, int LN,
-                                                           const T* __restrict__ b, T* __restrict__ x) {
-  __shared__ T part[DMV_WARPS][33];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int i0 = blockIdx.x * 32, k0 = warp * 32;
-  const int kl = k0 + lane;
-  const T bk = (kl < LN) ? b[kl] : T(0);
-  T acc;
-  if (TRANS) {
-    T a[32];
-#pragma unroll
-    for (int j = 0; j < 32; j++) {
-      const int i = i0 + j;
-      a[j] = (kl < LN && i < LN && kl <= i) ? U[kl + (i64)i * ldu] : T(0);
-    }
-#pragma unroll
-    for (int j = 0; j < 32; j++) a[j] *= bk;
-    dmv_fold<T, 16>(a, lane);  // keep half, pass half: lane l ends with index l
-    dmv_fold<T, 8>(a, lane);
-    dmv_fold<T, 4>(a, lane);
-    dmv_fold<T, 2>(a, lane);
-    dmv_fold<T, 1>(a, lane);
-    acc = a[0];
-  } else {
-    const int i = i0 + lane;
-    T v[32];
-#pragma unroll
-    for (int u = 0; u < 32; u++) {
-      const int k = k0 + u;
-      v[u] = (i < LN && k < LN && k >= i) ? U[i + (i64)k * ldu] : T(0);
-    }
-    acc = T(0);
-#pragma unroll
-    for (int u = 0; u < 32; u++) acc = fma(v[u], __shfl_sync(0xffffffffu, bk, u), acc);
-  }
-  part[warp][lane] = acc;
-  __syncthreads();
-  if (warp == 0 && i0 + lane < LN) {
-    T sum = part[0][lane];
-#pragma unroll
-    for (int w = 1; w < DMV_WARPS; w++) sum += part[w][lane];
-    x[i0 + lane] = sum;
   }
 }
 
@@ -1423,7 +1336,7 @@ int syrk_f32(int prec, const float* X, i64 ldx, float* C, i64 ldc, int m, int K,
 
 template <typename TA, typename TC>
 int gemm_nn_small(const TA* A, i64 lda, const TC* B, i64 ldb, TC* C, i64 ldc, int m, int k, int r, TC alpha, TC beta,
-                  cudaStream_t s, DevBuf* part, CopyOut<TC> co = CopyOut<TC>()) {
+                  cudaStream_t s, DevBuf* part) {
   if (m <= 0 || r <= 0) return OOC_OK;
   if (r > RMAX) return OOC_ERR_UNSUPPORTED;
   if (k <= 0) {
@@ -1442,11 +1355,11 @@ int gemm_nn_small(const TA* A, i64 lda, const TC* B, i64 ldb, TC* C, i64 ldc, in
     int rc = part->ensure((size_t)nslice * m * r * sizeof(TC));
     if (rc) return rc;
     NN_DISPATCH(r, (k_gemm_nn_small<TA, TC, RR><<<dim3(rows_blocks, nslice), 256, 0, s>>>(
-                       A, lda, B, ldb, C, ldc, m, k, r, kslice, (TC*)part->p, alpha, beta, co)));
+                       A, lda, B, ldb, C, ldc, m, k, r, kslice, (TC*)part->p, alpha, beta)));
     k_reduce_slices<TC><<<(m + 255) / 256, 256, 0, s>>>((const TC*)part->p, nslice, C, ldc, m, r, alpha, beta);
   } else {
     NN_DISPATCH(r, (k_gemm_nn_small<TA, TC, RR><<<dim3(rows_blocks, 1), 256, 0, s>>>(
-                       A, lda, B, ldb, C, ldc, m, k, r, k, nullptr, alpha, beta, co)));
+                       A, lda, B, ldb, C, ldc, m, k, r, k, nullptr, alpha, beta)));
   }
   OOC_CUDA_TRY(cudaGetLastError());
   return OOC_OK;
@@ -1454,11 +1367,11 @@ int gemm_nn_small(const TA* A, i64 lda, const TC* B, i64 ldb, TC* C, i64 ldc, in
 
 template <typename TA, typename TC>
 int gemm_tn_small(const TA* A, i64 lda, const TC* B, i64 ldb, TC* C, i64 ldc, int m, int k, int r, TC alpha, TC beta,
-                  cudaStream_t s, CopyOut<TC> co = CopyOut<TC>()) {
+                  cudaStream_t s) {
   if (m <= 0 || r <= 0) return OOC_OK;
   if (r > RMAX) return OOC_ERR_UNSUPPORTED;
   NN_DISPATCH(r, (k_gemm_tn_small<TA, TC, RR><<<(m + 7) / 8, 256, 0, s>>>(A, lda, B, ldb, C, ldc, m, k, r, alpha,
-                                                                        beta, co)));
+                                                                        beta)));
   OOC_CUDA_TRY(cudaGetLastError());
   return OOC_OK;
 }
@@ -1691,66 +1604,6 @@ struct Panels {
   }
 };
 
-// Solve L L^T X = B in place (B: n x r, ld ldb) using the inverses of the diagonal
-// tiles.  Dinv_J holds L_JJ^{-T} (column-major, upper), i.e. the transpose of
-// L_JJ^{-1}; tmp holds nb x r (nb = the widest panel).
-// B := (L L^T)^{-1} B with the factor's L and kept diagonal inverses (r <= 16 columns):
-// the dpotrs of the reference's VERIFY block (oocdag.cpp:439).  Two launches per block
-// step: the product with the block's inverse into tmp, then the panel product, whose
-// first CTA also moves tmp into place.
-template <typename T>
-int solve_with(const T* L, i64 ldl, const T* Dinv, const Panels& P, T* B, i64 ldb, int r, T* tmp, cudaStream_t s,
-               DevBuf* part) {
-  const i64 n = P.n;
-  const int nt = P.nb;  // ld of tmp
-  const int bb = P.count();
-  int rc;
-  // forward: L y = b
-  for (int J = 0; J < bb; J++) {
-    i64 J0, off;
-    int LN, ld;
-    P.get(J, &J0, &LN, &off, &ld);
-    if (r == 1 && LN <= DMV_WARPS * 32) {  // Dinv_J^T b_J
-      k_dinv_mv<T, true><<<(LN + 31) / 32, DMV_WARPS * 32, 0, s>>>(Dinv + off, ld, LN, B + J0, tmp);
-      OOC_CUDA_TRY(cudaGetLastError());
-    } else {
-      rc = gemm_tn_small<T, T>(Dinv + off, ld, B + J0, ldb, tmp, nt, LN, LN, r, T(1), T(0), s);
-      if (rc) return rc;
-    }
-    const i64 rows = n - J0 - LN;
-    if (rows > 0) {
-      rc = gemm_nn_small<T, T>(L + (J0 + LN) + J0 * ldl, ldl, tmp, nt, B + J0 + LN, ldb, (int)rows, LN, r, T(-1),
-                               T(1), s, part, CopyOut<T>{tmp, nt, B + J0, ldb, LN});
-      if (rc) return rc;
-    } else {
-      OOC_CUDA_TRY(cudaMemcpy2DAsync(B + J0, ldb * sizeof(T), tmp, nt * sizeof(T), LN * sizeof(T), r,
-                                     cudaMemcpyDeviceToDevice, s));
-    }
-  }
-  // backward: L^T x = y
-  for (int J = bb - 1; J >= 0; J--) {
-    i64 J0, off;
-    int LN, ld;
-    P.get(J, &J0, &LN, &off, &ld);
-    if (r == 1 && LN <= DMV_WARPS * 32) {  // Dinv_J y_J
-      k_dinv_mv<T, false><<<(LN + 31) / 32, DMV_WARPS * 32, 0, s>>>(Dinv + off, ld, LN, B + J0, tmp);
-      OOC_CUDA_TRY(cudaGetLastError());
-    } else {
-      rc = gemm_nn_small<T, T>(Dinv + off, ld, B + J0, ldb, tmp, nt, LN, LN, r, T(1), T(0), s, nullptr);
-      if (rc) return rc;
-    }
-    if (J0 > 0) {  // y_{<J} -= L_{J,<J}^T x_J
-      rc = gemm_tn_small<T, T>(L + J0, ldl, tmp, nt, B, ldb, (int)J0, LN, r, T(-1), T(1), s,
-                               CopyOut<T>{tmp, nt, B + J0, ldb, LN});
-      if (rc) return rc;
-    } else {
-      OOC_CUDA_TRY(cudaMemcpy2DAsync(B + J0, ldb * sizeof(T), tmp, nt * sizeof(T), LN * sizeof(T), r,
-                                     cudaMemcpyDeviceToDevice, s));
-    }
-  }
-  return OOC_OK;
-}
-
 }  // namespace
 
 // ---------------------------------------------------------------------------------
@@ -1782,18 +1635,18 @@ struct ooc_factor {
     P.nb2 = nb2 > 0 ? nb2 : nb;
     return P;
   }
-  double* tmp = nullptr;   // nb x 16
-  float* tmpf = nullptr;
   int* status = nullptr;   // device status word of the factorization
   int info = 0;
   // the handle's device-buffer cache (null: plain cudaMalloc / cudaFree); declared before
   // the DevBufs so that it outlives them
   std::shared_ptr<DevPool> pool;
-  DevBuf part, partf, work, scratch;
+  DevBuf part, work, scratch;
   DevBuf work2;  // BF16 planes of the panel before its tensor-core column solve
   // Solves share the buffers above: calls on one factor from several threads take turns.
   std::mutex solve_mu;
   DevBuf rws;    // refinement workspace (residual, FP32 correction, reductions), kept
+  DevBuf xch;    // exchange buffer of the triangular solves, zeroed when allocated
+  unsigned epoch = 0;  // launches on it since then
   DevBuf sws;    // FP32 right-hand sides of ooc_factor_solve on a reduced factor, kept
   DevBuf part2;  // partial sums of the refinement's norm (second stream)
   // FP64 copy of a host A's lower triangle (ld n), kept for the refinement
@@ -1825,23 +1678,58 @@ struct ooc_factor {
     release(Dinv);
     if (owns_Lf) release(Lf);
     release(Dinvf);
-    release(tmp);
-    release(tmpf);
     release(status);
   }
 };
 
 namespace {
 
+// B := (L L^T)^{-1} B with the factor's panels and kept inverses (r <= RMAX): the dpotrs of the
+// reference's VERIFY block (oocdag.cpp:439).  The caller holds solve_mu, and checks
+// solve_error once the stream is done.
+template <typename T>
+int factor_solve(ooc_factor* F, T* B, i64 ldb, int r, cudaStream_t s) {
+  const size_t need = trsolve_bytes(F->n, RMAX, sizeof(T));
+  if (F->xch.bytes < need) {
+    if (F->xch.ensure(need)) return OOC_ERR_NOMEM;
+    F->epoch = 0;
+  }
+  if (F->epoch == 0) OOC_CUDA_TRY(cudaMemsetAsync(F->xch.p, 0, F->xch.bytes, s));
+  const Panels P = F->panels();
+  TriSolve<T> a{P.n, nullptr, P.n, nullptr, P.tail0, P.nb, P.nb2, B, ldb, r, 3};
+  if constexpr (sizeof(T) == 4) {
+    a.L = F->Lf;
+    a.Dinv = F->Dinvf;
+  } else {
+    a.L = F->L;
+    a.Dinv = F->Dinv;
+  }
+  return launch_trsolve<T>(a, F->xch.p, ++F->epoch, s);
+}
+
+// Queues the read of a solve's error word; solve_status after the stream is done.
+int queue_solve_error(const void* exchange, int* err, cudaStream_t s) {
+  *err = 0;
+  OOC_CUDA_TRY(cudaMemcpyAsync(err, trsolve_error(exchange), sizeof(int), cudaMemcpyDeviceToHost, s));
+  return OOC_OK;
+}
+int solve_status(int err) {
+  if (!err) return OOC_OK;
+  ooc_set_last_message("triangular solve: a bounded wait between blocks ran out");
+  return OOC_ERR_TIMEOUT;
+}
+}  // namespace
+
+namespace {
+
 int alloc_factor(ooc_factor* F, i64 n, int nb, bool reduced) {
   const int bb = (int)((n + nb - 1) / nb);
   const size_t tiles = (size_t)bb * nb * nb;
-  bool ok = !F->alloc(&F->status, sizeof(int)) && !F->alloc(&F->tmp, (size_t)nb * RMAX * sizeof(double));
+  bool ok = !F->alloc(&F->status, sizeof(int));
   if (ok && !reduced)
     ok = !F->alloc(&F->L, (size_t)n * n * sizeof(double)) && !F->alloc(&F->Dinv, tiles * sizeof(double));
   if (ok && reduced)
-    ok = !F->alloc(&F->Lf, (size_t)n * n * sizeof(float)) && !F->alloc(&F->Dinvf, tiles * sizeof(float)) &&
-         !F->alloc(&F->tmpf, (size_t)nb * RMAX * sizeof(float));
+    ok = !F->alloc(&F->Lf, (size_t)n * n * sizeof(float)) && !F->alloc(&F->Dinvf, tiles * sizeof(float));
   return ok ? OOC_OK : OOC_ERR_NOMEM;
 }
 
@@ -2508,7 +2396,7 @@ static int create_impl(ooc_handle* h, const double* A, int64_t n, int64_t lda, b
     }
   }
   F->pool = ooc_handle_pool(h);
-  for (DevBuf* b : {&F->part, &F->partf, &F->work, &F->scratch, &F->work2, &F->part2, &F->rws, &F->sws})
+  for (DevBuf* b : {&F->part, &F->work, &F->scratch, &F->work2, &F->part2, &F->rws, &F->xch, &F->sws})
     b->pool = F->pool.get();
   int rc = alloc_factor(F, n, nb, reduced);
   if (rc) { delete F; return rc; }
@@ -2661,9 +2549,9 @@ extern "C" int ooc_factor_create_gen(ooc_handle* h, int64_t n, uint64_t seed, do
 extern "C" int64_t ooc_factor_bytes(int64_t n, int nb, int prec) {
   if (n <= 0 || nb <= 0) return 0;
   const int64_t bb = (n + nb - 1) / nb;
-  int64_t b = (int64_t)nb * 16 * 8 + 256;  // tmp, status
+  int64_t b = (int64_t)trsolve_bytes(n, RMAX, prec == OOC_PREC_FP64 ? 8 : 4) + 256;  // solve exchange, status
   if (prec == OOC_PREC_FP64) return b + n * n * 8 + bb * nb * nb * 8 + n * nb * 8 + (int64_t)nb * nb * 8;
-  b += n * n * 4 + bb * nb * nb * 4 + (int64_t)nb * 16 * 4 + 2 * (int64_t)nb * nb * 4;  // Lf, Dinvf, tmpf, scratch
+  b += n * n * 4 + bb * nb * nb * 4 + 2 * (int64_t)nb * nb * 4;  // Lf, Dinvf, scratch
   if (prec == OOC_PREC_BF16X3) {
     const int64_t planes = 2 * ((n + 127) / 128 * 128) * ((nb + 63) / 64 * 64) * 2 + 256;  // hi + lo
     b += planes;
@@ -2773,14 +2661,16 @@ extern "C" int ooc_factor_solve(ooc_handle* h, ooc_factor* F, double* B, int64_t
     float* bf = (float*)F->sws.p;
     const unsigned gb = (unsigned)((n + 255) / 256);
     k_to_f32_cols<<<gb, 256, 0, s>>>(B, ldb, bf, n, (int)n, nrhs);
-    rc = solve_with<float>(F->Lf, n, F->Dinvf, F->panels(), bf, n, nrhs, F->tmpf, s, &F->partf);
+    rc = factor_solve<float>(F, bf, n, nrhs, s);
     if (!rc) k_f32_to_f64_cols<<<gb, 256, 0, s>>>((const float*)bf, n, B, ldb, (int)n, nrhs);
-    if (!rc) rc = ooc_wait_stream(h, s);
-    return rc;
+  } else {
+    rc = factor_solve<double>(F, B, ldb, nrhs, s);
   }
-  rc = solve_with<double>(F->L, n, F->Dinv, F->panels(), B, ldb, nrhs, F->tmp, s, &F->part);
-  if (rc) return rc;
-  return ooc_wait_stream(h, s);
+  int err = 0;
+  if (!rc) rc = queue_solve_error(F->xch.p, &err, s);
+  const int wrc = ooc_wait_stream(h, s);
+  if (!rc) rc = wrc;
+  return rc ? rc : solve_status(err);
 }
 
 
@@ -2822,9 +2712,11 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
   const i64 tile = (i64)nb * nb;
   // workspace: status word, L_JJ^{-T}, nb x RMAX products, B's device copy, two panels
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  const size_t b_stat = 256, b_dinv = up(tile * 8), b_tmp = up((size_t)nb * RMAX * 8);
-  const size_t b_B = b_dev ? 0 : up((size_t)n * nrhs * 8), b_pan = l_dev ? 0 : up((size_t)n * nb * 8);
-  const size_t need = b_stat + b_dinv + b_tmp + b_B + 2 * b_pan;
+  // The budget is checked against the panel-wise solve's needs: two panels, an nb x nb inverse
+  // and nb x RMAX products.  (The 64 x 64 inverses and exchange words used below fit in that for
+  // nb >= 96 and exceed it by at most 40 KB for smaller nb.)
+  const size_t b_stat = 256, b_B = b_dev ? 0 : up((size_t)n * nrhs * 8), b_pan = l_dev ? 0 : up((size_t)n * nb * 8);
+  size_t need = b_stat + up(tile * 8) + up((size_t)nb * RMAX * 8) + b_B + 2 * b_pan;
   if (dev_budget > 0 && need > dev_budget) {
     char buf[200];
     snprintf(buf, sizeof(buf), "ooc_dpotrs_L: n=%lld nb=%d needs %zu device bytes (two panels), budget %zu",
@@ -2832,18 +2724,24 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
     ooc_set_last_message(buf);
     return OOC_ERR_BUDGET;
   }
+  // A device L whose whole-matrix workspace (an inverse per 64 rows, exchange words) fits the
+  // budget is solved in one launch; otherwise panel by panel.
+  const size_t w_dinv = up((size_t)((n + 63) / 64) * 64 * 64 * 8), w_x = up(trsolve_bytes(n, nrhs, 8));
+  const bool whole = l_dev && (dev_budget == 0 || b_stat + w_dinv + w_x + b_B <= dev_budget);
+  const size_t b_dinv = whole ? w_dinv : up((size_t)((nb + 63) / 64) * 64 * 64 * 8);
+  const size_t b_x = whole ? w_x : up(trsolve_bytes(nb, nrhs, 8));
+  need = b_stat + b_dinv + b_x + b_B + 2 * b_pan;
   GrowBuf* ws = ooc_handle_solve_ws(h);
   int rc = ws->ensure(need);
   if (rc) return rc;
   char* base = (char*)ws->p;
-  int* status = (int*)base;
   double* D = (double*)(base + b_stat);
-  double* tmp = (double*)(base + b_stat + b_dinv);
-  double* Bd = b_dev ? B : (double*)(base + b_stat + b_dinv + b_tmp);
+  void* xch = base + b_stat + b_dinv;
+  double* Bd = b_dev ? B : (double*)(base + b_stat + b_dinv + b_x);
   const i64 ldbd = b_dev ? ldb : n;
   double* Pbuf[2] = {nullptr, nullptr};
   if (!l_dev) {
-    Pbuf[0] = (double*)(base + b_stat + b_dinv + b_tmp + b_B);
+    Pbuf[0] = (double*)(base + b_stat + b_dinv + b_x + b_B);
     Pbuf[1] = (double*)((char*)Pbuf[0] + b_pan);
   }
   struct EvGuard {  // copied (per slot), slot free (per slot), inputs ready
@@ -2854,7 +2752,8 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
   cudaEvent_t* evc = ev.e;
   cudaEvent_t* evf = ev.e + 2;
   cudaEvent_t ev0 = ev.e[4];
-  OOC_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
+  OOC_CUDA_TRY(cudaMemsetAsync(xch, 0, b_x, s));
+  unsigned epoch = 0;
   if (!b_dev)
     OOC_CUDA_TRY(cudaMemcpy2DAsync(Bd, n * sizeof(double), B, ldb * sizeof(double), n * sizeof(double), nrhs,
                                    cudaMemcpyHostToDevice, s));
@@ -2877,7 +2776,11 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
     return OOC_OK;
   };
   int slot_uses[2] = {0, 0};
-  for (int sweep = 0; sweep < 2 && !rc; sweep++) {
+  if (whole) {
+    rc = launch_diag_inverses(L, ldl, n, D, s);
+    if (!rc) rc = launch_trsolve<double>(TriSolve<double>{n, L, ldl, D, n, 64, 64, Bd, ldbd, nrhs, 3}, xch, ++epoch, s);
+  }
+  for (int sweep = 0; sweep < 2 && !rc && !whole; sweep++) {
     // panel order: forward left to right, backward right to left
     auto pj = [&](int t) { return sweep == 0 ? t : bb - 1 - t; };
     if ((rc = fetch(pj(0), 0, slot_uses[0]))) break;
@@ -2898,37 +2801,18 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
         ldp = n;
       }
       const i64 rows = n - J0 - LN;
-      k_set_identity<double><<<dim3((LN + 255) / 256, std::min(LN, 1024)), 256, 0, s>>>(D, nb, LN);
-      rc = launch_trsm_col(Pj, ldp, TileCol{D, nb, tile}, 1, LN, LN, LN, status, s);  // D = L_JJ^{-T}
-      if (rc) break;
+      if ((rc = launch_diag_inverses(Pj, ldp, LN, D, s))) break;
+      TriSolve<double> tile{LN, Pj, ldp, D, LN, 64, 64, Bd + J0, ldbd, nrhs, sweep + 1};
       if (sweep == 0) {  // y_J = L_JJ^{-1} b_J, then b_below -= L_below y_J
-        if (nrhs == 1 && LN <= DMV_WARPS * 32) {
-          k_dinv_mv<double, true><<<(LN + 31) / 32, DMV_WARPS * 32, 0, s>>>(D, nb, LN, Bd + J0, tmp);
-          OOC_CUDA_TRY(cudaGetLastError());
-        } else if ((rc = gemm_tn_small<double, double>(D, nb, Bd + J0, ldbd, tmp, nb, LN, LN, nrhs, 1.0, 0.0, s))) {
+        if ((rc = launch_trsolve<double>(tile, xch, ++epoch, s))) break;
+        if (rows > 0 && (rc = gemm_nn_small<double, double>(Pj + LN, ldp, Bd + J0, ldbd, Bd + J0 + LN, ldbd, (int)rows, LN,
+                                                            nrhs, -1.0, 1.0, s, nullptr)))
           break;
-        }
-        if (rows > 0) {
-          rc = gemm_nn_small<double, double>(Pj + LN, ldp, tmp, nb, Bd + J0 + LN, ldbd, (int)rows, LN, nrhs, -1.0, 1.0,
-                                             s, nullptr, CopyOut<double>{tmp, nb, Bd + J0, ldbd, LN});
-          if (rc) break;
-        } else {
-          OOC_CUDA_TRY(cudaMemcpy2DAsync(Bd + J0, ldbd * sizeof(double), tmp, nb * sizeof(double), LN * sizeof(double),
-                                         nrhs, cudaMemcpyDeviceToDevice, s));
-        }
       } else {  // y_J -= L_below^T x_below, then x_J = L_JJ^{-T} y_J
         if (rows > 0 && (rc = gemm_tn_small<double, double>(Pj + LN, ldp, Bd + J0 + LN, ldbd, Bd + J0, ldbd, LN,
                                                             (int)rows, nrhs, -1.0, 1.0, s)))
           break;
-        if (nrhs == 1 && LN <= DMV_WARPS * 32) {
-          k_dinv_mv<double, false><<<(LN + 31) / 32, DMV_WARPS * 32, 0, s>>>(D, nb, LN, Bd + J0, tmp);
-          OOC_CUDA_TRY(cudaGetLastError());
-        } else if ((rc = gemm_nn_small<double, double>(D, nb, Bd + J0, ldbd, tmp, nb, LN, LN, nrhs, 1.0, 0.0, s,
-                                                       nullptr))) {
-          break;
-        }
-        OOC_CUDA_TRY(cudaMemcpy2DAsync(Bd + J0, ldbd * sizeof(double), tmp, nb * sizeof(double), LN * sizeof(double),
-                                       nrhs, cudaMemcpyDeviceToDevice, s));
+        if ((rc = launch_trsolve<double>(tile, xch, ++epoch, s))) break;
       }
       if (!l_dev) {
         OOC_CUDA_TRY(cudaEventRecord(evf[slot], s));
@@ -2939,8 +2823,11 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
   if (!rc && !b_dev)
     OOC_CUDA_TRY(cudaMemcpy2DAsync(B, ldb * sizeof(double), Bd, n * sizeof(double), n * sizeof(double), nrhs,
                                    cudaMemcpyDeviceToHost, s));
+  int solve_err = 0;
+  if (!rc) rc = queue_solve_error(xch, &solve_err, s);
   const int wrc = ooc_wait_stream(h, s);  // every queued use of the workspace is done
   if (!rc) rc = wrc;
+  if (!rc) rc = solve_status(solve_err);
   if (!rc) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -3013,33 +2900,7 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
     for (int q = 0; q < cols; q++) out[q] = host_max(hv, cols, q, nred);
     return OOC_OK;
   };
-  // The FP32 triangular solve on Rf is ~4 launches per block step: captured once into a
-  // CUDA graph and replayed for X0 and every correction (launch-bound otherwise).
-  cudaGraphExec_t solve_graph = nullptr;
-  bool graph_failed = false;
-  auto solve32 = [&]() -> int {
-    if (!solve_graph && !graph_failed) {
-      cudaGraph_t g = nullptr;
-      int crc = OOC_OK;
-      if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-        crc = OOC_ERR_CUDA;
-      } else {
-        crc = solve_with<float>(F->Lf, n, F->Dinvf, F->panels(), Rf, n, r, F->tmpf, s, nullptr);
-        if (cudaStreamEndCapture(s, &g) != cudaSuccess) crc = OOC_ERR_CUDA;
-      }
-      if (!crc && cudaGraphInstantiate(&solve_graph, g, 0) != cudaSuccess) {
-        solve_graph = nullptr;
-        crc = OOC_ERR_CUDA;
-      }
-      if (g) cudaGraphDestroy(g);
-      if (crc) {  // capture not available: launch directly from now on
-        cudaGetLastError();
-        graph_failed = true;
-      }
-    }
-    if (solve_graph) return cudaGraphLaunch(solve_graph, s) == cudaSuccess ? OOC_OK : OOC_ERR_CUDA;
-    return solve_with<float>(F->Lf, n, F->Dinvf, F->panels(), Rf, n, r, F->tmpf, s, &F->partf);
-  };
+  auto solve32 = [&]() -> int { return factor_solve<float>(F, Rf, n, r, s); };
   // ||A||_inf
   // ||A||_inf on the handle's second stream, beside X0's solve (a chain of small launches
   // that leaves most of the GPU idle): row sums into `rows`, their maximum per CTA into
@@ -3082,7 +2943,7 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
       ooc_set_last_error(e, "cudaMemcpy2DAsync (X := B)", __FILE__, __LINE__);
       rc = OOC_ERR_CUDA;
     } else {
-      rc = solve_with<double>(F->L, n, F->Dinv, F->panels(), X, ldx, r, F->tmp, s, &F->part);
+      rc = factor_solve<double>(F, X, ldx, r, s);
     }
   }
   if (!rc) rc = ooc_wait_stream(h, s2);
@@ -3125,16 +2986,18 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
       if (rc) break;
       k_add_f32_cols<<<gb, 256, 0, s>>>(X, ldx, Rf, n, (int)n, r);
     } else {
-      rc = solve_with<double>(F->L, n, F->Dinv, F->panels(), R, n, r, F->tmp, s, &F->part);
+      rc = factor_solve<double>(F, R, n, r, s);
       if (rc) break;
       k_axpy_cols<<<gb, 256, 0, s>>>(X, ldx, R, n, (int)n, r);
     }
     it++;
   }
+  int solve_err = 0;
+  if (!rc) rc = queue_solve_error(F->xch.p, &solve_err, s);
   if (!rc) rc = ooc_wait_stream(h, s);
+  if (!rc) rc = solve_status(solve_err);
   if (s2 != s) cudaStreamSynchronize(s2);  // the norm's buffers may go now
   if (ev_in) cudaEventDestroy(ev_in);
-  if (solve_graph) cudaGraphExecDestroy(solve_graph);
   if (Atmp) {
     cudaStreamSynchronize(s);
     F->release(Atmp);

@@ -1,0 +1,392 @@
+// Triangular solves L L^T X = B with a factor on the device: both sweeps in one launch.
+//
+// A sweep in panels (inverse product, then panel product, two launches per panel) is bound
+// by launches and by the few CTAs a panel fills: 11 us per 256 rows where the factor's bytes
+// take 0.7.  Here the rows are cut into blocks of BS and the CTAs take (sweep, block) tasks from
+// a ticket counter in dependence order, so a CTA only ever waits for tasks that others have
+// already started (no assumption on how many CTAs are resident).  Task (forward, i):
+//     y_i = L_ii^{-1} (b_i - sum_{j < i} L_ij y_j),     L_ij loaded before y_j is waited for,
+// and the same with L^T from the last block for the backward sweep.  A finished block goes to
+// the others as packets: 64-bit words of 32 data bits and a 32-bit tag (the launch's epoch), so
+// the arrival of the data is its own flag and one L2 round trip passes it on.
+// Bound by that chain: 2.2 us per 128 rows in FP32 (0.69 ms for both sweeps at n = 20000, where
+// the launches per panel took 1.7 ms), 5.7 us per 64 rows in FP64, most of it the FP64 pipe of one
+// SM (1.47 ms at n = 8192 with four right-hand sides); the factor streams from HBM beside it.
+// Sums are block by block in a fixed order, so results do not depend on scheduling.
+//
+// Every wait is bounded: one that runs out raises the buffer's error word, which ends the
+// other CTAs' waits too.
+
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "trsolve.cuh"
+
+namespace {
+
+constexpr int TS_RMAX = 8;                 // right-hand sides per task
+constexpr unsigned TS_POLLS = 1u << 22;    // polls before a wait is declared stuck
+constexpr size_t TS_CTL = 256;             // ticket, error word
+
+template <typename T>
+struct Cfg;
+template <>
+struct Cfg<float> { static constexpr int BS = 128, WORDS = 1; };
+template <>
+struct Cfg<double> { static constexpr int BS = 64, WORDS = 2; };
+
+__device__ __forceinline__ unsigned long long ld_packet(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_packet(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long pack(uint32_t bits, unsigned tag) {
+  return ((unsigned long long)tag << 32) | bits;
+}
+__device__ __forceinline__ void send(unsigned long long* x, i64 at, float v, unsigned tag) {
+  st_packet(x + at, pack(__float_as_uint(v), tag));
+}
+__device__ __forceinline__ void send(unsigned long long* x, i64 at, double v, unsigned tag) {
+  st_packet(x + 2 * at, pack((uint32_t)__double2loint(v), tag));
+  st_packet(x + 2 * at + 1, pack((uint32_t)__double2hiint(v), tag));
+}
+// One word, waiting (bounded) for its tag; 0 when the wait ends without it.
+__device__ __forceinline__ uint32_t take(const unsigned long long* p, unsigned tag, int* ctl) {
+  for (unsigned i = 0; i < TS_POLLS; i++) {
+    const unsigned long long v = ld_packet(p);
+    if ((unsigned)(v >> 32) == tag) return (uint32_t)v;
+    if ((i & 63) == 63 && *(volatile int*)(ctl + 1)) return 0;
+  }
+  atomicExch(ctl + 1, 1);
+  return 0;
+}
+__device__ __forceinline__ float receive(const unsigned long long* x, i64 at, unsigned tag, int* ctl, float) {
+  return __uint_as_float(take(x + at, tag, ctl));
+}
+__device__ __forceinline__ double receive(const unsigned long long* x, i64 at, unsigned tag, int* ctl, double) {
+  const uint32_t lo = take(x + 2 * at, tag, ctl), hi = take(x + 2 * at + 1, tag, ctl);
+  return __hiloint2double((int)hi, (int)lo);
+}
+
+// Rows of block b: start, count, and its diagonal inverse (ld).
+template <typename T>
+__device__ __forceinline__ void block_of(const TriSolve<T>& a, int b, i64* s, int* m, const T** U, int* ldu) {
+  constexpr int BS = Cfg<T>::BS;
+  const int hc = a.tail0 >= a.n ? (int)((a.n + a.nb - 1) / a.nb) : (int)(a.tail0 / a.nb);
+  const int pp = (a.nb + BS - 1) / BS, pp2 = (a.nb2 + BS - 1) / BS;
+  i64 J0, off;
+  int q, W;
+  if (b < hc * pp) {
+    const int p = b / pp;
+    q = b - p * pp;
+    J0 = (i64)p * a.nb;
+    off = (i64)p * a.nb * a.nb;
+    W = a.nb;
+  } else {
+    const int u = b - hc * pp, p = u / pp2;
+    q = u - p * pp2;
+    J0 = a.tail0 + (i64)p * a.nb2;
+    off = (i64)hc * a.nb * a.nb + (i64)p * a.nb2 * a.nb2;
+    W = a.nb2;
+  }
+  *ldu = W;
+  *U = a.Dinv + off + (i64)q * BS * (W + 1);
+  *s = J0 + (i64)q * BS;
+  *m = (int)min((i64)min(BS, W - q * BS), a.n - *s);
+}
+
+// v[0..V) summed over the warp's lanes; afterwards lane l holds the sums of indices
+// first(l) .. first(l) + V/32 - 1 (V < 32: of one index, the same in 32/V lanes).
+template <int V, typename T>
+__device__ __forceinline__ int warp_transpose_sum(T (&v)[V], int lane) {
+  int idx = 0;
+#pragma unroll
+  for (int st = 0; st < 5; st++) {
+    const int off = 16 >> st;
+    const int cnt = V >> st;  // values still held
+    if (cnt > 1) {
+      const bool hi = (lane & off) != 0;
+#pragma unroll
+      for (int j = 0; j < V / 2; j++)
+        if (j < cnt / 2) {
+          const T send = hi ? v[j] : v[j + cnt / 2];
+          const T keep = hi ? v[j + cnt / 2] : v[j];
+          v[j] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+      if (hi) idx += cnt / 2;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    }
+  }
+  return idx;
+}
+
+template <typename T, int R>
+__global__ void __launch_bounds__(Cfg<T>::BS * 4, sizeof(T) == 8 ? 2 : 1)
+    k_trsolve(const __grid_constant__ TriSolve<T> a, int nblk, int ngrp, unsigned long long* __restrict__ xch, int* ctl,
+              unsigned tag) {
+  constexpr int BS = Cfg<T>::BS, NT = BS * 4, KS = BS / 4, NW = NT / 32, CPW = BS / NW, RPL = BS / 32;
+  static_assert(CPW == 8, "eight columns per warp");
+  extern __shared__ __align__(16) unsigned char sm_raw[];
+  T* D = reinterpret_cast<T*>(sm_raw);   // the block's inverse, D[k + i * (BS + 1)] = U(k, i)
+  T* xs = D + (R == 1 ? 0 : BS * (BS + 1));  // arriving block, xs[buf][k * R + q]
+  T* red = xs + 2 * BS * R;              // partial sums, red[(slice * BS + row) * R + q]
+  T* ys = red + 4 * BS * R;              // ys[row * R + q]
+  __shared__ int s_ticket;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int row = t % BS, slice = t / BS;
+  const int nsw = a.sweeps == 3 ? 2 : 1;
+  const int total = nsw * nblk * ngrp;
+  const i64 dir_words = (i64)a.n * a.r * Cfg<T>::WORDS;
+  for (;;) {
+    __syncthreads();
+    if (t == 0) s_ticket = atomicAdd(ctl, 1);
+    __syncthreads();
+    const int tk = s_ticket;
+    if (tk >= total || *(volatile int*)(ctl + 1)) {
+      // the last CTA to stop leaves the counter at zero for the next launch
+      if (t == 0 && atomicAdd(ctl + 2, 1) == (int)gridDim.x - 1) {
+        ctl[0] = 0;
+        ctl[2] = 0;
+      }
+      return;
+    }
+    const int grp = tk % ngrp, u = tk / ngrp;
+    const bool fwd = a.sweeps != 2 && u < nblk;
+    const int i = fwd ? u : (nsw * nblk - 1 - u);
+    const int q0 = grp * R, rn = min(R, a.r - q0);  // this task's right-hand sides
+    i64 si;
+    int mi, ldu;
+    const T* U;
+    block_of(a, i, &si, &mi, &U, &ldu);
+    // The block's inverse, used only after the sums below (its loads overlap them): one
+    // right-hand side keeps the thread's elements in registers, more share them.
+    constexpr bool DREG = R == 1;
+    T dr[DREG ? KS : 1];
+    if constexpr (DREG) {
+#pragma unroll
+      for (int k = 0; k < KS; k++) {
+        const int kk = slice * KS + k;
+        dr[k] = T(0);
+        if (row < mi && kk < mi && (fwd ? kk <= row : kk >= row)) dr[k] = fwd ? U[kk + (i64)row * ldu] : U[row + (i64)kk * ldu];
+      }
+    } else {
+#pragma unroll 8
+      for (int idx = t; idx < BS * BS; idx += NT) {
+        const int k = idx % BS, c = idx / BS;
+        D[k + c * (BS + 1)] = (k <= c && c < mi) ? U[k + (i64)c * ldu] : T(0);
+      }
+    }
+    unsigned long long* out = xch + (fwd ? 0 : dir_words);
+    auto fetch = [&](int j, int buf) {  // block j of this sweep's solution into xs[buf]
+      i64 sj;
+      int mj, l2;
+      const T* u2;
+      block_of(a, j, &sj, &mj, &u2, &l2);
+      for (int idx = t; idx < BS * R; idx += NT) {
+        const int k = idx % BS, q = idx / BS;
+        T v = T(0);
+        if (k < mj && q < rn) v = receive(out, (i64)(q0 + q) * a.n + sj + k, tag, ctl, T(0));
+        xs[buf * BS * R + k * R + q] = v;
+      }
+    };
+    // b (forward) or y (backward) of the thread's element(s), off the chain
+    constexpr int PE = (BS * R + NT - 1) / NT;
+    T rhs[PE];
+#pragma unroll
+    for (int z = 0; z < PE; z++) {
+      const int idx = t + z * NT, rr = idx % BS, q = idx / BS;
+      rhs[z] = T(0);
+      if (q < rn && rr < mi) {
+        if (fwd || nsw == 1) rhs[z] = a.B[si + rr + (i64)(q0 + q) * a.ldb];
+        else rhs[z] = receive(xch, (i64)(q0 + q) * a.n + si + rr, tag, ctl, T(0));
+      }
+    }
+    int buf = 0;
+    if (fwd) {
+      T acc[R];
+#pragma unroll
+      for (int q = 0; q < R; q++) acc[q] = T(0);
+      const T* Lr = a.L + si + (row < mi ? row : 0);
+      for (int j = 0; j < i; j++, buf ^= 1) {
+        i64 sj;
+        int mj, l2;
+        const T* u2;
+        block_of(a, j, &sj, &mj, &u2, &l2);
+        T l[KS];
+#pragma unroll
+        for (int k = 0; k < KS; k++) {
+          const int c = slice * KS + k;
+          l[k] = (row < mi && c < mj) ? Lr[(sj + c) * a.ldl] : T(0);
+        }
+        fetch(j, buf);
+        __syncthreads();
+        const T* x = xs + buf * BS * R + slice * KS * R;
+        constexpr int PS = R == 1 ? 4 : 1;  // partial sums per right-hand side (a chain of KS FMAs otherwise)
+        T p[PS][R];
+#pragma unroll
+        for (int z = 0; z < PS; z++)
+#pragma unroll
+          for (int q = 0; q < R; q++) p[z][q] = T(0);
+#pragma unroll
+        for (int k = 0; k < KS; k++)
+#pragma unroll
+          for (int q = 0; q < R; q++) p[k % PS][q] = fma(l[k], x[k * R + q], p[k % PS][q]);
+#pragma unroll
+        for (int q = 0; q < R; q++) acc[q] += PS == 4 ? (p[0][q] + p[1 % PS][q]) + (p[2 % PS][q] + p[3 % PS][q]) : p[0][q];
+      }
+#pragma unroll
+      for (int q = 0; q < R; q++) red[t * R + q] = acc[q];
+      __syncthreads();
+#pragma unroll
+      for (int z = 0; z < PE; z++) {
+        const int idx = t + z * NT, rr = idx % BS, q = idx / BS;
+        if (q < R) {
+          T v = rhs[z];
+          if (rr < mi && q < rn)
+            v -= (red[rr * R + q] + red[(BS + rr) * R + q]) + (red[(2 * BS + rr) * R + q] + red[(3 * BS + rr) * R + q]);
+          ys[rr * R + q] = v;
+        }
+      }
+      __syncthreads();
+    } else {
+      T v[CPW * R];
+#pragma unroll
+      for (int z = 0; z < CPW * R; z++) v[z] = T(0);
+      for (int j = nblk - 1; j > i; j--, buf ^= 1) {
+        i64 sj;
+        int mj, l2;
+        const T* u2;
+        block_of(a, j, &sj, &mj, &u2, &l2);
+        T l[CPW * RPL];
+#pragma unroll
+        for (int c = 0; c < CPW; c++)
+#pragma unroll
+          for (int p = 0; p < RPL; p++) {
+            const int k = lane + 32 * p, cc = warp * CPW + c;
+            l[c * RPL + p] = (k < mj && cc < mi) ? a.L[sj + k + (si + cc) * a.ldl] : T(0);
+          }
+        fetch(j, buf);
+        __syncthreads();
+        const T* x = xs + buf * BS * R;
+        T w[R];
+#pragma unroll
+        for (int c = 0; c < CPW; c++) {
+#pragma unroll
+          for (int q = 0; q < R; q++) w[q] = T(0);
+#pragma unroll
+          for (int p = 0; p < RPL; p++)
+#pragma unroll
+            for (int q = 0; q < R; q++) w[q] = fma(l[c * RPL + p], x[(lane + 32 * p) * R + q], w[q]);
+#pragma unroll
+          for (int q = 0; q < R; q++) v[c * R + q] += w[q];
+        }
+      }
+      const int first = warp_transpose_sum<CPW * R>(v, lane);
+      constexpr int KEEP = CPW * R >= 32 ? CPW * R / 32 : 1;
+      if (CPW * R >= 32 || (lane & (32 / (CPW * R) - 1)) == 0) {
+#pragma unroll
+        for (int z = 0; z < KEEP; z++) red[(warp * CPW) * R + first + z] = v[z];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int z = 0; z < PE; z++) {
+        const int idx = t + z * NT, rr = idx % BS, q = idx / BS;
+        if (q < R) ys[rr * R + q] = rr < mi && q < rn ? rhs[z] - red[rr * R + q] : T(0);
+      }
+      __syncthreads();
+    }
+    // The block's inverse: forward x(row) = sum_{k <= row} U(k, row) y(k), backward x(row) =
+    // sum_{k >= row} U(row, k) y(k); thread (row, slice of k), warps outside the triangle idle.
+    T p[R];
+#pragma unroll
+    for (int q = 0; q < R; q++) p[q] = T(0);
+    const int wr = row & ~31, k0 = slice * KS;  // the warp's first row, the slice's first k
+    if (fwd ? k0 <= wr + 31 : k0 + KS > wr) {
+#pragma unroll
+      for (int k = 0; k < KS; k++) {
+        const T d = DREG ? dr[DREG ? k : 0] : fwd ? D[k0 + k + row * (BS + 1)] : D[row + (k0 + k) * (BS + 1)];
+#pragma unroll
+        for (int q = 0; q < R; q++) p[q] = fma(d, ys[(k0 + k) * R + q], p[q]);
+      }
+    }
+    // (red was last read before the barrier above)
+#pragma unroll
+    for (int q = 0; q < R; q++) red[t * R + q] = p[q];
+    __syncthreads();
+#pragma unroll
+    for (int z = 0; z < PE; z++) {
+      const int idx = t + z * NT, rr = idx % BS, q = idx / BS;
+      if (rr < mi && q < rn) {
+        const T x =
+            (red[rr * R + q] + red[(BS + rr) * R + q]) + (red[(2 * BS + rr) * R + q] + red[(3 * BS + rr) * R + q]);
+        send(out, (i64)(q0 + q) * a.n + si + rr, x, tag);
+        if (!fwd || nsw == 1) a.B[si + rr + (i64)(q0 + q) * a.ldb] = x;
+      }
+    }
+  }
+}
+
+template <typename T, int R>
+int launch_r(const TriSolve<T>& a, int nblk, int ngrp, void* exchange, unsigned epoch, cudaStream_t s) {
+  constexpr int BS = Cfg<T>::BS;
+  const size_t smem = (size_t)((R == 1 ? 0 : BS * (BS + 1)) + 2 * BS * R + 4 * BS * R + BS * R) * sizeof(T);
+  OOC_CUDA_TRY(cudaFuncSetAttribute(k_trsolve<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  int dev = 0, nsm = 0;
+  OOC_CUDA_TRY(cudaGetDevice(&dev));
+  OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int tasks = nblk * ngrp;  // tasks of one sweep
+  // FP64: two CTAs per SM, one's products beside the other's round trips
+  k_trsolve<T, R><<<std::max(1, std::min(tasks, (sizeof(T) == 8 ? 2 : 1) * nsm)), BS * 4, smem, s>>>(
+      a, nblk, ngrp, (unsigned long long*)((char*)exchange + TS_CTL), (int*)exchange, epoch);
+  OOC_CUDA_TRY(cudaGetLastError());
+  return OOC_OK;
+}
+
+}  // namespace
+
+size_t trsolve_bytes(i64 n, int r, int elem_size) {
+  return TS_CTL + (size_t)2 * (size_t)n * (size_t)r * (elem_size == 4 ? 8 : 16);
+}
+
+template <typename T>
+int launch_trsolve(const TriSolve<T>& a, void* exchange, unsigned epoch, cudaStream_t s) {
+  constexpr int BS = Cfg<T>::BS;
+  if (a.n <= 0 || a.r <= 0) return OOC_OK;
+  if (a.nb <= 0 || a.sweeps < 1 || a.sweeps > 3 || epoch == 0) return OOC_ERR_INTERNAL;
+  TriSolve<T> b = a;
+  if (b.tail0 >= b.n || b.nb2 <= 0) {
+    b.tail0 = b.n;
+    b.nb2 = b.nb;
+  }
+  const i64 hc = b.tail0 >= b.n ? (b.n + b.nb - 1) / b.nb : b.tail0 / b.nb;
+  const i64 pp = (b.nb + BS - 1) / BS, pp2 = (b.nb2 + BS - 1) / BS;
+  i64 nblk;  // whole panels, then the pieces of the last one
+  if (b.tail0 >= b.n) {
+    nblk = (hc - 1) * pp + (b.n - (hc - 1) * b.nb + BS - 1) / BS;
+  } else {
+    const i64 tc = (b.n - b.tail0 + b.nb2 - 1) / b.nb2;
+    nblk = hc * pp + (tc - 1) * pp2 + (b.n - b.tail0 - (tc - 1) * b.nb2 + BS - 1) / BS;
+  }
+  // FP64: one right-hand side per task.  A block step is FP64 work of one SM (64 x 64 products
+  // with L and with the inverse, 2.4 us at 1.75 FMAs per clock for each right-hand side), so
+  // the right-hand sides go side by side on different SMs; L comes from L2 for all but one.
+  const int r = b.r;
+  const int ngrp = sizeof(T) == 8 ? r : (r + TS_RMAX - 1) / TS_RMAX;
+  if (nblk * ngrp * 2 > 0x3fffffff) return OOC_ERR_INTERNAL;
+  if constexpr (sizeof(T) == 8) {
+    return launch_r<T, 1>(b, (int)nblk, ngrp, exchange, epoch, s);
+  } else {
+    if (r == 1) return launch_r<T, 1>(b, (int)nblk, 1, exchange, epoch, s);
+    if (r == 2) return launch_r<T, 2>(b, (int)nblk, 1, exchange, epoch, s);
+    if (r <= 4) return launch_r<T, 4>(b, (int)nblk, 1, exchange, epoch, s);
+    return launch_r<T, 8>(b, (int)nblk, ngrp, exchange, epoch, s);
+  }
+}
+template int launch_trsolve<float>(const TriSolve<float>&, void*, unsigned, cudaStream_t);
+template int launch_trsolve<double>(const TriSolve<double>&, void*, unsigned, cudaStream_t);
