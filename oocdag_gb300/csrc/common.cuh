@@ -51,6 +51,32 @@ struct TileCol {
     }                                                                   \
   } while (0)
 
+// ---- programmatic dependent launch ----------------------------------------------------
+// The FP64 factorization is a chain of kernels of 8 to 50 us on one stream.  Each is launched
+// so that its CTAs may be placed while the kernel before it in the stream still runs; pdl_wait
+// holds every thread until that kernel is done and its writes are visible, and is the first
+// statement of each kernel launched this way (a kernel that ended without it could let the
+// one after it start too early).
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s,
+                       Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 void ooc_set_last_error(cudaError_t e, const char* what, const char* file, int line);
 void ooc_set_last_message(const char* msg);
 

@@ -197,6 +197,7 @@ struct GemmBatch {
 
 template <bool VEC, int BMX = BM>
 __global__ void __launch_bounds__(GEMM_THREADS) k_gemm_batched(GemmBatch gb, const int* status) {
+  pdl_wait();
   if (status && *(volatile const int*)status) return;
   const int z = blockIdx.y;
   const int m = (z == gb.batch - 1) ? gb.m_last : gb.m;
@@ -251,10 +252,54 @@ __device__ __forceinline__ bool positive(double d) {  // d > 0 (false for NaN), 
   return (unsigned long long)__double_as_longlong(d) - 1ull < 0x7FF0000000000000ull;
 }
 
+// One column block: columns k .. k+15 of the rows from k on, LPR threads per row (threads t <
+// (64 - k) LPR; the others return at once).  More threads per row where rows are few: an
+// instruction costs a warp 64 clocks whatever its lanes.  Returns the columns that factored.
+template <int LPR>
+__device__ __forceinline__ int potrf_panel(double* S, int k) {
+  constexpr int XC = PB / LPR;  // columns per thread: k + LPR i + h
+  const int t = threadIdx.x;
+  const int r = k + t / LPR, h = t % LPR, nthr = (SB - k) * LPR;
+  if (r >= SB) return PB;
+  double x[XC];
+#pragma unroll
+  for (int i = 0; i < XC; i++) x[i] = S[(k + LPR * i + h) * SP + r];
+  int nfin = PB;
+#pragma unroll
+  for (int j = 0; j < PB; j++) {
+    asm volatile("bar.sync 1, %0;\n" ::"r"(nthr) : "memory");  // column j is in shared memory
+    const double* cb = S + (k + j) * SP;
+    const double d = cb[k + j];
+    if (nfin == PB) {
+      if (!positive(d)) {
+        nfin = j;
+      } else {
+        double u = cb[r];
+        if (recip_ok(d)) {
+          const double r0 = recip_seed(d), e = fma(-d, r0, 1.0), w = u * r0;
+          u = fma(w, fma(e, e, e), w);
+        } else {
+          u = slow_div(u, d);
+        }
+        if (j + 1 < PB) {  // the next column first: it is stored before the row's other FMAs
+          const int i1 = (j + 1) / LPR, h1 = (j + 1) % LPR;
+          if (h >= h1) x[i1] = fma(-u, cb[k + LPR * i1 + h], x[i1]);
+          if (h == h1) S[(k + j + 1) * SP + r] = x[i1];
+#pragma unroll
+          for (int i = i1 + 1; i < XC; i++) x[i] = fma(-u, cb[k + LPR * i + h], x[i]);
+        }
+      }
+    }
+  }
+  return nfin;
+}
+
 __global__ void __launch_bounds__(PT_THREADS) k_potrf_small(double* A, i64 ld, int n, i64 col0, int* status) {
+  pdl_wait();
   if (*(volatile int*)status) return;
   __shared__ double S[SB * SP];       // S[c * SP + r]
   __shared__ double sq[PB], rs[PB];
+  __shared__ int s_nfin;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   {  // 64 rows x 2 column groups; beyond n the identity
     const int r = t & (SB - 1), cg = t >> 6;
@@ -265,50 +310,23 @@ __global__ void __launch_bounds__(PT_THREADS) k_potrf_small(double* A, i64 ld, i
     }
   }
   __syncthreads();
-  const int r = t >> 1, h = t & 1;
   const int g = lane >> 2, tig = lane & 3;
-  int fail = -1;
-  for (int k = 0; k < n && fail < 0; k += PB) {
-    const bool act = r >= k;  // whole warps: warp w holds rows 16 w .. 16 w + 15
-    double x[PB / 2];         // columns k + 2 i + h of row r
-#pragma unroll
-    for (int i = 0; i < PB / 2; i++) x[i] = S[(k + 2 * i + h) * SP + r];
-    int nfin = PB;
-#pragma unroll
-    for (int j = 0; j < PB; j++) {
-      double* cb = S + (k + j) * SP;
-      if (act && h == (j & 1)) cb[r] = x[j >> 1];
-      __syncthreads();
-      if (nfin == PB) {
-        const double d = cb[k + j];
-        if (!positive(d)) {
-          nfin = j;
-        } else if (act) {
-          double u = cb[r];
-          if (recip_ok(d)) {
-            const double r0 = recip_seed(d), e = fma(-d, r0, 1.0), w = u * r0;
-            u = fma(w, fma(e, e, e), w);
-          } else {
-            u = slow_div(u, d);
-          }
-          const double* cc = cb + k + h;
-          if ((j & 1) == 0 && h == 1) x[j >> 1] = fma(-u, cc[j], x[j >> 1]);
-#pragma unroll
-          for (int i = (j >> 1) + 1; i < PB / 2; i++) x[i] = fma(-u, cc[2 * i], x[i]);
-        }
-      }
-    }
+  for (int k = 0; k < n; k += PB) {
+    int nfin = k < 32 ? potrf_panel<2>(S, k) : k < 48 ? potrf_panel<4>(S, k) : potrf_panel<8>(S, k);
+    if (t == 0) s_nfin = nfin;
     __syncthreads();
+    nfin = s_nfin;
     if (lane < PB && warp < 2) {  // the block's square roots and their reciprocals, a warp each
       const double d = S[(k + lane) * SP + k + lane];
       if (warp == 0) sq[lane] = lane < nfin ? sqrt(d) : 1.0;
       else rs[lane] = lane < nfin ? rsqrt(d) : 1.0;
     }
     __syncthreads();
-    if (act) {
+    {
+      const int r = t & (SB - 1), cg = t >> 6;
 #pragma unroll
       for (int i = 0; i < PB / 2; i++) {
-        const int c = 2 * i + h;
+        const int c = 2 * i + cg;
         double* e = S + (k + c) * SP + r;
         if (r == k + c && c < nfin) *e = sq[c];
         else if (r > k + c) *e *= rs[c];
@@ -316,8 +334,7 @@ __global__ void __launch_bounds__(PT_THREADS) k_potrf_small(double* A, i64 ld, i
     }
     __syncthreads();
     if (nfin < PB) {
-      fail = k + nfin;
-      if (t == 0) atomicCAS(status, 0, (int)(col0 + fail + 1));
+      if (t == 0) atomicCAS(status, 0, (int)(col0 + k + nfin + 1));
       break;
     }
     // rank-16 update of the lower triangle to the right, an 8 x 8 MMA tile per warp and turn
@@ -378,6 +395,7 @@ template <int R>
 __global__ void __launch_bounds__(TS_THREADS) k_trsm_small(const TrsmArgs a, const int* status) {
   constexpr int LPR = TS_THREADS / R;  // lanes per row
   constexpr int TC = SB / LPR;         // columns per lane
+  pdl_wait();
   if (status && *(volatile const int*)status) return;
   __shared__ __align__(16) double Ls[SB * SB];  // Ls[c * SB + r] = L(r, c)
   __shared__ double Rinv[SB];
@@ -438,6 +456,7 @@ __global__ void __launch_bounds__(TS_THREADS) k_trsm_small(const TrsmArgs a, con
 template <bool VEC, int BMX>
 __global__ void __launch_bounds__(GEMM_THREADS)
 k_half_update(const double* X, double* C, i64 ld, i64 stride, int nb, i64 org, int m, int w, int K, const int* status) {
+  pdl_wait();
   if (status && *(volatile const int*)status) return;
   const int cblocks = (w + BMX - 1) / BMX;
   const int rb = blockIdx.x / cblocks, cb = blockIdx.x % cblocks;
@@ -495,22 +514,23 @@ static int launch_gemm_batched(const GemmBatch& gb, const int* status, cudaStrea
   // one ~20 and a 16 x 16 one ~5: the blocks are as small as it takes to fill the GPU (up
   // to four 16 x 16 blocks per SM, which then take about as long as one 32 x 32 block).
   const i64 b64 = (i64)mb * nbk * gb.batch;
+  cudaError_t e;
   if (8 * b64 < 2LL * sm_count()) {
     const int mb16 = (max(gb.m, gb.m_last) + 15) / 16, nb16 = (gb.n + 15) / 16;
     dim3 g16(mb16 * nb16, gb.batch);
-    if (vec) k_gemm_batched<true, 16><<<g16, GEMM_THREADS, 0, s>>>(gb, status);
-    else k_gemm_batched<false, 16><<<g16, GEMM_THREADS, 0, s>>>(gb, status);
+    if (vec) e = launch_pdl(k_gemm_batched<true, 16>, g16, GEMM_THREADS, 0, s, gb, status);
+    else e = launch_pdl(k_gemm_batched<false, 16>, g16, GEMM_THREADS, 0, s, gb, status);
   } else if (b64 < 2LL * sm_count()) {
     const int mb32 = (max(gb.m, gb.m_last) + 31) / 32, nb32 = (gb.n + 31) / 32;
     dim3 g32(mb32 * nb32, gb.batch);
-    if (vec) k_gemm_batched<true, 32><<<g32, GEMM_THREADS, 0, s>>>(gb, status);
-    else k_gemm_batched<false, 32><<<g32, GEMM_THREADS, 0, s>>>(gb, status);
+    if (vec) e = launch_pdl(k_gemm_batched<true, 32>, g32, GEMM_THREADS, 0, s, gb, status);
+    else e = launch_pdl(k_gemm_batched<false, 32>, g32, GEMM_THREADS, 0, s, gb, status);
   } else if (vec) {
-    k_gemm_batched<true><<<grid, GEMM_THREADS, 0, s>>>(gb, status);
+    e = launch_pdl(k_gemm_batched<true, BM>, grid, GEMM_THREADS, 0, s, gb, status);
   } else {
-    k_gemm_batched<false><<<grid, GEMM_THREADS, 0, s>>>(gb, status);
+    e = launch_pdl(k_gemm_batched<false, BM>, grid, GEMM_THREADS, 0, s, gb, status);
   }
-  OOC_CUDA_TRY(cudaGetLastError());
+  OOC_CUDA_TRY(e);
   return OOC_OK;
 }
 
@@ -531,11 +551,12 @@ static int launch_trsm(const TrsmArgs& a, int batch, const int* status, cudaStre
   if (batch <= 0 || a.m <= 0 || (a.n <= 0 && a.n_last <= 0)) return OOC_OK;
   if (a.n > SB || a.n_last > SB || batch > 65535) return OOC_ERR_INTERNAL;
   const i64 rows = (i64)a.m * batch;
-  if (rows <= 4LL * sm_count()) k_trsm_small<4><<<dim3((a.m + 3) / 4, batch), TS_THREADS, 0, s>>>(a, status);
-  else if (rows <= 8LL * sm_count()) k_trsm_small<8><<<dim3((a.m + 7) / 8, batch), TS_THREADS, 0, s>>>(a, status);
-  else if (rows <= 16LL * sm_count()) k_trsm_small<16><<<dim3((a.m + 15) / 16, batch), TS_THREADS, 0, s>>>(a, status);
-  else k_trsm_small<32><<<dim3((a.m + 31) / 32, batch), TS_THREADS, 0, s>>>(a, status);
-  OOC_CUDA_TRY(cudaGetLastError());
+  cudaError_t e;
+  if (rows <= 4LL * sm_count()) e = launch_pdl(k_trsm_small<4>, dim3((a.m + 3) / 4, batch), TS_THREADS, 0, s, a, status);
+  else if (rows <= 8LL * sm_count()) e = launch_pdl(k_trsm_small<8>, dim3((a.m + 7) / 8, batch), TS_THREADS, 0, s, a, status);
+  else if (rows <= 16LL * sm_count()) e = launch_pdl(k_trsm_small<16>, dim3((a.m + 15) / 16, batch), TS_THREADS, 0, s, a, status);
+  else e = launch_pdl(k_trsm_small<32>, dim3((a.m + 31) / 32, batch), TS_THREADS, 0, s, a, status);
+  OOC_CUDA_TRY(e);
   return OOC_OK;
 }
 
@@ -567,8 +588,7 @@ int launch_diag_inverses(const double* L, i64 ldl, i64 n, double* Dinv, cudaStre
 int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStream_t s) {
   if (n <= 0) return OOC_OK;
   if (n > SB) return OOC_ERR_INTERNAL;
-  k_potrf_small<<<1, PT_THREADS, 0, s>>>(A, ld, n, col0, status);
-  OOC_CUDA_TRY(cudaGetLastError());
+  OOC_CUDA_TRY(launch_pdl(k_potrf_small, dim3(1), PT_THREADS, 0, s, A, ld, n, col0, status));
   return OOC_OK;
 }
 
@@ -581,14 +601,15 @@ int launch_half_update(const double* X, double* C, i64 ld, i64 stride, int nb, i
   const bool small = ((m + 15) / 16) * ((w + 15) / 16) <= 2LL * sm_count();
   const int bx = small ? 16 : 32;
   const unsigned grid = (unsigned)(((m + bx - 1) / bx) * ((w + bx - 1) / bx));
+  cudaError_t e;
   if (small) {
-    if (vec) k_half_update<true, 16><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
-    else k_half_update<false, 16><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
+    if (vec) e = launch_pdl(k_half_update<true, 16>, dim3(grid), GEMM_THREADS, 0, s, X, C, ld, stride, nb, org, (int)m, w, K, status);
+    else e = launch_pdl(k_half_update<false, 16>, dim3(grid), GEMM_THREADS, 0, s, X, C, ld, stride, nb, org, (int)m, w, K, status);
   } else {
-    if (vec) k_half_update<true, 32><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
-    else k_half_update<false, 32><<<grid, GEMM_THREADS, 0, s>>>(X, C, ld, stride, nb, org, (int)m, w, K, status);
+    if (vec) e = launch_pdl(k_half_update<true, 32>, dim3(grid), GEMM_THREADS, 0, s, X, C, ld, stride, nb, org, (int)m, w, K, status);
+    else e = launch_pdl(k_half_update<false, 32>, dim3(grid), GEMM_THREADS, 0, s, X, C, ld, stride, nb, org, (int)m, w, K, status);
   }
-  OOC_CUDA_TRY(cudaGetLastError());
+  OOC_CUDA_TRY(e);
   return OOC_OK;
 }
 

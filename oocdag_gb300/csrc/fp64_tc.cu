@@ -59,6 +59,7 @@ static_assert(NG * DC == 512, "the eight order sums fill the TMEM");
 __global__ void __launch_bounds__(256) k_digits(const double* __restrict__ X, i64 ldx, i64 stride, int nb, i64 org,
                                                 int rows, int Kall, uint8_t* __restrict__ planes, size_t slot,
                                                 const int* status) {
+  pdl_wait();
   if (status && *(volatile const int*)status) return;
   const int K = min(DIGIT_K, Kall - (int)blockIdx.y * DIGIT_K);  // blockIdx.y: run
   const int nst = (K + DK - 1) / DK;
@@ -151,14 +152,23 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                : "memory");
 }
 
-struct UpdateArgs {
+struct Operand {
   const uint8_t* planes[DIGIT_RUNS];  // each run's planes and row exponents, at the update's first row
   const int* exps[DIGIT_RUNS];
-  int nst[DIGIT_RUNS];                // its stages of DK columns
-  int nrun;
   const double* X;                    // the runs' elements (non-finite rows)
   i64 ldx, stride, org;
-  int nb, rows, K;
+  int nb, rows;
+  __device__ const double* row(int r) const {
+    const i64 g = org + r;
+    return X + (g / nb) * stride + g % nb;
+  }
+};
+struct UpdateArgs {
+  Operand a, b;                       // rows and columns of C
+  int nst[DIGIT_RUNS];                // a run's stages of DK columns
+  int nrun, K;
+  double alpha, beta;                 // general products only
+  int mask;
 };
 
 // The eight order sums of one element put together: sum_g G_g 2^(8 (5 - g)) as a 64-bit integer
@@ -190,12 +200,12 @@ __device__ __forceinline__ double digit_value(long long V, int es, bool& special
 // The same where the result is subnormal or overflows, and the plain sum for non-finite rows.
 __device__ __noinline__ double digit_value_special(long long V, int es, const UpdateArgs& X, int run, int r, int c) {
   if (es <= EXP_NONFINITE / 2) return scalbn((double)V, es - 54);
-  if (r >= X.rows || c >= X.rows) return 0.0;
-  const i64 gr = X.org + r, gc = X.org + c;
-  const double* a = X.X + (gr / X.nb) * X.stride + gr % X.nb + (i64)run * DIGIT_K * X.ldx;
-  const double* b = X.X + (gc / X.nb) * X.stride + gc % X.nb + (i64)run * DIGIT_K * X.ldx;
+  if (r >= X.a.rows || c >= X.b.rows) return 0.0;
+  const double* a = X.a.row(r) + (i64)run * DIGIT_K * X.a.ldx;
+  const double* b = X.b.row(c) + (i64)run * DIGIT_K * X.b.ldx;
   double v = 0.0;
-  for (int k = 0; k < X.nst[run] * DK && run * DIGIT_K + k < X.K; k++) v = fma(a[(i64)k * X.ldx], b[(i64)k * X.ldx], v);
+  for (int k = 0; k < X.nst[run] * DK && run * DIGIT_K + k < X.K; k++)
+    v = fma(a[(i64)k * X.a.ldx], b[(i64)k * X.b.ldx], v);
   return v;
 }
 
@@ -207,10 +217,11 @@ __device__ __noinline__ double digit_value_special(long long V, int es, const Up
 // clocks of MMAs (62 per 128 x 64 x 16 product, of which the tensor pipe needs 32), 6.0k until the
 // sums are out of TMEM; C overlaps with the next block.  A 4096 x 4096 lower triangle with
 // K = 128 takes 99 us (21.7 TFLOP/s of FP64 work); FP64 MMAs took 3.2 ms for K = 256.
+// GENERAL: C = beta C + alpha A B^T on all of C or a triangle (mask) instead, T columns of blocks.
+template <bool GENERAL>
 __global__ void __launch_bounds__(D_THREADS, 1)
     k_digit_update(const __grid_constant__ UpdateArgs X, TileMap Cm, int T, int bj_lo, int bj_hi, i64 nblk,
                    int* status) {
-  if (*(volatile int*)status) return;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + D_STAGES * D_STAGE);
@@ -246,6 +257,16 @@ __global__ void __launch_bounds__(D_THREADS, 1)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();  // (the set-up above touches no other kernel's data)
+  if (*(volatile int*)status) nblk = 0;
+  auto block_at = [&](i64 t, int* bi, int* bj) {
+    if constexpr (GENERAL) {
+      *bi = (int)(t / T);
+      *bj = (int)(t % T);
+    } else {
+      strip2_decode(t, T, bj_lo, bj_hi, bi, bj);
+    }
+  };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -253,11 +274,11 @@ __global__ void __launch_bounds__(D_THREADS, 1)
       bool ok = true;
       for (i64 t = blockIdx.x; ok && t < nblk; t += gridDim.x) {
         int bi, bj;
-        strip2_decode(t, T, bj_lo, bj_hi, &bi, &bj);
+        block_at(t, &bi, &bj);
         for (int run = 0; ok && run < X.nrun; run++) {
           const int nst = X.nst[run];
-          const uint8_t* ua = X.planes[run] + (i64)bi * nst * UNIT_STAGE;
-          const uint8_t* ub = X.planes[run] + (i64)(bj >> 1) * nst * UNIT_STAGE + (bj & 1) * B_DIG;
+          const uint8_t* ua = X.a.planes[run] + (i64)bi * nst * UNIT_STAGE;
+          const uint8_t* ub = X.b.planes[run] + (i64)(bj >> 1) * nst * UNIT_STAGE + (bj & 1) * B_DIG;
           for (int kc = 0; kc < nst; kc++, c++) {
             const int s = (int)(c % D_STAGES);
             if (!mbar_wait(&empty[s], (uint32_t)((c / D_STAGES) & 1) ^ 1u, abort_flag)) {
@@ -322,14 +343,14 @@ __global__ void __launch_bounds__(D_THREADS, 1)
     bool ok = true;
     for (i64 t = blockIdx.x; ok && t < nblk; t += gridDim.x) {
       int bi, bj;
-      strip2_decode(t, T, bj_lo, bj_hi, &bi, &bj);
+      block_at(t, &bi, &bj);
       const int row = bi * DR + quad * 32 + lane, col0 = bj * DC + half;
       double v[32];  // the runs' sum
 #pragma unroll
       for (int q = 0; q < 32; q++) v[q] = 0.0;
       for (int run = 0; run < X.nrun; run++, tl++) {
-        const int* exps = X.exps[run];
-        const int er = exps[row];
+        const int* exps = X.b.exps[run];
+        const int er = X.a.exps[run][row];
         const bool got = mbar_wait(tfull, (uint32_t)(tl & 1), abort_flag);
         if (!__all_sync(0xffffffffu, got)) {
           if (lane == 0) *abort_flag = 1;
@@ -367,8 +388,26 @@ __global__ void __launch_bounds__(D_THREADS, 1)
         if (lane == 0) mbar_arrive(tempty);  // the accumulators may be overwritten now
       }
       if (!ok) break;
-      if (row < X.rows) {
-        const i64 r = X.org + row, c = X.org + col0;
+      if constexpr (GENERAL) {
+        if (row < X.a.rows) {
+          const int q0 = X.mask == 2 ? max(0, row - col0) : 0;  // columns [q0, q1) of the warp's 32
+          const int q1 = min(32, X.mask == 1 ? min(row + 1, X.b.rows) - col0 : X.b.rows - col0);
+          double* p = Cm.base + row + (i64)col0 * Cm.ld;
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            double cv[16];
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+              cv[q] = X.beta != 0.0 && 16 * h + q >= q0 && 16 * h + q < q1 ? p[(i64)(16 * h + q) * Cm.ld] : 0.0;
+#pragma unroll
+            for (int q = 0; q < 16; q++)
+              if (16 * h + q >= q0 && 16 * h + q < q1)
+                p[(i64)(16 * h + q) * Cm.ld] =
+                    X.beta == 0.0 ? X.alpha * v[16 * h + q] : fma(X.alpha, v[16 * h + q], X.beta * cv[q]);
+          }
+        }
+      } else if (row < X.a.rows) {
+        const i64 r = X.a.org + row, c = X.a.org + col0;
         const i64 ti = r / nb, tj = c / nb;  // a block column lies in one tile column (64 divides nb)
         double* p = (Cm.packed ? Cm.base + packed_tile_index((int)ti, (int)tj, Cm.Ym) * (i64)nb * nb + (r - ti * nb) +
                                      (c - tj * nb) * Cm.ld
@@ -421,9 +460,45 @@ int launch_digits(DigitRuns& X, const int* status, cudaStream_t s) {
   const int nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
   if (nrun > DIGIT_RUNS || X.rows > (1 << 30)) return OOC_ERR_INTERNAL;
   for (int q = 0; q < nrun; q++) X.org_of[q] = X.org;
-  k_digits<<<dim3(2 * (unsigned)((X.rows + DR - 1) / DR), nrun), 256, 0, s>>>(
-      X.X, X.ldx, X.stride, X.nb, X.org, (int)X.rows, X.K, (uint8_t*)X.planes, X.slot, status);
-  OOC_CUDA_TRY(cudaGetLastError());
+  OOC_CUDA_TRY(launch_pdl(k_digits, dim3(2 * (unsigned)((X.rows + DR - 1) / DR), nrun), 256, 0, s, X.X, X.ldx, X.stride,
+                          X.nb, X.org, (int)X.rows, X.K, (uint8_t*)X.planes, X.slot, status));
+  return OOC_OK;
+}
+
+// The runs of X as an operand whose first row is X.org.
+static int operand_of(const DigitRuns& X, Operand* o, int* nst) {
+  const int nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
+  if (nrun > DIGIT_RUNS || X.rows > (1 << 30)) return OOC_ERR_INTERNAL;
+  for (int q = 0; q < nrun; q++) {
+    const i64 up = X.org - X.org_of[q];
+    if (up < 0 || up % DR != 0) return OOC_ERR_INTERNAL;
+    const int K = std::min(DIGIT_K, X.K - q * DIGIT_K);
+    const size_t units = (size_t)((X.rows + up + DR - 1) / DR);
+    nst[q] = (K + DK - 1) / DK;
+    const uint8_t* p = (const uint8_t*)X.planes + (size_t)q * X.slot;
+    o->planes[q] = p + (size_t)(up / DR) * nst[q] * UNIT_STAGE;
+    o->exps[q] = (const int*)(p + units * nst[q] * UNIT_STAGE) + up;
+  }
+  o->X = X.X;
+  o->ldx = X.ldx;
+  o->stride = X.stride;
+  o->org = X.org;
+  o->nb = X.nb;
+  o->rows = (int)X.rows;
+  return OOC_OK;
+}
+
+template <bool GENERAL>
+static int launch_blocks(const UpdateArgs& a, const TileMap& C, int T, int lo, int hi, i64 nblk, int* status,
+                         cudaStream_t s, int reserve_sms) {
+  if (nblk <= 0) return OOC_OK;
+  int dev = 0, nsm = 0;
+  OOC_CUDA_TRY(cudaGetDevice(&dev));
+  OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  OOC_CUDA_TRY(cudaFuncSetAttribute(k_digit_update<GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, D_SMEM));
+  const i64 grid = std::max<i64>(1, std::min<i64>(nblk, std::max(1, nsm - std::max(0, reserve_sms))));
+  OOC_CUDA_TRY(launch_pdl(k_digit_update<GENERAL>, dim3((unsigned)grid), D_THREADS, D_SMEM, s, a, C, T, lo, hi, nblk,
+                          status));
   return OOC_OK;
 }
 
@@ -431,35 +506,31 @@ int launch_digit_update(const DigitRuns& X, const TileMap& C, i64 c_lo, i64 c_hi
                         int reserve_sms) {
   c_hi = std::min(c_hi, X.rows);
   if (X.rows <= 0 || X.K <= 0 || c_lo >= c_hi) return OOC_OK;
+  if (!status || c_lo % DC != 0 || C.nb % DC != 0) return OOC_ERR_INTERNAL;
   UpdateArgs a{};
+  int rc = operand_of(X, &a.a, a.nst);
+  if (rc) return rc;
+  a.b = a.a;
   a.nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
-  if (!status || c_lo % DC != 0 || C.nb % DC != 0 || a.nrun > DIGIT_RUNS || X.rows > (1 << 30)) return OOC_ERR_INTERNAL;
-  for (int q = 0; q < a.nrun; q++) {
-    const i64 up = X.org - X.org_of[q];
-    if (up < 0 || up % DR != 0) return OOC_ERR_INTERNAL;
-    const int K = std::min(DIGIT_K, X.K - q * DIGIT_K);
-    const size_t units = (size_t)((X.rows + up + DR - 1) / DR);
-    a.nst[q] = (K + DK - 1) / DK;
-    const uint8_t* p = (const uint8_t*)X.planes + (size_t)q * X.slot;
-    a.planes[q] = p + (size_t)(up / DR) * a.nst[q] * UNIT_STAGE;
-    a.exps[q] = (const int*)(p + units * a.nst[q] * UNIT_STAGE) + up;
-  }
-  a.X = X.X;
-  a.ldx = X.ldx;
-  a.stride = X.stride;
-  a.org = X.org;
-  a.nb = X.nb;
-  a.rows = (int)X.rows;
   a.K = X.K;
   const int T = (int)((X.rows + DC - 1) / DC), lo = (int)(c_lo / DC), hi = (int)((c_hi + DC - 1) / DC);
-  const i64 nblk = count_blocks2(T, lo, hi);
-  if (nblk <= 0) return OOC_OK;
-  int dev = 0, nsm = 0;
-  OOC_CUDA_TRY(cudaGetDevice(&dev));
-  OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  OOC_CUDA_TRY(cudaFuncSetAttribute(k_digit_update, cudaFuncAttributeMaxDynamicSharedMemorySize, D_SMEM));
-  const i64 grid = std::max<i64>(1, std::min<i64>(nblk, std::max(1, nsm - std::max(0, reserve_sms))));
-  k_digit_update<<<(unsigned)grid, D_THREADS, D_SMEM, s>>>(a, C, T, lo, hi, nblk, const_cast<int*>(status));
-  OOC_CUDA_TRY(cudaGetLastError());
-  return OOC_OK;
+  return launch_blocks<false>(a, C, T, lo, hi, count_blocks2(T, lo, hi), const_cast<int*>(status), s, reserve_sms);
+}
+
+int launch_digit_gemm(const DigitRuns& A, const DigitRuns& B, double* C, i64 ldc, double alpha, double beta, int mask,
+                      int* status, cudaStream_t s) {
+  if (A.rows <= 0 || B.rows <= 0 || A.K <= 0) return OOC_OK;
+  if (!status || A.K != B.K) return OOC_ERR_INTERNAL;
+  UpdateArgs a{};
+  int rc = operand_of(A, &a.a, a.nst);
+  if (!rc) rc = operand_of(B, &a.b, a.nst);
+  if (rc) return rc;
+  a.nrun = (A.K + DIGIT_K - 1) / DIGIT_K;
+  a.K = A.K;
+  a.alpha = alpha;
+  a.beta = beta;
+  a.mask = mask;
+  const int T = (int)((B.rows + DC - 1) / DC);
+  // (a triangle's blocks on the other side of the diagonal are computed and not stored)
+  return launch_blocks<true>(a, TileMap{C, ldc, 0, 1, 0}, T, 0, 0, (A.rows + DR - 1) / DR * T, status, s, 0);
 }

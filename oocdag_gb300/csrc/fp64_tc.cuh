@@ -32,3 +32,9 @@ int launch_digits(DigitRuns& X, const int* status, cudaStream_t s);
 // where a row holds an infinity or NaN.
 int launch_digit_update(const DigitRuns& X, const TileMap& C, i64 c_lo, i64 c_hi, const int* status, cudaStream_t s,
                         int reserve_sms = 0);
+
+// C (A.rows x B.rows, ld ldc) = beta C + alpha (sum over the runs of A B^T) after launch_digits of both,
+// A.K == B.K, both with org 0: all of C (mask 0), its lower (1) or its upper (2) triangle.  A zero
+// beta leaves C unread.
+int launch_digit_gemm(const DigitRuns& A, const DigitRuns& B, double* C, i64 ldc, double alpha, double beta, int mask,
+                      int* status, cudaStream_t s);

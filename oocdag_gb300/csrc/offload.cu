@@ -14,6 +14,7 @@
 
 #include "../../include/ooc_offload.h"
 #include "common.cuh"
+#include "fp64_tc.cuh"
 
 namespace {
 
@@ -175,6 +176,8 @@ std::mutex g_mu;
 struct Slot {
   cudaStream_t s = nullptr;
   int* status = nullptr;
+  std::mutex mu;   // held by a call that uses ws until its work is done
+  GrowBuf ws;      // digit planes of the tensor-core products, kept across calls
 };
 Slot g_slot[MAX_R];
 thread_local int t_err = 0;
@@ -209,16 +212,49 @@ int finish(cudaStream_t s) {
   return OOC_OK;
 }
 
-void gemm_general(const double* A, i64 sar, i64 sak, const double* B, i64 sbr, i64 sbk, double* C, i64 ldc, int m,
-                  int n, int k, double alpha, double beta, int mask, cudaStream_t s) {
-  if (m <= 0 || n <= 0) return;
+// C = alpha opA opB^T + beta C (see k_gemm_general) on the slot's stream, done when it returns.
+// Tensor-core digit products (fp64_tc.cu) from DIGIT_FLOPS products on: a 256 x 256 x 256 product
+// takes GEMM_NEW us with its digits against GEMM_OLD us on the FP64 pipe; below, or without room
+// for the planes, FP64 MMAs.
+constexpr double DIGIT_PRODUCTS = 128.0 * 128.0 * 128.0;
+int gemm_general(Slot* sl, const double* A, i64 sar, i64 sak, const double* B, i64 sbr, i64 sbk, double* C, i64 ldc,
+                 int m, int n, int k, double alpha, double beta, int mask) {
+  if (m <= 0 || n <= 0) return OOC_OK;
+  cudaStream_t s = sl->s;
   if (k <= 0 || alpha == 0.0) {
     if (beta != 1.0)
       k_scale<<<dim3((m + 255) / 256, std::min(n, 4096)), 256, 0, s>>>(C, ldc, m, n, beta, mask);
-    return;
+    return finish(s);
+  }
+  if ((double)m * n * k >= DIGIT_PRODUCTS) {
+    std::lock_guard<std::mutex> lk(sl->mu);
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const int kp = std::min(k, DIGIT_K), runs = std::min(DIGIT_RUNS, (k + DIGIT_K - 1) / DIGIT_K);
+    const size_t sa = up(digit_plane_bytes(m, kp)), sb = up(digit_plane_bytes(n, kp));
+    if (sl->ws.ensure((sa + sb) * runs) == OOC_OK) {
+      int rc = OOC_OK;
+      cudaMemsetAsync(sl->status, 0, sizeof(int), s);
+      const bool same = A == B && sar == sbr && sak == sbk && m == n;  // a symmetric product
+      for (int k0 = 0; k0 < k && !rc; k0 += runs * DIGIT_K) {
+        const int K = std::min(runs * DIGIT_K, k - k0);
+        // element (r, k) at r * sr + k * sk: "tiles" of one row
+        DigitRuns Da{A + k0 * sak, sak, sar, 1, 0, m, K, sl->ws.p, sa, {}};
+        DigitRuns Db{B + k0 * sbk, sbk, sbr, 1, 0, n, K, (char*)sl->ws.p + sa * runs, sb, {}};
+        rc = launch_digits(Da, sl->status, s);
+        if (same) Db = Da;
+        else if (!rc) rc = launch_digits(Db, sl->status, s);
+        if (!rc) rc = launch_digit_gemm(Da, Db, C, ldc, alpha, k0 == 0 ? beta : 1.0, mask, sl->status, s);
+      }
+      int st = 0;
+      cudaMemcpyAsync(&st, sl->status, sizeof(int), cudaMemcpyDeviceToHost, s);
+      const int frc = finish(s);
+      if (rc || frc || st) t_err = rc ? rc : frc ? frc : OOC_ERR_TIMEOUT;
+      return rc ? rc : frc;
+    }
   }
   const int mb = (m + GBM - 1) / GBM, nbk = (n + GBM - 1) / GBM;
   k_gemm_general<<<mb * nbk, GTHR, 0, s>>>(A, sar, sak, B, sbr, sbk, C, ldc, m, n, k, alpha, beta, mask);
+  return finish(s);
 }
 
 }  // namespace
@@ -250,6 +286,7 @@ extern "C" void offload_destroy(void) {
   for (Slot& sl : g_slot) {
     if (sl.s) { cudaStreamSynchronize(sl.s); cudaStreamDestroy(sl.s); sl.s = nullptr; }
     if (sl.status) { cudaFree(sl.status); sl.status = nullptr; }
+    sl.ws.release();
   }
 }
 extern "C" void offload_destroy_(void) { offload_destroy(); }
@@ -281,7 +318,11 @@ static void vec_copy(int n, const double* x, int incx, double* y, int incy, int 
   if (incx <= 0 || incy <= 0) { t_err = -3; return; }
   Slot* sl = slot(r);
   if (!sl) return;
-  if (cudaMemcpy2DAsync(y, (size_t)incy * 8, x, (size_t)incx * 8, 8, n, kind, sl->s) != cudaSuccess) {
+  // contiguous vectors as one copy (a 2-D copy of n eight-byte rows takes 30 us for 65,536)
+  const cudaError_t e = incx == 1 && incy == 1
+                            ? cudaMemcpyAsync(y, x, (size_t)n * 8, kind, sl->s)
+                            : cudaMemcpy2DAsync(y, (size_t)incy * 8, x, (size_t)incx * 8, 8, n, kind, sl->s);
+  if (e != cudaSuccess) {
     cudaGetLastError();
     t_err = OOC_ERR_CUDA;
     return;
@@ -369,8 +410,7 @@ extern "C" void offload_dgemm(const char* transa, const char* transb, const MKL_
   const i64 sar = (ta == 'N') ? 1 : *lda, sak = (ta == 'N') ? *lda : 1;
   // opB as (n x k): opB(kk, j) = N -> b[kk + j*ldb], T -> b[j + kk*ldb]
   const i64 sbr = (tb == 'N') ? *ldb : 1, sbk = (tb == 'N') ? 1 : *ldb;
-  gemm_general(a, sar, sak, b, sbr, sbk, c, *ldc, *m, *n, *k, *alpha, *beta, 0, sl->s);
-  finish(sl->s);
+  gemm_general(sl, a, sar, sak, b, sbr, sbk, c, *ldc, *m, *n, *k, *alpha, *beta, 0);
 }
 
 extern "C" void offload_dsyrk(const char* uplo, const char* trans, const MKL_INT* n, const MKL_INT* k,
@@ -386,8 +426,7 @@ extern "C" void offload_dsyrk(const char* uplo, const char* trans, const MKL_INT
   if (!sl) return;
   // trans N: C = alpha A A^T + beta C, A n x k; trans T: C = alpha A^T A + beta C, A k x n
   const i64 sr = (t == 'N') ? 1 : *lda, sk = (t == 'N') ? *lda : 1;
-  gemm_general(a, sr, sk, a, sr, sk, c, *ldc, *n, *n, *k, *alpha, *beta, u == 'L' ? 1 : 2, sl->s);
-  finish(sl->s);
+  gemm_general(sl, a, sr, sk, a, sr, sk, c, *ldc, *n, *n, *k, *alpha, *beta, u == 'L' ? 1 : 2);
 }
 
 extern "C" void offload_dtrsm(const char* side, const char* uplo, const char* transa, const char* diag,
@@ -411,7 +450,7 @@ extern "C" void offload_dtrsm(const char* side, const char* uplo, const char* tr
   if (sd == 'R' && u == 'L' && t != 'N' && d == 'N') {
     // The form the reference uses (oocquark.cpp:407): B := alpha B L^-T, the library's
     // blocked column solve directly.
-    if (*alpha != 1.0) gemm_general(nullptr, 0, 0, nullptr, 0, 0, b, *ldb, *m, *n, 0, 0.0, *alpha, 0, s);
+    if (*alpha != 1.0) gemm_general(sl, nullptr, 0, 0, nullptr, 0, 0, b, *ldb, *m, *n, 0, 0.0, *alpha, 0);
     int rc = launch_trsm_col(a, *lda, TileCol{b, *ldb, 0}, 1, *m, *m, *n, sl->status, s);
     if (rc) t_err = rc;
     finish(s);
