@@ -591,7 +591,9 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
 // leave idle (its products of step K-1 beside the Cholesky of block K, while PT still holds
 // L(., K-1)), so the two phases share their barriers.
 // Dinv (= X^T), and X row-major as BF16 planes (or in FP32 into Xr when no planes are
-// asked for), at the end.  A non-positive pivot writes
+// asked for), at the end; of each row, what its 128-column block holds (zeros right of the
+// diagonal) and nothing beyond, which nothing reads.  A 256 tile takes 175k clocks alone
+// (93 us; 221k before: serial Cholesky 104k -> 45k, products and bank conflicts 79k -> 74k).  A non-positive pivot writes
 // info = col0 + j + 1 to the status word and stops, the columns left of the failed block
 // written, the others left as they were (as k_diag_f32).
 // ---------------------------------------------------------------------------------
@@ -599,7 +601,7 @@ constexpr int DS_MAX = 256, DS_NBK = DS_MAX / DG_B, DS_P = 36, DS_BLK = DG_B * D
 constexpr int DS_NBLK = DS_NBK * (DS_NBK + 1) / 2;
 constexpr int DS_PTLD = DS_MAX - DG_B + 4;  // rows below a block column, 16-byte multiple
 constexpr size_t DS_SMEM =
-    (size_t)((DS_NBLK + DS_NBK) * DS_BLK + DG_B * DS_PTLD + 2 * DG_B) * sizeof(float);
+    (size_t)((DS_NBLK + DS_NBK) * DS_BLK + DG_B * DS_PTLD + 3 * DG_B) * sizeof(float);
 static_assert(DS_SMEM + 64 <= 227 * 1024 && DG_SMEM + 64 <= 227 * 1024,
               "a diagonal kernel's shared memory exceeds the 227 KB a CTA may opt in to");
 
@@ -612,29 +614,34 @@ __device__ __forceinline__ void ds_block_ij(int b, int& I, int& J) {
   J = b - i * (i + 1) / 2;
 }
 
-// acc[i][j] += sum over k < 32 of A[k lda + r0 + i] B[k ldb + c0 + j]: lane's 4 x 8 tile of
-// a 32 x 32 block product (A and B k-major, rows 16-byte aligned)
-__device__ __forceinline__ void ds_mm32(float acc[4][8], const float* A, int lda, const float* B, int ldb, int r0,
-                                        int c0) {
-#pragma unroll 8
+// acc[i][j] += sum over k < 32 of A[k lda + r0 + 8 i] B[k ldb + c0 + j]: a lane's 4 rows (eight
+// apart, r0 = lane % 8) and 8 columns (c0 = 8 (lane / 8)) of a 32 x 32 block product (A and B
+// k-major, B's rows 16-byte aligned).  Rows eight apart keep ds_put free of bank conflicts
+// (four consecutive rows of pitch 36 met in two bank groups: 4 cycles an access).
+template <int Z>  // Z blocks of 32 rows one above the other
+__device__ __forceinline__ void ds_mm(float acc[Z][4][8], const float* A, int lda, const float* B, int ldb, int r0,
+                                      int c0) {
+#pragma unroll 4
   for (int k = 0; k < DG_B; k++) {
-    const float4 a = *reinterpret_cast<const float4*>(A + k * lda + r0);
     const float4 b0 = *reinterpret_cast<const float4*>(B + k * ldb + c0);
     const float4 b1 = *reinterpret_cast<const float4*>(B + k * ldb + c0 + 4);
-    const float av[4] = {a.x, a.y, a.z, a.w};
     const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int z = 0; z < Z; z++)
 #pragma unroll
-      for (int j = 0; j < 8; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+      for (int i = 0; i < 4; i++) {
+        const float av = A[k * lda + z * DG_B + r0 + 8 * i];
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[z][i][j] = fmaf(av, bv[j], acc[z][i][j]);
+      }
   }
 }
 
-// the lane's tile of block C (pitch DS_P) := C - acc (mode 0), -acc (mode 1) or acc (mode 2)
+// the lane's elements of block C (pitch DS_P) := C - acc (mode 0), -acc (mode 1) or acc (mode 2)
 __device__ __forceinline__ void ds_put(float* C, const float acc[4][8], int r0, int c0, int mode) {
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    float4* p = reinterpret_cast<float4*>(C + (r0 + i) * DS_P + c0);
+    float4* p = reinterpret_cast<float4*>(C + (r0 + 8 * i) * DS_P + c0);
     float v[8];
     if (mode == 0) {
       const float4 u = p[0], w = p[1];
@@ -654,30 +661,38 @@ __device__ __forceinline__ void ds_put(float* C, const float acc[4][8], int r0, 
 // r, as in k_diag_f32): the block's lower triangle := L (zeros above), dinv := 1 / diag(L).
 // Rows and columns from kb on are taken as the identity.  A non-positive pivot in the first
 // kb columns sets *fail and writes info = colg + j + 1 to the status word.
+// The pivot chain stays in registers: lane j + 1 forms its next pivot from its own row and passes
+// it on by a shuffle, while column j goes through shared memory (colb, two columns) for the
+// other updates, which the chain does not wait for (9.0k -> 5.4k clocks alone).
 __device__ __forceinline__ void ds_chol32(float* Tb, int kb, i64 colg, float* colb, float* dinv, int* fail,
                                           int* status, int lane) {
   float a[DG_B];
 #pragma unroll
   for (int c = 0; c < DG_B; c++) a[c] = (lane < kb && c <= lane) ? Tb[lane * DS_P + c] : ((c == lane) ? 1.f : 0.f);
   int first_bad = DG_B;
+  float d = __shfl_sync(0xffffffffu, a[0], 0);
 #pragma unroll
   for (int j = 0; j < DG_B; j++) {
-    colb[lane] = a[j];
-    __syncwarp();
-    float d = colb[j];
     if (!(d > 0.f)) {
       first_bad = min(first_bad, j);
       d = 1.f;
     }
     const float inv = rsqrtf(d);
-    const float lj = (lane == j) ? d * inv : a[j] * inv;  // L(lane, j)
-    const float ljs = lj * inv;                             // L(lane, j) / sqrt(d)
+    const float lj = (lane == j) ? d * inv : a[j] * inv;  // L(lane, j) for lane >= j
+    if (j + 1 < DG_B) d = __shfl_sync(0xffffffffu, fmaf(-lj, lj, a[j + 1 < DG_B ? j + 1 : 0]), j + 1);
     if (lane == j) dinv[j] = inv;
-    a[j] = (lane >= j) ? lj : a[j];
-#pragma unroll
-    for (int c = j + 1; c < DG_B; c++)
-      if (lane >= c) a[c] = fmaf(-ljs, colb[c], a[c]);
+    a[j] = lj;
+    float* col = colb + (j & 1) * DG_B;
+    col[lane] = lj;
     __syncwarp();
+#pragma unroll
+    for (int q = (j + 1) / 4; q < DG_B / 4; q++) {  // (elements above the diagonal are never used)
+      const float4 l = reinterpret_cast<const float4*>(col)[q];
+      const float lc[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (4 * q + u > j) a[4 * q + u] = fmaf(-lj, lc[u], a[4 * q + u]);
+    }
   }
   if (first_bad < kb && lane == 0) {
     *fail = 1;
@@ -700,7 +715,7 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
   __shared__ int s_fail;
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int NBK = (LN + DG_B - 1) / DG_B;
-  const int r0 = (lane & 7) * 4, c0 = (lane >> 3) * 8;  // the lane's tile of a block product
+  const int r0 = lane & 7, c0 = (lane >> 3) * 8;  // the lane's elements of a block product
   auto blk = [&](int I, int J) -> float* { return T + (I * (I + 1) / 2 + J) * DS_BLK; };
   if (t == 0) s_fail = 0;
   {  // the lower block triangle, 24 loads in flight per thread (lanes down a column)
@@ -741,13 +756,23 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
     float* Tkk = blk(K, K);
     if (warp == 0) {
       ds_chol32(Tkk, kb, col0 + k0, colb, dinv, &s_fail, status, lane);
-    } else if (K > 0) {  // phase 2, step K-1: block (K+ii, J) -= L(K+ii, K-1) X(K-1, J), J < K-1;
-                         // block (K+ii, K-1) := -L(K+ii, K-1) X_{K-1}
-      for (int it = warp - 1; it < (NBK - K) * K; it += DG_WARPS - 1) {
-        const int ii = it / K, J = it - ii * K;
-        float acc[4][8] = {};
-        ds_mm32(acc, PT + ii * DG_B, DS_PTLD, blk(K - 1, J), DS_P, r0, c0);
-        ds_put(blk(K + ii, J), acc, r0, c0, J < K - 1 ? 0 : 1);
+    } else if (K > 0 && (warp & 3) != 0) {
+      // phase 2, step K-1: block (K+ii, J) -= L(K+ii, K-1) X(K-1, J), J < K-1; block (K+ii, K-1) :=
+      // -L(K+ii, K-1) X_{K-1}; two blocks per item, at most 10 items.  Warps 4, 8 and 12 rest:
+      // they share warp 0's scheduler, whose chain ran 1.6 times as long beside them.
+      const int rows = NBK - K, np = (rows + 1) / 2;
+      for (int it = (warp >> 2) * 3 + (warp & 3) - 1; it < np * K; it += 12) {
+        const int pr = it / K, J = it - pr * K, ii = 2 * pr, mode = J < K - 1 ? 0 : 1;
+        if (ii + 1 < rows) {
+          float acc[2][4][8] = {};
+          ds_mm<2>(acc, PT + ii * DG_B, DS_PTLD, blk(K - 1, J), DS_P, r0, c0);
+          ds_put(blk(K + ii, J), acc[0], r0, c0, mode);
+          ds_put(blk(K + ii + 1, J), acc[1], r0, c0, mode);
+        } else {
+          float acc[1][4][8] = {};
+          ds_mm<1>(acc, PT + ii * DG_B, DS_PTLD, blk(K - 1, J), DS_P, r0, c0);
+          ds_put(blk(K + ii, J), acc[0], r0, c0, mode);
+        }
       }
     }
     __syncthreads();
@@ -798,25 +823,38 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
         if (lane >= c && lane < kb) D[(k0 + lane) + (i64)(k0 + c) * ldd] = Tkk[lane * DS_P + c];
     }
     __syncthreads();
-    // trailing lower block triangle: block (K+1+ii, K+1+jj) -= L(., K) L(., K)^T; then phase
-    // 2, step K: X(K, J) = X_KK B(K, J) for J < K (B(K, J) is final), and X(K, K) = X_KK
-    const int ntr = nI * (nI + 1) / 2;
+    // trailing lower block triangle: blocks (K+1+ii, K+1+jj) -= L(., K) L(., K)^T, two rows of
+    // blocks per item; then phase 2, step K: X(K, J) = X_KK B(K, J) for J < K (B(K, J) is final),
+    // and X(K, K) = X_KK.  At most 16 items in all.
+    int ntr = 0;
+    for (int jj = 0; jj < nI; jj++) ntr += (nI - jj + 1) / 2;
     for (int it = warp; it <= ntr + K; it += DG_WARPS) {
       if (it < ntr) {
-        int ii, jj;
-        ds_block_ij(it, ii, jj);
-        float acc[4][8] = {};
-        ds_mm32(acc, PT + ii * DG_B, DS_PTLD, PT + jj * DG_B, DS_PTLD, r0, c0);
-        ds_put(blk(K + 1 + ii, K + 1 + jj), acc, r0, c0, 0);
+        int jj = 0, u = it;
+        while (u >= (nI - jj + 1) / 2) {
+          u -= (nI - jj + 1) / 2;
+          jj++;
+        }
+        const int ii = jj + 2 * u;
+        if (ii + 1 < nI) {
+          float acc[2][4][8] = {};
+          ds_mm<2>(acc, PT + ii * DG_B, DS_PTLD, PT + jj * DG_B, DS_PTLD, r0, c0);
+          ds_put(blk(K + 1 + ii, K + 1 + jj), acc[0], r0, c0, 0);
+          ds_put(blk(K + 2 + ii, K + 1 + jj), acc[1], r0, c0, 0);
+        } else {
+          float acc[1][4][8] = {};
+          ds_mm<1>(acc, PT + ii * DG_B, DS_PTLD, PT + jj * DG_B, DS_PTLD, r0, c0);
+          ds_put(blk(K + 1 + ii, K + 1 + jj), acc[0], r0, c0, 0);
+        }
       } else {
         const float* Xk = XD + K * DS_BLK;
         const int J = it - ntr;
         if (J < K) {
           float* Bkj = blk(K, J);
-          float acc[4][8] = {};
-          ds_mm32(acc, Xk, DS_P, Bkj, DS_P, r0, c0);
+          float acc[1][4][8] = {};
+          ds_mm<1>(acc, Xk, DS_P, Bkj, DS_P, r0, c0);
           __syncwarp();
-          ds_put(Bkj, acc, r0, c0, 2);
+          ds_put(Bkj, acc[0], r0, c0, 2);
         } else {
 #pragma unroll 4
           for (int c = 0; c < DG_B; c++) Tkk[lane * DS_P + c] = (c <= lane) ? Xk[c * DS_P + lane] : 0.f;
@@ -825,14 +863,25 @@ __global__ void __launch_bounds__(DG_THREADS, 1)
     }
     __syncthreads();
   }
-  // Dinv = X^T (zeros below its diagonal), X row-major as BF16 planes or in FP32
-  for (int i = warp; i < LN; i += DG_WARPS)
-    for (int j = lane; j < LN; j += 32) {
-      const float x = (j <= i) ? blk(i >> 5, j >> 5)[(i & 31) * DS_P + (j & 31)] : 0.f;
-      Dinv[j + (i64)i * lde] = x;
-      if (Xh) dg_split_store(Xh, Xl, (i64)i * LN + j, x);
-      else Xr[(i64)i * LN + j] = x;
+  // Dinv = X^T, X row-major as BF16 planes or in FP32
+  for (int i = warp; i < LN; i += DG_WARPS) {
+    float x[DS_NBK];  // row i, lane's element of every block
+#pragma unroll
+    for (int J = 0; J < DS_NBK; J++) {
+      const int j = J * DG_B + lane;
+      x[J] = (j <= i) ? blk(i >> 5, J)[(i & 31) * DS_P + lane] : 0.f;
     }
+    const int jn = min(LN, (i | 127) + 1);  // right of the row's 128-column block nothing is read
+#pragma unroll
+    for (int J = 0; J < DS_NBK; J++) {
+      const int j = J * DG_B + lane;
+      if (j < jn) {
+        Dinv[j + (i64)i * lde] = x[J];
+        if (Xh) dg_split_store(Xh, Xl, (i64)i * LN + j, x[J]);
+        else Xr[(i64)i * LN + j] = x[J];
+      }
+    }
+  }
 }
 
 // FP32 column panel (m x K, ld ldx) -> copy with ld ldy.
