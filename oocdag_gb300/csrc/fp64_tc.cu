@@ -52,8 +52,8 @@ constexpr int EXP_NONFINITE = 1 << 28;        // row exponent of a row with an i
 static_assert(NG * DC == 512, "the eight order sums fill the TMEM");
 
 // ---- digits ----------------------------------------------------------------------
-// CTA: 64 rows, thread (row, stage of 32 columns).  Two passes over the thread's 32
-// elements: the row's largest exponent (the four threads of a row meet in shared memory),
+// CTA: 32 rows, thread (row, half stage of 16 columns).  Two passes over the thread's
+// elements: the row's largest exponent (the eight threads of a row meet in shared memory),
 // then the digits, eight columns at a time.  Integer arithmetic only.  Bound by HBM/L2:
 // 8 B in and 14 B out per element.
 __global__ void __launch_bounds__(256) k_digits(const double* __restrict__ X, i64 ldx, i64 stride, int nb, i64 org,
@@ -65,32 +65,34 @@ __global__ void __launch_bounds__(256) k_digits(const double* __restrict__ X, i6
   const int nst = (K + DK - 1) / DK;
   X += (i64)blockIdx.y * DIGIT_K * ldx;
   planes += (size_t)blockIdx.y * slot;
-  int* exps = reinterpret_cast<int*>(planes + (size_t)(gridDim.x / 2) * nst * UNIT_STAGE);
-  __shared__ int smax[4][64];
-  const int rl = threadIdx.x & 63, st = threadIdx.x >> 6;
-  const int row = blockIdx.x * 64 + rl;
+  int* exps = reinterpret_cast<int*>(planes + (size_t)(gridDim.x / 4) * nst * UNIT_STAGE);
+  constexpr int KT = DK / 2;  // columns per thread
+  __shared__ int smax[8][32];
+  const int rl = threadIdx.x & 31, cg = threadIdx.x >> 5, st = cg >> 1;
+  const int row = blockIdx.x * 32 + rl;
   const bool live = row < rows && st < nst;
   const i64 r = org + (row < rows ? row : 0);
-  const double* p = X + (r / nb) * stride + (r % nb) + (i64)st * DK * ldx;
-  const int kn = min(DK, K - st * DK);
-  unsigned long long v[DK];
+  const double* p = X + (r / nb) * stride + (r % nb) + (i64)cg * KT * ldx;
+  const int kn = min(KT, K - cg * KT);
+  unsigned long long v[KT];
   int bmax = 0;
 #pragma unroll
-  for (int k = 0; k < DK; k++) {
+  for (int k = 0; k < KT; k++) {
     v[k] = (live && k < kn) ? (unsigned long long)__double_as_longlong(p[(i64)k * ldx]) : 0ull;
   }
 #pragma unroll
-  for (int k = 0; k < DK; k++) bmax = max(bmax, (int)((v[k] >> 52) & 0x7FF));
-  smax[st][rl] = bmax;
+  for (int k = 0; k < KT; k++) bmax = max(bmax, (int)((v[k] >> 52) & 0x7FF));
+  smax[cg][rl] = bmax;
   __syncthreads();
-  bmax = max(max(smax[0][rl], smax[1][rl]), max(smax[2][rl], smax[3][rl]));
+#pragma unroll
+  for (int q = 0; q < 8; q++) bmax = max(bmax, smax[q][rl]);
   const int e = max(bmax, 1) - 1022;  // |x| < 2^e
-  if (st == 0) exps[row] = bmax == 0x7FF ? EXP_NONFINITE : e;
+  if (cg == 0) exps[row] = bmax == 0x7FF ? EXP_NONFINITE : e;
   if (st >= nst) return;
   uint8_t* base = planes + ((i64)(row >> 7) * nst + st) * UNIT_STAGE + (row & 127) * 64;
   const int swz = (row >> 1) & 3;  // 64-byte swizzle: 16-byte chunk c of a row sits at c ^ ((row / 2) % 4)
 #pragma unroll
-  for (int c = 0; c < 4; c++) {
+  for (int c = 0; c < 2; c++) {
     long long x[8];
 #pragma unroll
     for (int j = 0; j < 8; j++) {
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(256) k_digits(const double* __restrict__ X, i6
         // an integer of magnitude <= 128 is exact in BF16: the upper half of its FP32 encoding
         w[j / 2] = (__float_as_uint((float)d0) >> 16) | (__float_as_uint((float)d1) & 0xFFFF0000u);
       }
-      *reinterpret_cast<uint4*>(base + s * A_DIG + ((c ^ swz) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(base + s * A_DIG + (((2 * (cg & 1) + c) ^ swz) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
 }
@@ -132,26 +134,6 @@ __global__ void __launch_bounds__(256) k_digits(const double* __restrict__ X, i6
 // the same accumulator and shape (the pairs the tensor core keeps in issue order).
 constexpr uint32_t IDESC_D =
     (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(DC >> 3) << 17) | ((uint32_t)(DR >> 4) << 24);
-// USE: the A operand of the previous product is still in the collector buffer (0: read it and
-// keep it, 1: take it from there, 2: take it and let it go).
-template <int USE>
-__device__ __forceinline__ void umma_digit(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
-#define OOC_DIGIT_MMA(COLLECTOR)                                                                       \
-  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"                                          \
-               " tcgen05.mma.cta_group::1.kind::f16" COLLECTOR " [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d), \
-               "l"(da), "l"(db), "r"(IDESC_D), "r"(accumulate))
-  if constexpr (USE == 0) OOC_DIGIT_MMA(".collector::a::fill");
-  else if constexpr (USE == 1) OOC_DIGIT_MMA(".collector::a::use");
-  else OOC_DIGIT_MMA(".collector::a::lastuse");
-#undef OOC_DIGIT_MMA
-}
-__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   smem_u32(dst)),
-               "l"(src), "r"(bytes), "r"(smem_u32(bar))
-               : "memory");
-}
-
 struct Operand {
   const uint8_t* planes[DIGIT_RUNS];  // each run's planes and row exponents, at the update's first row
   const int* exps[DIGIT_RUNS];
@@ -323,9 +305,9 @@ __global__ void __launch_bounds__(D_THREADS, 1)
                 const uint32_t d = tmem + (uint32_t)((p + q) * DC);
                 const uint64_t da = umma_desc_sw64(a0 + p * A_DIG + kk * 32), db = umma_desc_sw64(b0 + q * B_DIG + kk * 32);
                 const uint32_t acc = (first && kc == 0) ? 0u : 1u;
-                if (q == 0) umma_digit<0>(d, da, db, acc);
-                else if (q + 1 < ND && p + q + 1 < NG) umma_digit<1>(d, da, db, acc);
-                else umma_digit<2>(d, da, db, acc);
+                if (q == 0) umma_collect<0>(IDESC_D, d, da, db, acc);
+                else if (q + 1 < ND && p + q + 1 < NG) umma_collect<1>(IDESC_D, d, da, db, acc);
+                else umma_collect<2>(IDESC_D, d, da, db, acc);
               }
           }
           umma_commit(&empty[s]);
@@ -460,7 +442,7 @@ int launch_digits(DigitRuns& X, const int* status, cudaStream_t s) {
   const int nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
   if (nrun > DIGIT_RUNS || X.rows > (1 << 30)) return OOC_ERR_INTERNAL;
   for (int q = 0; q < nrun; q++) X.org_of[q] = X.org;
-  OOC_CUDA_TRY(launch_pdl(k_digits, dim3(2 * (unsigned)((X.rows + DR - 1) / DR), nrun), 256, 0, s, X.X, X.ldx, X.stride,
+  OOC_CUDA_TRY(launch_pdl(k_digits, dim3(4 * (unsigned)((X.rows + DR - 1) / DR), nrun), 256, 0, s, X.X, X.ldx, X.stride,
                           X.nb, X.org, (int)X.rows, X.K, (uint8_t*)X.planes, X.slot, status));
   return OOC_OK;
 }

@@ -30,6 +30,7 @@
 
 #include "common.cuh"
 #include "devpool.cuh"
+#include "fp32_tc.cuh"
 #include "fp64_tc.cuh"
 #include "trsolve.cuh"
 
@@ -1328,11 +1329,30 @@ int syrk_lowprec(int prec, const double* X, i64 ldx, double* C, i64 ldc, int m, 
   return OOC_ERR_UNSUPPORTED;
 }
 
+// FP32 products as exact digit products (fp32_tc.cu): from K = 16 and half a block on.
+constexpr int DIGIT32_MIN_K = 16, DIGIT32_CHUNK = 512;
+
 // The same for the FP32 working matrix of a reduced-precision factor: C (FP32) -= X X^T
 // with X the FP32 column panel (no conversions).
 int syrk_f32(int prec, const float* X, i64 ldx, float* C, i64 ldc, int m, int K, const int* status, cudaStream_t s,
              DevBuf& work, int bj_lo = 0, int bj_hi = -1, int prepare = 1, int reserve_sms = 0) {
   if (m <= 0 || K <= 0) return OOC_OK;
+  if (prec == OOC_PREC_FP32 && K >= DIGIT32_MIN_K && m >= FB / 2) {
+    // digit products on the tensor cores, at most 512 columns at a time; without room for the planes
+    // the FP32 pipe (k_syrk_f32) does it
+    const int kc = std::min(K, DIGIT32_CHUNK);
+    bool ok = true;
+    if (prepare) ok = work.ensure(digit32_bytes(m, kc)) == OOC_OK;
+    if (ok) {
+      for (int k0 = 0; k0 < K; k0 += DIGIT32_CHUNK) {
+        const Digit32 D{X + (i64)k0 * ldx, ldx, m, std::min(kc, K - k0), work.p};
+        int rc = (prepare || K > DIGIT32_CHUNK) ? launch_digits32(D, status, s) : OOC_OK;
+        if (!rc) rc = launch_digit32_update(D, C, ldc, bj_lo, bj_hi, const_cast<int*>(status), s, reserve_sms);
+        if (rc) return rc;
+      }
+      return OOC_OK;
+    }
+  }
   if (prec == OOC_PREC_FP32) {
     const i64 T = ((i64)m + FB - 1) / FB;
     const i64 hi = std::min<i64>(bj_hi < 0 ? T : bj_hi, T);
@@ -3382,11 +3402,11 @@ extern "C" int ooc_spotrf_L(ooc_handle* h, float* A, int64_t n, int64_t lda, int
     OOC_CUDA_TRY(cudaMemcpy2DAsync(F.Lf, n * sizeof(float), A, lda * sizeof(float), n * sizeof(float), n,
                                    cudaMemcpyHostToDevice, s));
   }
-  if (cudaMalloc(&F.Dinvf, (size_t)bb * nb * nb * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&F.status, sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    return OOC_ERR_NOMEM;
-  }
+  // work buffers from the handle's cache: a cudaMalloc / cudaFree pair per call costs more than
+  // a small factorization
+  F.pool = ooc_handle_pool(h);
+  for (DevBuf* b : {&F.work, &F.scratch}) b->pool = F.pool.get();
+  if (F.alloc(&F.Dinvf, (size_t)bb * nb * nb * sizeof(float)) || F.alloc(&F.status, sizeof(int))) return OOC_ERR_NOMEM;
   OOC_CUDA_TRY(cudaMemsetAsync(F.status, 0, sizeof(int), s));
   cudaEvent_t e0, e1;
   OOC_CUDA_TRY(cudaEventCreate(&e0));

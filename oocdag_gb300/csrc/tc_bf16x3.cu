@@ -104,36 +104,6 @@ __global__ void k_split_bf16(const TX* __restrict__ X, i64 ldx, __nv_bfloat16* _
   }
 }
 
-// Block t of the lower-triangular block range [bj_lo, bj_hi) x rows (up to T), in strip
-// order: strips of STRIP block columns, and inside a strip row by row (the first rows of
-// a strip form its triangle).  Same set of blocks as ooc_lower_block_decode, other order.
-__device__ __forceinline__ void strip_block_decode(i64 t, int T, int bj_lo, int bj_hi, int* bi, int* bj) {
-  const int Tl = T - bj_lo, Wc = bj_hi - bj_lo;
-  for (int J0 = 0; J0 < Wc; J0 += STRIP) {
-    const i64 w = min(STRIP, Wc - J0);
-    const i64 tri = w * (w + 1) / 2;
-    const i64 cnt = tri + (i64)(Tl - J0 - w) * w;
-    if (t < cnt) {
-      int r, c;
-      if (t < tri) {
-        r = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);  // t < 136: exact enough, corrected below
-        while ((i64)(r + 1) * (r + 2) / 2 <= t) r++;
-        while ((i64)r * (r + 1) / 2 > t) r--;
-        c = (int)(t - (i64)r * (r + 1) / 2);
-      } else {
-        const i64 u = t - tri;
-        r = (int)(w + u / w);
-        c = (int)(u % w);
-      }
-      *bi = bj_lo + J0 + r;
-      *bj = bj_lo + J0 + c;
-      return;
-    }
-    t -= cnt;
-  }
-  *bi = *bj = 0;  // not reached for t < number of blocks
-}
-
 template <typename TC>
 __global__ void __launch_bounds__(THREADS, 1)
     k_syrk_bf16x3(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,

@@ -115,6 +115,57 @@ __device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr) {
   return d;
 }
 
+// One product of BF16 operands (kind::f16, instruction descriptor `idesc`).
+// USE: the A operand of the previous product is still in the collector buffer (0: read it and
+// keep it, 1: take it from there, 2: take it and let it go).
+template <int USE>
+__device__ __forceinline__ void umma_collect(uint32_t idesc, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
+#define OOC_DIGIT_MMA(COLLECTOR)                                                                       \
+  asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"                                          \
+               " tcgen05.mma.cta_group::1.kind::f16" COLLECTOR " [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem_d), \
+               "l"(da), "l"(db), "r"(idesc), "r"(accumulate))
+  if constexpr (USE == 0) OOC_DIGIT_MMA(".collector::a::fill");
+  else if constexpr (USE == 1) OOC_DIGIT_MMA(".collector::a::use");
+  else OOC_DIGIT_MMA(".collector::a::lastuse");
+#undef OOC_DIGIT_MMA
+}
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
+                   smem_u32(dst)),
+               "l"(src), "r"(bytes), "r"(smem_u32(bar))
+               : "memory");
+}
+
+// Block t of the lower-triangular block range [bj_lo, bj_hi) x rows (up to T), in strip
+// order: strips of STRIP block columns, and inside a strip row by row (the first rows of
+// a strip form its triangle).  Same set of blocks as ooc_lower_block_decode, other order.
+__device__ __forceinline__ void strip_block_decode(i64 t, int T, int bj_lo, int bj_hi, int* bi, int* bj) {
+  const int Tl = T - bj_lo, Wc = bj_hi - bj_lo;
+  for (int J0 = 0; J0 < Wc; J0 += STRIP) {
+    const i64 w = min(STRIP, Wc - J0);
+    const i64 tri = w * (w + 1) / 2;
+    const i64 cnt = tri + (i64)(Tl - J0 - w) * w;
+    if (t < cnt) {
+      int r, c;
+      if (t < tri) {
+        r = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);  // t < 136: exact enough, corrected below
+        while ((i64)(r + 1) * (r + 2) / 2 <= t) r++;
+        while ((i64)r * (r + 1) / 2 > t) r--;
+        c = (int)(t - (i64)r * (r + 1) / 2);
+      } else {
+        const i64 u = t - tri;
+        r = (int)(w + u / w);
+        c = (int)(u % w);
+      }
+      *bi = bj_lo + J0 + r;
+      *bj = bj_lo + J0 + c;
+      return;
+    }
+    t -= cnt;
+  }
+  *bi = *bj = 0;  // not reached for t < number of blocks
+}
+
 // Block t of the block columns [bj_lo, bj_hi) x row blocks bi2 (twice as high as a block column
 // is wide; T rows of the block columns' width) with 2 bi2 + 1 >= bj, in strips of STRIP block columns, row by row inside a strip.
 __device__ __forceinline__ void strip2_decode(i64 t, int T, int bj_lo, int bj_hi, int* bi2, int* bj) {
