@@ -43,111 +43,162 @@ constexpr int DK = 32;                        // K per stage
 constexpr int A_DIG = DR * DK * 2;            // 8 KB: one digit of 128 rows x 32 columns
 constexpr int B_DIG = DC * DK * 2;            // 4 KB
 constexpr int UNIT_STAGE = ND * A_DIG;        // 56 KB: one stage of a plane unit
-constexpr int D_STAGE = ND * (A_DIG + B_DIG); // 84 KB
-constexpr int D_STAGES = 2;
 constexpr int D_EPI_WARPS = 8;                // two per TMEM lane quadrant, 32 columns each
 constexpr int D_THREADS = 64 + 32 * D_EPI_WARPS;
-constexpr int D_SMEM = D_STAGES * D_STAGE + 1024 /*align*/ + 256 /*barriers*/;
+enum { UPDATE, GENERAL, NARROW };              // what a kernel computes (k_digit_update)
+__host__ __device__ constexpr int stage_bytes(int mode) { return UNIT_STAGE + (mode == NARROW ? 2 * ND * 16 * DK * 2 : ND * B_DIG); }
+__host__ __device__ constexpr int stages(int mode) { return mode == NARROW ? 3 : 2; }
+__host__ __device__ constexpr int d_smem(int mode) { return stages(mode) * stage_bytes(mode) + 1024 /*align*/ + 256 /*barriers*/; }
+// Of at most 16 columns (general products): the second operand's digits lie one below the other,
+// 16 rows each, between 6 x 16 and 16 rows of zeros.
+constexpr int NC = 16;                        // columns
+constexpr int N_SLAB = NC * DK * 2;           // 1 KB: one digit's rows, or zeros
 constexpr int EXP_NONFINITE = 1 << 28;        // row exponent of a row with an infinity or NaN
 static_assert(NG * DC == 512, "the eight order sums fill the TMEM");
+static_assert(stage_bytes(NARROW) == UNIT_STAGE + 2 * ND * N_SLAB, "six slabs of zeros, the digits, one of zeros");
 
 // ---- digits ----------------------------------------------------------------------
-// CTA: 32 rows, thread (row, half stage of 16 columns).  Two passes over the thread's
-// elements: the row's largest exponent (the eight threads of a row meet in shared memory),
-// then the digits, eight columns at a time.  Integer arithmetic only.  Bound by HBM/L2:
-// 8 B in and 14 B out per element.
-__global__ void __launch_bounds__(256) k_digits(const double* __restrict__ X, i64 ldx, i64 stride, int nb, i64 org,
-                                                int rows, int Kall, uint8_t* __restrict__ planes, size_t slot,
-                                                const int* status) {
-  pdl_wait();
-  if (status && *(volatile const int*)status) return;
-  const int K = min(DIGIT_K, Kall - (int)blockIdx.y * DIGIT_K);  // blockIdx.y: run
+// CTA: 32 rows x one run of 128 columns, thread (row, 8 columns): four lanes hold a row's 32
+// columns of a stage, so a warp reads eight full sectors of each column and writes 512
+// contiguous bytes per digit.  Two passes over the thread's elements: the row's largest
+// exponent (shuffles, then shared memory across the stages), then the digits.  Integer
+// arithmetic only, two instructions a digit and half a one to pack it: with 128 added at every
+// digit at once, the digits are the bytes of the sum less 128.
+// 16384 x 16384 elements of a symmetric matrix: 1.17 ms (5.0 TB/s of 8 B in and 14 B out per element), where a
+// thread per 16 columns that peeled the digits off one by one took 1.9 ms.
+struct DigitArgs {
+  const double* X;
+  i64 ldx, stride, org, k0;
+  int nb, rows, K, ksign, sym;
+  const int* kshift;
+  const int* only_if;
+  uint8_t* planes;
+  size_t slot;
+};
+
+// The byte of w that `sel` picks, less 128, as a float: 2^23 + byte is an FP32 number.
+template <int SEL>
+__device__ __forceinline__ uint32_t digit_float(uint32_t w) {
+  return __float_as_uint(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 | SEL)) - 8388736.f);
+}
+// The same digit of x0 and x1 as two BF16 (an integer of magnitude <= 128 is exact in it: the upper
+// half of its FP32 encoding).  Digit 0 is the top one, 0..256 before the 128 are taken off.
+template <int S>
+__device__ __forceinline__ uint32_t digit_pair(unsigned long long x0, unsigned long long x1) {
+  uint32_t f0, f1;
+  if constexpr (S == 0) {
+    f0 = __float_as_uint(__uint_as_float((uint32_t)(x0 >> 48) | 0x4B000000u) - 8388736.f);
+    f1 = __float_as_uint(__uint_as_float((uint32_t)(x1 >> 48) | 0x4B000000u) - 8388736.f);
+  } else {
+    constexpr int B = ND - 1 - S;
+    f0 = digit_float<(B & 3)>((uint32_t)(B < 4 ? x0 : x0 >> 32));
+    f1 = digit_float<(B & 3)>((uint32_t)(B < 4 ? x1 : x1 >> 32));
+  }
+  return __byte_perm(f0, f1, 0x7632);
+}
+template <int S>
+__device__ __forceinline__ void put_digits(const unsigned long long (&x)[8], uint8_t* p) {
+  *reinterpret_cast<uint4*>(p + S * A_DIG) = make_uint4(digit_pair<S>(x[0], x[1]), digit_pair<S>(x[2], x[3]),
+                                                        digit_pair<S>(x[4], x[5]), digit_pair<S>(x[6], x[7]));
+  if constexpr (S + 1 < ND) put_digits<S + 1>(x, p);
+}
+
+// SHIFT: exponents moved by kshift, and symmetric operands.
+template <bool SHIFT>
+__device__ __forceinline__ void digit_rows(const DigitArgs& a, int run) {
+  constexpr int KT = 8;  // columns per thread
+  __shared__ int smax[DIGIT_K / DK][32];
+  const int K = min(DIGIT_K, a.K - run * DIGIT_K);
   const int nst = (K + DK - 1) / DK;
-  X += (i64)blockIdx.y * DIGIT_K * ldx;
-  planes += (size_t)blockIdx.y * slot;
+  uint8_t* planes = a.planes + (size_t)run * a.slot;
   int* exps = reinterpret_cast<int*>(planes + (size_t)(gridDim.x / 4) * nst * UNIT_STAGE);
-  constexpr int KT = DK / 2;  // columns per thread
-  __shared__ int smax[8][32];
-  const int rl = threadIdx.x & 31, cg = threadIdx.x >> 5, st = cg >> 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int rl = 8 * (warp & 3) + (lane >> 2), ch = lane & 3, st = warp >> 2;
   const int row = blockIdx.x * 32 + rl;
-  const bool live = row < rows && st < nst;
-  const i64 r = org + (row < rows ? row : 0);
-  const double* p = X + (r / nb) * stride + (r % nb) + (i64)cg * KT * ldx;
-  const int kn = min(KT, K - cg * KT);
+  const bool live = row < a.rows;
+  const uint32_t r = (uint32_t)a.org + (live ? row : 0);
+  const int kc = st * DK + ch * KT;                      // the thread's first column in the run
+  const i64 kb = (i64)run * DIGIT_K + kc;
+  const int kn = live ? min(KT, K - kc) : 0;
+  const double* p = a.X + (a.sym ? 0 : (i64)(r / (uint32_t)a.nb) * a.stride + r % (uint32_t)a.nb + kb * a.ldx);
   unsigned long long v[KT];
-  int bmax = 0;
+  int sft[SHIFT ? KT : 1];
+  int bmax = -(1 << 20);  // of the nonzero elements
+  bool finite = true;
 #pragma unroll
   for (int k = 0; k < KT; k++) {
-    v[k] = (live && k < kn) ? (unsigned long long)__double_as_longlong(p[(i64)k * ldx]) : 0ull;
+    const double* q = p + (i64)k * a.ldx;
+    if (SHIFT && a.sym) {
+      const i64 c = a.k0 + kb + k;
+      q = a.X + (r >= c ? r + c * a.ldx : c + r * a.ldx);
+    }
+    v[k] = k < kn ? (unsigned long long)__double_as_longlong(*q) : 0ull;
+    if constexpr (SHIFT) sft[k] = k < kn ? a.ksign * a.kshift[a.k0 + kb + k] : 0;
   }
 #pragma unroll
-  for (int k = 0; k < KT; k++) bmax = max(bmax, (int)((v[k] >> 52) & 0x7FF));
-  smax[cg][rl] = bmax;
+  for (int k = 0; k < KT; k++) {
+    const int be = (int)((v[k] >> 52) & 0x7FF);
+    if (v[k] << 1) bmax = max(bmax, max(be, 1) + (SHIFT ? sft[SHIFT ? k : 0] : 0));
+    finite = finite && be != 0x7FF;
+  }
+  if (!finite) bmax = EXP_NONFINITE;
+  bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, 1));
+  bmax = max(bmax, __shfl_xor_sync(0xffffffffu, bmax, 2));
+  __syncthreads();  // (the last run's are read)
+  if (ch == 0) smax[st][rl] = bmax;
   __syncthreads();
 #pragma unroll
-  for (int q = 0; q < 8; q++) bmax = max(bmax, smax[q][rl]);
-  const int e = max(bmax, 1) - 1022;  // |x| < 2^e
-  if (cg == 0) exps[row] = bmax == 0x7FF ? EXP_NONFINITE : e;
+  for (int q = 0; q < DIGIT_K / DK; q++) bmax = max(bmax, smax[q][rl]);
+  const int e = bmax < -(1 << 19) ? 0 : bmax - 1022;  // |x| < 2^e (a row of zeros: any scale)
+  if (st == 0 && ch == 0) exps[row] = bmax >= EXP_NONFINITE ? EXP_NONFINITE : e;
   if (st >= nst) return;
-  uint8_t* base = planes + ((i64)(row >> 7) * nst + st) * UNIT_STAGE + (row & 127) * 64;
-  const int swz = (row >> 1) & 3;  // 64-byte swizzle: 16-byte chunk c of a row sits at c ^ ((row / 2) % 4)
+  unsigned long long x[KT];
 #pragma unroll
-  for (int c = 0; c < 2; c++) {
-    long long x[8];
-#pragma unroll
-    for (int j = 0; j < 8; j++) {
-      const unsigned long long b = v[8 * c + j];
-      const int be = (int)((b >> 52) & 0x7FF);
-      unsigned long long m = b & 0xFFFFFFFFFFFFFull;
-      if (be) m |= 1ull << 52;
-      const int sh = max(be, 1) - 1020 - e;  // X = m 2^sh, sh <= 2
-      if (sh >= 0) m <<= min(sh, 2);
-      else m = sh < -55 ? 0ull : (m + (1ull << (-sh - 1))) >> (-sh);
-      x[j] = (b >> 63) ? -(long long)m : (long long)m;
-    }
-#pragma unroll
-    for (int s = ND - 1; s >= 0; s--) {
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        int d0, d1;
-        if (s > 0) {
-          d0 = (int)((x[j] + 128) & 255) - 128;
-          d1 = (int)((x[j + 1] + 128) & 255) - 128;
-          x[j] = (x[j] - d0) >> 8;
-          x[j + 1] = (x[j + 1] - d1) >> 8;
-        } else {
-          d0 = (int)x[j];
-          d1 = (int)x[j + 1];
-        }
-        // an integer of magnitude <= 128 is exact in BF16: the upper half of its FP32 encoding
-        w[j / 2] = (__float_as_uint((float)d0) >> 16) | (__float_as_uint((float)d1) & 0xFFFF0000u);
-      }
-      *reinterpret_cast<uint4*>(base + s * A_DIG + (((2 * (cg & 1) + c) ^ swz) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-    }
+  for (int j = 0; j < KT; j++) {
+    const unsigned long long b = v[j];
+    const int be = (int)((b >> 52) & 0x7FF);
+    unsigned long long m = b & 0xFFFFFFFFFFFFFull;
+    if (be) m |= 1ull << 52;
+    const int sh = max(be, 1) + (SHIFT ? sft[SHIFT ? j : 0] : 0) - 1020 - e;  // X = m 2^sh, sh <= 2
+    if (sh >= 0) m <<= min(sh, 2);
+    else m = sh < -55 ? 0ull : (m + (1ull << (-sh - 1))) >> (-sh);
+    x[j] = ((b >> 63) ? 0ull - m : m) + 0x0080808080808080ull;
   }
+  // 64-byte swizzle: 16-byte chunk c of a row sits at c ^ ((row / 2) % 4)
+  put_digits<0>(x, planes + ((i64)(row >> 7) * nst + st) * UNIT_STAGE + (row & 127) * 64 + ((ch ^ ((row >> 1) & 3)) << 4));
+}
+template <bool SHIFT>
+__global__ void __launch_bounds__(512) k_digits(const __grid_constant__ DigitArgs a, const int* status) {
+  pdl_wait();
+  if (status && *(volatile const int*)status) return;
+  if (SHIFT && a.only_if && !*(volatile const int*)a.only_if) return;
+  for (int run = blockIdx.y; run * DIGIT_K < a.K; run += gridDim.y) digit_rows<SHIFT>(a, run);
 }
 
 // ---- update ----------------------------------------------------------------------
 // One product shape throughout: M = 128 rows, N = 64 columns, K = 16, each MMA adding into
 // one order's 64 TMEM columns, so that every pair of MMAs that shares an accumulator has
 // the same accumulator and shape (the pairs the tensor core keeps in issue order).
-constexpr uint32_t IDESC_D =
-    (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(DC >> 3) << 17) | ((uint32_t)(DR >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc_of(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(DR >> 4) << 24);
+}
 struct Operand {
   const uint8_t* planes[DIGIT_RUNS];  // each run's planes and row exponents, at the update's first row
   const int* exps[DIGIT_RUNS];
   const double* X;                    // the runs' elements (non-finite rows)
-  i64 ldx, stride, org;
-  int nb, rows;
-  __device__ const double* row(int r) const {
-    const i64 g = org + r;
-    return X + (g / nb) * stride + g % nb;
+  i64 ldx, stride, org, k0;
+  int nb, rows, sym, ksign;
+  const int* kshift;
+  size_t slot;                        // general products: bytes from one run's planes to the next
+  __device__ double at(int r, i64 k) const {
+    const i64 g = org + r, c = k0 + k;
+    const double v = sym ? X[g >= c ? g + c * ldx : c + g * ldx] : X[(g / nb) * stride + g % nb + k * ldx];
+    return kshift ? scalbn(v, ksign * kshift[c]) : v;
   }
 };
 struct UpdateArgs {
   Operand a, b;                       // rows and columns of C
-  int nst[DIGIT_RUNS];                // a run's stages of DK columns
+  int nst[DIGIT_RUNS];                // a run's stages of DK columns (general products: 4, but in the last)
   int nrun, K;
   double alpha, beta;                 // general products only
   int mask;
@@ -183,11 +234,9 @@ __device__ __forceinline__ double digit_value(long long V, int es, bool& special
 __device__ __noinline__ double digit_value_special(long long V, int es, const UpdateArgs& X, int run, int r, int c) {
   if (es <= EXP_NONFINITE / 2) return scalbn((double)V, es - 54);
   if (r >= X.a.rows || c >= X.b.rows) return 0.0;
-  const double* a = X.a.row(r) + (i64)run * DIGIT_K * X.a.ldx;
-  const double* b = X.b.row(c) + (i64)run * DIGIT_K * X.b.ldx;
   double v = 0.0;
-  for (int k = 0; k < X.nst[run] * DK && run * DIGIT_K + k < X.K; k++)
-    v = fma(a[(i64)k * X.a.ldx], b[(i64)k * X.b.ldx], v);
+  const int k1 = min(X.K, (run + 1) * DIGIT_K);
+  for (int k = run * DIGIT_K; k < k1; k++) v = fma(X.a.at(r, k), X.b.at(c, k), v);
   return v;
 }
 
@@ -200,17 +249,25 @@ __device__ __noinline__ double digit_value_special(long long V, int es, const Up
 // sums are out of TMEM; C overlaps with the next block.  A 4096 x 4096 lower triangle with
 // K = 128 takes 99 us (21.7 TFLOP/s of FP64 work); FP64 MMAs took 3.2 ms for K = 256.
 // GENERAL: C = beta C + alpha A B^T on all of C or a triangle (mask) instead, T columns of blocks.
-template <bool GENERAL>
+// NARROW: the same for C of at most 16 columns.  Products narrower than 64 columns cost what 64 do, so
+// one product takes digit p of A against the 128 rows of B from digit -p on, zeros standing for the
+// digits there are not: column 16 g + j of the one accumulator is order g of column j.  7 products per
+// K = 16 instead of 34; two accumulators, so that one run is put together beside the next one's
+// products, and three stages of 70 KB.  16384 x 16 with K = 16384 (3.8 GB of planes): 525 us
+// (7.2 TB/s, all that HBM gives), 1300 us as GENERAL.
+template <int MODE>
 __global__ void __launch_bounds__(D_THREADS, 1)
     k_digit_update(const __grid_constant__ UpdateArgs X, TileMap Cm, int T, int bj_lo, int bj_hi, i64 nblk,
                    int* status) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(smem + D_STAGES * D_STAGE);
-  uint64_t* empty = full + D_STAGES;
-  uint64_t* tfull = empty + D_STAGES;
-  uint64_t* tempty = tfull + 1;
-  uint64_t* done = tempty + 1;
+  constexpr int S_BYTES = stage_bytes(MODE), S_NUM = stages(MODE);
+  constexpr int S_ACC = MODE == NARROW ? 2 : 1;  // sets of order sums
+  uint64_t* full = (uint64_t*)(smem + S_NUM * S_BYTES);
+  uint64_t* empty = full + S_NUM;
+  uint64_t* tfull = empty + S_NUM;
+  uint64_t* tempty = tfull + 2;
+  uint64_t* done = tempty + 2;
   uint32_t* tmem_slot = (uint32_t*)(done + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
   volatile long long* n_issued = (volatile long long*)(tmem_slot + 2);
@@ -218,12 +275,14 @@ __global__ void __launch_bounds__(D_THREADS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < D_STAGES; s++) {
+    for (int s = 0; s < S_NUM; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(tfull, 1);
-    mbar_init(tempty, D_EPI_WARPS);
+    for (int s = 0; s < S_ACC; s++) {
+      mbar_init(&tfull[s], 1);
+      mbar_init(&tempty[s], D_EPI_WARPS);
+    }
     mbar_init(done, 1);
     *abort_flag = 0;
     *n_issued = 0;
@@ -235,14 +294,29 @@ __global__ void __launch_bounds__(D_THREADS, 1)
                  "r"(NG * DC));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
+  if constexpr (MODE == NARROW) {  // the zeros around each stage's digits (and those, until they are loaded)
+    constexpr int per = 2 * ND * N_SLAB / 16;
+    for (int i = threadIdx.x; i < S_NUM * per; i += D_THREADS)
+      *reinterpret_cast<uint4*>(smem + i / per * S_BYTES + UNIT_STAGE + i % per * 16) = make_uint4(0, 0, 0, 0);
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
   const uint32_t tmem = *tmem_slot;
   pdl_wait();  // (the set-up above touches no other kernel's data)
   if (*(volatile int*)status) nblk = 0;
+  auto run_stages = [&](int run) {
+    return MODE == UPDATE ? X.nst[run] : run + 1 < X.nrun ? DIGIT_K / DK : (X.K - run * DIGIT_K + DK - 1) / DK;
+  };
+  auto run_planes = [&](const Operand& o, int run) { return MODE != UPDATE ? o.planes[0] + (size_t)run * o.slot : o.planes[run]; };
+  auto run_exps = [&](const Operand& o, int run) {  // (the last run of a general product has fewer stages before them)
+    if constexpr (MODE == UPDATE) return o.exps[run];
+    const size_t units = (size_t)((o.rows + DR - 1) / DR);
+    return (const int*)(run_planes(o, run) + units * run_stages(run) * UNIT_STAGE);
+  };
   auto block_at = [&](i64 t, int* bi, int* bj) {
-    if constexpr (GENERAL) {
+    if constexpr (MODE != UPDATE) {
       *bi = (int)(t / T);
       *bj = (int)(t % T);
     } else {
@@ -258,20 +332,22 @@ __global__ void __launch_bounds__(D_THREADS, 1)
         int bi, bj;
         block_at(t, &bi, &bj);
         for (int run = 0; ok && run < X.nrun; run++) {
-          const int nst = X.nst[run];
-          const uint8_t* ua = X.a.planes[run] + (i64)bi * nst * UNIT_STAGE;
-          const uint8_t* ub = X.b.planes[run] + (i64)(bj >> 1) * nst * UNIT_STAGE + (bj & 1) * B_DIG;
+          const int nst = run_stages(run);
+          const uint8_t* ua = run_planes(X.a, run) + (i64)bi * nst * UNIT_STAGE;
+          const uint8_t* ub = run_planes(X.b, run) + (i64)(bj >> 1) * nst * UNIT_STAGE + (bj & 1) * B_DIG;
           for (int kc = 0; kc < nst; kc++, c++) {
-            const int s = (int)(c % D_STAGES);
-            if (!mbar_wait(&empty[s], (uint32_t)((c / D_STAGES) & 1) ^ 1u, abort_flag)) {
+            const int s = (int)(c % S_NUM);
+            if (!mbar_wait(&empty[s], (uint32_t)((c / S_NUM) & 1) ^ 1u, abort_flag)) {
               ok = false;
               break;
             }
-            uint8_t* st = smem + s * D_STAGE;
-            mbar_expect_tx(&full[s], D_STAGE);
+            uint8_t* st = smem + s * S_BYTES;
+            constexpr int bb = MODE == NARROW ? N_SLAB : B_DIG;
+            uint8_t* sb = st + UNIT_STAGE + (MODE == NARROW ? (ND - 1) * N_SLAB : 0);
+            mbar_expect_tx(&full[s], UNIT_STAGE + ND * bb);
             bulk_load(st, ua + (i64)kc * UNIT_STAGE, UNIT_STAGE, &full[s]);
             for (int q = 0; q < ND; q++)
-              bulk_load(st + UNIT_STAGE + q * B_DIG, ub + (i64)kc * UNIT_STAGE + q * A_DIG, B_DIG, &full[s]);
+              bulk_load(sb + q * bb, ub + (i64)kc * UNIT_STAGE + q * A_DIG, bb, &full[s]);
             *n_issued = c + 1;
           }
         }
@@ -284,18 +360,27 @@ __global__ void __launch_bounds__(D_THREADS, 1)
       int tl = 0;
       bool ok = true;
       for (i64 u = blockIdx.x * (i64)X.nrun; ok && u < nblk * X.nrun; tl++) {  // u: (block, run)
-        const int nst = X.nst[tl % X.nrun];
+        const int nst = run_stages(tl % X.nrun);
         u += (tl % X.nrun == X.nrun - 1) ? (i64)(gridDim.x - 1) * X.nrun + 1 : 1;
-        if (!mbar_wait(tempty, (uint32_t)(tl & 1) ^ 1u, abort_flag)) { ok = false; break; }
+        const int set = tl % S_ACC;
+        if (!mbar_wait(&tempty[set], (uint32_t)((tl / S_ACC) & 1) ^ 1u, abort_flag)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
         for (int kc = 0; kc < nst; kc++, c++) {
-          const int s = (int)(c % D_STAGES);
-          if (!mbar_wait(&full[s], (uint32_t)((c / D_STAGES) & 1), abort_flag)) { ok = false; break; }
+          const int s = (int)(c % S_NUM);
+          if (!mbar_wait(&full[s], (uint32_t)((c / S_NUM) & 1), abort_flag)) { ok = false; break; }
           *n_consumed = c + 1;
           asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-          const uint32_t a0 = smem_u32(smem + s * D_STAGE), b0 = a0 + UNIT_STAGE;
+          const uint32_t a0 = smem_u32(smem + s * S_BYTES), b0 = a0 + UNIT_STAGE;
 #pragma unroll
           for (int kk = 0; kk < DK / 16; kk++) {
+            if constexpr (MODE == NARROW) {
+#pragma unroll
+              for (int p = 0; p < ND; p++)
+                umma_collect<3>(idesc_of(NG * NC), tmem + (uint32_t)(set * NG * NC),
+                                umma_desc_sw64(a0 + p * A_DIG + kk * 32),
+                                umma_desc_sw64(b0 + (ND - 1 - p) * N_SLAB + kk * 32), kc == 0 && kk == 0 && p == 0 ? 0u : 1u);
+              continue;
+            }
 #pragma unroll
             for (int p = 0; p < ND; p++)
 #pragma unroll
@@ -305,21 +390,22 @@ __global__ void __launch_bounds__(D_THREADS, 1)
                 const uint32_t d = tmem + (uint32_t)((p + q) * DC);
                 const uint64_t da = umma_desc_sw64(a0 + p * A_DIG + kk * 32), db = umma_desc_sw64(b0 + q * B_DIG + kk * 32);
                 const uint32_t acc = (first && kc == 0) ? 0u : 1u;
-                if (q == 0) umma_collect<0>(IDESC_D, d, da, db, acc);
-                else if (q + 1 < ND && p + q + 1 < NG) umma_collect<1>(IDESC_D, d, da, db, acc);
-                else umma_collect<2>(IDESC_D, d, da, db, acc);
+                if (q == 0) umma_collect<0>(idesc_of(DC), d, da, db, acc);
+                else if (q + 1 < ND && p + q + 1 < NG) umma_collect<1>(idesc_of(DC), d, da, db, acc);
+                else umma_collect<2>(idesc_of(DC), d, da, db, acc);
               }
           }
           umma_commit(&empty[s]);
         }
         if (!ok) break;
-        umma_commit(tfull);
+        umma_commit(&tfull[set]);
       }
       if (!ok) *abort_flag = 1;
     }
   } else {
     const int quad = warp & 3;
-    const int half = ((warp - 2) >> 2) * 32;  // this warp's 32 of the block's 64 columns
+    constexpr int W = MODE == NARROW ? NC / 2 : DC / 2;  // this warp's columns of the block
+    const int half = ((warp - 2) >> 2) * W;
     const int nb = Cm.nb;
     int tl = 0;
     bool ok = true;
@@ -327,13 +413,14 @@ __global__ void __launch_bounds__(D_THREADS, 1)
       int bi, bj;
       block_at(t, &bi, &bj);
       const int row = bi * DR + quad * 32 + lane, col0 = bj * DC + half;
-      double v[32];  // the runs' sum
+      double v[W];  // the runs' sum
 #pragma unroll
-      for (int q = 0; q < 32; q++) v[q] = 0.0;
+      for (int q = 0; q < W; q++) v[q] = 0.0;
       for (int run = 0; run < X.nrun; run++, tl++) {
-        const int* exps = X.b.exps[run];
-        const int er = X.a.exps[run][row];
-        const bool got = mbar_wait(tfull, (uint32_t)(tl & 1), abort_flag);
+        const int* exps = run_exps(X.b, run);
+        const int er = run_exps(X.a, run)[row];
+        const int set = tl % S_ACC;
+        const bool got = mbar_wait(&tfull[set], (uint32_t)((tl / S_ACC) & 1), abort_flag);
         if (!__all_sync(0xffffffffu, got)) {
           if (lane == 0) *abort_flag = 1;
           ok = false;
@@ -341,14 +428,16 @@ __global__ void __launch_bounds__(D_THREADS, 1)
         }
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
 #pragma unroll
-        for (int b = 0; b < 4; b++) {  // eight columns at a time
+        for (int b = 0; b < W / 8; b++) {  // eight columns at a time
+          if (MODE != UPDATE && col0 + 8 * b >= X.b.rows) break;
           uint32_t g[NG][8];
 #pragma unroll
           for (int o = 0; o < NG; o++)
             asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
                          : "=r"(g[o][0]), "=r"(g[o][1]), "=r"(g[o][2]), "=r"(g[o][3]), "=r"(g[o][4]), "=r"(g[o][5]),
                            "=r"(g[o][6]), "=r"(g[o][7])
-                         : "r"(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(o * DC + half + 8 * b)));
+                         : "r"(tmem + ((uint32_t)(quad * 32) << 16) +
+                               (uint32_t)((set * NG + o) * (MODE == NARROW ? NC : DC) + half + 8 * b)));
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::);
           const int4 ea = *reinterpret_cast<const int4*>(exps + col0 + 8 * b);
           const int4 eb = *reinterpret_cast<const int4*>(exps + col0 + 8 * b + 4);
@@ -367,25 +456,26 @@ __global__ void __launch_bounds__(D_THREADS, 1)
         }
         asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
         __syncwarp();
-        if (lane == 0) mbar_arrive(tempty);  // the accumulators may be overwritten now
+        if (lane == 0) mbar_arrive(&tempty[set]);  // the accumulators may be overwritten now
       }
       if (!ok) break;
-      if constexpr (GENERAL) {
+      if constexpr (MODE != UPDATE) {
         if (row < X.a.rows) {
-          const int q0 = X.mask == 2 ? max(0, row - col0) : 0;  // columns [q0, q1) of the warp's 32
-          const int q1 = min(32, X.mask == 1 ? min(row + 1, X.b.rows) - col0 : X.b.rows - col0);
+          const int q0 = X.mask == 2 ? max(0, row - col0) : 0;  // columns [q0, q1) of the warp's
+          const int q1 = min(W, X.mask == 1 ? min(row + 1, X.b.rows) - col0 : X.b.rows - col0);
+          constexpr int H = W < 16 ? W : 16;
           double* p = Cm.base + row + (i64)col0 * Cm.ld;
 #pragma unroll
-          for (int h = 0; h < 2; h++) {
-            double cv[16];
+          for (int h = 0; h < W / H; h++) {
+            double cv[H];
 #pragma unroll
-            for (int q = 0; q < 16; q++)
-              cv[q] = X.beta != 0.0 && 16 * h + q >= q0 && 16 * h + q < q1 ? p[(i64)(16 * h + q) * Cm.ld] : 0.0;
+            for (int q = 0; q < H; q++)
+              cv[q] = X.beta != 0.0 && H * h + q >= q0 && H * h + q < q1 ? p[(i64)(H * h + q) * Cm.ld] : 0.0;
 #pragma unroll
-            for (int q = 0; q < 16; q++)
-              if (16 * h + q >= q0 && 16 * h + q < q1)
-                p[(i64)(16 * h + q) * Cm.ld] =
-                    X.beta == 0.0 ? X.alpha * v[16 * h + q] : fma(X.alpha, v[16 * h + q], X.beta * cv[q]);
+            for (int q = 0; q < H; q++)
+              if (H * h + q >= q0 && H * h + q < q1)
+                p[(i64)(H * h + q) * Cm.ld] =
+                    X.beta == 0.0 ? X.alpha * v[H * h + q] : fma(X.alpha, v[H * h + q], X.beta * cv[q]);
           }
         }
       } else if (row < X.a.rows) {
@@ -419,7 +509,7 @@ __global__ void __launch_bounds__(D_THREADS, 1)
     }
     if (warp == 0 && lane == 0) {  // let copies in flight land (bounded) before the shared memory goes away
       for (long long c = *n_consumed; c < *n_issued; c++)
-        (void)mbar_wait(&full[c % D_STAGES], (uint32_t)((c / D_STAGES) & 1), nullptr);
+        (void)mbar_wait(&full[c % S_NUM], (uint32_t)((c / S_NUM) & 1), nullptr);
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
@@ -440,18 +530,27 @@ size_t digit_plane_bytes(i64 rows, int K) {
 int launch_digits(DigitRuns& X, const int* status, cudaStream_t s) {
   if (X.rows <= 0 || X.K <= 0) return OOC_OK;
   const int nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
-  if (nrun > DIGIT_RUNS || X.rows > (1 << 30)) return OOC_ERR_INTERNAL;
-  for (int q = 0; q < nrun; q++) X.org_of[q] = X.org;
-  OOC_CUDA_TRY(launch_pdl(k_digits, dim3(4 * (unsigned)((X.rows + DR - 1) / DR), nrun), 256, 0, s, X.X, X.ldx, X.stride,
-                          X.nb, X.org, (int)X.rows, X.K, (uint8_t*)X.planes, X.slot, status));
+  if (X.rows > (1 << 30) || nrun > 65535) return OOC_ERR_INTERNAL;
+  for (int q = 0; q < std::min(nrun, DIGIT_RUNS); q++) X.org_of[q] = X.org;
+  const DigitArgs a{X.X, X.ldx, X.stride, X.org, X.k0, X.sym ? 1 : X.nb, (int)X.rows, X.K, X.ksign, X.sym, X.kshift, X.only_if,
+                    (uint8_t*)X.planes, X.slot};
+  const unsigned gx = 4 * (unsigned)((X.rows + DR - 1) / DR);
+  // planes that are seldom rewritten: few CTAs of many runs, since 65536 that only look at the word take 0.5 ms
+  const dim3 grid(gx, X.only_if ? std::min<unsigned>(nrun, std::max(1u, 2432 / gx)) : nrun);
+  if (X.sym || X.kshift) {
+    if (!X.kshift) return OOC_ERR_INTERNAL;
+    OOC_CUDA_TRY(launch_pdl(k_digits<true>, grid, 512, 0, s, a, status));
+  } else {
+    OOC_CUDA_TRY(launch_pdl(k_digits<false>, grid, 512, 0, s, a, status));
+  }
   return OOC_OK;
 }
 
 // The runs of X as an operand whose first row is X.org.
-static int operand_of(const DigitRuns& X, Operand* o, int* nst) {
+static int operand_of(const DigitRuns& X, Operand* o, int* nst, bool general) {
   const int nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
-  if (nrun > DIGIT_RUNS || X.rows > (1 << 30)) return OOC_ERR_INTERNAL;
-  for (int q = 0; q < nrun; q++) {
+  if ((!general && nrun > DIGIT_RUNS) || X.rows > (1 << 30)) return OOC_ERR_INTERNAL;
+  for (int q = 0; q < (general ? 1 : nrun); q++) {
     const i64 up = X.org - X.org_of[q];
     if (up < 0 || up % DR != 0) return OOC_ERR_INTERNAL;
     const int K = std::min(DIGIT_K, X.K - q * DIGIT_K);
@@ -467,19 +566,24 @@ static int operand_of(const DigitRuns& X, Operand* o, int* nst) {
   o->org = X.org;
   o->nb = X.nb;
   o->rows = (int)X.rows;
+  o->k0 = X.k0;
+  o->sym = X.sym;
+  o->ksign = X.ksign;
+  o->kshift = X.kshift;
+  o->slot = X.slot;
   return OOC_OK;
 }
 
-template <bool GENERAL>
+template <int MODE>
 static int launch_blocks(const UpdateArgs& a, const TileMap& C, int T, int lo, int hi, i64 nblk, int* status,
                          cudaStream_t s, int reserve_sms) {
   if (nblk <= 0) return OOC_OK;
   int dev = 0, nsm = 0;
   OOC_CUDA_TRY(cudaGetDevice(&dev));
   OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  OOC_CUDA_TRY(cudaFuncSetAttribute(k_digit_update<GENERAL>, cudaFuncAttributeMaxDynamicSharedMemorySize, D_SMEM));
+  OOC_CUDA_TRY(cudaFuncSetAttribute(k_digit_update<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, d_smem(MODE)));
   const i64 grid = std::max<i64>(1, std::min<i64>(nblk, std::max(1, nsm - std::max(0, reserve_sms))));
-  OOC_CUDA_TRY(launch_pdl(k_digit_update<GENERAL>, dim3((unsigned)grid), D_THREADS, D_SMEM, s, a, C, T, lo, hi, nblk,
+  OOC_CUDA_TRY(launch_pdl(k_digit_update<MODE>, dim3((unsigned)grid), D_THREADS, d_smem(MODE), s, a, C, T, lo, hi, nblk,
                           status));
   return OOC_OK;
 }
@@ -490,13 +594,13 @@ int launch_digit_update(const DigitRuns& X, const TileMap& C, i64 c_lo, i64 c_hi
   if (X.rows <= 0 || X.K <= 0 || c_lo >= c_hi) return OOC_OK;
   if (!status || c_lo % DC != 0 || C.nb % DC != 0) return OOC_ERR_INTERNAL;
   UpdateArgs a{};
-  int rc = operand_of(X, &a.a, a.nst);
+  int rc = operand_of(X, &a.a, a.nst, false);
   if (rc) return rc;
   a.b = a.a;
   a.nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
   a.K = X.K;
   const int T = (int)((X.rows + DC - 1) / DC), lo = (int)(c_lo / DC), hi = (int)((c_hi + DC - 1) / DC);
-  return launch_blocks<false>(a, C, T, lo, hi, count_blocks2(T, lo, hi), const_cast<int*>(status), s, reserve_sms);
+  return launch_blocks<UPDATE>(a, C, T, lo, hi, count_blocks2(T, lo, hi), const_cast<int*>(status), s, reserve_sms);
 }
 
 int launch_digit_gemm(const DigitRuns& A, const DigitRuns& B, double* C, i64 ldc, double alpha, double beta, int mask,
@@ -504,8 +608,8 @@ int launch_digit_gemm(const DigitRuns& A, const DigitRuns& B, double* C, i64 ldc
   if (A.rows <= 0 || B.rows <= 0 || A.K <= 0) return OOC_OK;
   if (!status || A.K != B.K) return OOC_ERR_INTERNAL;
   UpdateArgs a{};
-  int rc = operand_of(A, &a.a, a.nst);
-  if (!rc) rc = operand_of(B, &a.b, a.nst);
+  int rc = operand_of(A, &a.a, a.nst, true);
+  if (!rc) rc = operand_of(B, &a.b, a.nst, true);
   if (rc) return rc;
   a.nrun = (A.K + DIGIT_K - 1) / DIGIT_K;
   a.K = A.K;
@@ -514,5 +618,8 @@ int launch_digit_gemm(const DigitRuns& A, const DigitRuns& B, double* C, i64 ldc
   a.mask = mask;
   const int T = (int)((B.rows + DC - 1) / DC);
   // (a triangle's blocks on the other side of the diagonal are computed and not stored)
-  return launch_blocks<true>(a, TileMap{C, ldc, 0, 1, 0}, T, 0, 0, (A.rows + DR - 1) / DR * T, status, s, 0);
+  const TileMap map{C, ldc, 0, 1, 0};
+  const i64 nblk = (A.rows + DR - 1) / DR * T;
+  return B.rows <= NC ? launch_blocks<NARROW>(a, map, T, 0, 0, nblk, status, s, 0)
+                      : launch_blocks<GENERAL>(a, map, T, 0, 0, nblk, status, s, 0);
 }

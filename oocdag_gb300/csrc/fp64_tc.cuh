@@ -18,12 +18,21 @@ struct DigitRuns {
   void* planes;
   size_t slot;           // bytes between the runs' planes, >= digit_plane_bytes of each
   i64 org_of[DIGIT_RUNS];  // row each run's planes start at (org, or a multiple of 128 rows above it)
+  // Operands of launch_digit_gemm only.  kshift: element (r, k) enters as x 2^(ksign kshift[k]) (the
+  // other operand with the opposite sign).  sym: X is a symmetric matrix given by its lower
+  // triangle, rows 0.. and columns k0.. of it (org 0, ld ldx; stride and nb unused).
+  const int* kshift = nullptr;
+  int ksign = 0;
+  int sym = 0;
+  i64 k0 = 0;
+  const int* only_if = nullptr;  // planes are rewritten only where this word is not 0 (with kshift)
 };
 
 // Bytes of the digit planes and row exponents of `rows` rows of K columns.
 size_t digit_plane_bytes(i64 rows, int K);
 
-// The planes of every run of X for rows org.. (sets org_of).
+// The planes of every run of X for rows org.. (sets org_of; any number of runs for
+// launch_digit_gemm, at most DIGIT_RUNS for launch_digit_update).
 int launch_digits(DigitRuns& X, const int* status, cudaStream_t s);
 
 // C(org + r, org + c) -= sum over the runs of X(r) X(c)^T, for r < rows, c in [c_lo, c_hi), r >= c, after
@@ -34,7 +43,7 @@ int launch_digit_update(const DigitRuns& X, const TileMap& C, i64 c_lo, i64 c_hi
                         int reserve_sms = 0);
 
 // C (A.rows x B.rows, ld ldc) = beta C + alpha (sum over the runs of A B^T) after launch_digits of both,
-// A.K == B.K, both with org 0: all of C (mask 0), its lower (1) or its upper (2) triangle.  A zero
+// A.K == B.K, both with org 0 and any number of runs: all of C (mask 0), its lower (1) or its upper (2) triangle.  A zero
 // beta leaves C unread.
 int launch_digit_gemm(const DigitRuns& A, const DigitRuns& B, double* C, i64 ldc, double alpha, double beta, int mask,
                       int* status, cudaStream_t s);

@@ -1645,6 +1645,114 @@ int symv_lower(bool abs, const double* A, i64 lda, const double* X, i64 ldx, dou
   return OOC_OK;
 }
 
+// Exponents for the residual's digit products: cexp[q] = the exponent of column q's largest
+// element, then t[k] = max over q of (exponent of X(k, q)) - cexp[q] (<= 0; 0 for a row of zeros or
+// non-finite elements).
+__global__ void k_col_exponent(const double* __restrict__ X, i64 ldx, int n, int* __restrict__ cexp) {
+  __shared__ int sm[32];
+  int e = 0;
+  for (int k = threadIdx.x; k < n; k += blockDim.x) {
+    const int be = (__double2hiint(X[k + (i64)blockIdx.x * ldx]) >> 20) & 0x7FF;
+    if (be != 0x7FF) e = max(e, be);
+  }
+  e = __reduce_max_sync(0xffffffffu, e);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    e = __reduce_max_sync(0xffffffffu, threadIdx.x < blockDim.x / 32 ? sm[threadIdx.x] : 0);
+    if (threadIdx.x == 0) cexp[blockIdx.x] = e;
+  }
+}
+// stale is raised where a shift in use is more than SHIFT_SLACK from the row's t.
+constexpr int SHIFT_SLACK = 2;
+__global__ void k_row_shift(const double* __restrict__ X, i64 ldx, int n, int r, const int* __restrict__ cexp,
+                            const int* __restrict__ shift, int* __restrict__ t_of, int* __restrict__ stale) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  int t = -4096;
+  for (int q = 0; q < r; q++) {
+    const double x = X[k + (i64)q * ldx];
+    const int be = (__double2hiint(x) >> 20) & 0x7FF;
+    if (x != 0.0 && be != 0x7FF) t = max(t, be - cexp[q]);
+  }
+  t = t == -4096 ? 0 : max(t, -1000);
+  t_of[k] = t;
+  if (abs(t - shift[k]) > SHIFT_SLACK) *stale = 1;
+}
+__global__ void k_take_shift(const int* __restrict__ t_of, int* __restrict__ shift, int n, const int* __restrict__ stale) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n && *stale) shift[k] = t_of[k];
+}
+
+// R := R - A X (n x r, r <= 16, FP64) with A symmetric (lower triangle given, on the device) by
+// digit products on the tensor cores, as symv_lower does it on the FP64 pipe.  Column k of A is
+// scaled by 2^shift[k], the size of X(k, :), and X's row by its inverse, so that the one exponent
+// per row and run belongs to |a(i, k)| |x(k)|, not to |a(i, k)| alone.  Planes of all of A (14 bytes per
+// element, both triangles' elements read from the lower one) are kept through a refinement where they
+// take at most SYMM_KEEP bytes, and rewritten when the solution's rows have changed size by more than
+// 2^SHIFT_SLACK (the first correction may do that, later ones hardly); a larger A is taken in chunks of
+// columns whose planes fit SYMM_CHUNK bytes, each time.
+// Time of a whole step (residual, solve, norms), on the FP64 pipe and so, in ms; "first" with the planes:
+//   n = 16384  r = 16  first 9.4 / 3.7  then 9.0 / 2.1      r = 2  2.9 / 2.7  2.5 / 1.2     r = 1  1.5 / 2.7  1.1 / 1.2
+//   n = 4096   r = 16        1.42 / 0.76     1.30 / 0.58    r = 2  0.54 / 0.52  0.43 / 0.35  r = 1  0.39 / 0.51  0.26 / 0.32
+//   n = 3072                                                r = 2  0.40 / 0.42  0.33 / 0.28
+//   n = 2048   r = 5         0.72 / 0.41     0.64 / 0.29    r = 3  0.35 / 0.34  0.26 / 0.22  r = 2  0.32 / 0.33  0.25 / 0.24
+// One right-hand side has too few FMAs for the planes to pay.
+bool symm_by_digits(i64 n, int r) { return r >= 2 && n >= (r == 2 ? 3072 : 2048); }
+constexpr size_t SYMM_KEEP = 16ull << 30, SYMM_CHUNK = 512ull << 20;
+struct SymmDigits {
+  size_t sa, sx;  // planes of one run of A and of X
+  int runs;       // runs of A held at a time
+  bool kept;      // ... which are all of them
+  char *pa, *px;
+  int *shift, *t_of, *cexp, *stale;
+  int* status;    // of the products
+};
+// OOC_ERR_NOMEM without room for the planes.
+int symm_digits_begin(SymmDigits* D, DevBuf& buf, int n, int r, cudaStream_t s) {
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  D->sa = up(digit_plane_bytes(n, DIGIT_K));
+  D->sx = up(digit_plane_bytes(r, DIGIT_K));
+  const size_t ints = up((size_t)n * 4);
+  const int nrun = (n + DIGIT_K - 1) / DIGIT_K;
+  int rc = OOC_ERR_NOMEM;
+  D->kept = (D->sa + D->sx) * nrun <= SYMM_KEEP;
+  if (D->kept) rc = buf.ensure((D->sa + D->sx) * nrun + 2 * ints + 512);
+  if (rc) D->kept = false;
+  D->runs = D->kept ? nrun : (int)std::max<size_t>(1, std::min<size_t>(nrun, SYMM_CHUNK / (D->sa + D->sx)));
+  if (rc && buf.ensure((D->sa + D->sx) * D->runs + 2 * ints + 512)) return OOC_ERR_NOMEM;
+  D->pa = (char*)buf.p;
+  D->px = D->pa + D->sa * D->runs;
+  D->shift = (int*)(D->px + D->sx * D->runs);
+  D->t_of = (int*)((char*)D->shift + ints);
+  D->cexp = (int*)((char*)D->t_of + ints);
+  D->stale = (int*)((char*)D->cexp + 256);
+  D->status = D->stale + 1;
+  OOC_CUDA_TRY(cudaMemsetAsync(D->stale, 1, sizeof(int), s));  // no planes yet
+  OOC_CUDA_TRY(cudaMemsetAsync(D->status, 0, sizeof(int), s));
+  return OOC_OK;
+}
+int symm_digits(const SymmDigits& D, const double* A, i64 lda, const double* X, i64 ldx, double* R, i64 ldr, int n, int r,
+                cudaStream_t s) {
+  const unsigned g = (n + 255) / 256;
+  k_col_exponent<<<r, 1024, 0, s>>>(X, ldx, n, D.cexp);
+  k_row_shift<<<g, 256, 0, s>>>(X, ldx, n, r, D.cexp, D.shift, D.t_of, D.stale);
+  k_take_shift<<<g, 256, 0, s>>>(D.t_of, D.shift, n, D.stale);
+  OOC_CUDA_TRY(cudaGetLastError());
+  for (i64 c0 = 0; c0 < n; c0 += (i64)D.runs * DIGIT_K) {
+    const int K = (int)std::min<i64>((i64)D.runs * DIGIT_K, n - c0);
+    DigitRuns Da{A, lda, 0, 1, 0, n, K, D.pa, D.sa, {}, D.shift, 1, 1, c0, D.kept ? D.stale : nullptr};
+    // (row q, column k) of the second operand is X(c0 + k, q)
+    DigitRuns Dx{X + c0, 1, ldx, 1, 0, r, K, D.px, D.sx, {}, D.shift, -1, 0, c0};
+    int rc = launch_digits(Da, D.status, s);
+    if (!rc) rc = launch_digits(Dx, D.status, s);
+    if (!rc) rc = launch_digit_gemm(Da, Dx, R, ldr, -1.0, 1.0, 0, D.status, s);
+    if (rc) return rc;
+  }
+  if (D.kept) OOC_CUDA_TRY(cudaMemsetAsync(D.stale, 0, sizeof(int), s));
+  return OOC_OK;
+}
+
 // Panel schedule of a reduced-precision factor: nb-wide panels up to column tail0 (a
 // multiple of nb), then nb2-wide panels (tail0 = n: uniform nb).  Panel p starts at J0,
 // is LN wide, and its diagonal tile's inverse sits at Dinv + off with leading dimension ld
@@ -1716,6 +1824,7 @@ struct ooc_factor {
   DevBuf rws;    // refinement workspace (residual, FP32 correction, reductions), kept
   DevBuf xch;    // exchange buffer of the triangular solves, zeroed when allocated
   unsigned epoch = 0;  // launches on it since then
+  DevBuf dig;    // digit planes of A during a refinement
   DevBuf sws;    // FP32 right-hand sides of ooc_factor_solve on a reduced factor, kept
   DevBuf part2;  // partial sums of the refinement's norm (second stream)
   // FP64 copy of a host A's lower triangle (ld n), kept for the refinement
@@ -1784,7 +1893,7 @@ int queue_solve_error(const void* exchange, int* err, cudaStream_t s) {
 }
 int solve_status(int err) {
   if (!err) return OOC_OK;
-  ooc_set_last_message("triangular solve: a bounded wait between blocks ran out");
+  ooc_set_last_message("triangular solve or residual: a bounded wait ran out");
   return OOC_ERR_TIMEOUT;
 }
 }  // namespace
@@ -2465,7 +2574,7 @@ static int create_impl(ooc_handle* h, const double* A, int64_t n, int64_t lda, b
     }
   }
   F->pool = ooc_handle_pool(h);
-  for (DevBuf* b : {&F->part, &F->work, &F->scratch, &F->work2, &F->part2, &F->rws, &F->xch, &F->sws})
+  for (DevBuf* b : {&F->part, &F->work, &F->scratch, &F->work2, &F->part2, &F->rws, &F->xch, &F->dig, &F->sws})
     b->pool = F->pool.get();
   int rc = alloc_factor(F, n, nb, reduced);
   if (rc) { delete F; return rc; }
@@ -2955,6 +3064,13 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
       }
     }
   }
+  SymmDigits symm{};
+  bool by_digits = false;
+  if (!rc && !gen && symm_by_digits(n, r)) {
+    rc = symm_digits_begin(&symm, F->dig, (int)n, r, s);
+    by_digits = rc == OOC_OK;
+    if (rc == OOC_ERR_NOMEM) rc = OOC_OK;
+  }
   std::vector<double> hv((size_t)nred * r);
   const unsigned gb = (unsigned)((n + 255) / 256);
   // column slices of the generated products (enough CTAs to fill the GPU)
@@ -3036,7 +3152,8 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) { ooc_set_last_error(e, "generated residual", __FILE__, __LINE__); rc = OOC_ERR_CUDA; break; }
     } else {
-      rc = symv_lower(false, Astore, lda, X, ldx, R, n, (int)n, r, -1.0, 1.0, s, F->part);
+      rc = by_digits ? symm_digits(symm, Astore, lda, X, ldx, R, n, (int)n, r, s)
+                     : symv_lower(false, Astore, lda, X, ldx, R, n, (int)n, r, -1.0, 1.0, s, F->part);
       if (rc) break;
     }
     rc = colmax(R, n, r, nr);
@@ -3061,10 +3178,15 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
     }
     it++;
   }
-  int solve_err = 0;
+  int solve_err = 0, st = 0;
   if (!rc) rc = queue_solve_error(F->xch.p, &solve_err, s);
+  if (!rc && by_digits && cudaMemcpyAsync(&st, symm.status, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) rc = OOC_ERR_CUDA;
   if (!rc) rc = ooc_wait_stream(h, s);
-  if (!rc) rc = solve_status(solve_err);
+  if (!rc) rc = solve_status(solve_err | st);
+  if (by_digits) {
+    if (rc) cudaStreamSynchronize(s);
+    F->dig.release();
+  }
   if (s2 != s) cudaStreamSynchronize(s2);  // the norm's buffers may go now
   if (ev_in) cudaEventDestroy(ev_in);
   if (Atmp) {

@@ -117,7 +117,7 @@ __device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t saddr) {
 
 // One product of BF16 operands (kind::f16, instruction descriptor `idesc`).
 // USE: the A operand of the previous product is still in the collector buffer (0: read it and
-// keep it, 1: take it from there, 2: take it and let it go).
+// keep it, 1: take it from there, 2: take it and let it go; 3: the buffer is not used).
 template <int USE>
 __device__ __forceinline__ void umma_collect(uint32_t idesc, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t accumulate) {
 #define OOC_DIGIT_MMA(COLLECTOR)                                                                       \
@@ -126,7 +126,8 @@ __device__ __forceinline__ void umma_collect(uint32_t idesc, uint32_t tmem_d, ui
                "l"(da), "l"(db), "r"(idesc), "r"(accumulate))
   if constexpr (USE == 0) OOC_DIGIT_MMA(".collector::a::fill");
   else if constexpr (USE == 1) OOC_DIGIT_MMA(".collector::a::use");
-  else OOC_DIGIT_MMA(".collector::a::lastuse");
+  else if constexpr (USE == 2) OOC_DIGIT_MMA(".collector::a::lastuse");
+  else OOC_DIGIT_MMA("");
 #undef OOC_DIGIT_MMA
 }
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
