@@ -876,13 +876,13 @@ def forward_error_table(h, args, seed):
 # ----------------------------------------------------------------------------------
 def refine_launches(iters, npanels):
     """Kernels one ooc_solve_refine call launches on an FP32 or split-BF16 factor (device
-    A, up to 16 right-hand sides), from its structure: the norm of A (three residual-pass
-    kernels and a column maximum), the maximum of B, X0 (two conversions and a triangular
-    solve), per residual evaluation (iters + 1 of them) an initialisation, three pass
-    kernels and two column maxima, and per correction two conversions and a solve.  A
-    solve is one kernel, whatever the number of panels."""
+    A, one right-hand side), from its structure: the norm of A (three residual-pass
+    kernels), X0 (two conversions and a triangular solve), per residual evaluation
+    (iters + 1 of them) an initialisation, three pass kernels and one for all the column
+    maxima, and per correction two conversions and a solve.  A solve is one kernel,
+    whatever the number of panels."""
     solve = 1
-    return 4 + 1 + (2 + solve) + 6 * (iters + 1) + iters * (2 + solve)
+    return 3 + (2 + solve) + 5 * (iters + 1) + iters * (2 + solve)
 
 
 def panel_schedule(n, nb, prec, tail_order):
