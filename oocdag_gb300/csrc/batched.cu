@@ -8,9 +8,8 @@
 // diagonal block factored by one warp in registers, the panel solved a row per thread in
 // registers and kept transposed in shared memory, the trailing update by 32 x 32 blocks
 // with a 4 x 8 register tile per lane, the forward substitution inside the factorization
-// and the backward sweep on the vector in shared memory.  FP64 (factor_one): the diagonal
-// block column by column by the CTA, the panel solve a row per thread, the trailing update
-// from a row copy of the panel with 4 x 4 register tiles, then both sweeps (solve_one).
+// and the backward sweep on the vector in shared memory.  FP64 (factor_f64): the same steps with the
+// trailing update by digit products on the tensor cores, the diagonal block by four warps.
 // Per-matrix LAPACK info goes to an array; a failed matrix is skipped.  The panel width is
 // chosen per size bucket by the autotuner (oocdag_gb300/autotune.py).
 //
@@ -28,6 +27,8 @@
 #include <vector>
 
 #include "common.cuh"
+#include "digits.cuh"
+#include "fp64_panel.cuh"
 
 namespace {
 
@@ -43,34 +44,28 @@ struct Item {
   int mode;   // 0: factor + solve, 1: solve with an L already in `a`
 };
 
-template <typename T>
-__device__ __forceinline__ T tsqrt(T x) { return sqrt(x); }
-template <>
-__device__ __forceinline__ float tsqrt<float>(float x) { return sqrtf(x); }
-
 // Cholesky of the kb x kb (kb <= 32) block at rows/columns off.. of D (lower, column-major,
 // ld 65) in one warp: lane r holds row r in registers, and the current column is published
 // through the padding slots D[c * 65 + 64] (row 64 of D is never data), so the warp needs no
 // block-wide barrier.  A non-positive pivot is replaced by 1 so the steps stay finite;
 // returns the first one (kb if none), and writes the block back only if it factored.
-template <typename T>
-__device__ int chol32_warp(T* D, int off, int kb, int lane) {
-  T a[32];
+__device__ int chol32_warp(float* D, int off, int kb, int lane) {
+  float a[32];
 #pragma unroll
   for (int c = 0; c < 32; c++)
-    a[c] = (lane < kb && c <= lane) ? D[(off + c) * 65 + off + lane] : ((c == lane) ? T(1) : T(0));
+    a[c] = (lane < kb && c <= lane) ? D[(off + c) * 65 + off + lane] : ((c == lane) ? 1.f : 0.f);
   int bad = kb;
 #pragma unroll
   for (int j = 0; j < 32; j++) {
     D[lane * 65 + 64] = a[j];  // column j as it stands
     __syncwarp();
-    T d = D[j * 65 + 64];
-    if (!(d > T(0))) {
+    float d = D[j * 65 + 64];
+    if (!(d > 0.f)) {
       if (j < kb) bad = min(bad, j);
-      d = T(1);
+      d = 1.f;
     }
-    const T sq = tsqrt(d), inv = T(1) / sq;
-    const T lj = (lane == j) ? sq : a[j] * inv;  // L(lane, j)
+    const float sq = sqrtf(d), inv = 1.f / sq;
+    const float lj = (lane == j) ? sq : a[j] * inv;  // L(lane, j)
     if (lane >= j) a[j] = lj;
 #pragma unroll
     for (int c = j + 1; c < 32; c++)  // A(lane, c) -= L(lane, j) L(c, j)
@@ -83,116 +78,6 @@ __device__ int chol32_warp(T* D, int off, int kb, int lane) {
       if (lane < kb && c <= lane) D[(off + c) * 65 + off + lane] = a[c];
   }
   return bad;
-}
-
-// FP64 factorization of one matrix by the CTA.  Shared layout: D[64][65] (diagonal block),
-// P[NMAX][blk+1] (panel copy).  BLK is the panel width (a compile-time constant, so that
-// the panel solve keeps its row in registers).
-template <typename T, int BLK>
-__device__ int factor_one(T* __restrict__ A, int n, T* D, T* P, int* s_fail) {
-  constexpr int blk = BLK;
-  const int t = threadIdx.x;
-  const int ldp = blk + 1;
-  for (int k = 0; k < n; k += blk) {
-    const int kb = min(blk, n - k);
-    // 1. diagonal block -> shared, unblocked right-looking Cholesky
-    for (int idx = t; idx < kb * kb; idx += BT) {
-      const int c = idx / kb, r = idx % kb;
-      if (r >= c) D[c * 65 + r] = A[(k + r) + (i64)(k + c) * n];
-    }
-    if (t == 0) *s_fail = 0;
-    __syncthreads();
-    // column by column over the CTA (a warp form would spill its doubles)
-    for (int j = 0; j < kb; j++) {
-      if (t == 0) {
-        const T d = D[j * 65 + j];
-        if (!(d > T(0))) *s_fail = k + j + 1;
-        else D[j * 65 + j] = tsqrt(d);
-      }
-      __syncthreads();
-      if (*s_fail) break;
-      const T inv = T(1) / D[j * 65 + j];
-      for (int r = j + 1 + t; r < kb; r += BT) D[j * 65 + r] *= inv;
-      __syncthreads();
-      const int w = kb - j - 1;
-      for (int idx = t; idx < w * w; idx += BT) {
-        const int c = j + 1 + idx / w, r = j + 1 + idx % w;
-        if (r >= c) D[c * 65 + r] -= D[j * 65 + r] * D[j * 65 + c];
-      }
-      __syncthreads();
-    }
-    for (int idx = t; idx < kb * kb; idx += BT) {
-      const int c = idx / kb, r = idx % kb;
-      if (r >= c) A[(k + r) + (i64)(k + c) * n] = D[c * 65 + r];
-    }
-    const int fail = *s_fail;
-    __syncthreads();
-    if (fail) return fail;
-    const int m = n - k - kb;
-    if (m <= 0) break;
-    // 2. panel: rows below, B := B L_kk^-T, one thread per row held in registers (the
-    // dependent chain then waits on FMAs, not on shared-memory loads); result kept in P.
-    // Columns c >= kb are computed from stale D entries and discarded.
-    for (int i = t; i < m; i += BT) {
-      const int gi = k + kb + i;
-      T r[BLK];
-#pragma unroll
-      for (int c = 0; c < BLK; c++) r[c] = (c < kb) ? A[gi + (i64)(k + c) * n] : T(0);
-#pragma unroll
-      for (int c = 0; c < BLK; c++) {
-        T v = r[c];
-#pragma unroll
-        for (int q = 0; q < c; q++) v -= r[q] * D[q * 65 + c];
-        r[c] = (c < kb) ? v / D[c * 65 + c] : T(0);
-      }
-      T* row = P + i * ldp;
-#pragma unroll
-      for (int c = 0; c < BLK; c++)
-        if (c < kb) {
-          row[c] = r[c];
-          A[gi + (i64)(k + c) * n] = r[c];
-        }
-    }
-    __syncthreads();
-    // 3. trailing update of the lower triangle from P (4 x 4 tiles per thread)
-    const int Tt = (m + 3) / 4;
-    const int ntile = Tt * (Tt + 1) / 2;
-    for (int tile = t; tile < ntile; tile += BT) {
-      int ti = (int)((sqrtf(8.f * (float)tile + 1.f) - 1.f) * 0.5f);
-      while ((ti + 1) * (ti + 2) / 2 <= tile) ti++;
-      while (ti * (ti + 1) / 2 > tile) ti--;
-      const int tj = tile - ti * (ti + 1) / 2;
-      T acc[4][4];
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) acc[a][b] = T(0);
-      const int r0 = ti * 4, c0 = tj * 4;
-      for (int q = 0; q < kb; q++) {
-        T ra[4], cb[4];
-#pragma unroll
-        for (int a = 0; a < 4; a++) ra[a] = (r0 + a < m) ? P[(r0 + a) * ldp + q] : T(0);
-#pragma unroll
-        for (int b = 0; b < 4; b++) cb[b] = (c0 + b < m) ? P[(c0 + b) * ldp + q] : T(0);
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-          for (int b = 0; b < 4; b++) acc[a][b] = fma(ra[a], cb[b], acc[a][b]);
-      }
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++) {
-          const int r = r0 + a, c = c0 + b;
-          if (r < m && c < m && c <= r) {
-            T* p = A + (k + kb + r) + (i64)(k + kb + c) * n;
-            *p -= acc[a][b];
-          }
-        }
-    }
-    __syncthreads();
-  }
-  return 0;
 }
 
 // FP32 factorization of one matrix by the CTA, in steps of BLK (16 or 32) columns:
@@ -388,63 +273,394 @@ __device__ void solve_back_f32(const float* __restrict__ L, int n, float* bs) {
   }
 }
 
-// L L^T x = b in place (b in global), blocks of 32 rows: one warp solves the diagonal
-// block with shuffles, all threads update the rest.
-template <typename T>
-__device__ void solve_one(const T* __restrict__ L, int n, T* __restrict__ b) {
+// ---- FP64 ----------------------------------------------------------------------------
+// One matrix by a CTA of NT threads, in steps of blk columns (8, 16 or 32; KS = K / 16 of a step's
+// products).  The FP64 pipe does ~1.75 FMAs per clock per SM and was all of the time (57 % of its
+// peak), so the n^3 / 6 of the trailing updates go to the tensor cores as exact digit products (the
+// method: fp64_tc.cu):
+//   1. four warps factor the diagonal block (two 16-column blocks of potrf_panel), from the second
+//      step on inside the previous step's trailing update, while the other warps update the rest;
+//   2. every row below solves against L_kk^T, a thread per row with the row in registers; it goes to
+//      the matrix and, as seven BF16 digits with one exponent per row, to shared memory (448 bytes per
+//      row of 32 columns; the 64-byte rows of a digit are swizzled for ldmatrix);
+//   3. the trailing lower triangle takes the products by 16 x 8 blocks, a warp a block: 34 MMAs of
+//      m16n8k16 per 16 columns into the eight order sums (32 registers), put together in integers and
+//      taken off the matrix with one FP64 addition per element and step.
+// mma.sync, not tcgen05: a step's operands are at most 480 rows by 32 columns, written by the CTA's own
+// threads, and its results are wanted in registers at once; 16 x 8 blocks keep the triangle's
+// waste small at these orders.
+// 1200 matrices of 16..512: 7.4 ms against 26.7 ms with FP64 FMAs.
+__device__ __forceinline__ void bar_group() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }  // warps 0..3
+constexpr int DP = 33;          // column pitch of the diagonal block
+constexpr int F64_GROUP = 4;    // 8-column blocks per task of the trailing update
+
+// v / d from ri = 1 / d rounded: one Newton step, as accurate as the division.
+__device__ __forceinline__ double div_by(double v, double d, double ri) {
+  const double q = v * ri;
+  return fma(fma(-q, d, v), ri, q);
+}
+
+struct Shared64 {
+  double D[32 * DP];            // the diagonal block, identity beyond its order
+  double rinv[32];              // the reciprocals of its diagonal
+  double sq[16], rs[16];
+  int nfin, fail, task, idx;
+};
+
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr));
+}
+__device__ __forceinline__ void ldsm2(uint32_t (&r)[2], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];\n" : "=r"(r[0]), "=r"(r[1]) : "r"(addr));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+
+// Digit planes of a step's rows: row i's 16-byte chunk c (8 columns) of digit s at s plane + row_at(i, c).
+template <int KS>
+__device__ __forceinline__ int row_at(int i, int c) {
+  return KS == 2 ? i * 64 + ((c ^ ((i >> 1) & 3)) << 4) : i * 32 + ((c ^ ((i >> 2) & 1)) << 4);
+}
+
+// Cholesky of the diagonal block in S.D (kb of 32) by warps 0..3; S.fail gets the first bad
+// pivot's 1-based index.  Then L_kk (the columns before that pivot) to the matrix, and y_k = L_kk^{-1} b_k.
+__device__ __forceinline__ void diag_f64(Shared64& S, double* __restrict__ A, int n, int k, int kb, double* bs) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  // forward
-  for (int k = 0; k < n; k += 32) {
-    const int kb = min(32, n - k);
-    if (warp == 0) {
-      T v = (lane < kb) ? b[k + lane] : T(0);
-      for (int j = 0; j < kb; j++) {
-        T yj = __shfl_sync(0xffffffffu, v, j);
-        if (lane == j) { yj = v / L[(k + j) + (i64)(k + j) * n]; v = yj; }
-        yj = __shfl_sync(0xffffffffu, v, j);
-        if (lane > j && lane < kb) v -= L[(k + lane) + (i64)(k + j) * n] * yj;
-      }
-      if (lane < kb) b[k + lane] = v;
+  int fail = 0, done = 32;  // columns that factored
+  for (int o = 0; o < kb; o += PB) {
+    int nf = o == 0 ? potrf_panel<4, 32, DP>(S.D, 0) : potrf_panel<8, 32, DP>(S.D, PB);
+    if (t == 0) S.nfin = nf;
+    bar_group();
+    nf = S.nfin;
+    if (lane < PB && warp < 2) {
+      const double d = S.D[(o + lane) * DP + o + lane];
+      if (warp == 0) S.sq[lane] = lane < nf ? sqrt(d) : 1.0;
+      else S.rs[lane] = lane < nf ? rsqrt(d) : 1.0;
     }
-    __syncthreads();
-    for (int i = k + kb + t; i < n; i += BT) {
-      T s = T(0);
-      for (int j = 0; j < kb; j++) s = fma(L[i + (i64)(k + j) * n], b[k + j], s);
-      b[i] -= s;
+    bar_group();
+    for (int i = t; i < PB * 32; i += 128) {
+      const int c = i >> 5, r = i & 31;
+      double* e = S.D + (o + c) * DP + r;
+      if (r == o + c && c < nf) *e = S.sq[c];
+      else if (r > o + c) *e *= S.rs[c];
+    }
+    bar_group();
+    if (nf < PB) {
+      done = o + nf;
+      fail = k + done + 1;
+      break;
+    }
+    if (o == 0 && kb > PB) {  // the lower right 16 x 16
+      for (int i = t; i < PB * PB; i += 128) {
+        const int c = PB + (i >> 4), r = PB + (i & 15);
+        double v = S.D[c * DP + r];
+#pragma unroll
+        for (int q = 0; q < PB; q++) v = fma(-S.D[q * DP + r], S.D[q * DP + c], v);
+        if (r >= c) S.D[c * DP + r] = v;
+      }
+      bar_group();
+    }
+  }
+  if (t == 0) S.fail = fail;
+  if (warp == 0 && !fail) S.rinv[lane] = 1.0 / S.D[lane * DP + lane];
+  for (int i = t; i < 32 * 32; i += 128) {
+    const int c = i >> 5, r = i & 31;
+    if (r >= c && r < kb && c < done) A[(k + r) + (i64)(k + c) * n] = S.D[c * DP + r];
+  }
+  if (warp == 0 && bs && !fail) {  // (b_k is final: every earlier step has taken its share off)
+    __syncwarp();
+    double v = lane < kb ? bs[k + lane] : 0.0;
+    const double ri = S.rinv[lane], d = S.D[lane * DP + lane];
+#pragma unroll 8
+    for (int j = 0; j < 32; j++) {
+      const double y = __shfl_sync(0xffffffffu, div_by(v, d, ri), j);
+      v = lane == j ? y : lane > j ? fma(-S.D[j * DP + lane], y, v) : v;
+    }
+    if (lane < kb) bs[k + lane] = v;
+  }
+}
+
+// The diagonal block at column k from the matrix into S.D, by warps 0..3.
+__device__ __forceinline__ void load_diag_f64(Shared64& S, const double* A, int n, int k, int kb) {
+  for (int i = threadIdx.x; i < 32 * 32; i += 128) {
+    const int c = i >> 5, r = i & 31;
+    S.D[c * DP + r] = (r >= c && r < kb) ? A[(k + r) + (i64)(k + c) * n] : (r == c ? 1.0 : 0.0);
+  }
+}
+
+// An element of the product where digits do not serve: a result out of the normal range, or a row with
+// an infinity or NaN (the plain sum; X: the step's first column of the trailing rows).
+__device__ __noinline__ double product_special(long long V, int es, const double* X, int n, int m, int kb, int r, int c) {
+  if (es <= EXP_NONFINITE / 2) return scalbn((double)V, es - 54);
+  if (r >= m || c >= m) return 0.0;
+  double v = 0.0;
+  for (int q = 0; q < kb; q++) v = fma(X[r + (i64)q * n], X[c + (i64)q * n], v);
+  return v;
+}
+
+// The 16 x 8 block at strip I and column block J of the trailing triangle (m x m at C, column pitch n).
+template <int KS>
+__device__ __forceinline__ void update_block(double* __restrict__ C, const double* X, int n, int m, int kb, int I, int J,
+                                             uint32_t planes, int plane, const int* exps, int lane) {
+  const int r0 = 16 * I + (lane >> 2), c0 = 8 * J + 2 * (lane & 3);
+  double cv[4];
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const int r = r0 + 8 * (e >> 1), c = c0 + (e & 1);
+    cv[e] = (r < m && c <= r) ? C[r + (i64)c * n] : 0.0;
+  }
+  float acc[NG][4];
+#pragma unroll
+  for (int o = 0; o < NG; o++)
+#pragma unroll
+    for (int e = 0; e < 4; e++) acc[o][e] = 0.f;
+  const int ra = 16 * I + (lane & 15), rb = 8 * J + (lane & 7);
+#pragma unroll
+  for (int kk = 0; kk < KS; kk++) {
+    uint32_t b[ND][2];
+    const uint32_t pb = planes + row_at<KS>(rb, 2 * kk + ((lane >> 3) & 1)), pa = planes + row_at<KS>(ra, 2 * kk + (lane >> 4));
+#pragma unroll
+    for (int q = 0; q < ND; q++) ldsm2(b[q], pb + q * plane);
+#pragma unroll
+    for (int p = 0; p < ND; p++) {
+      uint32_t a[4];
+      ldsm4(a, pa + p * plane);
+#pragma unroll
+      for (int q = 0; q < ND && p + q < NG; q++) mma_bf16(acc[p + q], a, b[q]);
+    }
+  }
+  const int er[2] = {exps[r0], exps[r0 + 8]}, ec[2] = {exps[c0], exps[c0 + 1]};
+  double w[4];
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    uint32_t g[NG];
+#pragma unroll
+    for (int o = 0; o < NG; o++) g[o] = __float_as_uint(acc[o][e]);
+    const long long V = digit_sum<true>(g, 1);
+    bool special = false;
+    w[e] = digit_value(V, er[e >> 1] + ec[e & 1], special);
+    if (special) w[e] = product_special(V, er[e >> 1] + ec[e & 1], X, n, m, kb, r0 + 8 * (e >> 1), c0 + (e & 1));
+  }
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const int r = r0 + 8 * (e >> 1), c = c0 + (e & 1);
+    if (r < m && c <= r) C[r + (i64)c * n] = cv[e] - w[e];
+  }
+}
+
+template <int NT, int KS>
+__device__ int factor_f64(double* __restrict__ A, int n, int blk, Shared64& S, double* bs, uint8_t* planes, int* exps) {
+  constexpr int W = 16 * KS;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int zero = n >> 30;  // n <= 512
+  {
+    if (t < 128) {
+      load_diag_f64(S, A, n, 0, min(blk, n));
+      bar_group();
+      diag_f64(S, A, n, 0, min(blk, n), bs);
     }
     __syncthreads();
   }
-  // backward: L^T x = y
-  for (int k = ((n - 1) / 32) * 32; k >= 0; k -= 32) {
-    const int kb = min(32, n - k);
-    if (warp == 0) {
-      T v = (lane < kb) ? b[k + lane] : T(0);
-      for (int j = kb - 1; j >= 0; j--) {
-        T xj = __shfl_sync(0xffffffffu, v, j);
-        if (lane == j) { xj = v / L[(k + j) + (i64)(k + j) * n]; v = xj; }
-        xj = __shfl_sync(0xffffffffu, v, j);
-        if (lane < j) v -= L[(k + j) + (i64)(k + lane) * n] * xj;  // (L^T)(lane, j) = L(j, lane)
+  const uint32_t pl = (uint32_t)__cvta_generic_to_shared(planes);
+  for (int k = 0; k < n; k += blk) {
+    if (S.fail) return S.fail;
+    const int kb = min(blk, n - k), m = n - k - kb;
+    if (m <= 0) break;
+    const int m16 = (m + 15) & ~15, plane = m16 * (32 * KS);
+    double* X = A + (k + kb) + (i64)k * n;
+    if (t == 0) S.task = 0;
+    for (int i = t; i < m16; i += NT) {
+      const bool live = i < m;
+      double r[W];
+#pragma unroll
+      for (int c = 0; c < W; c++) r[c] = (live && c < kb) ? X[i + (i64)c * n] : 0.0;
+      double fw = 0.0;  // b_i -= L(i, k..) y_k
+      const double* yk = bs ? bs + k : S.rinv;
+      int be = 0;
+      bool any = false;
+#pragma unroll
+      for (int c = 0; c < W; c++) {
+        r[c] *= S.rinv[c];
+        // zero at run time: column c's loads of L_kk wait for r[c] (not all hoisted into registers)
+        const int z = zero & __double2loint(r[c]);
+        const double* lc = S.D + c * DP + z;
+#pragma unroll
+        for (int q = c + 1; q < W; q++) r[q] = fma(-r[c], lc[q], r[q]);
+        if (live && c < kb) {
+          X[i + (i64)c * n] = r[c];
+          fw = fma(r[c], yk[c + z], fw);
+        }
+        const int hi = __double2hiint(r[c]) & 0x7FFFFFFF;
+        be = max(be, hi >> 20);
+        any = any || (hi | __double2loint(r[c])) != 0;
       }
-      if (lane < kb) b[k + lane] = v;
+      if (bs && live) bs[k + kb + i] -= fw;
+      const int e = any ? max(be, 1) - 1022 : 0;  // |x| < 2^e
+      exps[i] = be == 0x7FF ? EXP_NONFINITE : e;
+#pragma unroll
+      for (int c = 0; c < W / 8; c++) {
+        unsigned long long x[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) x[j] = digit_fixed((unsigned long long)__double_as_longlong(r[8 * c + j]), -e);
+        put_digits<0>(x, planes + row_at<KS>(i, c), plane);
+      }
     }
     __syncthreads();
-    for (int i = t; i < k; i += BT) {
-      T s = T(0);
-      for (int j = 0; j < kb; j++) s = fma(L[(k + j) + (i64)i * n], b[k + j], s);
-      b[i] -= s;
+    // Strips of 16 rows.  Warps 0..3 take strips 0 and 1 (they hold the next diagonal block) and factor it at
+    // once; the others, and these four after it, take groups of up to four blocks of the later
+    // strips: strips 2 j and 2 j + 1 have j + 1 groups each.
+    double* C = A + (k + kb) + (i64)(k + kb) * n;
+    const int ns = m16 / 16;
+    if (warp < 4) {
+      for (int b = warp; b < 6; b += 4) {
+        const int I = b >= 2, J = b - 2 * I;
+        if (I < ns) update_block<KS>(C, X, n, m, kb, I, J, pl, plane, exps, lane);
+      }
+      bar_group();
+      const int kn = min(blk, m);
+      load_diag_f64(S, A, n, k + kb, kn);
+      bar_group();
+      diag_f64(S, A, n, k + kb, kn, bs);
+    }
+    const int np = ns / 2, ntask = ns < 3 ? 0 : np * np + np - 2 + ((ns & 1) ? np + 1 : 0);
+    for (;;) {
+      int x = 0;
+      if (lane == 0) x = atomicAdd(&S.task, 1);
+      x = __shfl_sync(0xffffffffu, x, 0);
+      if (x >= ntask) break;
+      int j = (int)((sqrtf(4.f * (float)x + 9.f) - 1.f) * 0.5f);  // j^2 + j - 2 <= x
+      if ((j + 1) * (j + 1) + (j + 1) - 2 <= x) j++;
+      if (j * j + j - 2 > x) j--;
+      const int rem = x - (j * j + j - 2), I = 2 * j + (rem > j), g = rem > j ? rem - j - 1 : rem;
+      for (int J = F64_GROUP * g; J < min(F64_GROUP * (g + 1), 2 * (I + 1)); J++)
+        update_block<KS>(C, X, n, m, kb, I, J, pl, plane, exps, lane);
+    }
+    __syncthreads();
+  }
+  return 0;
+}
+
+// Sweeps on the vector in shared memory, blocks of 32 rows: warp 0 solves the diagonal block with
+// shuffles and reciprocals, then every thread takes the block's share off its rows.
+template <int NT>
+__device__ void solve_forward_f64(const double* __restrict__ L, int n, double* bs) {
+  const int t = threadIdx.x, lane = t & 31;
+  for (int k = 0; k < n; k += 32) {
+    const int kb = min(32, n - k);
+    if (t < 32) {
+      double v = lane < kb ? bs[k + lane] : 0.0;
+      const double d = lane < kb ? L[(k + lane) + (i64)(k + lane) * n] : 1.0, ri = 1.0 / d;
+      const double* l = L + (k + lane) + (i64)k * n;
+#pragma unroll 8
+      for (int j = 0; j < 32; j++) {
+        const double c = (lane > j && lane < kb) ? l[(i64)j * n] : 0.0;
+        const double y = __shfl_sync(0xffffffffu, div_by(v, d, ri), j);
+        v = lane == j ? y : fma(-c, y, v);
+      }
+      if (lane < kb) bs[k + lane] = v;
+    }
+    __syncthreads();
+    for (int i = k + kb + t; i < n; i += NT) {
+      double s0 = 0.0, s1 = 0.0;
+      const double* l = L + i + (i64)k * n;
+#pragma unroll 8
+      for (int j = 0; j < 32; j += 2) {  // (rows below: the block is full)
+        s0 = fma(l[(i64)j * n], bs[k + j], s0);
+        s1 = fma(l[(i64)(j + 1) * n], bs[k + j + 1], s1);
+      }
+      bs[i] -= s0 + s1;
+    }
+    __syncthreads();
+  }
+}
+template <int NT>
+__device__ void solve_back_f64(const double* __restrict__ L, int n, double* bs) {
+  const int t = threadIdx.x, lane = t & 31;
+  for (int k = (n - 1) / 32 * 32; k >= 0; k -= 32) {
+    const int kb = min(32, n - k);
+    if (t < 32) {
+      double v = lane < kb ? bs[k + lane] : 0.0;
+      const double* l = L + k + (i64)(k + (lane < kb ? lane : 0)) * n;  // (L^T)(lane, j) = L(j, lane)
+      const double d = lane < kb ? l[lane] : 1.0, ri = 1.0 / d;
+#pragma unroll 8
+      for (int j = 31; j >= 0; j--) {
+        const double c = (j < kb && lane < j) ? l[j] : 0.0;
+        const double x = __shfl_sync(0xffffffffu, div_by(v, d, ri), j);
+        v = lane == j ? x : fma(-c, x, v);
+      }
+      if (lane < kb) bs[k + lane] = v;
+    }
+    __syncthreads();
+    for (int i = t; i < k; i += NT) {
+      const double* l = L + k + (i64)i * n;
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll 8
+      for (int j = 0; j + 1 < kb; j += 2) {
+        s0 = fma(l[j], bs[k + j], s0);
+        s1 = fma(l[j + 1], bs[k + j + 1], s1);
+      }
+      if (kb & 1) s0 = fma(l[kb - 1], bs[k + kb - 1], s0);
+      bs[i] -= s0 + s1;
     }
     __syncthreads();
   }
 }
 
-// MINB resident CTAs per SM requested from the register allocator: 2 for FP32 (whose
-// shared memory, sized per size class, lets two CTAs share an SM up to n = 256), 1 for FP64.
-template <typename T, int MINB>
-__global__ void __launch_bounds__(BT, MINB) k_batched_posv(const Item* __restrict__ items, int count, int* info,
-                                                           int* counter, int do_solve, int ldt) {
+// Shared memory of a launch whose matrices have orders <= nmax: bytes of digits for rows below a
+// step, their exponents, the right-hand side, Shared64.
+__host__ __device__ inline size_t digit_bytes_f64(int n, int blk) {
+  const int m = n > blk ? (n - blk + 15) / 16 * 16 : 0;
+  return (size_t)m * ND * (blk <= 16 ? 32 : 64);
+}
+inline size_t smem_f64(size_t digits, int nmax) { return digits + (size_t)((nmax + 31) / 32 * 32) * 12 + sizeof(Shared64); }
+
+// A persistent CTA takes the next matrix until there are none.  512, 256 or 128 threads and 1, 2 or 4 CTAs per
+// SM, by the class's largest order: wide enough to have a row per thread, as many CTAs as the digits leave room
+// for, since the diagonal blocks and the sweeps are chains.
+template <int NT>
+__global__ void __launch_bounds__(NT, 512 / NT) k_batched_f64(const Item* __restrict__ items, int count, int* info,
+                                                             int* counter, int do_solve, int nmax, int digits) {
+  extern __shared__ __align__(128) uint8_t smem64_raw[];
+  double* bs = (double*)(smem64_raw + digits);
+  int* exps = (int*)(bs + nmax);
+  Shared64& S = *(Shared64*)(exps + nmax);
+  for (;;) {
+    if (threadIdx.x == 0) S.idx = atomicAdd(counter, 1);
+    __syncthreads();
+    const int idx = S.idx;
+    if (idx >= count) break;
+    const Item it = items[idx];
+    double *a = (double*)it.a, *b = (double*)it.b;
+    if (do_solve)
+      for (int i = threadIdx.x; i < it.n; i += NT) bs[i] = b[i];
+    __syncthreads();
+    int f = 0;
+    if (it.mode == 0)
+      f = it.blk <= 16 ? factor_f64<NT, 1>(a, it.n, it.blk, S, do_solve ? bs : nullptr, smem64_raw, exps)
+                       : factor_f64<NT, 2>(a, it.n, it.blk, S, do_solve ? bs : nullptr, smem64_raw, exps);
+    else if (do_solve)
+      solve_forward_f64<NT>(a, it.n, bs);
+    if (threadIdx.x == 0) info[idx] = f;
+    if (f == 0 && do_solve) {
+      solve_back_f64<NT>(a, it.n, bs);
+      for (int i = threadIdx.x; i < it.n; i += NT) b[i] = bs[i];
+    }
+    __syncthreads();
+  }
+}
+
+// Two resident CTAs per SM requested from the register allocator (the shared memory, sized per size
+// class, lets two CTAs share an SM up to n = 256).
+__global__ void __launch_bounds__(BT, 2) k_batched_f32(const Item* __restrict__ items, int count, int* info, int* counter,
+                                                       int do_solve, int ldt) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  T* D = (T*)smem_raw;
-  T* P = D + 64 * 65;
+  float* D = (float*)smem_raw;
+  float* P = D + 64 * 65;
   __shared__ int s_idx, s_fail;
   for (;;) {
     if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1);
@@ -453,35 +669,22 @@ __global__ void __launch_bounds__(BT, MINB) k_batched_posv(const Item* __restric
     __syncthreads();
     if (idx >= count) break;
     const Item it = items[idx];
-    T* a = (T*)it.a;
+    float* a = (float*)it.a;
     int f = 0;
-    bool solved = false;
-    if (it.mode == 0) {
-      if constexpr (sizeof(T) == 4) {  // 16- or 32-wide steps (the autotuner's choice)
-        // the right-hand side in shared memory: the forward sweep runs inside the
-        // factorization, the backward sweep after it
-        float* bs = do_solve ? P + 32 * ldt : nullptr;
-        if (bs) {
-          for (int i = threadIdx.x; i < it.n; i += BT) bs[i] = ((const float*)it.b)[i];
-          __syncthreads();
-        }
-        if (it.blk <= 16) f = factor_f32<16>(a, it.n, D, P, ldt, bs, &s_fail);
-        else f = factor_f32<32>(a, it.n, D, P, ldt, bs, &s_fail);
-        if (bs && f == 0) {
-          solve_back_f32(a, it.n, bs);
-          for (int i = threadIdx.x; i < it.n; i += BT) ((float*)it.b)[i] = bs[i];
-        }
-        solved = true;
-      } else {
-        switch (it.blk) {  // the widths the autotuner chooses from (others fall back to 32)
-          case 8: f = factor_one<T, 8>(a, it.n, D, P, &s_fail); break;
-          case 16: f = factor_one<T, 16>(a, it.n, D, P, &s_fail); break;
-          default: f = factor_one<T, 32>(a, it.n, D, P, &s_fail); break;
-        }
-      }
+    // 16- or 32-wide steps (the autotuner's choice); the right-hand side in shared memory: the
+    // forward sweep runs inside the factorization, the backward sweep after it
+    float* bs = do_solve ? P + 32 * ldt : nullptr;
+    if (bs) {
+      for (int i = threadIdx.x; i < it.n; i += BT) bs[i] = ((const float*)it.b)[i];
+      __syncthreads();
+    }
+    if (it.blk <= 16) f = factor_f32<16>(a, it.n, D, P, ldt, bs, &s_fail);
+    else f = factor_f32<32>(a, it.n, D, P, ldt, bs, &s_fail);
+    if (bs && f == 0) {
+      solve_back_f32(a, it.n, bs);
+      for (int i = threadIdx.x; i < it.n; i += BT) ((float*)it.b)[i] = bs[i];
     }
     if (threadIdx.x == 0) info[idx] = f;
-    if (f == 0 && do_solve && !solved) solve_one<T>(a, it.n, (T*)it.b);
     __syncthreads();
   }
 }
@@ -492,18 +695,24 @@ __global__ void k_scatter_info(const int* sorted_info, const int* order, int cou
   if (i < count) out[order[i]] = sorted_info[i];
 }
 
-// Shared memory of a launch whose matrices have orders <= nmax and panel widths <= blk.
-// FP32 keeps the panel transposed (up to 32 rows of ldt floats, ldt = the class's largest
-// order rounded up to 32, plus 4) and the right-hand side (ldt floats); FP64 keeps the
-// panel row by row (nmax rows of blk + 1).
+// Shared memory of an FP32 launch whose matrices have orders <= nmax: the panel transposed (32 rows
+// of ldt floats, ldt = nmax rounded up to 32, plus 4), the right-hand side (ldt floats), D.
 inline int ldt_for(int nmax) { return (nmax + 31) / 32 * 32 + 4; }
-template <typename T>
-size_t smem_for(int blk, int nmax = NMAX) {
-  if (sizeof(T) == 4) return (size_t)(64 * 65 + 33 * ldt_for(nmax)) * sizeof(T);  // D, PT (<= 32 rows), b
-  return (size_t)(64 * 65 + nmax * (blk + 1)) * sizeof(T);
+inline size_t smem_f32(int nmax) { return (size_t)(64 * 65 + 33 * ldt_for(nmax)) * sizeof(float); }
+
+// One size class on the stream: items [0, count) on the device, orders <= nmax.
+template <typename K, typename... Args>
+int launch_class(K kernel, int threads, size_t smem, int nsm, int ctas_per_sm, int count, cudaStream_t s, Args... args) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    cudaGetLastError();
+    return OOC_ERR_UNSUPPORTED;
+  }
+  int occ = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
+  const int per = std::max(1, std::min(ctas_per_sm > 0 ? ctas_per_sm : occ, std::max(occ, 1)));
+  kernel<<<std::max(1, std::min(count, nsm * per)), threads, smem, s>>>(args...);
+  return OOC_OK;
 }
-template <typename T>
-constexpr int minb() { return sizeof(T) == 4 ? 2 : 1; }
 
 template <typename T>
 int run_items(cudaStream_t s, int dev, std::vector<Item>& items_in, int* info_host, const int* blk_table,
@@ -584,30 +793,31 @@ int run_items(cudaStream_t s, int dev, std::vector<Item>& items_in, int* info_ho
     cudaEventCreate(&e1);
     cudaEventRecord(e0, s);
     for (int ci = 0; ci < ncls && !rc; ci++) {
-      const int i0 = classes[ci].first, i1 = classes[ci].second;
-      int cmax = 1, cblk = 1;
-      for (int i = i0; i < i1; i++) {
+      const int i0 = classes[ci].first, cnt = classes[ci].second - i0;
+      int cmax = 1;
+      size_t digits = 0;
+      for (int i = i0; i < i0 + cnt; i++) {
         cmax = std::max(cmax, items[i].n);
-        cblk = std::max(cblk, items[i].blk);
+        if (sizeof(T) == 8) digits = std::max(digits, digit_bytes_f64(items[i].n, items[i].blk));
       }
-      const size_t sm = smem_for<T>(cblk, cmax);
-      if (cudaFuncSetAttribute(k_batched_posv<T, minb<T>()>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
-          cudaSuccess) {
-        cudaGetLastError();
-        rc = OOC_ERR_UNSUPPORTED;
-        break;
+      auto go = [&](auto kernel, int threads, size_t smem, auto... more) {
+        return launch_class(kernel, threads, smem, nsm, ctas_per_sm, cnt, s, (const Item*)d_items + i0, cnt, d_info + i0,
+                            d_counter + ci, do_solve, more...);
+      };
+      if constexpr (sizeof(T) == 4) {
+        rc = go(k_batched_f32, BT, smem_f32(cmax), ldt_for(cmax));
+      } else {
+        const int nmax = (cmax + 31) / 32 * 32;
+        const size_t sm = smem_f64(digits, cmax);
+        rc = cmax <= 128   ? go(k_batched_f64<128>, 128, sm, nmax, (int)digits)
+             : cmax <= 256 ? go(k_batched_f64<256>, 256, sm, nmax, (int)digits)
+                           : go(k_batched_f64<512>, 512, sm, nmax, (int)digits);
       }
-      int occ = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batched_posv<T, minb<T>()>, BT, sm);
-      const int per = std::max(1, std::min(ctas_per_sm > 0 ? ctas_per_sm : occ, std::max(occ, 1)));
-      const int grid = std::max(1, std::min(i1 - i0, nsm * per));
-      k_batched_posv<T, minb<T>()><<<grid, BT, sm, s>>>(d_items + i0, i1 - i0, d_info + i0, d_counter + ci, do_solve,
-                                                         ldt_for(cmax));
     }
     cudaEventRecord(e1, s);
     if (!rc) k_scatter_info<<<(count + 255) / 256, 256, 0, s>>>(d_info, d_order, count, d_out);
     cudaError_t e = cudaGetLastError();
-    if (!rc && e != cudaSuccess) { ooc_set_last_error(e, "k_batched_posv", __FILE__, __LINE__); rc = OOC_ERR_CUDA; }
+    if (!rc && e != cudaSuccess) { ooc_set_last_error(e, "batched factor and solve", __FILE__, __LINE__); rc = OOC_ERR_CUDA; }
   }
   if (!rc) {
     cudaMemcpyAsync(info_host, d_out, sizeof(int) * count, cudaMemcpyDeviceToHost, s);

@@ -30,13 +30,12 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "digits.cuh"
 #include "fp64_tc.cuh"
 #include "tc_ptx.cuh"
 
 namespace {
 
-constexpr int ND = 7;                         // digits per element
-constexpr int NG = 8;                         // product orders kept
 constexpr int DR = 128;                       // rows per plane unit and output block
 constexpr int DC = 64;                        // columns per output block
 constexpr int DK = 32;                        // K per stage
@@ -53,7 +52,6 @@ __host__ __device__ constexpr int d_smem(int mode) { return stages(mode) * stage
 // 16 rows each, between 6 x 16 and 16 rows of zeros.
 constexpr int NC = 16;                        // columns
 constexpr int N_SLAB = NC * DK * 2;           // 1 KB: one digit's rows, or zeros
-constexpr int EXP_NONFINITE = 1 << 28;        // row exponent of a row with an infinity or NaN
 static_assert(NG * DC == 512, "the eight order sums fill the TMEM");
 static_assert(stage_bytes(NARROW) == UNIT_STAGE + 2 * ND * N_SLAB, "six slabs of zeros, the digits, one of zeros");
 
@@ -75,33 +73,6 @@ struct DigitArgs {
   uint8_t* planes;
   size_t slot;
 };
-
-// The byte of w that `sel` picks, less 128, as a float: 2^23 + byte is an FP32 number.
-template <int SEL>
-__device__ __forceinline__ uint32_t digit_float(uint32_t w) {
-  return __float_as_uint(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 | SEL)) - 8388736.f);
-}
-// The same digit of x0 and x1 as two BF16 (an integer of magnitude <= 128 is exact in it: the upper
-// half of its FP32 encoding).  Digit 0 is the top one, 0..256 before the 128 are taken off.
-template <int S>
-__device__ __forceinline__ uint32_t digit_pair(unsigned long long x0, unsigned long long x1) {
-  uint32_t f0, f1;
-  if constexpr (S == 0) {
-    f0 = __float_as_uint(__uint_as_float((uint32_t)(x0 >> 48) | 0x4B000000u) - 8388736.f);
-    f1 = __float_as_uint(__uint_as_float((uint32_t)(x1 >> 48) | 0x4B000000u) - 8388736.f);
-  } else {
-    constexpr int B = ND - 1 - S;
-    f0 = digit_float<(B & 3)>((uint32_t)(B < 4 ? x0 : x0 >> 32));
-    f1 = digit_float<(B & 3)>((uint32_t)(B < 4 ? x1 : x1 >> 32));
-  }
-  return __byte_perm(f0, f1, 0x7632);
-}
-template <int S>
-__device__ __forceinline__ void put_digits(const unsigned long long (&x)[8], uint8_t* p) {
-  *reinterpret_cast<uint4*>(p + S * A_DIG) = make_uint4(digit_pair<S>(x[0], x[1]), digit_pair<S>(x[2], x[3]),
-                                                        digit_pair<S>(x[4], x[5]), digit_pair<S>(x[6], x[7]));
-  if constexpr (S + 1 < ND) put_digits<S + 1>(x, p);
-}
 
 // SHIFT: exponents moved by kshift, and symmetric operands.
 template <bool SHIFT>
@@ -155,17 +126,11 @@ __device__ __forceinline__ void digit_rows(const DigitArgs& a, int run) {
   unsigned long long x[KT];
 #pragma unroll
   for (int j = 0; j < KT; j++) {
-    const unsigned long long b = v[j];
-    const int be = (int)((b >> 52) & 0x7FF);
-    unsigned long long m = b & 0xFFFFFFFFFFFFFull;
-    if (be) m |= 1ull << 52;
-    const int sh = max(be, 1) + (SHIFT ? sft[SHIFT ? j : 0] : 0) - 1020 - e;  // X = m 2^sh, sh <= 2
-    if (sh >= 0) m <<= min(sh, 2);
-    else m = sh < -55 ? 0ull : (m + (1ull << (-sh - 1))) >> (-sh);
-    x[j] = ((b >> 63) ? 0ull - m : m) + 0x0080808080808080ull;
+    x[j] = digit_fixed(v[j], (SHIFT ? sft[SHIFT ? j : 0] : 0) - e);
   }
   // 64-byte swizzle: 16-byte chunk c of a row sits at c ^ ((row / 2) % 4)
-  put_digits<0>(x, planes + ((i64)(row >> 7) * nst + st) * UNIT_STAGE + (row & 127) * 64 + ((ch ^ ((row >> 1) & 3)) << 4));
+  put_digits<0>(x, planes + ((i64)(row >> 7) * nst + st) * UNIT_STAGE + (row & 127) * 64 + ((ch ^ ((row >> 1) & 3)) << 4),
+                A_DIG);
 }
 template <bool SHIFT>
 __global__ void __launch_bounds__(512) k_digits(const __grid_constant__ DigitArgs a, const int* status) {
@@ -204,32 +169,6 @@ struct UpdateArgs {
   int mask;
 };
 
-// The eight order sums of one element put together: sum_g G_g 2^(8 (5 - g)) as a 64-bit integer
-// (|G_0| <= 2^21, so it stays below 2^62).  Orders 5..7 are added in FP32 first, to within one
-// unit of order 5, 2^-54 of 2^(e(i) + e(j)): an FP64 chain over the K products errs by several
-// times that.
-__device__ __forceinline__ long long digit_sum(const uint32_t* g, int stride) {
-  auto f = [&](int o) { return __uint_as_float(g[o * stride]); };
-  const int t = __float2int_rn(fmaf(f(7), 0x1.0p-16f, fmaf(f(6), 0x1.0p-8f, f(5))));
-  // |G_0| <= 2^21 and |G_1| <= 2^22: an FP32 addition of 1.5 2^23 leaves the integer in the low bits
-  // (a conversion instruction issues at a quarter of the rate)
-  auto small_int = [](float x) { return __float_as_int(x + 12582912.f) - 0x4B400000; };
-  const int a1 = small_int(f(0)) * 256 + small_int(f(1));  // < 2^30
-  const int a2 = __float2int_rn(f(2)) * 256 + __float2int_rn(f(3));  // < 2^31
-  return ((long long)a1 << 32) + ((long long)a2 * 65536 + ((long long)__float2int_rn(f(4)) * 256 + t));
-}
-// V 2^(es - 54) rounded to FP64 (es = e(i) + e(j)), on the integer pipe and without branches:
-// `special` is raised where the result needs digit_value_special.
-__device__ __forceinline__ double digit_value(long long V, int es, bool& special) {
-  const unsigned long long sg = (unsigned long long)(V >> 63);
-  const unsigned long long a = ((unsigned long long)V ^ sg) - sg;
-  const int lz = __clzll((long long)a);
-  const int be = es + 1023 + 9 - lz;  // V = 1.x 2^(63 - lz)
-  special = special || (a != 0 && (unsigned)(be - 1) > 2044u) || es > EXP_NONFINITE / 2;
-  const unsigned long long M = a << (lz & 63);
-  const unsigned long long r = (M >> 11) + ((M >> 10) & 1u) + ((unsigned long long)(uint32_t)((be - 1) << 20) << 32);
-  return a == 0 ? 0.0 : __longlong_as_double((long long)(r | (sg << 63)));
-}
 // The same where the result is subnormal or overflows, and the plain sum for non-finite rows.
 __device__ __noinline__ double digit_value_special(long long V, int es, const UpdateArgs& X, int run, int r, int c) {
   if (es <= EXP_NONFINITE / 2) return scalbn((double)V, es - 54);
