@@ -2056,6 +2056,16 @@ int factor_mixed(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int6
 // product on the CUDA cores (k_colsolve_f32) and the update splits the panel itself.
 constexpr int kChainSMs = 1;  // the diagonal kernel is one CTA
 
+// Panel width of an FP32 factorization whose tiles are nb wide.  The chain of diagonal tiles sets the time of
+// small orders (one of 512 columns takes 450 us, of 256 108 us, of 128 40 us), the updates' passes over the matrix
+// that of large ones.  ms with panels of 128, 256 and 512 columns: n = 1000 0.64, 0.69, 1.80;
+// n = 4000 2.44, 2.65, 7.17; n = 6001 3.98, 4.24, 11.1; n = 10000 8.74, 7.64, 19.5; n = 16000 23.0, 17.8, 34.8.
+// A tile's width stays what the caller gave where 128 does not divide it, or the matrix is one such tile.
+int panel_width_f32(int64_t n, int nb) {
+  if (nb % 128 || nb <= 128 || n <= 256) return nb;
+  return n > 6144 && nb % 256 == 0 ? 256 : 128;
+}
+
 int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_t* launches, MixedProf* prof) {
   const i64 n = F->n;
   const int nb = F->nb;
@@ -2585,6 +2595,10 @@ static int create_impl(ooc_handle* h, const double* A, int64_t n, int64_t lda, b
     // automatic: 4096-column blocks for device and page-locked host matrices of more
     // than two blocks (faster long-K updates; for a host matrix, copies overlapped)
     bcols = opt >= 0 ? opt : ((pinned || on_device) && n > 2 * 4096 ? 4096 : 0);
+  }
+  if (prec == OOC_PREC_FP32 && panel_width_f32(n, nb) < nb) {
+    F->tail0 = 0;
+    F->nb2 = panel_width_f32(n, nb);
   }
   const bool lb = !gen && bcols > 0 && prec == OOC_PREC_BF16X3 && nb % 128 == 0 && n > nb && (on_device || pinned);
   if (lb && nb % 256 == 0) {  // left-looking blocks: nb/2-wide panels throughout
@@ -3441,8 +3455,9 @@ int spotrf_host_ooc(ooc_handle* h, float* A, i64 n, i64 lda, int nb, size_t budg
       launches++;
     }
     // in-core factorization of the panel, right-looking inside it (ooc_incore)
-    for (i64 q0 = 0; q0 < Wp; q0 += nb) {
-      const int LN = (int)std::min<i64>(nb, Wp - q0);
+    const int w = panel_width_f32(n, nb);
+    for (i64 q0 = 0; q0 < Wp; q0 += w) {
+      const int LN = (int)std::min<i64>(w, Wp - q0);
       float* Djj = P + q0 + q0 * n;
       if (LN <= DS_MAX)
         k_diag_s256<<<1, DG_THREADS, DS_SMEM, s>>>(Djj, n, LN, J0 + q0, Dinv, LN, Xr, nullptr, nullptr, status);
@@ -3517,6 +3532,8 @@ extern "C" int ooc_spotrf_L(ooc_handle* h, float* A, int64_t n, int64_t lda, int
   F.device = ooc_device(h);
   F.n = n;
   F.nb = nb;
+  F.tail0 = panel_width_f32(n, nb) < nb ? 0 : n;
+  F.nb2 = panel_width_f32(n, nb);
   F.prec = OOC_PREC_FP32;
   F.owns_Lf = on_device ? false : true;
   const int bb = (int)((n + nb - 1) / nb);
