@@ -44,54 +44,94 @@ struct Item {
   int mode;   // 0: factor + solve, 1: solve with an L already in `a`
 };
 
-// Cholesky of the kb x kb (kb <= 32) block at rows/columns off.. of D (lower, column-major,
-// ld 65) in one warp: lane r holds row r in registers, and the current column is published
-// through the padding slots D[c * 65 + 64] (row 64 of D is never data), so the warp needs no
-// block-wide barrier.  A non-positive pivot is replaced by 1 so the steps stay finite;
-// returns the first one (kb if none), and writes the block back only if it factored.
-__device__ int chol32_warp(float* D, int off, int kb, int lane) {
+// sqrt(d) and its reciprocal, each within an ulp, from the approximate reciprocal root and one Newton step
+// (a square root and a division are ~150 clocks of the chain, this 40); the functions themselves outside
+// the range where d's square root and its square are normal.
+__device__ __forceinline__ void root_f32(float d, float& sq, float& inv) {
+  if (d > 0x1p-100f && d < 0x1p100f) {
+    const float r = rsqrtf(d), s = d * r;
+    sq = fmaf(fmaf(-s, s, d), 0.5f * r, s);
+    inv = fmaf(fmaf(-sq, r, 1.f), r, r);
+  } else {
+    sq = sqrtf(d);
+    inv = 1.f / sq;
+  }
+}
+
+// v / d from ri = 1 / d rounded: one Newton step, as accurate as the division.
+template <typename T>
+__device__ __forceinline__ T div_by(T v, T d, T ri) {
+  const T q = v * ri;
+  return fma(fma(-q, d, v), ri, q);
+}
+
+// The kb x kb (kb <= 32) diagonal block at column k of the matrix, by one warp: lane r holds row r of
+// D (column-major, pitch 65) in registers; the pivots pass by shuffles, column j to the other rows'
+// updates through colb (two columns of 32 floats, 16-byte aligned), which the chain does not wait for.
+// L_kk goes to D and the matrix, 1 / diag to rinv, and b_k := L_kk^{-1} b_k beside it (bs not null). A
+// non-positive pivot is replaced by 1 so the steps stay finite; returns the first one (kb if
+// none), and writes the block back only if it factored.  As loops over shared memory with a square root and a
+// division per column it took 57k clocks a step, all the other warps waiting: this, whole-sector
+// accesses in the trailing update and back_block's loads ahead took the kernel from 6.6 to 3.9 ms for 4000
+// matrices of 16..512.
+__device__ __forceinline__ int diag_f32(float* D, float* A, int n, int k, int kb, float* colb, float* rinv, float* bs,
+                                        int lane) {
   float a[32];
 #pragma unroll
-  for (int c = 0; c < 32; c++)
-    a[c] = (lane < kb && c <= lane) ? D[(off + c) * 65 + off + lane] : ((c == lane) ? 1.f : 0.f);
+  for (int c = 0; c < 32; c++) a[c] = (lane < kb && c <= lane) ? D[c * 65 + lane] : (c == lane ? 1.f : 0.f);
+  float v = (bs && lane < kb) ? bs[k + lane] : 0.f, rv = 1.f;
   int bad = kb;
+  float d = __shfl_sync(0xffffffffu, a[0], 0);
 #pragma unroll
   for (int j = 0; j < 32; j++) {
-    D[lane * 65 + 64] = a[j];  // column j as it stands
-    __syncwarp();
-    float d = D[j * 65 + 64];
     if (!(d > 0.f)) {
-      if (j < kb) bad = min(bad, j);
+      bad = min(bad, j);
       d = 1.f;
     }
-    const float sq = sqrtf(d), inv = 1.f / sq;
-    const float lj = (lane == j) ? sq : a[j] * inv;  // L(lane, j)
-    if (lane >= j) a[j] = lj;
-#pragma unroll
-    for (int c = j + 1; c < 32; c++)  // A(lane, c) -= L(lane, j) L(c, j)
-      if (lane >= c) a[c] -= lj * (D[c * 65 + 64] * inv);
+    float sq, inv;
+    root_f32(d, sq, inv);
+    const float lj = lane == j ? sq : a[j] * inv;  // L(lane, j) for lane >= j
+    if (j + 1 < 32) d = __shfl_sync(0xffffffffu, fmaf(-lj, lj, a[j + 1 < 32 ? j + 1 : 0]), j + 1);
+    const float y = __shfl_sync(0xffffffffu, div_by(v, sq, inv), j);
+    v = lane == j ? y : lane > j ? fmaf(-lj, y, v) : v;
+    if (lane == j) rv = inv;
+    a[j] = lj;
+    float* col = colb + (j & 1) * 32;
+    col[lane] = lj;
     __syncwarp();
+#pragma unroll
+    for (int q = (j + 1) / 4; q < 8; q++) {  // (elements above the diagonal are never used)
+      const float4 l = reinterpret_cast<const float4*>(col)[q];
+      const float lc[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (4 * q + u > j) a[4 * q + u] = fmaf(-lj, lc[u], a[4 * q + u]);
+    }
   }
+  rinv[lane] = rv;
   if (bad == kb) {
 #pragma unroll
     for (int c = 0; c < 32; c++)
-      if (lane < kb && c <= lane) D[(off + c) * 65 + off + lane] = a[c];
+      if (lane < kb && c <= lane) {
+        D[c * 65 + lane] = a[c];
+        A[(k + lane) + (i64)(k + c) * n] = a[c];
+      }
+    if (bs && lane < kb) bs[k + lane] = v;
   }
   return bad;
 }
 
 // FP32 factorization of one matrix by the CTA, in steps of BLK (16 or 32) columns:
-//   1. the diagonal block is factored by one warp in registers (chol32_warp), and the
+//   1. the diagonal block is factored by one warp in registers (diag_f32), and the
 //      reciprocals of its diagonal are kept; from the second step on this happens inside
 //      the previous step's trailing update (warp 0 updates the block that holds it and
-//      factors it while the other warps update the rest);
+//      factors it while the other warps update the rest, then helps them);
 //   2. every row below solves against L_kk^T, one thread per row with the row in registers,
 //      right-looking (each column's FMAs independent of the others'); the result goes to
 //      the matrix and, transposed, to PT (PT[c ldt + i] = L(k + kb + i, k + c)), zero-padded
 //      to a multiple of 32 rows;
 //   3. the trailing lower triangle is updated by 32 x 32 blocks, a warp a block, each lane a
-//      4 x 8 register tile fed by 16-byte shared loads of PT (ten FMAs per shared load); the
-//      block's elements of the matrix are loaded before the products and stored after.
+//      4 x 8 register tile fed by shared loads of PT; the block's elements of the matrix are loaded before the products and stored after.
 // The trailing matrix stays in global memory (up to 1 MB per matrix); every element of it is
 // read and written once per step.
 __device__ __forceinline__ void bt_block_ij(int b, int& I, int& J) {
@@ -105,32 +145,16 @@ __device__ __forceinline__ void bt_block_ij(int b, int& I, int& J) {
 template <int BLK>
 __device__ int factor_f32(float* __restrict__ A, int n, float* D, float* PT, int ldt, float* bs, int* s_fail) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  float* rinv = D + 40 * 65;  // a column of D that a <= 32-wide block never uses
-  const int r0 = (lane & 7) * 4, c0 = (lane >> 3) * 8;
+  float* rinv = D + 40 * 65;  // columns of D that a <= 32-wide block never uses
+  float* colb = D + 44 * 65;  // (a multiple of 4)
+  int* task = (int*)(D + 48 * 65);
+  // a lane's elements of a 32 x 32 block: rows r0 + 8 i, so that a column's load or store is a whole
+  // sector for eight lanes, columns c0 + j
+  const int r0 = lane & 7, c0 = (lane >> 3) * 8;
   const int zero = n >> 30;  // n <= 512
-  // warp 0: factor the kb x kb diagonal block at column k (already in D), keep the
-  // reciprocals of its diagonal and write L_kk to the matrix
-  auto diag = [&](int k, int kb) {
-    const int b = chol32_warp(D, 0, kb, lane);
+  auto diag = [&](int k, int kb) {  // warp 0: the block already in D
+    const int b = diag_f32(D, A, n, k, kb, colb, rinv, bs, lane);
     if (lane == 0) *s_fail = (b < kb) ? k + b + 1 : 0;
-    const float ri = (lane < kb) ? 1.f / D[lane * 65 + lane] : 0.f;
-    if (lane < BLK) rinv[lane] = ri;
-    if (b == kb) {
-      for (int idx = lane; idx < kb * kb; idx += 32) {
-        const int c = idx / kb, r = idx % kb;
-        if (r >= c) A[(k + r) + (i64)(k + c) * n] = D[c * 65 + r];
-      }
-      if (bs) {  // forward sweep, this block: y_k = L_kk^{-1} b_k (b_k is final: every
-                 // earlier step's row solve has already subtracted its panel's share)
-        float v = (lane < kb) ? bs[k + lane] : 0.f;
-        for (int j = 0; j < kb; j++) {
-          const float yj = __shfl_sync(0xffffffffu, v * ri, j);
-          if (lane == j) v = yj;
-          else if (lane > j) v = fmaf(-D[j * 65 + lane], yj, v);
-        }
-        if (lane < kb) bs[k + lane] = v;
-      }
-    }
   };
   {
     const int kb = min(BLK, n);
@@ -149,6 +173,7 @@ __device__ int factor_f32(float* __restrict__ A, int n, float* D, float* PT, int
     const int m = n - k - kb;
     if (m <= 0) break;
     const int m32 = (m + 31) & ~31;
+    if (t == 0) *task = 1;
     for (int i = t; i < m32; i += BT) {
       float r[BLK];
       float* g = A + (k + kb + i);
@@ -174,12 +199,17 @@ __device__ int factor_f32(float* __restrict__ A, int n, float* D, float* PT, int
     }
     __syncthreads();
     // Trailing update.  Warp 0 takes block (0, 0), which holds the next diagonal block: it
-    // also leaves that block's kn x kn corner in D and factors it at once, while warps
-    // 1.. update the other blocks; the next step's row solve follows the barrier directly.
+    // also leaves that block's kn x kn corner in D and factors it at once, while the other warps, and it
+    // after that, take the other blocks in turn; the next step's row solve follows the barrier directly.
     const int nb32 = m32 >> 5, nblk = nb32 * (nb32 + 1) / 2;
     const int kn = min(BLK, m);
     float* C = A + (k + kb) + (i64)(k + kb) * n;
-    for (int b = (warp == 0) ? 0 : warp; b < nblk; b += (warp == 0) ? nblk : BT / 32 - 1) {
+    auto next = [&]() {
+      int x = 0;
+      if (lane == 0) x = atomicAdd(task, 1);
+      return __shfl_sync(0xffffffffu, x, 0);
+    };
+    for (int b = (warp == 0) ? 0 : next(); b < nblk; b = next()) {
       int I, J;
       bt_block_ij(b, I, J);
       const int rb = I * 32 + r0, cb = J * 32 + c0;
@@ -188,16 +218,16 @@ __device__ int factor_f32(float* __restrict__ A, int n, float* D, float* PT, int
       for (int ii = 0; ii < 4; ii++)
 #pragma unroll
         for (int jj = 0; jj < 8; jj++) {
-          const int row = rb + ii, col = cb + jj;
+          const int row = rb + 8 * ii, col = cb + jj;
           cv[ii][jj] = (row < m && col <= row) ? C[row + (i64)col * n] : 0.f;
         }
       float acc[4][8] = {};
 #pragma unroll 8
       for (int q = 0; q < BLK; q++) {
-        const float4 a = *reinterpret_cast<const float4*>(PT + q * ldt + rb);
         const float4 b0 = *reinterpret_cast<const float4*>(PT + q * ldt + cb);
         const float4 b1 = *reinterpret_cast<const float4*>(PT + q * ldt + cb + 4);
-        const float av[4] = {a.x, a.y, a.z, a.w};
+        const float* ar = PT + q * ldt + rb;
+        const float av[4] = {ar[0], ar[8], ar[16], ar[24]};
         const float bv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
         for (int ii = 0; ii < 4; ii++)
@@ -208,17 +238,17 @@ __device__ int factor_f32(float* __restrict__ A, int n, float* D, float* PT, int
       for (int ii = 0; ii < 4; ii++)
 #pragma unroll
         for (int jj = 0; jj < 8; jj++) {
-          const int row = rb + ii, col = cb + jj;
+          const int row = rb + 8 * ii, col = cb + jj;
           if (row < m && col <= row) {
             const float v = cv[ii][jj] - acc[ii][jj];
             C[row + (i64)col * n] = v;
             if (b == 0 && row < kn) D[col * 65 + row] = v;
           }
         }
-    }
-    if (warp == 0) {
-      __syncwarp();
-      diag(k + kb, kn);
+      if (b == 0) {
+        __syncwarp();
+        diag(k + kb, kn);
+      }
     }
     __syncthreads();
   }
@@ -243,14 +273,20 @@ __device__ __forceinline__ void back_share(const float* __restrict__ L, int n, f
   bs[i] -= s0 + s1;
 }
 
+// (The block's 32 loads come first, then a chain of shuffles: with a load and a division in each step it took
+// a sixth of the kernel.)
 __device__ __forceinline__ void back_block(const float* __restrict__ L, int n, float* bs, int k, int lane) {
   const int kb = min(32, n - k);
+  const float* l = L + k + (i64)(k + (lane < kb ? lane : 0)) * n;  // (L^T)(lane, j) = L(j, lane)
+  float c[32];
+#pragma unroll
+  for (int j = 0; j < 32; j++) c[j] = (j < kb && lane <= j) ? l[j] : 0.f;
   float v = (lane < kb) ? bs[k + lane] : 0.f;
-  const float ljj = (lane < kb) ? L[(k + lane) + (i64)(k + lane) * n] : 1.f;
-  for (int j = kb - 1; j >= 0; j--) {
-    const float xj = __shfl_sync(0xffffffffu, v / ljj, j);
-    if (lane == j) v = xj;
-    else if (lane < j) v = fmaf(-L[(k + j) + (i64)(k + lane) * n], xj, v);  // (L^T)(lane, j) = L(j, lane)
+  const float d = (lane < kb) ? l[lane] : 1.f, ri = 1.f / d;
+#pragma unroll
+  for (int j = 31; j >= 0; j--) {
+    const float x = __shfl_sync(0xffffffffu, div_by(v, d, ri), j);
+    v = lane == j ? x : lane < j ? fmaf(-c[j], x, v) : v;
   }
   if (lane < kb) bs[k + lane] = v;
 }
@@ -289,16 +325,11 @@ __device__ void solve_back_f32(const float* __restrict__ L, int n, float* bs) {
 // mma.sync, not tcgen05: a step's operands are at most 480 rows by 32 columns, written by the CTA's own
 // threads, and its results are wanted in registers at once; 16 x 8 blocks keep the triangle's
 // waste small at these orders.
-// 1200 matrices of 16..512: 7.4 ms against 26.7 ms with FP64 FMAs.
+// 1200 matrices of 16..512: 5.9 ms against 26.7 ms with FP64 FMAs (7.4 with every class in steps of 32 columns and
+// no class beside another's tail).
 __device__ __forceinline__ void bar_group() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }  // warps 0..3
 constexpr int DP = 33;          // column pitch of the diagonal block
 constexpr int F64_GROUP = 4;    // 8-column blocks per task of the trailing update
-
-// v / d from ri = 1 / d rounded: one Newton step, as accurate as the division.
-__device__ __forceinline__ double div_by(double v, double d, double ri) {
-  const double q = v * ri;
-  return fma(fma(-q, d, v), ri, q);
-}
 
 struct Shared64 {
   double D[32 * DP];            // the diagonal block, identity beyond its order
@@ -611,6 +642,13 @@ __device__ void solve_back_f64(const double* __restrict__ L, int n, double* bs) 
   }
 }
 
+// Step width where the caller gives none: 16 columns need half the FP64 work of 32 in the panel's solve and
+// half the shared memory, 32 fewer passes over the matrix.  Kernel ms for 16 and 32: n in 64..128 (1000 matrices) 0.50,
+// 0.54; 256..384 (608) 2.77 (two CTAs per SM), 3.33; 400..512 (608) 7.04, 6.61 (one CTA either way); up to 64, one step
+// of 32 and the rest: 0.36, 0.34.
+inline int default_blk_f64(int n) { return n > 64 && n <= 448 ? 16 : 32; }
+constexpr size_t F64_TWO = 113 * 1024;  // shared memory that lets two CTAs share an SM
+
 // Shared memory of a launch whose matrices have orders <= nmax: bytes of digits for rows below a
 // step, their exponents, the right-hand side, Shared64.
 __host__ __device__ inline size_t digit_bytes_f64(int n, int blk) {
@@ -619,9 +657,14 @@ __host__ __device__ inline size_t digit_bytes_f64(int n, int blk) {
 }
 inline size_t smem_f64(size_t digits, int nmax) { return digits + (size_t)((nmax + 31) / 32 * 32) * 12 + sizeof(Shared64); }
 
-// A persistent CTA takes the next matrix until there are none.  512, 256 or 128 threads and 1, 2 or 4 CTAs per
-// SM, by the class's largest order: wide enough to have a row per thread, as many CTAs as the digits leave room
-// for, since the diagonal blocks and the sweeps are chains.
+// The size classes' launches do not depend on one another: each lets the next one's CTAs take the places that
+// its own leave (a class's tail beside the next class), and ends after the one before it.
+__device__ __forceinline__ void class_begin() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void class_end() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// A persistent CTA takes the next matrix until there are none.  128 threads and 4 CTAs per SM up to n = 128,
+// 256 and 2 where the digits leave room for two CTAs, else 512 and 1: one matrix's FP64 panel solve and chains run
+// beside another's products.
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) k_batched_f64(const Item* __restrict__ items, int count, int* info,
                                                              int* counter, int do_solve, int nmax, int digits) {
@@ -629,6 +672,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_batched_f64(const Item* __rest
   double* bs = (double*)(smem64_raw + digits);
   int* exps = (int*)(bs + nmax);
   Shared64& S = *(Shared64*)(exps + nmax);
+  class_begin();
   for (;;) {
     if (threadIdx.x == 0) S.idx = atomicAdd(counter, 1);
     __syncthreads();
@@ -652,6 +696,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_batched_f64(const Item* __rest
     }
     __syncthreads();
   }
+  class_end();
 }
 
 // Two resident CTAs per SM requested from the register allocator (the shared memory, sized per size
@@ -662,6 +707,7 @@ __global__ void __launch_bounds__(BT, 2) k_batched_f32(const Item* __restrict__ 
   float* D = (float*)smem_raw;
   float* P = D + 64 * 65;
   __shared__ int s_idx, s_fail;
+  class_begin();
   for (;;) {
     if (threadIdx.x == 0) s_idx = atomicAdd(counter, 1);
     __syncthreads();
@@ -687,6 +733,7 @@ __global__ void __launch_bounds__(BT, 2) k_batched_f32(const Item* __restrict__ 
     if (threadIdx.x == 0) info[idx] = f;
     __syncthreads();
   }
+  class_end();
 }
 
 // Scatter per-matrix info from sorted order back to the caller's order.
@@ -700,9 +747,11 @@ __global__ void k_scatter_info(const int* sorted_info, const int* order, int cou
 inline int ldt_for(int nmax) { return (nmax + 31) / 32 * 32 + 4; }
 inline size_t smem_f32(int nmax) { return (size_t)(64 * 65 + 33 * ldt_for(nmax)) * sizeof(float); }
 
-// One size class on the stream: items [0, count) on the device, orders <= nmax.
+// One size class on the stream: items [0, count) on the device, orders <= nmax.  `first`: the launch
+// tables before it in the stream are its inputs, so it waits for them.
 template <typename K, typename... Args>
-int launch_class(K kernel, int threads, size_t smem, int nsm, int ctas_per_sm, int count, cudaStream_t s, Args... args) {
+int launch_class(K kernel, int threads, size_t smem, int nsm, int ctas_per_sm, int count, bool first, cudaStream_t s,
+                 Args... args) {
   if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
     cudaGetLastError();
     return OOC_ERR_UNSUPPORTED;
@@ -710,7 +759,9 @@ int launch_class(K kernel, int threads, size_t smem, int nsm, int ctas_per_sm, i
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, smem);
   const int per = std::max(1, std::min(ctas_per_sm > 0 ? ctas_per_sm : occ, std::max(occ, 1)));
-  kernel<<<std::max(1, std::min(count, nsm * per)), threads, smem, s>>>(args...);
+  const unsigned grid = (unsigned)std::max(1, std::min(count, nsm * per));
+  if (first) kernel<<<grid, threads, smem, s>>>(args...);
+  else OOC_CUDA_TRY(launch_pdl(kernel, dim3(grid), threads, smem, s, args...));
   return OOC_OK;
 }
 
@@ -744,17 +795,17 @@ int run_items(cudaStream_t s, int dev, std::vector<Item>& items_in, int* info_ho
   for (int i = 0; i < count; i++) {
     const int j = order[i];
     const int bucket = std::min(NBUCKETS - 1, items_in[j].n / 32);
-    int blk = blk_table ? blk_table[bucket] : (sizeof(T) == 8 ? 32 : 64);
+    int blk = blk_table ? blk_table[bucket] : (sizeof(T) == 8 ? default_blk_f64(items_in[j].n) : 64);
     blk = std::max(1, std::min(blk, 32));
     blk = sizeof(T) == 4 ? (blk <= 16 ? 16 : 32) : (blk <= 8 ? 8 : blk <= 16 ? 16 : 32);  // the compiled widths
     items[i] = items_in[j];
     items[i].blk = blk;
   }
-  // Size classes (orders in (0,64], (64,128], (128,256], (256,384], (384,512]; the items
+  // Size classes (orders in (0,64], (64,128], (128,256], (256,384], (384,512], FP64 448 for 384; the items
   // are sorted by decreasing order, so a class is a contiguous range): one persistent
   // launch each, its shared memory sized for the class's largest order and panel width,
   // so that the small classes fit several CTAs per SM.
-  const int bounds[] = {512, 384, 256, 128, 64};
+  const int bounds[] = {512, sizeof(T) == 8 ? 448 : 384, 256, 128, 64};
   std::vector<std::pair<int, int>> classes;  // [first, one past the last) in sorted order
   {
     int i = 0;
@@ -801,7 +852,7 @@ int run_items(cudaStream_t s, int dev, std::vector<Item>& items_in, int* info_ho
         if (sizeof(T) == 8) digits = std::max(digits, digit_bytes_f64(items[i].n, items[i].blk));
       }
       auto go = [&](auto kernel, int threads, size_t smem, auto... more) {
-        return launch_class(kernel, threads, smem, nsm, ctas_per_sm, cnt, s, (const Item*)d_items + i0, cnt, d_info + i0,
+        return launch_class(kernel, threads, smem, nsm, ctas_per_sm, cnt, ci == 0, s, (const Item*)d_items + i0, cnt, d_info + i0,
                             d_counter + ci, do_solve, more...);
       };
       if constexpr (sizeof(T) == 4) {
@@ -809,9 +860,9 @@ int run_items(cudaStream_t s, int dev, std::vector<Item>& items_in, int* info_ho
       } else {
         const int nmax = (cmax + 31) / 32 * 32;
         const size_t sm = smem_f64(digits, cmax);
-        rc = cmax <= 128   ? go(k_batched_f64<128>, 128, sm, nmax, (int)digits)
-             : cmax <= 256 ? go(k_batched_f64<256>, 256, sm, nmax, (int)digits)
-                           : go(k_batched_f64<512>, 512, sm, nmax, (int)digits);
+        rc = cmax <= 128     ? go(k_batched_f64<128>, 128, sm, nmax, (int)digits)
+             : sm <= F64_TWO ? go(k_batched_f64<256>, 256, sm, nmax, (int)digits)
+                             : go(k_batched_f64<512>, 512, sm, nmax, (int)digits);
       }
     }
     cudaEventRecord(e1, s);
