@@ -920,9 +920,15 @@ def update_schedule(n, nb, prec, tail_order, block_cols, device_matrix=True):
     lb = prec == "bf16x3" and nb % 128 == 0 and n > nb and bc > 0
     if not lb:
         panels = panel_schedule(n, nb, prec, tail_order)
-        if prec == "fp32" and nb % 128 == 0 and nb > 128 and n > 256:  # narrower panels than the tiles
-            w = 256 if n > 6144 and nb % 256 == 0 else 128
-            panels = [(J0, min(w, n - J0)) for J0 in range(0, n, w)]
+        w = nb if nb <= 256 or nb % 128 else 128 if nb % 256 else 256
+        if prec == "fp32" and w < nb:  # panels inside the tiles, then the tile as one
+            panels, launches = [(J0, min(w, n - J0)) for J0 in range(0, n, w)], []
+            for J0, LN in panels:
+                G0, m = J0 // nb * nb, n - J0 - LN
+                G1 = min(G0 + nb, n)
+                if m > 0:
+                    launches.append((m, LN, G1 - J0 - LN) if J0 + LN < G1 else (m, G1 - G0, m))
+            return {"kind": "right-looking tiles", "panels": panels, "launches": launches}
         return {"kind": "right-looking", "panels": panels,
                 "launches": [(n - J0 - LN, LN, n - J0 - LN) for J0, LN in panels if n - J0 - LN > 0]}
     w = nb // 2 if nb % 256 == 0 else nb

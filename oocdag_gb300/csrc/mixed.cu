@@ -2056,14 +2056,24 @@ int factor_mixed(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int6
 // product on the CUDA cores (k_colsolve_f32) and the update splits the panel itself.
 constexpr int kChainSMs = 1;  // the diagonal kernel is one CTA
 
-// Panel width of an FP32 factorization whose tiles are nb wide.  The chain of diagonal tiles sets the time of
-// small orders (one of 512 columns takes 450 us, of 256 108 us, of 128 40 us), the updates' passes over the matrix
-// that of large ones.  ms with panels of 128, 256 and 512 columns: n = 1000 0.64, 0.69, 1.80;
-// n = 4000 2.44, 2.65, 7.17; n = 6001 3.98, 4.24, 11.1; n = 10000 8.74, 7.64, 19.5; n = 16000 23.0, 17.8, 34.8.
-// A tile's width stays what the caller gave where 128 does not divide it, or the matrix is one such tile.
-int panel_width_f32(int64_t n, int nb) {
-  if (nb % 128 || nb <= 128 || n <= 256) return nb;
-  return n > 6144 && nb % 256 == 0 ? 256 : 128;
+// Lower-triangle elements of an m x m trailing matrix in columns [a, b): the useful
+// outputs of an update restricted to those columns (2 K flops each).
+double lower_elems(i64 m, i64 a, i64 b) {
+  b = std::min(b, m);
+  if (a >= b) return 0.0;
+  return (double)(b - a) * (double)m - ((double)b * (double)(b - 1) - (double)a * (double)(a - 1)) / 2.0;
+}
+
+// Panel width of an FP32 factorization whose tiles are nb wide: the one-CTA diagonal tiles are a chain (one of 512
+// columns takes 450 us, of 256 108 us).  Panels narrower than the tile are updated inside it one by one, and
+// the columns right of the tile take it whole (K = nb), so that an element is rounded as often as with panels
+// of nb columns: with an update per panel of 128 the error against 64 bits at n = 6001 was 1.06e-7 instead of 0.88e-7.
+// Tiles of 512 in one panel and in panels of 256 (and 128), ms: n = 600 1.04, 0.44 (0.41); n = 2000 3.58, 1.44 (1.39);
+// n = 6001 11.1, 4.30 (4.22); n = 16000 35.0, 19.7 (20.3).  Tiles of 256 in panels of 128 gain nothing (n = 1000 0.68,
+// 0.78; n = 6001 4.19, 4.07; n = 16000 17.9, 20.1).
+int panel_width_f32(int nb) {
+  if (nb <= 256 || nb % 128) return nb;
+  return nb % 256 ? 128 : 256;
 }
 
 int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_t* launches, MixedProf* prof) {
@@ -2103,6 +2113,7 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
     return LN;
   };
   OOC_CUDA_TRY(cudaEventRecord(evA, s0));  // the matrix was filled on s0
+  const bool grouped = prec == OOC_PREC_FP32 && P.tail0 == 0 && P.nb2 < nb;  // panels narrower than the tiles
   if (tc_solve) {  // panel 0 below its diagonal tile, beside the first diagonal kernel
     const int w0 = width(0);
     rc = launch_split_bf16_f32(A + w0, lda, (int)(n - w0), w0, F->work2.p, F->work2.bytes, s0);
@@ -2142,10 +2153,24 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
         prof->mark(s0);
         prof->mark(s0);
         prof->kind.push_back(1);
-        prof->flops.push_back((double)m * (double)(m + 1) * LN);
+        const i64 G0 = J0 / nb * nb, G1 = std::min<i64>(G0 + nb, n);
+        prof->flops.push_back(!grouped        ? (double)m * (double)(m + 1) * LN
+                              : J0 + LN < G1 ? 2.0 * lower_elems(m, 0, G1 - J0 - LN) * LN
+                                             : (double)m * (double)(m + 1) * (double)(G1 - G0));
       }
       float* C = A + (J0 + LN) * (1 + lda);
-      if (tc_solve) {  // the planes come from the solve
+      const i64 G0 = J0 / nb * nb, G1 = std::min<i64>(G0 + nb, n);  // the panel's tile
+      if (grouped && J0 + LN < G1) {  // the rest of the tile
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, (int)((G1 - J0 - LN + 127) / 128));
+        if (rc) return rc;
+        OOC_CUDA_TRY(cudaEventRecord(evA, s0));
+      } else if (grouped) {  // everything right of the tile, the next panel first
+        float* Xg = A + G1 + G0 * lda;
+        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, 0, bjn, 1, 0);
+        if (rc) return rc;
+        OOC_CUDA_TRY(cudaEventRecord(evA, s0));
+        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, bjn, -1, 0, kChainSMs);
+      } else if (tc_solve) {  // the planes come from the solve
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 0, 0);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
@@ -2173,14 +2198,6 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
   OOC_CUDA_TRY(cudaEventRecord(evP, s1));
   OOC_CUDA_TRY(cudaStreamWaitEvent(s0, evP, 0));
   return OOC_OK;
-}
-
-// Lower-triangle elements of an m x m trailing matrix in columns [a, b): the useful
-// outputs of an update restricted to those columns (2 K flops each).
-double lower_elems(i64 m, i64 a, i64 b) {
-  b = std::min(b, m);
-  if (a >= b) return 0.0;
-  return (double)(b - a) * (double)m - ((double)b * (double)(b - 1) - (double)a * (double)(a - 1)) / 2.0;
 }
 
 // Where the columns of a left-looking factorization come from: a page-locked host matrix
@@ -2596,9 +2613,9 @@ static int create_impl(ooc_handle* h, const double* A, int64_t n, int64_t lda, b
     // than two blocks (faster long-K updates; for a host matrix, copies overlapped)
     bcols = opt >= 0 ? opt : ((pinned || on_device) && n > 2 * 4096 ? 4096 : 0);
   }
-  if (prec == OOC_PREC_FP32 && panel_width_f32(n, nb) < nb) {
+  if (prec == OOC_PREC_FP32 && n > panel_width_f32(nb) && panel_width_f32(nb) < nb) {
     F->tail0 = 0;
-    F->nb2 = panel_width_f32(n, nb);
+    F->nb2 = panel_width_f32(nb);
   }
   const bool lb = !gen && bcols > 0 && prec == OOC_PREC_BF16X3 && nb % 128 == 0 && n > nb && (on_device || pinned);
   if (lb && nb % 256 == 0) {  // left-looking blocks: nb/2-wide panels throughout
@@ -3455,9 +3472,8 @@ int spotrf_host_ooc(ooc_handle* h, float* A, i64 n, i64 lda, int nb, size_t budg
       launches++;
     }
     // in-core factorization of the panel, right-looking inside it (ooc_incore)
-    const int w = panel_width_f32(n, nb);
-    for (i64 q0 = 0; q0 < Wp; q0 += w) {
-      const int LN = (int)std::min<i64>(w, Wp - q0);
+    for (i64 q0 = 0; q0 < Wp; q0 += nb) {
+      const int LN = (int)std::min<i64>(nb, Wp - q0);
       float* Djj = P + q0 + q0 * n;
       if (LN <= DS_MAX)
         k_diag_s256<<<1, DG_THREADS, DS_SMEM, s>>>(Djj, n, LN, J0 + q0, Dinv, LN, Xr, nullptr, nullptr, status);
@@ -3532,8 +3548,8 @@ extern "C" int ooc_spotrf_L(ooc_handle* h, float* A, int64_t n, int64_t lda, int
   F.device = ooc_device(h);
   F.n = n;
   F.nb = nb;
-  F.tail0 = panel_width_f32(n, nb) < nb ? 0 : n;
-  F.nb2 = panel_width_f32(n, nb);
+  F.nb2 = panel_width_f32(nb);
+  F.tail0 = n > F.nb2 && F.nb2 < nb ? 0 : n;
   F.prec = OOC_PREC_FP32;
   F.owns_Lf = on_device ? false : true;
   const int bb = (int)((n + nb - 1) / nb);

@@ -1,4 +1,4 @@
-"""FP32 factorizations in panels narrower than the caller's tiles (128 columns, 256 above n = 6144).
+"""FP32 factorizations in panels narrower than the caller's tiles (256 columns, or 128 where 256 does not divide it).
 
 |A - L L^T|(i, j) <= c n eps sqrt(a_ii a_jj) with eps = 2^-24 and c = 2 (the column solve multiplies by an
 explicit inverse of a well-conditioned 128- or 256-column diagonal tile, so its rounding errors grow by that
