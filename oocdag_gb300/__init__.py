@@ -332,20 +332,31 @@ class Handle:
         matrix i at element offset a_off[i] with ld = ns[i], right-hand side at b_off[i]).
         prec: 'fp64' or 'fp32' (the storage and arithmetic type of A and B).  Returns
         (info list, kernel seconds)."""
+        import numpy as np
+
         count = len(ns)
-        n_arr = (ctypes.c_int * count)(*[int(x) for x in ns])
-        ao = (ctypes.c_int64 * count)(*[int(x) for x in a_off])
-        bo = (ctypes.c_int64 * count)(*[int(x) for x in b_off])
-        info = (ctypes.c_int * count)()
+
+        # one conversion per table (4000 systems took 1.2 ms as Python integers one by one)
+        def table(values, dtype):
+            if not isinstance(values, (list, tuple, np.ndarray)):
+                values = [int(x) for x in values]
+            out, v = np.zeros(max(count, 1), dtype=dtype), np.array(values).astype(np.int64)
+            out[: len(v)] = v.astype(dtype)  # (an error if there are more than `count`)
+            return out
+
+        n_arr, ao, bo = table(ns, np.int32), table(a_off, np.int64), table(b_off, np.int64)
+        info = np.zeros(max(count, 1), dtype=np.int32)
         tbl = None
         if blk_table is not None:
             tbl = (ctypes.c_int * 16)(*[int(x) for x in blk_table])
         sec = ctypes.c_double(0)
         self._after_torch(A, B)
         fn = load().ooc_batched_dposv if prec == "fp64" else load().ooc_batched_sposv
-        _check(fn(self._h, count, n_arr, ao, bo, _ptr(A), _ptr(B), info, tbl, ctas_per_sm, ctypes.byref(sec)),
+        i32, i64 = ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int64)
+        _check(fn(self._h, count, n_arr.ctypes.data_as(i32), ao.ctypes.data_as(i64), bo.ctypes.data_as(i64), _ptr(A), _ptr(B),
+                  info.ctypes.data_as(i32), tbl, ctypes.c_int(ctas_per_sm), ctypes.byref(sec)),
                "ooc_batched_posv")
-        return list(info), sec.value
+        return info[:count].tolist(), sec.value
 
     def fp64_peak(self, ms: float = 200.0) -> float:
         r = ctypes.c_double()
