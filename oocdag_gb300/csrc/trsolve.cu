@@ -376,16 +376,25 @@ int launch_trsolve(const TriSolve<T>& a, void* exchange, unsigned epoch, cudaStr
   // FP64: one right-hand side per task.  A block step is FP64 work of one SM (64 x 64 products
   // with L and with the inverse, 2.4 us at 1.75 FMAs per clock for each right-hand side), so
   // the right-hand sides go side by side on different SMs; L comes from L2 for all but one.
+  // FP32: R per task.  Fewer make a block step of the chain shorter, more make the groups, which all read
+  // L, fewer: the smallest R whose tasks still fit the SMs, 4 while they are at most four to an SM.  us
+  // for R = 1, 2, 4, 8:  n = 2048  r = 8 117 119 134 195,  r = 16 144 121 133 207
+  //                      n = 6000  r = 4 266 245 283 445,  r = 16 592 401 321 496
+  //                      n = 16384 r = 2 789 636 714 1226, r = 16 3611 2118 1380 1471
+  //                      n = 30000 r = 8 6238 3542 2381 2676, r = 16 11591 6503 4005 3703
   const int r = b.r;
-  const int ngrp = sizeof(T) == 8 ? r : (r + TS_RMAX - 1) / TS_RMAX;
-  if (nblk * ngrp * 2 > 0x3fffffff) return OOC_ERR_INTERNAL;
+  if (nblk * r * 2 > 0x3fffffff) return OOC_ERR_INTERNAL;
   if constexpr (sizeof(T) == 8) {
-    return launch_r<T, 1>(b, (int)nblk, ngrp, exchange, epoch, s);
+    return launch_r<T, 1>(b, (int)nblk, r, exchange, epoch, s);
   } else {
-    if (r == 1) return launch_r<T, 1>(b, (int)nblk, 1, exchange, epoch, s);
-    if (r == 2) return launch_r<T, 2>(b, (int)nblk, 1, exchange, epoch, s);
-    if (r <= 4) return launch_r<T, 4>(b, (int)nblk, 1, exchange, epoch, s);
-    return launch_r<T, 8>(b, (int)nblk, ngrp, exchange, epoch, s);
+    int dev = 0, nsm = 0;
+    OOC_CUDA_TRY(cudaGetDevice(&dev));
+    OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    auto groups = [&](int R) { return (r + R - 1) / R; };
+    if (r == 1 || nblk * r <= nsm) return launch_r<T, 1>(b, (int)nblk, r, exchange, epoch, s);
+    if (r == 2 || 4 * nblk * groups(2) <= 5 * nsm) return launch_r<T, 2>(b, (int)nblk, groups(2), exchange, epoch, s);
+    if (r <= 4 || nblk * groups(4) <= 4 * nsm) return launch_r<T, 4>(b, (int)nblk, groups(4), exchange, epoch, s);
+    return launch_r<T, TS_RMAX>(b, (int)nblk, groups(TS_RMAX), exchange, epoch, s);
   }
 }
 template int launch_trsolve<float>(const TriSolve<float>&, void*, unsigned, cudaStream_t);

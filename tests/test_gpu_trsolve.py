@@ -72,3 +72,22 @@ def test_dpotrs(handle, where, n, nb, r, budget):
         X = B.copy(order="F")
         handle.dpotrs_L(L, n, n, nb, X, n, r, budget=budget)
     assert _berr(A, X, B) <= 1e-14
+
+
+@pytest.mark.parametrize("n,r", [(2300, 8), (2500, 9), (3100, 16), (5000, 3), (19600, 16), (19700, 10)])
+def test_right_hand_sides_per_task(handle, n, r):
+    # FP32: 1, 2, 4 or 8 right-hand sides per task by the number of tasks; orders where that changes
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(n)
+    A = torch.empty(n, n, dtype=torch.float64, device="cuda").uniform_(-0.5, 0.5, generator=g)
+    A = torch.tril(A) + torch.tril(A, -1).T
+    A.diagonal().add_(n**0.5)
+    B = torch.randn(r, n, dtype=torch.float64, device="cuda", generator=g)
+    with handle.factor(A, n, n, 256, "fp32") as F:
+        assert F.info == 0
+        X = B.clone()
+        F.solve(X, n, r)
+    R, nA = B - X @ A, A.abs().sum(dim=1).max()
+    be = (R.abs().amax(dim=1) / (nA * X.abs().amax(dim=1) + B.abs().amax(dim=1))).max().item()
+    assert be <= n * 2.0**-23 + 2.0**-20
