@@ -1,21 +1,23 @@
 // Mixed-precision factorization and FP64 solves with iterative refinement.
 //
 // Factor objects.  OOC_PREC_FP64 is the plain path's right-looking factorization (device
-// potrf, inverse-based column solve and DMMA updates).  The reduced precisions keep the
+// potrf, inverse-based column solve, updates by digit products).  The reduced precisions keep the
 // reference's per-panel structure (diagonal-tile potrf, column solve, trailing syrk/gemm:
 // oocquark.cpp:393-410, 346, 351) on an FP32 working matrix that becomes the factor:
 //   diagonal tile  : FP32 Cholesky and inverse in one CTA (k_diag_s256 for tiles of up to
 //                    256 columns, held in shared memory; k_diag_f32 for wider ones);
 //   column solve   : the panel times the tile's inverse, in FP32 (k_colsolve_f32) or as
 //                    three split-BF16 tensor-core products (k_trsm2_bf16x3, tc_bf16x3.cu);
-//   trailing update: OOC_PREC_FP32 - FP32 FFMA products (k_syrk_f32);
+//   trailing update: OOC_PREC_FP32 - exact products of BF16 digits (fp32_tc.cu; k_syrk_f32 on
+//                    the FP32 pipe for a few columns or without room for the digits);
 //                    OOC_PREC_BF16X3 - hi/lo BF16 planes of the panel, three tensor-core
 //                    products (hi*hi + hi*lo + lo*hi) accumulated in FP32 in TMEM and added
 //                    into the FP32 trailing matrix by TMA reductions (k_syrk2_bf16x3).
 // Split-BF16 factors use nb/2-wide panels for the last OOC_OPT_TAIL_ORDER orders.
 // Solves use the kept inverses of the diagonal tiles (trsolve.cu).  The refinement
 // computes residuals in FP64 against the FP64 matrix (device, or the lower triangle of a
-// host matrix copied once), and corrects with the FP32 factor until the normwise backward
+// host matrix copied once), on the FP64 pipe for one right-hand side and by digit products for
+// several, and corrects with the FP32 factor until the normwise backward
 // error ||b - A x||_inf / (||A||_inf ||x||_inf + ||b||_inf) reaches the tolerance.
 
 #include <cuda_bf16.h>
@@ -1964,7 +1966,12 @@ struct MixedProf {
 // B := W (L_jj^{-1})^T with W a copy of B and the triangular half of K skipped.
 // Look-ahead on two streams: the diagonal work of panel j (potrf, inverse, column solve)
 // runs on `s1` while `s0` performs the bulk of the trailing update of panel j-1; `s0` first
-// updates only the next panel's columns and signals `s1`, then updates the rest.
+// updates only the next panel's columns and signals `s1`, then updates the rest.  Where 64 divides nb the
+// updates are digit products on the tensor cores (fp64_tc.cu), FP64_CHUNK columns of the panel at a time (one
+// rounding into C each); otherwise, or without room for the digits, FP64 MMAs (launch_panel_update).
+// n = 8192, nb = 512: 43 ms, 200 with FP64 MMAs; n = 16384: 160 and 1392.
+constexpr int FP64_CHUNK = DIGIT_RUNS * DIGIT_K;
+constexpr int kMixedChainSMs = 16;  // SMs the bulk update leaves to the next panel's kernels
 int factor_mixed(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_t* launches, MixedProf* prof) {
   const i64 n = F->n;
   const int nb = F->nb;
@@ -1977,6 +1984,8 @@ int factor_mixed(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int6
   double* W = (double*)F->scratch.p;   // copy of the column panel (m x nb, ld n)
   double* E = W + (size_t)n * nb;      // L_jj^{-1} (lower, ld nb)
   (void)prec;
+  const size_t slot = (digit_plane_bytes(n, DIGIT_K) + 255) / 256 * 256;
+  const bool digits = nb % 64 == 0 && n > nb && F->work.ensure((size_t)DIGIT_RUNS * slot) == OOC_OK;
   cudaEvent_t evA, evP;  // A: next panel's columns updated (s0 -> s1); P: panel solved (s1 -> s0)
   OOC_CUDA_TRY(cudaEventCreateWithFlags(&evA, cudaEventDisableTiming));
   OOC_CUDA_TRY(cudaEventCreateWithFlags(&evP, cudaEventDisableTiming));
@@ -2021,10 +2030,25 @@ int factor_mixed(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int6
         prof->flops.push_back((double)m * (double)(m + 1) * LN);
       }
       TileMap Cm{C, lda, 0, below, nb};
-      rc = launch_panel_update(TileCol{Pn, lda, nb}, Cm, below, 1, m, m, LN, F->status, s0);
-      if (rc) return rc;
-      OOC_CUDA_TRY(cudaEventRecord(evA, s0));
-      if (below > 1) {
+      const TileMap whole{A, lda, 0, bb, nb};
+      const i64 narrow = std::min<i64>(nb, m);
+      for (int c0 = 0; digits && c0 < LN; c0 += FP64_CHUNK) {
+        const bool last = c0 + FP64_CHUNK >= LN;
+        DigitRuns X{A + (J0 + c0) * lda, lda, nb, nb, J0 + LN, m, std::min(FP64_CHUNK, LN - c0), F->work.p, slot, {}};
+        if ((rc = launch_digits(X, F->status, s0)) || (rc = launch_digit_update(X, whole, 0, last ? narrow : m, F->status, s0)))
+          return rc;
+        if (last) {
+          OOC_CUDA_TRY(cudaEventRecord(evA, s0));
+          if (m > nb) rc = launch_digit_update(X, whole, nb, m, F->status, s0, kMixedChainSMs);
+        }
+        if (rc) return rc;
+      }
+      if (!digits) {
+        rc = launch_panel_update(TileCol{Pn, lda, nb}, Cm, below, 1, m, m, LN, F->status, s0);
+        if (rc) return rc;
+        OOC_CUDA_TRY(cudaEventRecord(evA, s0));
+      }
+      if (!digits && below > 1) {
         TileMap Cr{C + nb * (1 + lda), lda, 0, below - 1, nb};
         rc = launch_panel_update(TileCol{Pn + nb, lda, nb}, Cr, below - 1, below - 1, m - nb, m - nb, LN,
                                  F->status, s0);
@@ -3381,7 +3405,7 @@ extern "C" int ooc_dsyrk_ln(ooc_handle* h, int prec, int n, int k, const double*
 
 // ---------------------------------------------------------------------------------
 // FP32 Cholesky of a caller's matrix, in place (the reference has no FP32 entry): the
-// reduced-precision factor pipeline with FP32 trailing updates (k_syrk_f32), on the
+// reduced-precision factor pipeline with FP32 trailing updates (syrk_f32), on the
 // matrix itself (device) or on a device copy of it (host, when it fits in dev_budget).
 // ---------------------------------------------------------------------------------
 namespace {
@@ -3389,7 +3413,7 @@ namespace {
 // left-looking panel loop (oocdag.cpp:59-87) with panels of W columns (W from the budget:
 // the panel and two copies of earlier columns, each n x W floats).  Per panel, on the
 // compute stream s: the panel's lower part arrives (copy stream sc), every earlier panel's
-// columns arrive W at a time through two X buffers and update it (FP32 k_syrk_f32 restricted
+// columns arrive W at a time through two X buffers and update it (FP32 syrk_f32 restricted
 // to the panel's columns: the A2X + ooc_syrk tasks, oocquark.cpp:301-356), then the panel is
 // factored in core right-looking (FP32 diagonal tile, column solve, updates inside the
 // panel: ooc_incore, oocquark.cpp:358-421) and copied back (stream sd) before any later

@@ -101,3 +101,22 @@ def test_factor_is_schedule_invariant(oracle_mod, handle, n, nb, tiles):
     np.testing.assert_array_equal(H, L)
     Lo = np.linalg.cholesky(A)
     np.testing.assert_allclose(np.tril(L), Lo, rtol=0, atol=1e-12 * np.abs(Lo).max())
+
+
+@pytest.mark.parametrize("n,nb", [(65, 64), (129, 64), (500, 192), (1000, 128), (1300, 1088), (1201, 576), (700, 100)])
+def test_factor_object(handle, n, nb):
+    # factor objects in FP64: panels of up to 512 columns per update, tiles wider than that in several, and one
+    # that 64 does not divide (FP64 MMAs).  |A - L L^T| <= 4 n eps sqrt(a_ii a_jj): the column solve multiplies by the
+    # explicit inverse of a diagonal tile whose condition number is below 3.
+    rng = np.random.default_rng(n)
+    R = rng.uniform(-0.5, 0.5, (n, n))
+    A = (R + R.T) / 2 + np.sqrt(n) * np.eye(n)
+    import torch
+
+    L = np.asfortranarray(np.empty((n, n)))
+    with handle.factor(torch.from_numpy(np.ascontiguousarray(A)).cuda(), n, n, nb, "fp64") as F:
+        assert F.info == 0
+        F.copy_L(L, n)
+    L, s = np.tril(L).astype(np.longdouble), np.sqrt(np.diag(A))
+    err = np.abs(np.tril(A - L @ L.T) / s[:, None] / s[None, :]).max()
+    assert err <= 4 * n * 2.0**-53, float(err)
