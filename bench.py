@@ -41,15 +41,30 @@ sys.path.insert(0, ROOT)
 
 METRIC = "Cholesky TFLOP/s (n^3/3 flops), mixed vs FP64 at backward err<=1e-14; p99 ms"
 
-# DRAM bytes per algorithmic flop of k_panel_update, from one ncu capture of two launches
-# at n=8192, nb=1024 (dram__bytes_read.sum + dram__bytes_write.sum = 348.1 MB for
-# 44.02 GFLOP).  The kernel's traffic is the operand and C tiles, which scale with the
-# flops of a launch at fixed nb.
-UPDATE_DRAM_BYTES_PER_FLOP = 348.1e6 / 44.02e9
 # ncu DRAM bytes / algorithmic bytes of one long-K catch-up launch (k_syrk2t_bf16x3, n=16384,
 # m=12032, 3840 columns, K=4096: 698.1 + 140.1 MB measured against 8 B per lower element of
 # C plus 4 B per plane element, 507.8 MB); the catch-ups carry 90 % of the update flops
 UPDATE_TRAFFIC_RATIO = (698.1 + 140.1) / 507.8
+
+
+# Products of BF16 digits per FP64 product in the tensor-core updates (csrc/fp64_tc.cu)
+DIGIT_PRODUCTS = 34
+
+
+def fp64_update_roofline(tflops, fp64_peak, nb):
+    """Roofline entry of the FP64 trailing updates at `tflops` (algorithmic): digit products on the tensor
+    cores where 64 divides the tile width, the FP64 pipe otherwise."""
+    pipe = {"fp64_pipe_peak": fp64_peak, "times_fp64_pipe": tflops / fp64_peak if tflops else None,
+            "fp64_pipe_source": "measured live: FP64 DMMA issue loop on all SMs (ooc_fp64_peak_probe)"}
+    if nb % 64:
+        return {"bound": "fp64-dmma", "kernel": "k_panel_update (syrk+gemm, FP64 mma.sync m8n8k4)", "achieved": tflops,
+                "peak": fp64_peak, "unit": "TFLOP/s", "frac": tflops / fp64_peak if tflops else None} | pipe
+    path = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    peak = json.load(open(path)).get("bf16_tflops") if os.path.exists(path) else None
+    return {"bound": "tensor", "kernel": "k_digit_update (tcgen05, exact products of BF16 digits)", "achieved": tflops,
+            "peak": peak / DIGIT_PRODUCTS if peak else None, "unit": "TFLOP/s",
+            "frac": tflops * DIGIT_PRODUCTS / peak if tflops and peak else None,
+            "peak_source": f"MEASURED_PEAKS.json bf16_tflops / {DIGIT_PRODUCTS} products"} | pipe
 
 
 def parse():
@@ -373,16 +388,11 @@ def run_fp64_ooc(args):
 
     # ---- roofline of the dominant kernel -----------------------------------------
     achieved = upd_flops / (upd_ms / 1e3) / 1e12 if upd_ms > 0 else None
-    roofline = {"bound": "fp64-dmma", "kernel": "k_panel_update (syrk+gemm, FP64 mma.sync m8n8k4)",
-                "achieved": achieved, "peak": peak_tf, "unit": "TFLOP/s",
-                "frac": (achieved / peak_tf) if achieved else None,
-                "peak_source": "measured live: FP64 DMMA issue loop on all SMs (ooc_fp64_peak_probe); "
-                               "MEASURED_PEAKS.json has no FP64 entry",
+    roofline = fp64_update_roofline(achieved, peak_tf, nb) | {
                 "launches": upd_launch, "avg_launch_ms": upd_ms / max(1, upd_launch),
                 "share_of_step": upd_ms / (ms_local * args.steps) if ms_local > 0 else None,
-                "traffic": (UPDATE_DRAM_BYTES_PER_FLOP * upd_flops / upd_launch) if upd_launch else None,
-                "traffic_unit": "bytes per launch (ncu capture at n=8192 scaled by flops per launch)",
-                "algorithmic_bytes_note": "operand tiles read once + C tiles read and written"}
+                "traffic": None,
+                "algorithmic_bytes_note": "14 bytes of digit planes per element of X + C tiles read and written"}
 
     # ---- CPU baseline (rank 0, N=1 only) -----------------------------------------
     cpu = None
@@ -468,11 +478,8 @@ def run_fp64_ooc_host(args):
                    "form": "fp64-ooc-host", "n": n, "nb": nb, "budget_mb": args.budget_mb},
         "panels": st["npanels"], "h2d_bytes": st["h2d_bytes"], "d2h_bytes": st["d2h_bytes"],
         "host_link_gbs_achieved": (st["h2d_bytes"] + st["d2h_bytes"]) / (ms / 1e3) / 1e9, "host_link_probe": link,
-        "roofline": {"bound": "fp64-dmma", "kernel": "k_panel_update (syrk+gemm, FP64 mma.sync m8n8k4)",
-                     "achieved": upd, "peak": peak_tf, "unit": "TFLOP/s", "frac": upd / peak_tf if upd else None,
-                     "step_frac": value / peak_tf, "launches": st["update_launches"],
-                     "share_of_step": st["update_ms"] / ms if ms else None,
-                     "peak_source": "measured live: FP64 DMMA issue loop on all SMs (ooc_fp64_peak_probe)"},
+        "roofline": fp64_update_roofline(upd, peak_tf, nb) | {
+                     "launches": st["update_launches"], "share_of_step": st["update_ms"] / ms if ms else None},
         "clocks": clk, "gpu_launches": st["kernel_launches"],
     }
     print(json.dumps(line), flush=True)
@@ -617,8 +624,8 @@ def run_mixed(args):
         X64 = X[:nrhs].clone()
         fp64 = {"value": flops / t64 / 1e12, "unit": "TFLOP/s", "ms_per_step": t64 * 1e3, "steps": 1,
                 "warmup": 0, "backward_error": be64, "factor_seconds": st64["seconds"],
-                "note": "plain FP64 path (DMMA updates, FP64 solve), same A and b, measured once",
-                "fp64_dmma_peak_tflops": fp64_peak, "frac_of_fp64_peak": (flops / t64 / 1e12) / fp64_peak,
+                "note": "plain FP64 path (FP64 factor object, FP64 solve), same A and b, measured once",
+                "fp64_pipe_peak_tflops": fp64_peak, "times_fp64_pipe": (flops / t64 / 1e12) / fp64_peak,
                 "speedup_mixed_over_fp64": (value / world) / (flops / t64 / 1e12)}
 
     # ---- errors of every solve form, per delta (untimed) --------------------------------
@@ -735,14 +742,14 @@ def run_mixed(args):
     share_upd = upd_ms / (ms_local * args.steps)
     share_fac = fac_ms / (ms_local * args.steps)
     bf16_peak = peaks.get("bf16_tflops_sustained") or peaks.get("bf16_tflops")
-    mult = 3 if args.prec == "bf16x3" else 1
+    mult = 3 if args.prec == "bf16x3" else 10  # BF16 products per product
     upd_roof = {"kernel": "k_syrk2t_bf16x3 (long-K catch-ups: N=256 tcgen05 MMAs, C transposed in TMEM, four-stage "
                           "K=32 operand ring) + k_syrk2_bf16x3<float> (in-block K=256 updates): persistent split-BF16 "
                           "trailing updates, 256x128 blocks, FP32 C updated by TMA reductions"
-                if args.prec == "bf16x3" else "k_syrk_f32<float> (FP32 FFMA trailing update)",
-                "bound": "tensor" if args.prec == "bf16x3" else "fp32-simt",
+                if args.prec == "bf16x3" else "k_digit32 (tcgen05, exact products of BF16 digits of FP32 panels)",
+                "bound": "tensor",
                 "achieved": upd_flops / (upd_ms / 1e3) / 1e12 if upd_ms else None,
-                "peak": bf16_peak if args.prec == "bf16x3" else None, "unit": "TFLOP/s",
+                "peak": bf16_peak, "unit": "TFLOP/s",
                 "flops_convention": "algorithmic: 2 K per lower-triangle output element (m(m+1)K for a whole "
                                     "trailing matrix), the Cholesky's own flops",
                 "launches": upd_launch, "avg_launch_ms": upd_ms / max(1, upd_launch), "share_of_step": share_upd,

@@ -10,8 +10,10 @@
  *   - `r` (the QUARK worker rank, ooc_offload.cpp:99) selects a per-worker CUDA stream;
  *     every call returns when its work on that stream has finished, as the reference's
  *     offload regions did;
- *   - the BLAS/LAPACK calls run the library's own sm_103a kernels (FP64 DMMA contraction,
- *     device potrf, blocked column solve); no cuBLAS/cuSOLVER.
+ *   - the BLAS/LAPACK calls run the library's own sm_103a kernels (FP64 contraction by
+ *     exact digit products on the tensor cores or DMMA, device potrf, blocked column solve); no
+ *     cuBLAS/cuSOLVER.  A product's error is relative to the largest element of its operand
+ *     rows per 128 columns of k, at or below that of an FP64 sum over them.
  * MKL_INT is the LP64 int.  All functions have C linkage (the reference's were C++ except
  * offload_init_/offload_destroy_).  Errors: the BLAS-style calls return void as in the
  * reference; ooc_offload_last_error() reports the last failure (0 = none).

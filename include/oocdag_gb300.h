@@ -120,6 +120,9 @@ int ooc_get_stream(ooc_handle* h, int which, void** stream);
  *           ooc_incore (oocquark.cpp:253-421, prototypes oocdag.h:119-123).
  * A: host memory (pageable or pinned; streamed through a device budget of dev_budget
  *    bytes) or device memory (factored in place, in core).  Upper triangle untouched.
+ *    Where 64 divides nb the trailing updates go through digit planes on the tensor cores:
+ *    28 bytes per row of a panel for each of up to 512 columns, device memory beside
+ *    dev_budget that the handle keeps; without room for it the FP64 pipe does them.
  * *info: 0, or k > 0 if the leading minor of order k is not positive definite.      */
 int ooc_dpotrf_L(ooc_handle* h, double* A, int64_t n, int64_t lda, int nb, size_t dev_budget,
                  int* info, ooc_stats* stats);
@@ -177,8 +180,8 @@ int ooc_panel_plan(int64_t n, int nb, int64_t memBlock, int nx, int* out, int ca
  * the tile's inverse) in FP32 for OOC_PREC_FP32 and with the update's three BF16 tensor
  * products for OOC_PREC_BF16X3 (nb a multiple of 128).                               */
 enum {
-  OOC_PREC_FP64 = 0,  /* FP64 DMMA updates (the plain path)                        */
-  OOC_PREC_FP32 = 1,  /* FP32 operands, FP32 FFMA accumulation                      */
+  OOC_PREC_FP64 = 0,  /* FP64 updates (the plain path)                             */
+  OOC_PREC_FP32 = 1,  /* FP32 operands, sums exact or in FP32                       */
   OOC_PREC_BF16X3 = 2 /* hi/lo BF16 splits, 3 tensor-core products, FP32 accumulate */
 };
 

@@ -8,12 +8,13 @@
 //                                            page-locked host matrix into the packed panel
 //   A2X   H2D task per tile of column jjb      s_h2d: same, into X buffer jjb % 2, waiting
 //         (single X buffer: WAR on X)          on the update that last read that buffer
-//   ooc_syrk  dsyrk/dgemm task per tile pair   s_comp: ONE launch per X column covering
-//                                            every tile pair of the panel (FP64 DMMA)
-//   ooc_incore  host dpotrf round trip,        s_comp: device potrf of the diagonal tile,
-//               dtrsm + D2H per tile,          one column solve launch sequence, trailing
-//               trailing ooc_syrk              update launch; s_d2h copies each finished
-//                                            column back while s_comp moves on
+//   ooc_syrk  dsyrk/dgemm task per tile pair   s_comp: per X column its digits and ONE launch
+//                                            covering every tile pair of the panel (tensor
+//                                            cores; FP64 DMMA where 64 does not divide nb)
+//   ooc_incore  host dpotrf round trip,        s_h2d: chain of 64-column diagonal blocks, row
+//               dtrsm + D2H per tile,          solves and narrow updates; s_comp: the bulk of
+//               trailing ooc_syrk              the trailing update; s_d2h copies each finished
+//                                            column back meanwhile
 //   QUARK_Barrier                              one bounded wait at the end
 //
 // Hazards QUARK tracked by tile address become events: Y is reused across panels
@@ -77,7 +78,7 @@ struct ooc_handle {
   std::shared_ptr<DevPool> pool;  // device buffers of the handle's factor objects
   GrowBuf batch_ws;               // launch tables of the batched solvers
   GrowBuf solve_ws;               // panels and vectors of ooc_dpotrs_L
-  GrowBuf digit_ws;               // digit planes of the tensor-core FP64 updates (two runs of 128 columns)
+  GrowBuf digit_ws;               // digit planes of the tensor-core FP64 updates (two sets of up to four runs of 128 columns)
   int last_info = 0;
   std::vector<cudaEvent_t> ev_pool;  // reusable timing-free events
   size_t ev_next = 0;
