@@ -2854,11 +2854,6 @@ __global__ void k_add_f32_cols(double* X, i64 ldx, const float* D, i64 ldd, int 
   for (int q = 0; q < r; q++) X[i + q * ldx] += ooc_f32_to_f64(D[i + q * ldd]);
 }
 
-double host_max(const std::vector<double>& v, int r, int q, int nb) {
-  double m = 0;
-  for (int b = 0; b < nb; b++) m = std::max(m, v[(size_t)b * r + q]);
-  return m;
-}
 }  // namespace
 
 extern "C" int ooc_factor_copy_L(ooc_factor* F, double* L, int64_t ldl) {
