@@ -225,10 +225,11 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm_batched(GemmBatch gb, con
 //     refined by one cubic Newton step (e = 1 - d r0, a r0 (1 + e + e^2): error e^3 <
 //     2^-66), four dependent FP64 instructions where a square root and a division took
 //     twenty; one barrier per column;
-//   * the 16 square roots and their reciprocals are taken side by side at the block's end;
-//   * the columns to the right take the block as one rank-16 update on the FP64 MMA.
+//   * the columns to the right take the block as one rank-16 update on the FP64 MMA, from the
+//     unscaled columns and the quotients;
+//   * the 64 square roots and their reciprocals are taken side by side at the end.
 // Measured on a 64 x 64 block: 90 us with a square root and a division per column on the
-// barrier-to-barrier path, 50 us now.
+// barrier-to-barrier path, 50 us with the roots and a scaling pass per 16 columns, 46 us now.
 // LAPACK convention: a pivot that is not > 0 (or is NaN) stops the factorization and reports
 // info = col0 + j + 1; the columns before it are written back.
 // ---------------------------------------------------------------------------------
@@ -239,8 +240,9 @@ constexpr int SP = SB + 1;           // column pitch in shared memory
 __global__ void __launch_bounds__(PT_THREADS) k_potrf_small(double* A, i64 ld, int n, i64 col0, int* status) {
   pdl_wait();
   if (*(volatile int*)status) return;
-  __shared__ double S[SB * SP];       // S[c * SP + r]
-  __shared__ double sq[PB], rs[PB];
+  __shared__ double S[SB * SP];       // S[c * SP + r], unscaled until the end
+  __shared__ double U[PB * SP];       // a block's columns over their pivots
+  __shared__ double sq[SB], rs[SB];
   __shared__ int s_nfin;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   {  // 64 rows x 2 column groups; beyond n the identity
@@ -253,30 +255,15 @@ __global__ void __launch_bounds__(PT_THREADS) k_potrf_small(double* A, i64 ld, i
   }
   __syncthreads();
   const int g = lane >> 2, tig = lane & 3;
+  int done = SB;  // columns that factored
   for (int k = 0; k < n; k += PB) {
-    int nfin = k < 32 ? potrf_panel<2, SB, SP>(S, k) : k < 48 ? potrf_panel<4, SB, SP>(S, k) : potrf_panel<8, SB, SP>(S, k);
+    int nfin = k < 32 ? potrf_panel<2, SB, SP>(S, k, U) : k < 48 ? potrf_panel<4, SB, SP>(S, k, U) : potrf_panel<8, SB, SP>(S, k, U);
     if (t == 0) s_nfin = nfin;
     __syncthreads();
     nfin = s_nfin;
-    if (lane < PB && warp < 2) {  // the block's square roots and their reciprocals, a warp each
-      const double d = S[(k + lane) * SP + k + lane];
-      if (warp == 0) sq[lane] = lane < nfin ? sqrt(d) : 1.0;
-      else rs[lane] = lane < nfin ? rsqrt(d) : 1.0;
-    }
-    __syncthreads();
-    {
-      const int r = t & (SB - 1), cg = t >> 6;
-#pragma unroll
-      for (int i = 0; i < PB / 2; i++) {
-        const int c = 2 * i + cg;
-        double* e = S + (k + c) * SP + r;
-        if (r == k + c && c < nfin) *e = sq[c];
-        else if (r > k + c) *e *= rs[c];
-      }
-    }
-    __syncthreads();
     if (nfin < PB) {
-      if (t == 0) atomicCAS(status, 0, (int)(col0 + k + nfin + 1));
+      done = k + nfin;
+      if (t == 0) atomicCAS(status, 0, (int)(col0 + done + 1));
       break;
     }
     // rank-16 update of the lower triangle to the right, an 8 x 8 MMA tile per warp and turn
@@ -290,18 +277,25 @@ __global__ void __launch_bounds__(PT_THREADS) k_potrf_small(double* A, i64 ld, i
       double c0 = S[(col + 2 * tig) * SP + row], c1 = S[(col + 2 * tig + 1) * SP + row];
 #pragma unroll
       for (int q = 0; q < PB; q += 4)
-        dmma884(c0, c1, -S[(k + q + tig) * SP + row], S[(k + q + tig) * SP + col + g]);
+        dmma884(c0, c1, -U[(q + tig) * SP + row], S[(k + q + tig) * SP + col + g]);
       S[(col + 2 * tig) * SP + row] = c0;
       S[(col + 2 * tig + 1) * SP + row] = c1;
     }
     __syncthreads();
   }
+  {  // every square root and its reciprocal, side by side, scale the columns on their way out
+    const int c = t & (SB - 1);
+    const double d = c < done ? S[c * SP + c] : 1.0;
+    if (t < SB) sq[c] = sqrt(d);
+    else rs[c] = rsqrt(d);
+  }
+  __syncthreads();
   {
     const int rr = t & (SB - 1), cg = t >> 6;
 #pragma unroll 16
     for (int i = 0; i < SB / 2; i++) {
       const int c = cg + 2 * i;
-      if (rr < n && c <= rr) A[rr + (i64)c * ld] = S[c * SP + rr];
+      if (rr < n && c <= rr) A[rr + (i64)c * ld] = rr == c && c < done ? sq[c] : S[c * SP + rr] * rs[c];
     }
   }
 }

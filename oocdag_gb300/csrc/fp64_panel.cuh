@@ -32,8 +32,10 @@ __device__ __forceinline__ bool positive(double d) {  // d > 0 (false for NaN), 
 // (S[c SP + r]), LPR threads per row (threads t <
 // (SB - k) LPR; the others return at once).  More threads per row where rows are few: an
 // instruction costs a warp 64 clocks whatever its lanes.  Returns the columns that factored.
+// U, where given (PB columns of pitch SP), gets a(r, j) / d(j): the other factor of an update by the
+// unscaled columns.
 template <int LPR, int SB, int SP>
-__device__ __forceinline__ int potrf_panel(double* S, int k) {
+__device__ __forceinline__ int potrf_panel(double* S, int k, double* U = nullptr) {
   constexpr int XC = PB / LPR;  // columns per thread: k + LPR i + h
   const int t = threadIdx.x;
   const int r = k + t / LPR, h = t % LPR, nthr = (SB - k) * LPR;
@@ -58,6 +60,7 @@ __device__ __forceinline__ int potrf_panel(double* S, int k) {
         } else {
           u = slow_div(u, d);
         }
+        if (U && h == 0) U[j * SP + r] = u;
         if (j + 1 < PB) {  // the next column first: it is stored before the row's other FMAs
           const int i1 = (j + 1) / LPR, h1 = (j + 1) % LPR;
           if (h >= h1) x[i1] = fma(-u, cb[k + LPR * i1 + h], x[i1]);
