@@ -325,7 +325,7 @@ __device__ void solve_back_f32(const float* __restrict__ L, int n, float* bs) {
 // mma.sync, not tcgen05: a step's operands are at most 480 rows by 32 columns, written by the CTA's own
 // threads, and its results are wanted in registers at once; 16 x 8 blocks keep the triangle's
 // waste small at these orders.
-// 1200 matrices of 16..512: 5.9 ms against 26.7 ms with FP64 FMAs (7.4 with every class in steps of 32 columns and
+// 1200 matrices of 16..512: 5.7 ms against 26.7 ms with FP64 FMAs (7.4 with every class in steps of 32 columns and
 // no class beside another's tail).
 __device__ __forceinline__ void bar_group() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }  // warps 0..3
 constexpr int DP = 33;          // column pitch of the diagonal block
@@ -358,12 +358,15 @@ __device__ __forceinline__ int row_at(int i, int c) {
   return KS == 2 ? i * 64 + ((c ^ ((i >> 1) & 3)) << 4) : i * 32 + ((c ^ ((i >> 2) & 1)) << 4);
 }
 
-// Cholesky of the diagonal block in S.D (kb of 32) by warps 0..3; S.fail gets the first bad
+// Cholesky of the diagonal block in S.D by warps 0..3 (KS = 2: kb of 32 columns; KS = 1: kb of 16, in the
+// lower right corner, where the panel step has eight threads a row); S.fail gets the first bad
 // pivot's 1-based index.  Then L_kk (the columns before that pivot) to the matrix, and y_k = L_kk^{-1} b_k.
+template <int KS>
 __device__ __forceinline__ void diag_f64(Shared64& S, double* __restrict__ A, int n, int k, int kb, double* bs) {
+  constexpr int O = KS == 1 ? PB : 0, W = 16 * KS;
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  int fail = 0, done = 32;  // columns that factored
-  for (int o = 0; o < kb; o += PB) {
+  int fail = 0, done = W;  // columns that factored
+  for (int o = O; o < O + kb; o += PB) {
     int nf = o == 0 ? potrf_panel<4, 32, DP>(S.D, 0) : potrf_panel<8, 32, DP>(S.D, PB);
     if (t == 0) S.nfin = nf;
     bar_group();
@@ -380,9 +383,10 @@ __device__ __forceinline__ void diag_f64(Shared64& S, double* __restrict__ A, in
       if (r == o + c && c < nf) *e = S.sq[c];
       else if (r > o + c) *e *= S.rs[c];
     }
+    if (t < PB) S.rinv[o - O + t] = S.rs[t];
     bar_group();
     if (nf < PB) {
-      done = o + nf;
+      done = o - O + nf;
       fail = k + done + 1;
       break;
     }
@@ -398,30 +402,32 @@ __device__ __forceinline__ void diag_f64(Shared64& S, double* __restrict__ A, in
     }
   }
   if (t == 0) S.fail = fail;
-  if (warp == 0 && !fail) S.rinv[lane] = 1.0 / S.D[lane * DP + lane];
-  for (int i = t; i < 32 * 32; i += 128) {
+  for (int i = t; i < W * 32; i += 128) {
     const int c = i >> 5, r = i & 31;
-    if (r >= c && r < kb && c < done) A[(k + r) + (i64)(k + c) * n] = S.D[c * DP + r];
+    if (r >= c && r < kb && c < done) A[(k + r) + (i64)(k + c) * n] = S.D[(O + c) * DP + O + r];
   }
   if (warp == 0 && bs && !fail) {  // (b_k is final: every earlier step has taken its share off)
-    __syncwarp();
+    const int l = min(lane, W - 1);
     double v = lane < kb ? bs[k + lane] : 0.0;
-    const double ri = S.rinv[lane], d = S.D[lane * DP + lane];
+    const double d = S.D[(O + l) * DP + O + l], ri = 1.0 / d;
 #pragma unroll 8
-    for (int j = 0; j < 32; j++) {
+    for (int j = 0; j < W; j++) {
       const double y = __shfl_sync(0xffffffffu, div_by(v, d, ri), j);
-      v = lane == j ? y : lane > j ? fma(-S.D[j * DP + lane], y, v) : v;
+      v = lane == j ? y : lane > j && lane < W ? fma(-S.D[(O + j) * DP + O + l], y, v) : v;
     }
     if (lane < kb) bs[k + lane] = v;
   }
 }
 
 // The diagonal block at column k from the matrix into S.D, by warps 0..3.
+template <int KS>
 __device__ __forceinline__ void load_diag_f64(Shared64& S, const double* A, int n, int k, int kb) {
-  for (int i = threadIdx.x; i < 32 * 32; i += 128) {
-    const int c = i >> 5, r = i & 31;
-    S.D[c * DP + r] = (r >= c && r < kb) ? A[(k + r) + (i64)(k + c) * n] : (r == c ? 1.0 : 0.0);
+  constexpr int O = KS == 1 ? PB : 0, W = 16 * KS;
+  for (int i = threadIdx.x; i < W * W; i += 128) {
+    const int c = i / W, r = i % W;
+    S.D[(O + c) * DP + O + r] = (r >= c && r < kb) ? A[(k + r) + (i64)(k + c) * n] : (r == c ? 1.0 : 0.0);
   }
+  if (KS == 2 && threadIdx.x < 32) S.rinv[threadIdx.x] = 1.0;  // (columns that no panel step reaches)
 }
 
 // An element of the product where digits do not serve: a result out of the normal range, or a row with
@@ -486,14 +492,14 @@ __device__ __forceinline__ void update_block(double* __restrict__ C, const doubl
 
 template <int NT, int KS>
 __device__ int factor_f64(double* __restrict__ A, int n, int blk, Shared64& S, double* bs, uint8_t* planes, int* exps) {
-  constexpr int W = 16 * KS;
+  constexpr int W = 16 * KS, O = KS == 1 ? PB : 0;  // (O: the diagonal block's place in S.D)
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int zero = n >> 30;  // n <= 512
   {
     if (t < 128) {
-      load_diag_f64(S, A, n, 0, min(blk, n));
+      load_diag_f64<KS>(S, A, n, 0, min(blk, n));
       bar_group();
-      diag_f64(S, A, n, 0, min(blk, n), bs);
+      diag_f64<KS>(S, A, n, 0, min(blk, n), bs);
     }
     __syncthreads();
   }
@@ -519,7 +525,7 @@ __device__ int factor_f64(double* __restrict__ A, int n, int blk, Shared64& S, d
         r[c] *= S.rinv[c];
         // zero at run time: column c's loads of L_kk wait for r[c] (not all hoisted into registers)
         const int z = zero & __double2loint(r[c]);
-        const double* lc = S.D + c * DP + z;
+        const double* lc = S.D + (O + c) * DP + O + z;
 #pragma unroll
         for (int q = c + 1; q < W; q++) r[q] = fma(-r[c], lc[q], r[q]);
         if (live && c < kb) {
@@ -554,9 +560,9 @@ __device__ int factor_f64(double* __restrict__ A, int n, int blk, Shared64& S, d
       }
       bar_group();
       const int kn = min(blk, m);
-      load_diag_f64(S, A, n, k + kb, kn);
+      load_diag_f64<KS>(S, A, n, k + kb, kn);
       bar_group();
-      diag_f64(S, A, n, k + kb, kn, bs);
+      diag_f64<KS>(S, A, n, k + kb, kn, bs);
     }
     const int np = ns / 2, ntask = ns < 3 ? 0 : np * np + np - 2 + ((ns & 1) ? np + 1 : 0);
     for (;;) {
