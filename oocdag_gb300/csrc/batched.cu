@@ -649,10 +649,10 @@ __device__ void solve_back_f64(const double* __restrict__ L, int n, double* bs) 
 }
 
 // Step width where the caller gives none: 16 columns need half the FP64 work of 32 in the panel's solve and
-// half the shared memory, 32 fewer passes over the matrix.  Kernel ms for 16 and 32: n in 64..128 (1000 matrices) 0.50,
-// 0.54; 256..384 (608) 2.77 (two CTAs per SM), 3.33; 400..512 (608) 7.04, 6.61 (one CTA either way); up to 64, one step
-// of 32 and the rest: 0.36, 0.34.
-inline int default_blk_f64(int n) { return n > 64 && n <= 448 ? 16 : 32; }
+// half the shared memory, 32 fewer passes over the matrix.  Kernel ms for 16 and 32: n in 16..64 (2000 matrices) 0.31,
+// 0.34; 64..128 (1000) 0.45, 0.54; 128..256 (1000) 1.75, 1.88; 256..384 (608) 2.67 (two CTAs per SM), 3.33;
+// 400..512 (608) 7.78, 6.54 (one CTA either way above 448).
+inline int default_blk_f64(int n) { return n <= 448 ? 16 : 32; }
 constexpr size_t F64_TWO = 113 * 1024;  // shared memory that lets two CTAs share an SM
 
 // Shared memory of a launch whose matrices have orders <= nmax: bytes of digits for rows below a
