@@ -2757,7 +2757,7 @@ static int create_impl(ooc_handle* h, const double* A, int64_t n, int64_t lda, b
   }
   int st = 0;
   if (!rc) rc = read_int(F->status, &st, s);
-  if (lb) F->work.release();  // the plane store: the factor is complete
+  if (lb || prec != OOC_PREC_BF16X3) F->work.release();  // the plane store, the digits: the factor is complete
   if (!rc) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { ooc_set_last_error(e, "mixed factorization", __FILE__, __LINE__); rc = OOC_ERR_CUDA; }
