@@ -70,8 +70,9 @@ __global__ void __launch_bounds__(256) k_digits32(const Op32 o, uint8_t* __restr
   bool any = false;  // a row of zeros has scale 1 (any scale does), a subnormal one 2^-125
 #pragma unroll
   for (int k = 0; k < FKS; k++) any = any || (v[k] & 0x7FFFFFFFu) != 0;
-  const bool zero = bmax == 0 && !__syncthreads_or(any && bmax == 0 ? 1 : 0);
-  const int e = zero ? 0 : max(bmax, 1) - 126;  // |x| < 2^e
+  // (a barrier, so every thread of the CTA takes it: rows of zeros, padding among them, share warps with others)
+  const bool subnormal = __syncthreads_or(any && bmax == 0 ? 1 : 0);
+  const int e = bmax == 0 && !subnormal ? 0 : max(bmax, 1) - 126;  // |x| < 2^e
   if (cg == 0) exps[(i64)run * o.pad + row] = bmax == 0xFF ? F_NONFINITE : e;
   const int swz = (row >> 1) & 3;
   {
