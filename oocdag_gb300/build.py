@@ -39,7 +39,7 @@ def _sources() -> list[str]:
 
 
 def _deps() -> list[str]:
-    return _sources() + sorted(glob.glob(os.path.join(CSRC, "*.cuh"))) + sorted(
+    return _sources() + sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h"))) + sorted(
         glob.glob(os.path.join(INCLUDE, "*.h"))) + [CLI_SRC]
 
 

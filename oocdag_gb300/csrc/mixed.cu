@@ -34,6 +34,7 @@
 #include "devpool.cuh"
 #include "fp32_tc.cuh"
 #include "fp64_tc.cuh"
+#include "syrk32_way.h"
 #include "trsolve.cuh"
 
 namespace {
@@ -1361,17 +1362,31 @@ int syrk_lowprec(int prec, const double* X, i64 ldx, double* C, i64 ldc, int m, 
 constexpr int DIGIT32_MIN_K = 16, DIGIT32_CHUNK = 512;
 
 // The same for the FP32 working matrix of a reduced-precision factor: C (FP32) -= X X^T
-// with X the FP32 column panel (no conversions).
+// with X the FP32 column panel (no conversions).  OOC_PREC_FP32 in several calls on one X: `way` takes the
+// prepared call's choice to the others.
 int syrk_f32(int prec, const float* X, i64 ldx, float* C, i64 ldc, int m, int K, const int* status, cudaStream_t s,
-             DevBuf& work, int bj_lo = 0, int bj_hi = -1, int prepare = 1, int reserve_sms = 0) {
+             DevBuf& work, int bj_lo = 0, int bj_hi = -1, int prepare = 1, int reserve_sms = 0,
+             Syrk32Way* way = nullptr) {
   if (m <= 0 || K <= 0) return OOC_OK;
-  if (prec == OOC_PREC_FP32 && K >= DIGIT32_MIN_K && m >= FB / 2) {
-    // digit products on the tensor cores, at most 512 columns at a time; without room for the planes
-    // the FP32 pipe (k_syrk_f32) does it
+  if (prec == OOC_PREC_FP32) {
+    // digit products on the tensor cores, at most 512 columns at a time; k_syrk_f32 stages X with 16-byte
+    // copies: a panel whose base or leading dimension is not 16-byte compatible is first copied to an
+    // aligned buffer (once per panel)
     const int kc = std::min(K, DIGIT32_CHUNK);
-    bool ok = true;
-    if (prepare) ok = work.ensure(digit32_bytes(m, kc)) == OOC_OK;
-    if (ok) {
+    const i64 lds = ((i64)m + 3) / 4 * 4;
+    Syrk32Way one = Syrk32Way::kNone;
+    if (!way) way = &one;
+    if (prepare) {
+      const bool aligned = reinterpret_cast<uintptr_t>(X) % 16 == 0 && ldx % 4 == 0;
+      int rc = syrk32_choose(work, K >= DIGIT32_MIN_K && m >= FB / 2, digit32_bytes(m, kc), aligned,
+                             (size_t)lds * K * sizeof(float), way);
+      if (rc) return rc;
+      if (*way == Syrk32Way::kCopied)
+        k_copy_f32<<<dim3((unsigned)((m + 255) / 256), (unsigned)std::min(K, 1024)), 256, 0, s>>>(X, ldx, (float*)work.p,
+                                                                                              lds, m, K);
+    }
+    if (*way == Syrk32Way::kNone) return OOC_ERR_INTERNAL;
+    if (*way == Syrk32Way::kDigits) {
       for (int k0 = 0; k0 < K; k0 += DIGIT32_CHUNK) {
         const Digit32 D{X + (i64)k0 * ldx, ldx, m, std::min(kc, K - k0), work.p};
         int rc = (prepare || K > DIGIT32_CHUNK) ? launch_digits32(D, status, s) : OOC_OK;
@@ -1380,28 +1395,14 @@ int syrk_f32(int prec, const float* X, i64 ldx, float* C, i64 ldc, int m, int K,
       }
       return OOC_OK;
     }
-  }
-  if (prec == OOC_PREC_FP32) {
     const i64 T = ((i64)m + FB - 1) / FB;
     const i64 hi = std::min<i64>(bj_hi < 0 ? T : bj_hi, T);
     if (bj_lo >= hi) return OOC_OK;
     const i64 nblk = ooc_lower_blocks_before(hi, T) - ooc_lower_blocks_before(bj_lo, T);
     if (nblk > 0x7fffffff) return OOC_ERR_INTERNAL;
-    // k_syrk_f32 stages X with 16-byte copies: a panel whose base or leading dimension is
-    // not 16-byte compatible is first copied to an aligned buffer (once per panel).
-    const float* Xs = X;
-    i64 lds = ldx;
-    if ((reinterpret_cast<uintptr_t>(X) % 16) != 0 || (ldx % 4) != 0) {
-      lds = ((i64)m + 3) / 4 * 4;
-      if (prepare) {
-        int rc = work.ensure((size_t)lds * K * sizeof(float));
-        if (rc) return rc;
-        k_copy_f32<<<dim3((unsigned)((m + 255) / 256), (unsigned)std::min(K, 1024)), 256, 0, s>>>(X, ldx, (float*)work.p,
-                                                                                              lds, m, K);
-      }
-      Xs = (const float*)work.p;
-    }
-    k_syrk_f32<float><<<(unsigned)nblk, FTHR, 0, s>>>(Xs, lds, C, ldc, m, K, (int)T, bj_lo, status);
+    const bool copied = *way == Syrk32Way::kCopied;
+    k_syrk_f32<float><<<(unsigned)nblk, FTHR, 0, s>>>(copied ? (const float*)work.p : X, copied ? lds : ldx, C, ldc, m, K,
+                                                      (int)T, bj_lo, status);
     OOC_CUDA_TRY(cudaGetLastError());
     return OOC_OK;
   }
@@ -2184,16 +2185,18 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
       }
       float* C = A + (J0 + LN) * (1 + lda);
       const i64 G0 = J0 / nb * nb, G1 = std::min<i64>(G0 + nb, n);  // the panel's tile
+      Syrk32Way way = Syrk32Way::kNone;                             // of the updates below
       if (grouped && J0 + LN < G1) {  // the rest of the tile
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, (int)((G1 - J0 - LN + 127) / 128));
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
       } else if (grouped) {  // everything right of the tile, the next panel first
         float* Xg = A + G1 + G0 * lda;
-        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, 0, bjn, 1, 0);
+        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, 0, bjn, 1, 0, &way);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
-        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, bjn, -1, 0, kChainSMs);
+        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, bjn, -1, 0, kChainSMs,
+                      &way);
       } else if (tc_solve) {  // the planes come from the solve
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 0, 0);
         if (rc) return rc;
@@ -2205,10 +2208,10 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
         }
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, bjn, -1, 0, kChainSMs);
       } else if (split) {
-        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 1, 0);
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 1, 0, &way);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
-        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, bjn, -1, 0, kChainSMs);
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, bjn, -1, 0, kChainSMs, &way);
       } else {
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work);
         if (rc) return rc;

@@ -1,0 +1,77 @@
+"""The FP32 trailing update's choice between digit planes and the FP32 pipe (syrk32_way.h), on the host with a buffer
+whose growth can be made to fail: a panel's later block-column ranges follow the choice made when it was prepared, so planes
+that found no room are never read."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "oocdag_gb300", "csrc")
+
+PROGRAM = r"""
+#include "syrk32_way.h"
+#include <cstdio>
+#include <initializer_list>
+struct Buf {
+  size_t limit, bytes = 0;
+  int ensure(size_t b) {  // like a device buffer: a failed growth leaves none
+    if (b <= bytes) return 0;
+    bytes = 0;
+    if (b > limit) return -5;
+    bytes = b;
+    return 0;
+  }
+};
+int main() {
+  const size_t digits = 4096, copy = 2048;
+  for (size_t limit : {(size_t)0, copy, digits})
+    for (int serve = 0; serve < 2; serve++)
+      for (int aligned = 0; aligned < 2; aligned++) {
+        Buf b{limit};
+        Syrk32Way way = Syrk32Way::kNone;
+        const int rc = syrk32_choose(b, serve, digits, aligned, copy, &way);
+        printf("%zu %d %d: %d %d %zu\n", limit, serve, aligned, rc, (int)way, b.bytes);
+      }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def table(tmp_path_factory):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if not cxx:
+        pytest.skip("no C++ compiler")
+    d = tmp_path_factory.mktemp("way")
+    (d / "t.cpp").write_text(PROGRAM)
+    subprocess.run([cxx, "-std=c++17", "-I" + CSRC, str(d / "t.cpp"), "-o", str(d / "t")], check=True)
+    out = subprocess.run([str(d / "t")], check=True, capture_output=True, text=True).stdout
+    rows = [line.split(": ") for line in out.strip().splitlines()]
+    return {tuple(map(int, k.split())): tuple(map(int, v.split())) for k, v in rows}
+
+
+NONE, DIRECT, COPIED, DIGITS = range(4)
+
+
+def test_every_choice(table):
+    assert len(table) == 12
+    for (limit, serve, aligned), (rc, way, held) in table.items():
+        if serve and limit >= 4096:
+            want = (0, DIGITS, 4096)
+        elif aligned:
+            want = (0, DIRECT, 0)
+        elif limit >= 2048:
+            want = (0, COPIED, 2048)
+        else:
+            want = (-5, NONE, 0)
+        assert (rc, way, held) == want, (limit, serve, aligned)
+
+
+def test_later_ranges_take_the_prepared_way():
+    """Every syrk_f32 call without preparation on an FP32 panel passes the way of the call that prepared it."""
+    text = open(os.path.join(CSRC, "mixed.cu")).read()
+    body = text[text.index("int factor_f32(ooc_factor* F") : text.index("int factor_f32_lb(")]
+    for branch in ("} else if (grouped) {", "} else if (split) {"):
+        part = body[body.index(branch) + len(branch) :]
+        part = part[: part.index("} else")]
+        assert part.count("syrk_f32(") == 2 and part.count("&way)") == 2
