@@ -175,8 +175,9 @@ int g_device = 0;
 std::mutex g_mu;
 struct Slot {
   cudaStream_t s = nullptr;
-  int* status = nullptr;
-  std::mutex mu;   // held by a call that uses ws until its work is done
+  int* status = nullptr;  // of dpotrf and dtrsm
+  int* prod = nullptr;    // of the tensor-core products (another thread's factorization may be under way)
+  std::mutex mu;   // held by a call that uses ws and prod until its work is done
   GrowBuf ws;      // digit planes of the tensor-core products, kept across calls
 };
 Slot g_slot[MAX_R];
@@ -192,11 +193,12 @@ Slot* slot(int r) {
   Slot& sl = g_slot[r];
   if (!sl.s) {
     if (cudaStreamCreateWithFlags(&sl.s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&sl.status, sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&sl.status, 2 * sizeof(int)) != cudaSuccess) {
       cudaGetLastError();
       t_err = OOC_ERR_CUDA;
       return nullptr;
     }
+    sl.prod = sl.status + 1;
   }
   return &sl;
 }
@@ -233,20 +235,20 @@ int gemm_general(Slot* sl, const double* A, i64 sar, i64 sak, const double* B, i
     const size_t sa = up(digit_plane_bytes(m, kp)), sb = up(digit_plane_bytes(n, kp));
     if (sl->ws.ensure((sa + sb) * runs) == OOC_OK) {
       int rc = OOC_OK;
-      cudaMemsetAsync(sl->status, 0, sizeof(int), s);
+      cudaMemsetAsync(sl->prod, 0, sizeof(int), s);
       const bool same = A == B && sar == sbr && sak == sbk && m == n;  // a symmetric product
       for (int k0 = 0; k0 < k && !rc; k0 += runs * DIGIT_K) {
         const int K = std::min(runs * DIGIT_K, k - k0);
         // element (r, k) at r * sr + k * sk: "tiles" of one row
         DigitRuns Da{A + k0 * sak, sak, sar, 1, 0, m, K, sl->ws.p, sa, {}};
         DigitRuns Db{B + k0 * sbk, sbk, sbr, 1, 0, n, K, (char*)sl->ws.p + sa * runs, sb, {}};
-        rc = launch_digits(Da, sl->status, s);
+        rc = launch_digits(Da, sl->prod, s);
         if (same) Db = Da;
-        else if (!rc) rc = launch_digits(Db, sl->status, s);
-        if (!rc) rc = launch_digit_gemm(Da, Db, C, ldc, alpha, k0 == 0 ? beta : 1.0, mask, sl->status, s);
+        else if (!rc) rc = launch_digits(Db, sl->prod, s);
+        if (!rc) rc = launch_digit_gemm(Da, Db, C, ldc, alpha, k0 == 0 ? beta : 1.0, mask, sl->prod, s);
       }
       int st = 0;
-      cudaMemcpyAsync(&st, sl->status, sizeof(int), cudaMemcpyDeviceToHost, s);
+      cudaMemcpyAsync(&st, sl->prod, sizeof(int), cudaMemcpyDeviceToHost, s);
       const int frc = finish(s);
       if (rc || frc || st) t_err = rc ? rc : frc ? frc : OOC_ERR_TIMEOUT;
       return rc ? rc : frc;
@@ -285,7 +287,7 @@ extern "C" void offload_destroy(void) {
   cudaSetDevice(g_device);
   for (Slot& sl : g_slot) {
     if (sl.s) { cudaStreamSynchronize(sl.s); cudaStreamDestroy(sl.s); sl.s = nullptr; }
-    if (sl.status) { cudaFree(sl.status); sl.status = nullptr; }
+    if (sl.status) { cudaFree(sl.status); sl.status = sl.prod = nullptr; }
     sl.ws.release();
   }
 }
