@@ -11,9 +11,10 @@
  *     every call returns when its work on that stream has finished, as the reference's
  *     offload regions did;
  *   - the BLAS/LAPACK calls run the library's own sm_103a kernels (FP64 contraction by
- *     exact digit products on the tensor cores or DMMA, device potrf, blocked column solve); no
- *     cuBLAS/cuSOLVER.  A product's error is relative to the largest element of its operand
- *     rows per 128 columns of k, at or below that of an FP64 sum over them.
+ *     digit products on the tensor cores or DMMA, device potrf, blocked column solve); no
+ *     cuBLAS/cuSOLVER.  A product's error is bounded like that of an FP64 sum, by a multiple of
+ *     2^-53 sum |a| |b|: the tensor cores take operands whose rows are even in size (at most
+ *     2^-43 sum |a| |b|, and less than an FP64 sum's error for uniform or normal values), DMMA the others.
  * MKL_INT is the LP64 int.  All functions have C linkage (the reference's were C++ except
  * offload_init_/offload_destroy_).  Errors: the BLAS-style calls return void as in the
  * reference; ooc_offload_last_error() reports the last failure (0 = none).

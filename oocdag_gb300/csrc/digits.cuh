@@ -19,8 +19,8 @@ __device__ __forceinline__ unsigned long long digit_fixed(unsigned long long b, 
   const int be = (int)((b >> 52) & 0x7FF);
   unsigned long long m = b & 0xFFFFFFFFFFFFFull;
   if (be) m |= 1ull << 52;
-  const int sh = max(be, 1) - 1020 + shift;  // X = m 2^sh, sh <= 2
-  if (sh >= 0) m <<= min(sh, 2);
+  const int sh = max(be, 1) - 1020 + shift;  // X = m 2^sh < 2^55: sh <= 2 but for subnormal elements
+  if (sh >= 0) m <<= min(sh, 63);
   else m = sh < -55 ? 0ull : (m + (1ull << (-sh - 1))) >> (-sh);
   return ((b >> 63) ? 0ull - m : m) + 0x0080808080808080ull;
 }

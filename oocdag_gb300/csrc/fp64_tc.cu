@@ -22,6 +22,18 @@
 // plain bulk copies without tensor maps; k_digit_update is the update.
 //
 // An element whose row or column of X holds an infinity or NaN takes the plain FP64 sum.
+//
+// Operands that are not a Cholesky factor's panels are checked first (DigitCheck).  What digits lose is
+// relative to the largest elements of the two rows, what an FP64 sum loses to sum |a| |b|, which may be far less:
+// operands graded along k in opposite directions, (A D)(D^-1 B), meet large with small throughout.  So k_digits notes, for
+// each row and run, which elements are within 2^-5 of the row's scale 2^e, and which columns are not all zero;
+// k_uneven counts.  If both rows have 5/8 of the columns that matter (not all zero in either operand) there, at
+// least a quarter of these have a product of at least 2^(e(i) + e(j) - 10), so the loss, 2^-55 of 2^(e(i) + e(j)) per
+// column, stays below 2^-43 of sum |a| |b| whatever the values; for uniform and normal ones it is below what an FP64
+// sum rounds off.  A last run of at most 32 columns is too short to count: its rows have to be within a
+// factor of 2 of the run before it, whose sum then covers its loss.  Where a row fails, the FP64 pipe takes the product.
+// 2^-5 and 5/8: of 128 normally distributed elements 80 % or more are that large; a row that is mostly zeros, or a
+// few large elements, fails.
 
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -70,12 +82,22 @@ struct DigitArgs {
   int nb, rows, K, ksign, sym;
   const int* kshift;
   const int* only_if;
+  DigitCheck chk;
   uint8_t* planes;
   size_t slot;
 };
+constexpr int WIDE_BITS = 5;   // "large": at least 2^-5 of the row's scale
+constexpr int SHORT_RUN = 32;  // columns of a run that is compared with the one before it
 
-// SHIFT: exponents moved by kshift, and symmetric operands.
-template <bool SHIFT>
+// 1023 + the exponent of the nonzero finite element with bits b, counting a subnormal's leading zeros.
+__device__ __forceinline__ int true_exponent(unsigned long long b) {
+  const int be = (int)((b >> 52) & 0x7FF);
+  return be ? be : 12 - __clzll((long long)(b << 12 >> 12));
+}
+
+// SHIFT: exponents moved by kshift, and symmetric operands.  CHECK: the rows' large elements and the nonzero columns
+// are noted.
+template <bool SHIFT, bool CHECK>
 __device__ __forceinline__ void digit_rows(const DigitArgs& a, int run) {
   constexpr int KT = 8;  // columns per thread
   __shared__ int smax[DIGIT_K / DK][32];
@@ -109,7 +131,7 @@ __device__ __forceinline__ void digit_rows(const DigitArgs& a, int run) {
 #pragma unroll
   for (int k = 0; k < KT; k++) {
     const int be = (int)((v[k] >> 52) & 0x7FF);
-    if (v[k] << 1) bmax = max(bmax, max(be, 1) + (SHIFT ? sft[SHIFT ? k : 0] : 0));
+    if (v[k] << 1) bmax = max(bmax, (CHECK ? true_exponent(v[k]) : max(be, 1)) + (SHIFT ? sft[SHIFT ? k : 0] : 0));
     finite = finite && be != 0x7FF;
   }
   if (!finite) bmax = EXP_NONFINITE;
@@ -122,6 +144,21 @@ __device__ __forceinline__ void digit_rows(const DigitArgs& a, int run) {
   for (int q = 0; q < DIGIT_K / DK; q++) bmax = max(bmax, smax[q][rl]);
   const int e = bmax < -(1 << 19) ? 0 : bmax - 1022;  // |x| < 2^e (a row of zeros: any scale)
   if (st == 0 && ch == 0) exps[row] = bmax >= EXP_NONFINITE ? EXP_NONFINITE : e;
+  if constexpr (CHECK) {
+    uint32_t large = 0, some = 0;
+#pragma unroll
+    for (int k = 0; k < KT; k++)
+      if (v[k] << 1) {
+        some |= 1u << (KT * ch + k);
+        if (true_exponent(v[k]) + (SHIFT ? sft[SHIFT ? k : 0] : 0) > bmax - WIDE_BITS) large |= 1u << (KT * ch + k);
+      }
+    if (bmax >= EXP_NONFINITE) large = ~0u;  // (plain sums: nothing to lose)
+    large |= __shfl_xor_sync(0xffffffffu, large, 1);
+    large |= __shfl_xor_sync(0xffffffffu, large, 2);
+    if (ch == 0) a.chk.large[((i64)run * (gridDim.x * 32) + row) * (DIGIT_K / DK) + st] = large;
+    some = __reduce_or_sync(0xffffffffu, some);
+    if (lane == 0 && some) atomicOr(a.chk.cols + run * (DIGIT_K / DK) + st, some);
+  }
   if (st >= nst) return;
   unsigned long long x[KT];
 #pragma unroll
@@ -132,13 +169,52 @@ __device__ __forceinline__ void digit_rows(const DigitArgs& a, int run) {
   put_digits<0>(x, planes + ((i64)(row >> 7) * nst + st) * UNIT_STAGE + (row & 127) * 64 + ((ch ^ ((row >> 1) & 3)) << 4),
                 A_DIG);
 }
-template <bool SHIFT>
+template <bool SHIFT, bool CHECK>
 __global__ void __launch_bounds__(512) k_digits(const __grid_constant__ DigitArgs a, const int* status) {
   pdl_wait();
   if (status && *(volatile const int*)status) return;
   if (SHIFT && a.only_if && !*(volatile const int*)a.only_if) return;
-  for (int run = blockIdx.y; run * DIGIT_K < a.K; run += gridDim.y) digit_rows<SHIFT>(a, run);
+  for (int run = blockIdx.y; run * DIGIT_K < a.K; run += gridDim.y) digit_rows<SHIFT, CHECK>(a, run);
 }
+
+// Raises *wide where a row of A or B (blockIdx.z) is too uneven in run blockIdx.y.
+struct UnevenArgs {
+  const uint32_t* large[2];
+  const int* exps[2];  // the first run's; `step` ints to the next one's, but the last run's sit at last_exps
+  size_t step[2];
+  const int* last_exps[2];
+  const uint32_t* cols[2];
+  int rows[2], pad[2];
+  int nrun, K;
+  int* wide;
+};
+__global__ void __launch_bounds__(128) k_uneven(const __grid_constant__ UnevenArgs a) {
+  pdl_wait();
+  constexpr int W = DIGIT_K / DK;
+  const int row = blockIdx.x * 128 + threadIdx.x, run = blockIdx.y, z = blockIdx.z;
+  if (row >= a.rows[z]) return;
+  auto words = [&](int q) { return reinterpret_cast<const uint4*>(a.large[z])[(i64)q * a.pad[z] + row]; };
+  const uint4 l = words(run);
+  if (!(l.x | l.y | l.z | l.w)) return;  // a row of zeros
+  bool ok;
+  if (run > 0 && a.K - run * DIGIT_K <= SHORT_RUN) {
+    const uint4 b = words(run - 1);
+    ok = (b.x | b.y | b.z | b.w) && a.last_exps[z][row] <= a.exps[z][(run - 1) * a.step[z] + row] + 1;
+    ok = ok || a.last_exps[z][row] == EXP_NONFINITE;
+  } else {
+    const uint32_t lw[W] = {l.x, l.y, l.z, l.w};
+    int n = 0, c = 0;
+#pragma unroll
+    for (int q = 0; q < W; q++) {
+      const uint32_t both = a.cols[0][run * W + q] & a.cols[1][run * W + q];
+      n += __popc(both);
+      c += __popc(lw[q] & both);
+    }
+    ok = 8 * c >= 5 * n;
+  }
+  if (!ok) *a.wide = 1;
+}
+static_assert(DIGIT_K / DK == 4, "a row's large elements in a run: one uint4");
 
 // ---- update ----------------------------------------------------------------------
 // One product shape throughout: M = 128 rows, N = 64 columns, K = 16, each MMA adding into
@@ -165,6 +241,7 @@ struct UpdateArgs {
   Operand a, b;                       // rows and columns of C
   int nst[DIGIT_RUNS];                // a run's stages of DK columns (general products: 4, but in the last)
   int nrun, K;
+  const int* unless;                  // nothing is done where this word is not 0 (may be null)
   double alpha, beta;                 // general products only
   int mask;
 };
@@ -244,7 +321,7 @@ __global__ void __launch_bounds__(D_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
   const uint32_t tmem = *tmem_slot;
   pdl_wait();  // (the set-up above touches no other kernel's data)
-  if (*(volatile int*)status) nblk = 0;
+  if (*(volatile int*)status || (X.unless && *(volatile const int*)X.unless)) nblk = 0;
   auto run_stages = [&](int run) {
     return MODE == UPDATE ? X.nst[run] : run + 1 < X.nrun ? DIGIT_K / DK : (X.K - run * DIGIT_K + DK - 1) / DK;
   };
@@ -472,16 +549,46 @@ int launch_digits(DigitRuns& X, const int* status, cudaStream_t s) {
   if (X.rows > (1 << 30) || nrun > 65535) return OOC_ERR_INTERNAL;
   for (int q = 0; q < std::min(nrun, DIGIT_RUNS); q++) X.org_of[q] = X.org;
   const DigitArgs a{X.X, X.ldx, X.stride, X.org, X.k0, X.sym ? 1 : X.nb, (int)X.rows, X.K, X.ksign, X.sym, X.kshift, X.only_if,
-                    (uint8_t*)X.planes, X.slot};
+                    X.chk, (uint8_t*)X.planes, X.slot};
   const unsigned gx = 4 * (unsigned)((X.rows + DR - 1) / DR);
   // planes that are seldom rewritten: few CTAs of many runs, since 65536 that only look at the word take 0.5 ms
   const dim3 grid(gx, X.only_if ? std::min<unsigned>(nrun, std::max(1u, 2432 / gx)) : nrun);
-  if (X.sym || X.kshift) {
-    if (!X.kshift) return OOC_ERR_INTERNAL;
-    OOC_CUDA_TRY(launch_pdl(k_digits<true>, grid, 512, 0, s, a, status));
-  } else {
-    OOC_CUDA_TRY(launch_pdl(k_digits<false>, grid, 512, 0, s, a, status));
+  const bool check = X.chk.large != nullptr;
+  if (X.sym && (!X.kshift || check)) return OOC_ERR_INTERNAL;
+  auto* kernel = X.kshift ? (check ? k_digits<true, true> : k_digits<true, false>)
+                          : (check ? k_digits<false, true> : k_digits<false, false>);
+  OOC_CUDA_TRY(launch_pdl(kernel, grid, 512, 0, s, a, status));
+  return OOC_OK;
+}
+
+size_t digit_check_bytes(i64 rows, int K) {
+  return (size_t)((rows + DR - 1) / DR) * DR * ((K + DIGIT_K - 1) / DIGIT_K) * sizeof(uint4);
+}
+size_t digit_cols_bytes(int K) { return (size_t)((K + DIGIT_K - 1) / DIGIT_K) * sizeof(uint4); }
+
+int launch_digit_check(const DigitRuns& A, const DigitRuns& B, cudaStream_t s) {
+  const int nrun = (A.K + DIGIT_K - 1) / DIGIT_K;
+  if (A.rows <= 0 || B.rows <= 0 || nrun <= 0) return OOC_OK;
+  if (!A.chk.large || !B.chk.large || A.chk.wide != B.chk.wide || A.K != B.K || nrun > 65535) return OOC_ERR_INTERNAL;
+  const bool same = A.chk.large == B.chk.large;
+  UnevenArgs a{};
+  for (int z = 0; z < 2; z++) {
+    const DigitRuns& X = z ? B : A;
+    const size_t units = (size_t)((X.rows + DR - 1) / DR);
+    const int last = (X.K - (nrun - 1) * DIGIT_K + DK - 1) / DK;
+    a.large[z] = X.chk.large;
+    a.cols[z] = X.chk.cols;
+    a.exps[z] = (const int*)((const uint8_t*)X.planes + units * (nrun > 1 ? DIGIT_K / DK : last) * UNIT_STAGE);
+    a.step[z] = X.slot / sizeof(int);
+    a.last_exps[z] = (const int*)((const uint8_t*)X.planes + (size_t)(nrun - 1) * X.slot + units * last * UNIT_STAGE);
+    a.rows[z] = (int)X.rows;
+    a.pad[z] = (int)(units * DR);
   }
+  a.nrun = nrun;
+  a.K = A.K;
+  a.wide = A.chk.wide;
+  const unsigned gx = (unsigned)((std::max(A.rows, same ? A.rows : B.rows) + 127) / 128);
+  OOC_CUDA_TRY(launch_pdl(k_uneven, dim3(gx, nrun, same ? 1 : 2), 128, 0, s, a));
   return OOC_OK;
 }
 
@@ -538,6 +645,7 @@ int launch_digit_update(const DigitRuns& X, const TileMap& C, i64 c_lo, i64 c_hi
   a.b = a.a;
   a.nrun = (X.K + DIGIT_K - 1) / DIGIT_K;
   a.K = X.K;
+  a.unless = X.chk.wide;
   const int T = (int)((X.rows + DC - 1) / DC), lo = (int)(c_lo / DC), hi = (int)((c_hi + DC - 1) / DC);
   return launch_blocks<UPDATE>(a, C, T, lo, hi, count_blocks2(T, lo, hi), const_cast<int*>(status), s, reserve_sms);
 }
@@ -552,6 +660,7 @@ int launch_digit_gemm(const DigitRuns& A, const DigitRuns& B, double* C, i64 ldc
   if (rc) return rc;
   a.nrun = (A.K + DIGIT_K - 1) / DIGIT_K;
   a.K = A.K;
+  a.unless = A.chk.wide;
   a.alpha = alpha;
   a.beta = beta;
   a.mask = mask;

@@ -1,10 +1,22 @@
 // FP64 updates on the tensor cores by exact digit products (fp64_tc.cu).
 #pragma once
 
+#include <cstdint>
+
 #include "common.cuh"
 
 constexpr int DIGIT_K = 128;    // columns of X per run (one exponent per row and run)
 constexpr int DIGIT_RUNS = 4;   // most runs an update sums before it rounds into C
+
+// Notes of an operand whose values are not known to suit digits (fp64_tc.cu): which elements of a row are large
+// (digit_check_bytes(rows, K)), which columns are not all zero (digit_cols_bytes(K), zeroed before launch_digits), and the word that
+// launch_digit_check raises (to 1, never lowers) where the rows are too uneven for a product to be as
+// accurate as an FP64 sum; an update with such an operand then does nothing.
+struct DigitCheck {
+  uint32_t* large = nullptr;
+  uint32_t* cols = nullptr;
+  int* wide = nullptr;
+};
 
 // Runs of at most DIGIT_K columns of a column of tiles: element (r, k), r = org .. org + rows - 1,
 // k < K, of run q sits at X + (r / nb) * stride + r % nb + (q DIGIT_K + k) * ldx (stride = nb for a plain
@@ -26,6 +38,7 @@ struct DigitRuns {
   int sym = 0;
   i64 k0 = 0;
   const int* only_if = nullptr;  // planes are rewritten only where this word is not 0 (with kshift)
+  DigitCheck chk;  // (launch_digit_update's operands as well)
 };
 
 // Bytes of the digit planes and row exponents of `rows` rows of K columns.
@@ -34,6 +47,11 @@ size_t digit_plane_bytes(i64 rows, int K);
 // The planes of every run of X for rows org.. (sets org_of; any number of runs for
 // launch_digit_gemm, at most DIGIT_RUNS for launch_digit_update).
 int launch_digits(DigitRuns& X, const int* status, cudaStream_t s);
+
+size_t digit_check_bytes(i64 rows, int K);
+size_t digit_cols_bytes(int K);
+// After launch_digits of both operands of a product (the same one twice for a symmetric product), org 0.
+int launch_digit_check(const DigitRuns& A, const DigitRuns& B, cudaStream_t s);
 
 // C(org + r, org + c) -= sum over the runs of X(r) X(c)^T, for r < rows, c in [c_lo, c_hi), r >= c, after
 // launch_digits: one rounding into C per call.  64 divides C.nb, org and c_lo; columns are

@@ -3375,15 +3375,27 @@ extern "C" int ooc_dsyrk_ln(ooc_handle* h, int prec, int n, int k, const double*
   cudaMemsetAsync(status, 0, sizeof(int), s);
   DevBuf work;
   int rc;
+  const int group = std::min(k, DIGIT_RUNS * DIGIT_K);
   const size_t slot = (digit_plane_bytes(n, std::min(k, DIGIT_K)) + 255) / 256 * 256;
-  if (prec == OOC_PREC_FP64 && n > 64 && k >= 16 && !work.ensure(slot * std::min(DIGIT_RUNS, (k + DIGIT_K - 1) / DIGIT_K))) {
-    // digit products on the tensor cores (from one block and half a stage on: fp64_tc.cu)
+  const size_t planes = slot * ((group + DIGIT_K - 1) / DIGIT_K), notes = digit_check_bytes(n, group), cols = digit_cols_bytes(k);
+  if (prec == OOC_PREC_FP64 && n > 64 && k >= 16 && !work.ensure(planes + notes + cols + 256)) {
+    // digit products on the tensor cores (from one block and half a stage on: fp64_tc.cu); the columns from
+    // the first group on in which the caller's rows are too uneven for them on the FP64 pipe
     const int nb = (n + 63) / 64 * 64;  // one tile
+    char* base = (char*)work.p;
+    int* flag = (int*)(base + planes + notes + cols);
+    int wide = 0;
+    cudaMemsetAsync(base + planes + notes, 0, cols + 256, s);
     rc = OOC_OK;
-    for (int k0 = 0; k0 < k && !rc; k0 += DIGIT_RUNS * DIGIT_K) {
-      DigitRuns D{A + (i64)k0 * lda, lda, nb, nb, 0, n, std::min(DIGIT_RUNS * DIGIT_K, k - k0), work.p, slot, {}};
+    for (int k0 = 0; k0 < k && !rc && !wide; k0 += DIGIT_RUNS * DIGIT_K) {
+      const double* Ak = A + (i64)k0 * lda;
+      DigitRuns D{Ak, lda, nb, nb, 0, n, std::min(DIGIT_RUNS * DIGIT_K, k - k0), base, slot, {}};
+      D.chk = DigitCheck{(uint32_t*)(base + planes), (uint32_t*)(base + planes + notes + digit_cols_bytes(k0)), flag};
       rc = launch_digits(D, status, s);
+      if (!rc) rc = launch_digit_check(D, D, s);
       if (!rc) rc = launch_digit_update(D, TileMap{C, ldc, 0, 1, nb}, 0, n, status, s);
+      if (!rc) rc = read_int(flag, &wide, s);
+      if (!rc && wide) rc = launch_gemm_nt(Ak, lda, Ak, lda, C, ldc, n, n, k - k0, 1, -1.0, status, s);
     }
   } else if (prec == OOC_PREC_FP64) {
     rc = launch_gemm_nt(A, lda, A, lda, C, ldc, n, n, k, 1, -1.0, status, s);

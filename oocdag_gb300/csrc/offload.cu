@@ -52,7 +52,8 @@ __device__ __forceinline__ void load_strided(double* S, const double* M, i64 sr,
 __global__ void __launch_bounds__(GTHR) k_gemm_general(const double* __restrict__ A, i64 sar, i64 sak,
                                                        const double* __restrict__ B, i64 sbr, i64 sbk,
                                                        double* __restrict__ C, i64 ldc, int m, int n, int k,
-                                                       double alpha, double beta, int mask) {
+                                                       double alpha, double beta, int mask, const int* only_if) {
+  if (only_if && !*(volatile const int*)only_if) return;
   __shared__ __align__(16) double As[GBK * GLDS];
   __shared__ __align__(16) double Bs[GBK * GLDS];
   const int mblocks = (m + GBM - 1) / GBM;
@@ -176,9 +177,9 @@ std::mutex g_mu;
 struct Slot {
   cudaStream_t s = nullptr;
   int* status = nullptr;  // of dpotrf and dtrsm
-  int* prod = nullptr;    // of the tensor-core products (another thread's factorization may be under way)
-  std::mutex mu;   // held by a call that uses ws and prod until its work is done
-  GrowBuf ws;      // digit planes of the tensor-core products, kept across calls
+  std::mutex mu;   // held by a call that uses ws until its work is done
+  GrowBuf ws;      // of the tensor-core products, kept across calls: their own status (another thread's
+                   // factorization may be under way), notes on the operands, digit planes
 };
 Slot g_slot[MAX_R];
 thread_local int t_err = 0;
@@ -193,12 +194,11 @@ Slot* slot(int r) {
   Slot& sl = g_slot[r];
   if (!sl.s) {
     if (cudaStreamCreateWithFlags(&sl.s, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaMalloc(&sl.status, 2 * sizeof(int)) != cudaSuccess) {
+        cudaMalloc(&sl.status, sizeof(int)) != cudaSuccess) {
       cudaGetLastError();
       t_err = OOC_ERR_CUDA;
       return nullptr;
     }
-    sl.prod = sl.status + 1;
   }
   return &sl;
 }
@@ -216,8 +216,9 @@ int finish(cudaStream_t s) {
 
 // C = alpha opA opB^T + beta C (see k_gemm_general) on the slot's stream, done when it returns.
 // Tensor-core digit products (fp64_tc.cu) from DIGIT_PRODUCTS on: a 256 x 256 x 256 product
-// takes 43 us with its digits against 332 us on the FP64 pipe; below, or without room
-// for the planes, FP64 MMAs.
+// takes 43 us with its digits against 332 us on the FP64 pipe, and 9 us more for the check of
+// its operands; below, without room for the planes, or for the columns of operands whose
+// rows are too uneven, FP64 MMAs.
 constexpr double DIGIT_PRODUCTS = 128.0 * 128.0 * 128.0;
 int gemm_general(Slot* sl, const double* A, i64 sar, i64 sak, const double* B, i64 sbr, i64 sbk, double* C, i64 ldc,
                  int m, int n, int k, double alpha, double beta, int mask) {
@@ -228,34 +229,51 @@ int gemm_general(Slot* sl, const double* A, i64 sar, i64 sak, const double* B, i
       k_scale<<<dim3((m + 255) / 256, std::min(n, 4096)), 256, 0, s>>>(C, ldc, m, n, beta, mask);
     return finish(s);
   }
+  // columns [k0, k0 + K) on the FP64 pipe (where *only_if is not 0)
+  auto on_fp64_pipe = [&](int k0, int K, const int* only_if) {
+    const int mb = (m + GBM - 1) / GBM, nbk = (n + GBM - 1) / GBM;
+    k_gemm_general<<<mb * nbk, GTHR, 0, s>>>(A + k0 * sak, sar, sak, B + k0 * sbk, sbr, sbk, C, ldc, m, n, K, alpha,
+                                             k0 == 0 ? beta : 1.0, mask, only_if);
+  };
   if ((double)m * n * k >= DIGIT_PRODUCTS) {
     std::lock_guard<std::mutex> lk(sl->mu);
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     const int kp = std::min(k, DIGIT_K), runs = std::min(DIGIT_RUNS, (k + DIGIT_K - 1) / DIGIT_K);
     const size_t sa = up(digit_plane_bytes(m, kp)), sb = up(digit_plane_bytes(n, kp));
-    if (sl->ws.ensure((sa + sb) * runs) == OOC_OK) {
+    // status and wide words, the columns' notes (zeroed), the rows' notes, the planes
+    const size_t cols = up(digit_cols_bytes(k)), zeroed = 256 + 2 * cols;
+    const size_t la = up(digit_check_bytes(m, std::min(k, DIGIT_RUNS * DIGIT_K)));
+    const size_t lb = up(digit_check_bytes(n, std::min(k, DIGIT_RUNS * DIGIT_K)));
+    if (sl->ws.ensure(zeroed + la + lb + (sa + sb) * runs) == OOC_OK) {
       int rc = OOC_OK;
-      cudaMemsetAsync(sl->prod, 0, sizeof(int), s);
+      char* base = (char*)sl->ws.p;
+      char* planes = base + zeroed + la + lb;
+      int* status = (int*)base;
+      cudaMemsetAsync(base, 0, zeroed, s);
       const bool same = A == B && sar == sbr && sak == sbk && m == n;  // a symmetric product
       for (int k0 = 0; k0 < k && !rc; k0 += runs * DIGIT_K) {
         const int K = std::min(runs * DIGIT_K, k - k0);
         // element (r, k) at r * sr + k * sk: "tiles" of one row
-        DigitRuns Da{A + k0 * sak, sak, sar, 1, 0, m, K, sl->ws.p, sa, {}};
-        DigitRuns Db{B + k0 * sbk, sbk, sbr, 1, 0, n, K, (char*)sl->ws.p + sa * runs, sb, {}};
-        rc = launch_digits(Da, sl->prod, s);
+        DigitRuns Da{A + k0 * sak, sak, sar, 1, 0, m, K, planes, sa, {}};
+        DigitRuns Db{B + k0 * sbk, sbk, sbr, 1, 0, n, K, planes + sa * runs, sb, {}};
+        const size_t co = digit_cols_bytes(k0);
+        Da.chk = DigitCheck{(uint32_t*)(base + zeroed), (uint32_t*)(base + 256 + co), status + 1};
+        Db.chk = DigitCheck{(uint32_t*)(base + zeroed + la), (uint32_t*)(base + 256 + cols + co), status + 1};
+        rc = launch_digits(Da, status, s);
         if (same) Db = Da;
-        else if (!rc) rc = launch_digits(Db, sl->prod, s);
-        if (!rc) rc = launch_digit_gemm(Da, Db, C, ldc, alpha, k0 == 0 ? beta : 1.0, mask, sl->prod, s);
+        else if (!rc) rc = launch_digits(Db, status, s);
+        if (!rc) rc = launch_digit_check(Da, Db, s);
+        if (!rc) rc = launch_digit_gemm(Da, Db, C, ldc, alpha, k0 == 0 ? beta : 1.0, mask, status, s);
+        if (!rc) on_fp64_pipe(k0, K, Da.chk.wide);
       }
       int st = 0;
-      cudaMemcpyAsync(&st, sl->prod, sizeof(int), cudaMemcpyDeviceToHost, s);
+      cudaMemcpyAsync(&st, status, sizeof(int), cudaMemcpyDeviceToHost, s);
       const int frc = finish(s);
       if (rc || frc || st) t_err = rc ? rc : frc ? frc : OOC_ERR_TIMEOUT;
       return rc ? rc : frc;
     }
   }
-  const int mb = (m + GBM - 1) / GBM, nbk = (n + GBM - 1) / GBM;
-  k_gemm_general<<<mb * nbk, GTHR, 0, s>>>(A, sar, sak, B, sbr, sbk, C, ldc, m, n, k, alpha, beta, mask);
+  on_fp64_pipe(0, k, nullptr);
   return finish(s);
 }
 
@@ -287,7 +305,7 @@ extern "C" void offload_destroy(void) {
   cudaSetDevice(g_device);
   for (Slot& sl : g_slot) {
     if (sl.s) { cudaStreamSynchronize(sl.s); cudaStreamDestroy(sl.s); sl.s = nullptr; }
-    if (sl.status) { cudaFree(sl.status); sl.status = sl.prod = nullptr; }
+    if (sl.status) { cudaFree(sl.status); sl.status = nullptr; }
     sl.ws.release();
   }
 }
