@@ -1150,13 +1150,16 @@ __global__ void k_colmax_abs(const double* V, i64 ld, int n, int r, double* out 
 // that all that a refinement's stopping rule needs is one launch, one small copy and one wait.
 // At n = 1000 and one right-hand side a refinement of two corrections takes 340 us, and 415 with a launch, a
 // copy of 152 partial maxima per column and a wait for each block.
+// The words at `flags` (may be null) go after them: out[gridDim.y RMAX] = flags[0], the next flags[1].
 struct ColMax {
   const double* V[4];
   i64 ld[4];
   int cols[4];
+  const int* flags;
 };
 __global__ void __launch_bounds__(1024) k_col_max(const ColMax a, int n, double* __restrict__ out) {
   const int q = blockIdx.x, w = blockIdx.y;
+  if (q == 0 && w == 0 && threadIdx.x < 2) out[gridDim.y * RMAX + threadIdx.x] = a.flags ? a.flags[threadIdx.x] : 0;
   if (q >= a.cols[w]) return;
   __shared__ double sm[32];
   const double* v = a.V[w] + (i64)q * a.ld[w];
@@ -1727,6 +1730,8 @@ __global__ void k_take_shift(const int* __restrict__ t_of, int* __restrict__ shi
 //   n = 3072                                                r = 2  0.40 / 0.42  0.33 / 0.28
 //   n = 2048   r = 5         0.72 / 0.41     0.64 / 0.29    r = 3  0.35 / 0.34  0.26 / 0.22  r = 2  0.32 / 0.33  0.25 / 0.24
 // One right-hand side has too few FMAs for the planes to pay.
+// The one shift per row suits solutions whose columns are of a kind.  Columns graded differently leave X 2^-shift
+// uneven in some column and run (fp64_tc.cu), which raises `wide`: the caller forms such a residual by symv_lower.
 bool symm_by_digits(i64 n, int r) { return r >= 2 && n >= (r == 2 ? 3072 : 2048); }
 constexpr size_t SYMM_KEEP = 16ull << 30, SYMM_CHUNK = 512ull << 20;
 struct SymmDigits {
@@ -1735,21 +1740,23 @@ struct SymmDigits {
   bool kept;      // ... which are all of them
   char *pa, *px;
   int *shift, *t_of, *cexp, *stale;
-  int* status;    // of the products
+  int* status;    // of the products; the word after it: X was too uneven for them
+  DigitCheck chk; // of X
 };
 // OOC_ERR_NOMEM without room for the planes.
 int symm_digits_begin(SymmDigits* D, DevBuf& buf, int n, int r, cudaStream_t s) {
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   D->sa = up(digit_plane_bytes(n, DIGIT_K));
   D->sx = up(digit_plane_bytes(r, DIGIT_K));
-  const size_t ints = up((size_t)n * 4);
   const int nrun = (n + DIGIT_K - 1) / DIGIT_K;
+  const size_t ints = up((size_t)n * 4), cols = up(digit_cols_bytes(n)), large = up(digit_check_bytes(r, n));
+  const size_t rest = 2 * ints + 512 + cols + large;
   int rc = OOC_ERR_NOMEM;
   D->kept = (D->sa + D->sx) * nrun <= SYMM_KEEP;
-  if (D->kept) rc = buf.ensure((D->sa + D->sx) * nrun + 2 * ints + 512);
+  if (D->kept) rc = buf.ensure((D->sa + D->sx) * nrun + rest);
   if (rc) D->kept = false;
   D->runs = D->kept ? nrun : (int)std::max<size_t>(1, std::min<size_t>(nrun, SYMM_CHUNK / (D->sa + D->sx)));
-  if (rc && buf.ensure((D->sa + D->sx) * D->runs + 2 * ints + 512)) return OOC_ERR_NOMEM;
+  if (rc && buf.ensure((D->sa + D->sx) * D->runs + rest)) return OOC_ERR_NOMEM;
   D->pa = (char*)buf.p;
   D->px = D->pa + D->sa * D->runs;
   D->shift = (int*)(D->px + D->sx * D->runs);
@@ -1757,8 +1764,9 @@ int symm_digits_begin(SymmDigits* D, DevBuf& buf, int n, int r, cudaStream_t s) 
   D->cexp = (int*)((char*)D->t_of + ints);
   D->stale = (int*)((char*)D->cexp + 256);
   D->status = D->stale + 1;
+  D->chk = DigitCheck{(uint32_t*)((char*)D->stale + 256 + cols), (uint32_t*)((char*)D->stale + 256), D->status + 1};
   OOC_CUDA_TRY(cudaMemsetAsync(D->stale, 1, sizeof(int), s));  // no planes yet
-  OOC_CUDA_TRY(cudaMemsetAsync(D->status, 0, sizeof(int), s));
+  OOC_CUDA_TRY(cudaMemsetAsync(D->status, 0, 2 * sizeof(int), s));
   return OOC_OK;
 }
 int symm_digits(const SymmDigits& D, const double* A, i64 lda, const double* X, i64 ldx, double* R, i64 ldr, int n, int r,
@@ -1768,13 +1776,17 @@ int symm_digits(const SymmDigits& D, const double* A, i64 lda, const double* X, 
   k_row_shift<<<g, 256, 0, s>>>(X, ldx, n, r, D.cexp, D.shift, D.t_of, D.stale);
   k_take_shift<<<g, 256, 0, s>>>(D.t_of, D.shift, n, D.stale);
   OOC_CUDA_TRY(cudaGetLastError());
+  OOC_CUDA_TRY(cudaMemsetAsync(D.chk.cols, 0, digit_cols_bytes(n), s));
   for (i64 c0 = 0; c0 < n; c0 += (i64)D.runs * DIGIT_K) {
     const int K = (int)std::min<i64>((i64)D.runs * DIGIT_K, n - c0);
     DigitRuns Da{A, lda, 0, 1, 0, n, K, D.pa, D.sa, {}, D.shift, 1, 1, c0, D.kept ? D.stale : nullptr};
     // (row q, column k) of the second operand is X(c0 + k, q)
     DigitRuns Dx{X + c0, 1, ldx, 1, 0, r, K, D.px, D.sx, {}, D.shift, -1, 0, c0};
+    Dx.chk = D.chk;
+    Dx.chk.cols += digit_cols_bytes((int)c0) / sizeof(uint32_t);
     int rc = launch_digits(Da, D.status, s);
     if (!rc) rc = launch_digits(Dx, D.status, s);
+    if (!rc) rc = launch_digit_check(Dx, Dx, s);
     if (!rc) rc = launch_digit_gemm(Da, Dx, R, ldr, -1.0, 1.0, 0, D.status, s);
     if (rc) return rc;
   }
@@ -3110,7 +3122,7 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
   // the factor's workspace (sized once for RMAX columns and kept across calls)
   const size_t bR = (size_t)n * RMAX * sizeof(double), bRf = ((size_t)n * RMAX * sizeof(float) + 255) / 256 * 256;
   const size_t bRows = ((size_t)n * sizeof(double) + 255) / 256 * 256;
-  if (F->rws.ensure(bR + bRf + bRows + 4 * RMAX * sizeof(double))) return OOC_ERR_NOMEM;
+  if (F->rws.ensure(bR + bRf + bRows + (4 * RMAX + 2) * sizeof(double))) return OOC_ERR_NOMEM;
   double* R = (double*)F->rws.p;
   float* Rf = (float*)((char*)F->rws.p + bR);
   double* rows = (double*)((char*)F->rws.p + bR + bRf);
@@ -3180,7 +3192,7 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
     }
     if (!rc && s2 != s && (cudaEventRecord(ev_in, s2) != cudaSuccess)) rc = OOC_ERR_CUDA;
   }
-  double hmax[4 * RMAX];                                 // the maxima of R, X, B and rows
+  double hmax[4 * RMAX + 2];                             // the maxima of R, X, B and rows, symm's status and wide words
   const double *nr = hmax, *nx = hmax + RMAX;
   std::vector<double> nb_(r);
   if (!rc && F->Lf) {  // X0 from the FP32 factor
@@ -3217,12 +3229,20 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
       if (rc) break;
     }
     const int blocks = it == 0 ? 4 : 2;  // (B's and A's norms once)
-    k_col_max<<<dim3(r, blocks), 1024, 0, s>>>(ColMax{{R, X, B, rows}, {n, ldx, ldb, n}, {r, r, r, 1}}, (int)n, red);
+    k_col_max<<<dim3(r, blocks), 1024, 0, s>>>(
+        ColMax{{R, X, B, rows}, {n, ldx, ldb, n}, {r, r, r, 1}, by_digits ? symm.status : nullptr}, (int)n, red);
     cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(hmax, red, blocks * RMAX * sizeof(double), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(hmax, red, (blocks * RMAX + 2) * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) { ooc_set_last_error(e, "refinement norms", __FILE__, __LINE__); rc = OOC_ERR_CUDA; break; }
     rc = ooc_wait_stream(h, s);
+    if (!rc && hmax[blocks * RMAX] != 0) rc = solve_status(1);
     if (rc) break;
+    if (hmax[blocks * RMAX + 1] != 0) {  // columns graded differently: this residual and the next ones on the FP64 pipe
+      by_digits = false;
+      F->dig.release();
+      continue;
+    }
     if (it == 0) {
       nb_.assign(hmax + 2 * RMAX, hmax + 2 * RMAX + r);
       normA = hmax[3 * RMAX];
@@ -3245,11 +3265,10 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
     }
     it++;
   }
-  int solve_err = 0, st = 0;
+  int solve_err = 0;
   if (!rc) rc = queue_solve_error(F->xch.p, &solve_err, s);
-  if (!rc && by_digits && cudaMemcpyAsync(&st, symm.status, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) rc = OOC_ERR_CUDA;
   if (!rc) rc = ooc_wait_stream(h, s);
-  if (!rc) rc = solve_status(solve_err | st);
+  if (!rc) rc = solve_status(solve_err);
   if (by_digits) {
     if (rc) cudaStreamSynchronize(s);
     F->dig.release();
