@@ -32,6 +32,7 @@
 
 #include "common.cuh"
 #include "devpool.cuh"
+#include "exchange_epoch.h"
 #include "fp32_tc.cuh"
 #include "fp64_tc.cuh"
 #include "syrk32_way.h"
@@ -1863,8 +1864,8 @@ struct ooc_factor {
   // Solves share the buffers above: calls on one factor from several threads take turns.
   std::mutex solve_mu;
   DevBuf rws;    // refinement workspace (residual, FP32 correction, reductions), kept
-  DevBuf xch;    // exchange buffer of the triangular solves, zeroed when allocated
-  unsigned epoch = 0;  // launches on it since then
+  DevBuf xch;    // exchange buffer of the triangular solves
+  ExchangeEpoch epoch;
   DevBuf dig;    // digit planes of A during a refinement
   DevBuf sws;    // FP32 right-hand sides of ooc_factor_solve on a reduced factor, kept
   DevBuf part2;  // partial sums of the refinement's norm (second stream)
@@ -1911,9 +1912,11 @@ int factor_solve(ooc_factor* F, T* B, i64 ldb, int r, cudaStream_t s) {
   const size_t need = trsolve_bytes(F->n, RMAX, sizeof(T));
   if (F->xch.bytes < need) {
     if (F->xch.ensure(need)) return OOC_ERR_NOMEM;
-    F->epoch = 0;
+    F->epoch.restart();
   }
-  if (F->epoch == 0) OOC_CUDA_TRY(cudaMemsetAsync(F->xch.p, 0, F->xch.bytes, s));
+  bool clear = false;
+  const unsigned tag = F->epoch.next(&clear);
+  if (clear) OOC_CUDA_TRY(cudaMemsetAsync(F->xch.p, 0, F->xch.bytes, s));
   const Panels P = F->panels();
   TriSolve<T> a{P.n, nullptr, P.n, nullptr, P.tail0, P.nb, P.nb2, B, ldb, r, 3};
   if constexpr (sizeof(T) == 4) {
@@ -1923,7 +1926,7 @@ int factor_solve(ooc_factor* F, T* B, i64 ldb, int r, cudaStream_t s) {
     a.L = F->L;
     a.Dinv = F->Dinv;
   }
-  return launch_trsolve<T>(a, F->xch.p, ++F->epoch, s);
+  return launch_trsolve<T>(a, F->xch.p, tag, s);
 }
 
 // Queues the read of a solve's error word; solve_status after the stream is done.
@@ -1936,6 +1939,13 @@ int solve_status(int err) {
   if (!err) return OOC_OK;
   ooc_set_last_message("triangular solve or residual: a bounded wait ran out");
   return OOC_ERR_TIMEOUT;
+}
+// The status of a solve with F: rc, or what its error word says (read when the stream was done).  After a
+// failure the next solve starts on a zeroed buffer.
+int factor_solve_status(ooc_factor* F, int rc, int err) {
+  if (!rc) rc = solve_status(err);
+  if (rc) F->epoch.restart();
+  return rc;
 }
 }  // namespace
 
@@ -2939,7 +2949,7 @@ extern "C" int ooc_factor_solve(ooc_handle* h, ooc_factor* F, double* B, int64_t
   if (!rc) rc = queue_solve_error(F->xch.p, &err, s);
   const int wrc = ooc_wait_stream(h, s);
   if (!rc) rc = wrc;
-  return rc ? rc : solve_status(err);
+  return factor_solve_status(F, rc, err);
 }
 
 
@@ -3268,7 +3278,7 @@ static int refine_impl(ooc_handle* h, ooc_factor* F, const double* Astore, i64 l
   int solve_err = 0;
   if (!rc) rc = queue_solve_error(F->xch.p, &solve_err, s);
   if (!rc) rc = ooc_wait_stream(h, s);
-  if (!rc) rc = solve_status(solve_err);
+  rc = factor_solve_status(F, rc, solve_err);
   if (by_digits) {
     if (rc) cudaStreamSynchronize(s);
     F->dig.release();
