@@ -122,7 +122,8 @@ int ooc_get_stream(ooc_handle* h, int which, void** stream);
  *    bytes) or device memory (factored in place, in core).  Upper triangle untouched.
  *    Where 64 divides nb the trailing updates go through digit planes on the tensor cores:
  *    28 bytes per row of a panel for each of up to 512 columns, device memory beside
- *    dev_budget that the handle keeps; without room for it the FP64 pipe does them.
+ *    dev_budget, taken after it, of which the handle keeps at most 256 MiB; without room
+ *    for it the FP64 pipe does them.
  * *info: 0, or k > 0 if the leading minor of order k is not positive definite.      */
 int ooc_dpotrf_L(ooc_handle* h, double* A, int64_t n, int64_t lda, int nb, size_t dev_budget,
                  int* info, ooc_stats* stats);

@@ -83,6 +83,11 @@ struct DevPool {
     cap = c;
     if (cached > cap) flush_locked();
   }
+  // Frees what is cached (for an allocation outside the pool that found no room).
+  void flush() {
+    std::lock_guard<std::mutex> g(mu);
+    flush_locked();
+  }
   void flush_locked() {
     for (auto& kv : idle) cudaFree(kv.second);
     idle.clear();

@@ -680,8 +680,25 @@ int sync_all(ooc_handle* h) {
   return rc;
 }
 
+// The digit planes of a factorization's tensor-core updates, two sets, where 64 divides nb (their blocks are
+// 64 columns wide) and there is a trailing matrix.  Other tile sizes, and a device without room for the
+// planes (28 bytes per row and column of a group), keep the FP64-pipe updates.  Taken after the panel
+// buffer, so that the caller's budget never fails for them, and kept by the handle up to KEEP_PLANES bytes
+// (a larger set is allocated and freed in under a thousandth of its factorization's time).
+constexpr size_t KEEP_PLANES = 256ull << 20;
+void take_planes(Run& R, i64 n, int nb) {
+  ooc_handle* h = R.h;
+  if (nb % 64 != 0 || n <= 64) return;
+  R.slot = (digit_plane_bytes(n, std::min(nb, DIGIT_K)) + 255) / 256 * 256;
+  const size_t bytes = R.slot * ((std::min(group_cols(nb), nb) + DIGIT_K - 1) / DIGIT_K);
+  if (h->digit_ws.ensure(2 * bytes) != OOC_OK) return;
+  R.planes[0] = h->digit_ws.p;
+  R.planes[1] = (char*)h->digit_ws.p + bytes;
+}
+
 // In-core: A is device memory.  One panel covering the whole matrix, factored in place.
 int dpotrf_device(Run& R, double* A, i64 n, i64 lda, int nb) {
+  take_planes(R, n, nb);
   const int bb = (int)((n + nb - 1) / nb);
   TileMap P{A, lda, 0, bb, nb};
   R.st.npanels = 1;
@@ -717,11 +734,19 @@ int dpotrf_host(Run& R, double* A, i64 n, i64 lda, int nb, size_t budget) {
     h->d_buf_bytes = 0;
     if (cudaMalloc(&h->d_buf, need) != cudaSuccess) {
       cudaGetLastError();
-      g_last_error = "device panel buffer allocation failed";
-      return OOC_ERR_NOMEM;
+      h->d_buf = nullptr;
+      h->digit_ws.release();  // what the handle keeps beside it
+      h->pool->flush();
+      if (cudaMalloc(&h->d_buf, need) != cudaSuccess) {
+        cudaGetLastError();
+        h->d_buf = nullptr;
+        g_last_error = "device panel buffer allocation failed";
+        return OOC_ERR_NOMEM;
+      }
     }
     h->d_buf_bytes = need;
   }
+  take_planes(R, n, nb);
   double* Y = h->d_buf;
   int state = 0;
   cudaEvent_t ev_prev_comp = nullptr, ev_prev_d2h = nullptr;
@@ -849,22 +874,12 @@ extern "C" int ooc_dpotrf_L(ooc_handle* h, double* A, int64_t n, int64_t lda, in
   }
   *h->h_status = 0;
   if (!rc) rc = ooc_wait_stream(h, h->s_comp);
-  // Tensor-core updates where 64 divides nb (their blocks are 64 columns wide) and there is a
-  // trailing matrix; other tile sizes, and a device without room for the planes (28 bytes per
-  // row and column of a group), keep the FP64-pipe updates.
-  if (!rc && nb % 64 == 0 && n > 64) {
-    R.slot = (digit_plane_bytes(n, std::min(nb, DIGIT_K)) + 255) / 256 * 256;
-    const size_t bytes = R.slot * ((std::min(group_cols(nb), nb) + DIGIT_K - 1) / DIGIT_K);
-    if (h->digit_ws.ensure(2 * bytes) == OOC_OK) {
-      R.planes[0] = h->digit_ws.p;
-      R.planes[1] = (char*)h->digit_ws.p + bytes;
-    }
-  }
   auto t0 = std::chrono::steady_clock::now();
   if (!rc) rc = on_device ? dpotrf_device(R, A, n, lda, nb) : dpotrf_host(R, A, n, lda, nb, dev_budget);
   int rc2 = sync_all(h);
   if (!rc) rc = rc2;
   auto t1 = std::chrono::steady_clock::now();
+  if (h->digit_ws.bytes > KEEP_PLANES) h->digit_ws.release();
   int st = 0;
   if (!rc) rc = read_status(h, &st);
   if (!rc && h->profile) rc = finish_profile(R);
