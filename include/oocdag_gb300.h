@@ -134,7 +134,9 @@ int ooc_dpotrf_L(ooc_handle* h, double* A, int64_t n, int64_t lda, int nb, size_
  * A on the host: on a device copy when it fits dev_budget bytes (0 = 3/4 of free device
  * memory); otherwise out of core, left-looking over panels of W columns with
  * 3 n W floats <= dev_budget (the panel and two buffers of earlier columns streamed from
- * the host, oocdag.cpp:59-87), OOC_ERR_BUDGET if not even W = nb fits.
+ * the host, oocdag.cpp:59-87), OOC_ERR_BUDGET if not even W = nb fits.  On the host route
+ * the updates' digit planes (8 bytes per row for each of up to 512 columns) count against the
+ * budget too: where it has no room for them the FP32 pipe makes the updates.
  * *info as for ooc_dpotrf_L.                                                          */
 int ooc_spotrf_L(ooc_handle* h, float* A, int64_t n, int64_t lda, int nb, size_t dev_budget,
                  int* info, ooc_stats* stats);

@@ -1367,10 +1367,10 @@ constexpr int DIGIT32_MIN_K = 16, DIGIT32_CHUNK = 512;
 
 // The same for the FP32 working matrix of a reduced-precision factor: C (FP32) -= X X^T
 // with X the FP32 column panel (no conversions).  OOC_PREC_FP32 in several calls on one X: `way` takes the
-// prepared call's choice to the others.
+// prepared call's choice to the others.  planes: false where the caller's budget has no room for them.
 int syrk_f32(int prec, const float* X, i64 ldx, float* C, i64 ldc, int m, int K, const int* status, cudaStream_t s,
              DevBuf& work, int bj_lo = 0, int bj_hi = -1, int prepare = 1, int reserve_sms = 0,
-             Syrk32Way* way = nullptr) {
+             Syrk32Way* way = nullptr, bool planes = true) {
   if (m <= 0 || K <= 0) return OOC_OK;
   if (prec == OOC_PREC_FP32) {
     // digit products on the tensor cores, at most 512 columns at a time; k_syrk_f32 stages X with 16-byte
@@ -1382,7 +1382,7 @@ int syrk_f32(int prec, const float* X, i64 ldx, float* C, i64 ldc, int m, int K,
     if (!way) way = &one;
     if (prepare) {
       const bool aligned = reinterpret_cast<uintptr_t>(X) % 16 == 0 && ldx % 4 == 0;
-      int rc = syrk32_choose(work, K >= DIGIT32_MIN_K && m >= FB / 2, digit32_bytes(m, kc), aligned,
+      int rc = syrk32_choose(work, planes && K >= DIGIT32_MIN_K && m >= FB / 2, digit32_bytes(m, kc), aligned,
                              (size_t)lds * K * sizeof(float), way);
       if (rc) return rc;
       if (*way == Syrk32Way::kCopied)
@@ -1854,6 +1854,7 @@ struct ooc_factor {
     P.nb2 = nb2 > 0 ? nb2 : nb;
     return P;
   }
+  bool planes = true;      // FP32 and FP64: updates may use digit planes (false: the caller's budget has no room)
   int* status = nullptr;   // device status word of the factorization
   int info = 0;
   // the handle's device-buffer cache (null: plain cudaMalloc / cudaFree); declared before
@@ -2209,12 +2210,13 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
       const i64 G0 = J0 / nb * nb, G1 = std::min<i64>(G0 + nb, n);  // the panel's tile
       Syrk32Way way = Syrk32Way::kNone;                             // of the updates below
       if (grouped && J0 + LN < G1) {  // the rest of the tile
-        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, (int)((G1 - J0 - LN + 127) / 128));
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, (int)((G1 - J0 - LN + 127) / 128), 1,
+                      0, nullptr, F->planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
       } else if (grouped) {  // everything right of the tile, the next panel first
         float* Xg = A + G1 + G0 * lda;
-        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, 0, bjn, 1, 0, &way);
+        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, 0, bjn, 1, 0, &way, F->planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
         rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, bjn, -1, 0, kChainSMs,
@@ -2230,12 +2232,12 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
         }
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, bjn, -1, 0, kChainSMs);
       } else if (split) {
-        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 1, 0, &way);
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 1, 0, &way, F->planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, bjn, -1, 0, kChainSMs, &way);
       } else {
-        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work);
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, -1, 1, 0, nullptr, F->planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
       }
@@ -3450,7 +3452,8 @@ extern "C" int ooc_dsyrk_ln(ooc_handle* h, int prec, int n, int k, const double*
 namespace {
 // FP32 lower Cholesky of a HOST matrix through `budget` device bytes: the reference's
 // left-looking panel loop (oocdag.cpp:59-87) with panels of W columns (W from the budget:
-// the panel and two copies of earlier columns, each n x W floats).  Per panel, on the
+// the panel and two copies of earlier columns, each n x W floats, and the digit planes of an
+// update, spotrf_ooc_width).  Per panel, on the
 // compute stream s: the panel's lower part arrives (copy stream sc), every earlier panel's
 // columns arrive W at a time through two X buffers and update it (FP32 syrk_f32 restricted
 // to the panel's columns: the A2X + ooc_syrk tasks, oocquark.cpp:301-356), then the panel is
@@ -3458,7 +3461,8 @@ namespace {
 // panel: ooc_incore, oocquark.cpp:358-421) and copied back (stream sd) before any later
 // panel reads its columns from the host.
 int spotrf_host_ooc(ooc_handle* h, float* A, i64 n, i64 lda, int nb, size_t budget, int* info, ooc_stats* stats) {
-  const i64 W = (i64)(budget / ((size_t)3 * n * sizeof(float))) / nb * nb;
+  bool planes = false;
+  const i64 W = spotrf_ooc_width(n, nb, budget, digit32_bytes, DIGIT32_CHUNK, &planes);
   if (W < nb) {
     char buf[200];
     snprintf(buf, sizeof(buf), "ooc_spotrf_L: budget %zu bytes below one panel (3 n nb floats = %zu)", budget,
@@ -3529,7 +3533,9 @@ int spotrf_host_ooc(ooc_handle* h, float* A, i64 n, i64 lda, int nb, size_t budg
       OOC_CUDA_TRY(cudaEventRecord(evXin[sl], sc));
       h2d += (double)m * Kw * 4;
       OOC_CUDA_TRY(cudaStreamWaitEvent(s, evXin[sl], 0));
-      if ((rc = syrk_f32(OOC_PREC_FP32, X, n, P, n, (int)m, (int)Kw, status, s, work, 0, bjp))) return rc;
+      if ((rc = syrk_f32(OOC_PREC_FP32, X, n, P, n, (int)m, (int)Kw, status, s, work, 0, bjp, 1, 0, nullptr,
+                         planes)))
+        return rc;
       OOC_CUDA_TRY(cudaEventRecord(evXfree[sl], s));
       xuses[sl]++;
       launches++;
@@ -3553,7 +3559,7 @@ int spotrf_host_ooc(ooc_handle* h, float* A, i64 n, i64 lda, int nb, size_t budg
       const i64 wrest = Wp - q0 - LN;  // the panel's columns right of this step
       if (wrest > 0) {
         if ((rc = syrk_f32(OOC_PREC_FP32, Pn, n, Pn + LN * n, n, (int)mq, LN, status, s, work, 0,
-                           (int)((wrest + 127) / 128))))
+                           (int)((wrest + 127) / 128), 1, 0, nullptr, planes)))
           return rc;
         launches++;
       }
@@ -3629,6 +3635,7 @@ extern "C" int ooc_spotrf_L(ooc_handle* h, float* A, int64_t n, int64_t lda, int
     }
     if (bytes > budget)  // out of core: left-looking panels streamed through the budget
       return spotrf_host_ooc(h, A, n, lda, nb, budget, info, stats);
+    F.planes = bytes + digit32_bytes(n, nb) <= budget;
     if (cudaMalloc(&F.Lf, bytes) != cudaSuccess) { cudaGetLastError(); F.Lf = nullptr; return OOC_ERR_NOMEM; }
     F.ld = n;
     OOC_CUDA_TRY(cudaMemcpy2DAsync(F.Lf, n * sizeof(float), A, lda * sizeof(float), n * sizeof(float), n,

@@ -1,8 +1,10 @@
-// How the FP32 trailing updates of one panel are made, chosen when the panel is prepared and
-// kept for its later block-column ranges: what the work buffer holds afterwards depends on it.
+// How the FP32 trailing updates of one panel are made, and what room they get in a budget.  The
+// choice is made when the panel is prepared and kept for its later block-column ranges: what the
+// work buffer holds afterwards depends on it.
 #pragma once
 
 #include <cstddef>
+#include <cstdint>
 
 enum class Syrk32Way {
   kNone,    // nothing prepared
@@ -23,4 +25,21 @@ int syrk32_choose(Buf& work, bool digits_serve, size_t digit_bytes, bool aligned
   const int rc = aligned ? 0 : work.ensure(copy_bytes);
   if (rc) *way = Syrk32Way::kNone;
   return rc;
+}
+
+// Panel width of an out-of-core FP32 factorization (0: not even nb columns fit): the widest multiple of nb with 3 n W
+// floats within the budget.  *planes: an update's digit planes (plane_bytes(rows, columns), at most `chunk`
+// columns at a time) fit beside them.  Up to a quarter of the width is given for them: the update by
+// tensor cores takes a third of the FP32 pipe's time, but a narrower panel reads the earlier columns more often.
+template <typename PlaneBytes>
+int64_t spotrf_ooc_width(int64_t n, int nb, size_t budget, PlaneBytes plane_bytes, int chunk, bool* planes) {
+  const size_t per_column = (size_t)3 * n * sizeof(float);
+  const int64_t widest = (int64_t)(budget / per_column) / nb * nb;
+  *planes = false;
+  for (int64_t W = widest; W >= nb && 4 * W >= 3 * widest; W -= nb)
+    if (per_column * W + plane_bytes(n, (int)(W < chunk ? W : chunk)) <= budget) {
+      *planes = true;
+      return W;
+    }
+  return widest < nb ? 0 : widest;
 }

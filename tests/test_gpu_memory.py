@@ -25,3 +25,49 @@ def test_dpotrf_keeps_at_most_256_mib_of_planes(ooc):
         assert h.dpotrf_L(A, n, n, nb, 0).info == 0
         assert before - _free() <= 0
     assert torch.equal(A.diagonal(), torch.full((n,), 2.0, dtype=torch.float64, device="cuda"))
+
+
+def _spd32(n, lda):
+    import numpy as np
+
+    rng = np.random.default_rng(n)
+    A = np.full((lda, n), 5.0, dtype=np.float32, order="F")
+    R = rng.uniform(-0.5, 0.5, (n, n)).astype(np.float32)
+    A[:n] = np.tril(R) + np.tril(R, -1).T + np.float32(n**0.5) * np.eye(n, dtype=np.float32)
+    return A
+
+
+def _check32(A, L, n):
+    """|A - L L^T| <= 4 (n + 2) 2^-24 sqrt(a_ii a_jj), the bar of test_gpu_fp32_digits.py."""
+    import torch
+
+    A, L = (torch.from_numpy(M[:n].copy()).cuda().double().tril() for M in (A, L))
+    d = A.diagonal().sqrt()
+    err = ((A - (L @ L.T).tril()).abs() / d[:, None] / d[None, :]).max().item()
+    assert err <= 4 * (n + 2) * 2.0**-24, err
+
+
+@pytest.mark.parametrize("n,nb,extra", [(6000, 512, 0), (6000, 512, 30 << 20), (5001, 256, 4096), (4000, 512, 1 << 20)])
+def test_spotrf_out_of_core_stays_within_its_budget(ooc, n, nb, extra):
+    """Buffers (kept by the handle after the call, so what is free tells) within the budget, two tiles and the allocator's
+    2 MiB a buffer."""
+    A = _spd32(n, n)
+    L = A.copy(order="F")
+    budget = 12 * n * nb + extra
+    with ooc.Handle(0) as h:
+        assert h.spotrf_L(_spd32(600, 600), 600, 600, nb).info == 0  # modules loaded
+        before = _free()
+        r = h.spotrf_L(L, n, n, nb, budget)
+        assert r.info == 0 and r.stats["npanels"] >= 2
+        copies = 4 * n * 512 if n % 4 else 0  # (an aligned copy of an odd-order panel for the FP32 pipe)
+        assert before - _free() <= budget + copies + 8 * nb * nb + (5 << 21)
+    _check32(A, L, n)
+
+
+@pytest.mark.parametrize("n,lda,nb", [(777, 777, 512), (1100, 1101, 512), (1000, 1000, 256), (701, 703, 128), (300, 300, 100)])
+def test_spotrf_in_core_budget_without_room_for_planes(ooc, handle, n, lda, nb):
+    """The matrix fits the budget exactly: the FP32 pipe makes the updates, in both calls of a split one."""
+    A = _spd32(n, lda)
+    L = A.copy(order="F")
+    assert handle.spotrf_L(L, n, lda, nb, 4 * n * n).info == 0
+    _check32(A, L, n)

@@ -25,13 +25,21 @@ struct Buf {
 };
 int main() {
   const size_t digits = 4096, copy = 2048;
+  auto planes_of = [](int64_t rows, int k) { return (size_t)rows * k * 8; };
+  for (int64_t n : {100, 1000, 6000})
+    for (int nb : {64, 100, 512})
+      for (size_t budget = 0; budget <= (size_t)12 * n * 8 * nb; budget += (size_t)n * nb) {
+        bool planes = false;
+        const int64_t W = spotrf_ooc_width(n, nb, budget, planes_of, 512, &planes);
+        printf("w %lld %d %zu: %lld %d\n", (long long)n, nb, budget, (long long)W, (int)planes);
+      }
   for (size_t limit : {(size_t)0, copy, digits})
     for (int serve = 0; serve < 2; serve++)
       for (int aligned = 0; aligned < 2; aligned++) {
         Buf b{limit};
         Syrk32Way way = Syrk32Way::kNone;
         const int rc = syrk32_choose(b, serve, digits, aligned, copy, &way);
-        printf("%zu %d %d: %d %d %zu\n", limit, serve, aligned, rc, (int)way, b.bytes);
+        printf("c %zu %d %d: %d %d %zu\n", limit, serve, aligned, rc, (int)way, b.bytes);
       }
 }
 """
@@ -47,15 +55,16 @@ def table(tmp_path_factory):
     subprocess.run([cxx, "-std=c++17", "-I" + CSRC, str(d / "t.cpp"), "-o", str(d / "t")], check=True)
     out = subprocess.run([str(d / "t")], check=True, capture_output=True, text=True).stdout
     rows = [line.split(": ") for line in out.strip().splitlines()]
-    return {tuple(map(int, k.split())): tuple(map(int, v.split())) for k, v in rows}
+    return {(k[0], *map(int, k[2:].split())): tuple(map(int, v.split())) for k, v in rows}
 
 
 NONE, DIRECT, COPIED, DIGITS = range(4)
 
 
 def test_every_choice(table):
-    assert len(table) == 12
-    for (limit, serve, aligned), (rc, way, held) in table.items():
+    choices = {k[1:]: v for k, v in table.items() if k[0] == "c"}
+    assert len(choices) == 12
+    for (limit, serve, aligned), (rc, way, held) in choices.items():
         if serve and limit >= 4096:
             want = (0, DIGITS, 4096)
         elif aligned:
@@ -74,4 +83,16 @@ def test_later_ranges_take_the_prepared_way():
     for branch in ("} else if (grouped) {", "} else if (split) {"):
         part = body[body.index(branch) + len(branch) :]
         part = part[: part.index("} else")]
-        assert part.count("syrk_f32(") == 2 and part.count("&way)") == 2
+        assert part.count("syrk_f32(") == 2 and part.count("&way") == 2
+
+
+def test_out_of_core_width_and_planes_stay_within_the_budget(table):
+    rows = {k[1:]: v for k, v in table.items() if k[0] == "w"}
+    assert len(rows) > 500 and {p for _, p in rows.values()} == {0, 1}
+    for (n, nb, budget), (W, planes) in rows.items():
+        widest = budget // (12 * n) // nb * nb
+        assert W % nb == 0 and (W == 0) == (widest < nb)  # what was accepted stays accepted
+        if W == 0:
+            continue
+        fits = [w for w in range(nb, widest + 1, nb) if 4 * w >= 3 * widest and 12 * n * w + 8 * n * min(w, 512) <= budget]
+        assert (W, planes) == ((max(fits), 1) if fits else (widest, 0)), (n, nb, budget)
