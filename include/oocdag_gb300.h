@@ -207,7 +207,10 @@ int ooc_factor_solve(ooc_handle* h, ooc_factor* F, double* B, int64_t ldb, int n
  * factor), until the normwise backward error ||R||_inf/(||A||_inf ||X||_inf + ||B||_inf)
  * <= tol or maxiter corrections.  A: device or host, lower triangle read (the residual
  * and the norm use A's symmetry; a host A is copied to the device, lower triangle only,
- * unless the factor kept it, OOC_OPT_KEEP_A).  B, X: device, nrhs <= 16.            */
+ * unless the factor kept it, OOC_OPT_KEEP_A).  B, X: device, nrhs <= 16.
+ * From n = 2048 on and with several right-hand sides the residual takes digit planes of A where there is
+ * room (14 n^2 bytes up to 16 GiB, else 512 MiB at a time), which go back to the handle's
+ * cache (OOC_OPT_POOL_BYTES) before the call returns.                                */
 int ooc_solve_refine(ooc_handle* h, ooc_factor* F, const double* A, int64_t lda, const double* B,
                      int64_t ldb, double* X, int64_t ldx, int nrhs, double tol, int maxiter, int* iters,
                      double* berr);
@@ -222,7 +225,8 @@ int ooc_factor_create_gen(ooc_handle* h, int64_t n, uint64_t seed, double alpha,
 int ooc_solve_refine_gen(ooc_handle* h, ooc_factor* F, uint64_t seed, double alpha, const double* B,
                          int64_t ldb, double* X, int64_t ldx, int nrhs, double tol, int maxiter, int* iters,
                          double* berr);
-/* Device bytes a factor object of order n, tile nb and precision prec holds.         */
+/* Device bytes a factor object of order n, tile nb and precision prec holds, those of the
+ * digit planes that its updates take while it is made included.                        */
 int64_t ooc_factor_bytes(int64_t n, int nb, int prec);
 /* B (n x nrhs, device) := N(0,1) samples of stream `seed` (Box-Muller on SplitMix64).  */
 int ooc_gen_normal(ooc_handle* h, double* B, int64_t n, int64_t ldb, int nrhs, uint64_t seed);

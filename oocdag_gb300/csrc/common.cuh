@@ -165,6 +165,14 @@ struct GrowBuf {
 };
 // The handle's workspace for the batched solvers' launch tables.
 GrowBuf* ooc_handle_batch_ws(ooc_handle* h);
+// Digit planes of the tensor-core updates: whether the handle's next factorizations may take them (default:
+// yes; without them the FP64 and FP32 pipes make the updates), the bytes they take in ooc_dpotrf_L and while a
+// factor object is made, and the return of those that the handle keeps.
+void ooc_handle_set_planes(ooc_handle* h, bool on);
+bool ooc_handle_planes(ooc_handle* h);
+int64_t ooc_dpotrf_plane_bytes(int64_t n, int nb);
+int64_t ooc_factor_plane_bytes(int64_t n, int nb, int prec);
+void ooc_handle_release_planes(ooc_handle* h);
 // The handle's workspace for solves with a stored factor (ooc_dpotrs_L).
 GrowBuf* ooc_handle_solve_ws(ooc_handle* h);
 // Backward error of a solution x of A x = b (device vectors) for the uniform test matrix

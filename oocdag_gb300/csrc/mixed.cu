@@ -1995,6 +1995,7 @@ struct MixedProf {
 // rounding into C each); otherwise, or without room for the digits, FP64 MMAs (launch_panel_update).
 // n = 8192, nb = 512: 43 ms, 200 with FP64 MMAs; n = 16384: 160 and 1392.
 constexpr int FP64_CHUNK = DIGIT_RUNS * DIGIT_K;
+size_t fp64_slot(i64 n) { return (digit_plane_bytes(n, DIGIT_K) + 255) / 256 * 256; }  // planes of one run
 constexpr int kMixedChainSMs = 16;  // SMs the bulk update leaves to the next panel's kernels
 int factor_mixed(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_t* launches, MixedProf* prof) {
   const i64 n = F->n;
@@ -2008,8 +2009,8 @@ int factor_mixed(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int6
   double* W = (double*)F->scratch.p;   // copy of the column panel (m x nb, ld n)
   double* E = W + (size_t)n * nb;      // L_jj^{-1} (lower, ld nb)
   (void)prec;
-  const size_t slot = (digit_plane_bytes(n, DIGIT_K) + 255) / 256 * 256;
-  const bool digits = nb % 64 == 0 && n > nb && F->work.ensure((size_t)DIGIT_RUNS * slot) == OOC_OK;
+  const size_t slot = fp64_slot(n);
+  const bool digits = F->planes && nb % 64 == 0 && n > nb && F->work.ensure((size_t)DIGIT_RUNS * slot) == OOC_OK;
   cudaEvent_t evA, evP;  // A: next panel's columns updated (s0 -> s1); P: panel solved (s1 -> s0)
   OOC_CUDA_TRY(cudaEventCreateWithFlags(&evA, cudaEventDisableTiming));
   OOC_CUDA_TRY(cudaEventCreateWithFlags(&evP, cudaEventDisableTiming));
@@ -2682,6 +2683,7 @@ static int create_impl(ooc_handle* h, const double* A, int64_t n, int64_t lda, b
     }
   }
   F->pool = ooc_handle_pool(h);
+  F->planes = ooc_handle_planes(h);
   for (DevBuf* b : {&F->part, &F->work, &F->scratch, &F->work2, &F->part2, &F->rws, &F->xch, &F->dig, &F->sws})
     b->pool = F->pool.get();
   int rc = alloc_factor(F, n, nb, reduced);
@@ -2832,10 +2834,20 @@ extern "C" int ooc_factor_create_gen(ooc_handle* h, int64_t n, uint64_t seed, do
   return create_impl(h, nullptr, n, n, true, seed, alpha, nb, prec, out, info, stats);
 }
 
+// While the factor is made (given back afterwards): FP32's planes of up to 512 columns of a panel, FP64's of
+// DIGIT_RUNS runs.
+int64_t ooc_factor_plane_bytes(int64_t n, int nb, int prec) {
+  if (n <= 0 || nb <= 0) return 0;
+  if (prec == OOC_PREC_FP32) return n > panel_width_f32(nb) ? (int64_t)digit32_bytes(n, std::min(nb, DIGIT32_CHUNK)) : 0;
+  if (prec == OOC_PREC_FP64) return nb % 64 == 0 && n > nb ? (int64_t)(DIGIT_RUNS * fp64_slot(n)) : 0;
+  return 0;
+}
+
 extern "C" int64_t ooc_factor_bytes(int64_t n, int nb, int prec) {
   if (n <= 0 || nb <= 0) return 0;
   const int64_t bb = (n + nb - 1) / nb;
   int64_t b = (int64_t)trsolve_bytes(n, RMAX, prec == OOC_PREC_FP64 ? 8 : 4) + 256;  // solve exchange, status
+  b += ooc_factor_plane_bytes(n, nb, prec);
   if (prec == OOC_PREC_FP64) return b + n * n * 8 + bb * nb * nb * 8 + n * nb * 8 + (int64_t)nb * nb * 8;
   b += n * n * 4 + bb * nb * nb * 4 + 2 * (int64_t)nb * nb * 4;  // Lf, Dinvf, scratch
   if (prec == OOC_PREC_BF16X3) {

@@ -78,6 +78,7 @@ struct ooc_handle {
   std::shared_ptr<DevPool> pool;  // device buffers of the handle's factor objects
   GrowBuf batch_ws;               // launch tables of the batched solvers
   GrowBuf solve_ws;               // panels and vectors of ooc_dpotrs_L
+  bool planes = true;             // factorizations may take digit planes
   GrowBuf digit_ws;               // digit planes of the tensor-core FP64 updates (two sets of up to four runs of 128 columns)
   int last_info = 0;
   std::vector<cudaEvent_t> ev_pool;  // reusable timing-free events
@@ -686,12 +687,15 @@ int sync_all(ooc_handle* h) {
 // buffer, so that the caller's budget never fails for them, and kept by the handle up to KEEP_PLANES bytes
 // (a larger set is allocated and freed in under a thousandth of its factorization's time).
 constexpr size_t KEEP_PLANES = 256ull << 20;
+size_t plane_set_bytes(i64 n, int nb, size_t* slot) {
+  if (nb % 64 != 0 || n <= 64) return 0;
+  *slot = (digit_plane_bytes(n, std::min(nb, DIGIT_K)) + 255) / 256 * 256;
+  return *slot * ((std::min(group_cols(nb), nb) + DIGIT_K - 1) / DIGIT_K);
+}
 void take_planes(Run& R, i64 n, int nb) {
   ooc_handle* h = R.h;
-  if (nb % 64 != 0 || n <= 64) return;
-  R.slot = (digit_plane_bytes(n, std::min(nb, DIGIT_K)) + 255) / 256 * 256;
-  const size_t bytes = R.slot * ((std::min(group_cols(nb), nb) + DIGIT_K - 1) / DIGIT_K);
-  if (h->digit_ws.ensure(2 * bytes) != OOC_OK) return;
+  const size_t bytes = plane_set_bytes(n, nb, &R.slot);
+  if (!h->planes || !bytes || h->digit_ws.ensure(2 * bytes) != OOC_OK) return;
   R.planes[0] = h->digit_ws.p;
   R.planes[1] = (char*)h->digit_ws.p + bytes;
 }
@@ -895,6 +899,14 @@ extern "C" int ooc_dpotrf_L(ooc_handle* h, double* A, int64_t n, int64_t lda, in
   if (stats) *stats = R.st;
   return OOC_OK;
 }
+
+void ooc_handle_set_planes(ooc_handle* h, bool on) { h->planes = on; }
+bool ooc_handle_planes(ooc_handle* h) { return !h || h->planes; }
+int64_t ooc_dpotrf_plane_bytes(int64_t n, int nb) {
+  size_t slot = 0;
+  return n > 0 && nb > 0 ? (int64_t)(2 * plane_set_bytes(n, nb, &slot)) : 0;
+}
+void ooc_handle_release_planes(ooc_handle* h) { h->digit_ws.release(); }
 
 // ---------------------------------------------------------------------------------
 // Reference-shaped entry points.

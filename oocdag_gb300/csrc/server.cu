@@ -98,6 +98,7 @@ struct Job {
   int64_t factor_bytes = 0;  // part of `reserve` that stays resident afterwards
   bool small = false;
   bool ooc = false;          // factored out of core (host-resident matrix, capped device budget)
+  bool planes = true;        // the factorization's digit planes are part of `reserve` (false: no room, it does without)
   bool hit = false;          // solved with a resident factor
 };
 
@@ -205,11 +206,14 @@ struct ooc_server {
         const int64_t n = j.r.n;
         // out of core: the factor lives in host memory; the device holds the panel budget
         // and the solve's two panels
-        const int64_t need_f = hit || j.ooc ? 0 : (j.small ? 8 * n * n : ooc_factor_bytes(n, cfg.nb, cfg.prec));
+        // the factor stays; its digit planes are held while it is made, and given up where the budget has no room
+        const int64_t planes = hit || j.small ? 0 : j.ooc ? ooc_dpotrf_plane_bytes(n, cfg.nb) : ooc_factor_plane_bytes(n, cfg.nb, cfg.prec);
+        const int64_t need_f = hit || j.ooc ? 0 : (j.small ? 8 * n * n : ooc_factor_bytes(n, cfg.nb, cfg.prec) - planes);
         const int64_t need_w = j.small ? 64 * n
                                : j.ooc ? cfg.ooc_budget + 16 * n * cfg.nb + 64 * n + (64LL << 20)
                                        : 64 * n + (64LL << 20);
-        const int64_t need = need_f + need_w;
+        j.planes = need_f + need_w + planes <= budget;
+        const int64_t need = need_f + need_w + (j.planes ? planes : 0);
         if (need > budget) {  // can never fit this device budget
           Job jj = j;
           pending.erase(pending.begin() + i);
@@ -271,8 +275,11 @@ struct ooc_server {
         }
       }
       if (status == OOC_OK) status = ooc_dmatgen_uniform(h, ooc_host, n, n, j.r.matrix_seed, alpha);
-      if (status == OOC_OK)
+      if (status == OOC_OK) {
+        ooc_handle_set_planes(h, j.planes);
         status = ooc_dpotrf_L(h, ooc_host, n, n, cfg.nb, (size_t)cfg.ooc_budget, &info, nullptr);
+        ooc_handle_release_planes(h);
+      }
       double *B = nullptr, *X = nullptr;
       if (status == OOC_OK && info == 0 && (status = wbuf.ensure((size_t)n * 16)) == OOC_OK) {
         B = (double*)wbuf.p;
@@ -323,6 +330,7 @@ struct ooc_server {
       std::vector<double> x;
       bool made = false;
       if (!F) {
+        ooc_handle_set_planes(h, j.planes);
         status = ooc_factor_create_gen(h, n, j.r.matrix_seed, alpha, cfg.nb, cfg.prec, &F, &info, nullptr);
         made = (status == OOC_OK);
       }

@@ -71,3 +71,31 @@ def test_spotrf_in_core_budget_without_room_for_planes(ooc, handle, n, lda, nb):
     L = A.copy(order="F")
     assert handle.spotrf_L(L, n, lda, nb, 4 * n * n).info == 0
     _check32(A, L, n)
+
+
+@pytest.mark.parametrize("kind", ["fp32", "fp64", "out of core"])
+def test_server_admits_by_what_a_request_holds(ooc, kind):
+    """A budget with room for all of a request but its digit planes: admitted, factored without them; one byte less is
+    refused.  The planes: FP32 8 bytes a row for each of nb columns and 8 bytes of exponents, FP64 14 bytes
+    for each of 512 columns and 16 of exponents, which factor_bytes counts; out of core twice that, per job."""
+    from oocdag_gb300.server import Server
+
+    n, nb = 4096, 512
+    prec = "fp32" if kind == "fp32" else "fp64"
+    planes = n * (8 * nb + 8) if kind == "fp32" else n * (14 * 512 + 16)
+    assert ooc.factor_bytes(n, nb, prec) >= (4 if kind == "fp32" else 8) * n * n + planes
+    if kind == "out of core":
+        opts = dict(ooc_min_n=n, ooc_budget=96 << 20)
+        least = (96 << 20) + 16 * n * nb + 64 * n + (64 << 20)
+    else:
+        opts, least = {}, ooc.factor_bytes(n, nb, prec) - planes + 64 * n + (64 << 20)
+    for budget, status in ((least + 2 * planes, 0), (least, 0), (least - 1, ooc.OOC_ERR_BUDGET)):
+        with Server(workers=1, nb=nb, prec=prec, hbm_budget=budget, **opts) as S:
+            i = S.submit(n=n, matrix_seed=1, rhs_seed=2, key=1)
+            done = []
+            for _ in range(120):
+                done = S.poll(wait_ms=1000)
+                if done:
+                    break
+            assert [d["id"] for d in done] == [i] and done[0]["status"] == status, (budget, done, S.last_error())
+            assert status or done[0]["backward_error"] <= 1e-14
