@@ -119,7 +119,7 @@ int launch_potrf_block(double* A, i64 ld, int n, i64 col0, int* status, cudaStre
 int launch_trsm_rows(const double* L, i64 ldl, double* B, i64 ldb, i64 stride, int nb, i64 org, i64 m, int n,
                      const int* status, cudaStream_t s);
 // The inverses L_bb^{-T} of the 64 x 64 diagonal blocks of L (n x n lower), one after another
-// (64 x 64 each, column-major; the last may hold fewer columns).
+// (64 x 64 each, column-major; the last may hold fewer columns; n < 64: one block with ld n).
 int launch_diag_inverses(const double* L, i64 ldl, i64 n, double* Dinv, cudaStream_t s);
 // C(i, c) -= X(i) X(c)^T, c < w <= 64, i >= c, with X (K columns) and C (w columns) addressed by the
 // same rows; 32 divides nb and org.

@@ -510,6 +510,8 @@ int launch_trsm_rows(const double* L, i64 ldl, double* B, i64 ldb, i64 stride, i
 }
 
 int launch_diag_inverses(const double* L, i64 ldl, i64 n, double* Dinv, cudaStream_t s) {
+  if (n > 0 && n < SB)
+    return launch_trsm(TrsmArgs{L, ldl, 0, Dinv, n, 0, 0, SB, 0, (int)n, (int)n, (int)n, 1}, 1, nullptr, s);
   const i64 nblk = (n + SB - 1) / SB;
   for (i64 z = 0; z < nblk; z += 65535) {
     const int batch = (int)min(nblk - z, (i64)65535);

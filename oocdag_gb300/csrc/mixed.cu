@@ -32,6 +32,7 @@
 
 #include "common.cuh"
 #include "devpool.cuh"
+#include "dpotrs_plan.h"
 #include "exchange_epoch.h"
 #include "fp32_tc.cuh"
 #include "fp64_tc.cuh"
@@ -3002,40 +3003,26 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
   const bool l_dev = on_device(L), b_dev = on_device(B);
   nb = (int)std::min<i64>(nb, n);
   const int bb = (int)((n + nb - 1) / nb);
-  const i64 tile = (i64)nb * nb;
-  // workspace: status word, L_JJ^{-T}, nb x RMAX products, B's device copy, two panels
-  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  // The budget is checked against the panel-wise solve's needs: two panels, an nb x nb inverse
-  // and nb x RMAX products.  (The 64 x 64 inverses and exchange words used below fit in that for
-  // nb >= 96 and exceed it by at most 40 KB for smaller nb.)
-  const size_t b_stat = 256, b_B = b_dev ? 0 : up((size_t)n * nrhs * 8), b_pan = l_dev ? 0 : up((size_t)n * nb * 8);
-  size_t need = b_stat + up(tile * 8) + up((size_t)nb * RMAX * 8) + b_B + 2 * b_pan;
-  if (dev_budget > 0 && need > dev_budget) {
+  const DpotrsPlan plan = dpotrs_plan(n, nb, nrhs, l_dev, b_dev, dev_budget, [](i64 m, int r, int sweeps) { return trsolve_bytes(m, r, 8, sweeps); });
+  if (!plan.ok) {
     char buf[200];
     snprintf(buf, sizeof(buf), "ooc_dpotrs_L: n=%lld nb=%d needs %zu device bytes (two panels), budget %zu",
-             (long long)n, nb, need, dev_budget);
+             (long long)n, nb, plan.least, dev_budget);
     ooc_set_last_message(buf);
     return OOC_ERR_BUDGET;
   }
-  // A device L whose whole-matrix workspace (an inverse per 64 rows, exchange words) fits the
-  // budget is solved in one launch; otherwise panel by panel.
-  const size_t w_dinv = up((size_t)((n + 63) / 64) * 64 * 64 * 8), w_x = up(trsolve_bytes(n, nrhs, 8));
-  const bool whole = l_dev && (dev_budget == 0 || b_stat + w_dinv + w_x + b_B <= dev_budget);
-  const size_t b_dinv = whole ? w_dinv : up((size_t)((nb + 63) / 64) * 64 * 64 * 8);
-  const size_t b_x = whole ? w_x : up(trsolve_bytes(nb, nrhs, 8));
-  need = b_stat + b_dinv + b_x + b_B + 2 * b_pan;
+  const bool whole = plan.whole;
   GrowBuf* ws = ooc_handle_solve_ws(h);
-  int rc = ws->ensure(need);
+  int rc = ws->ensure(plan.need);
   if (rc) return rc;
-  char* base = (char*)ws->p;
-  double* D = (double*)(base + b_stat);
-  void* xch = base + b_stat + b_dinv;
-  double* Bd = b_dev ? B : (double*)(base + b_stat + b_dinv + b_x);
+  char* xch = (char*)ws->p;
+  double* D = (double*)(xch + plan.inverses);
+  double* Bd = b_dev ? B : (double*)(xch + plan.b);
   const i64 ldbd = b_dev ? ldb : n;
   double* Pbuf[2] = {nullptr, nullptr};
   if (!l_dev) {
-    Pbuf[0] = (double*)(base + b_stat + b_dinv + b_x + b_B);
-    Pbuf[1] = (double*)((char*)Pbuf[0] + b_pan);
+    Pbuf[0] = (double*)(xch + plan.panels);
+    Pbuf[1] = (double*)(xch + plan.panels + plan.panel);
   }
   struct EvGuard {  // copied (per slot), slot free (per slot), inputs ready
     cudaEvent_t e[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -3045,7 +3032,7 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
   cudaEvent_t* evc = ev.e;
   cudaEvent_t* evf = ev.e + 2;
   cudaEvent_t ev0 = ev.e[4];
-  OOC_CUDA_TRY(cudaMemsetAsync(xch, 0, b_x, s));
+  OOC_CUDA_TRY(cudaMemsetAsync(xch, 0, plan.inverses, s));
   unsigned epoch = 0;
   if (!b_dev)
     OOC_CUDA_TRY(cudaMemcpy2DAsync(Bd, n * sizeof(double), B, ldb * sizeof(double), n * sizeof(double), nrhs,
@@ -3071,7 +3058,8 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
   int slot_uses[2] = {0, 0};
   if (whole) {
     rc = launch_diag_inverses(L, ldl, n, D, s);
-    if (!rc) rc = launch_trsolve<double>(TriSolve<double>{n, L, ldl, D, n, 64, 64, Bd, ldbd, nrhs, 3}, xch, ++epoch, s);
+    const int w = (int)std::min<i64>(DPOTRS_BLOCK, n);
+    if (!rc) rc = launch_trsolve<double>(TriSolve<double>{n, L, ldl, D, n, w, w, Bd, ldbd, nrhs, 3}, xch, ++epoch, s);
   }
   for (int sweep = 0; sweep < 2 && !rc && !whole; sweep++) {
     // panel order: forward left to right, backward right to left
@@ -3095,9 +3083,17 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
       }
       const i64 rows = n - J0 - LN;
       if ((rc = launch_diag_inverses(Pj, ldp, LN, D, s))) break;
-      TriSolve<double> tile{LN, Pj, ldp, D, LN, 64, 64, Bd + J0, ldbd, nrhs, sweep + 1};
+      auto solve_tile = [&]() -> int {
+        const int w = std::min(DPOTRS_BLOCK, LN);
+        int e = OOC_OK;
+        for (int q = 0; q < nrhs && !e; q += plan.group)
+          e = launch_trsolve<double>(TriSolve<double>{LN, Pj, ldp, D, LN, w, w, Bd + J0 + q * ldbd, ldbd,
+                                                      std::min(plan.group, nrhs - q), sweep + 1},
+                                     xch, ++epoch, s);
+        return e;
+      };
       if (sweep == 0) {  // y_J = L_JJ^{-1} b_J, then b_below -= L_below y_J
-        if ((rc = launch_trsolve<double>(tile, xch, ++epoch, s))) break;
+        if ((rc = solve_tile())) break;
         if (rows > 0 && (rc = gemm_nn_small<double, double>(Pj + LN, ldp, Bd + J0, ldbd, Bd + J0 + LN, ldbd, (int)rows, LN,
                                                             nrhs, -1.0, 1.0, s, nullptr)))
           break;
@@ -3105,7 +3101,7 @@ extern "C" int ooc_dpotrs_L(ooc_handle* h, const double* L, int64_t n, int64_t l
         if (rows > 0 && (rc = gemm_tn_small<double, double>(Pj + LN, ldp, Bd + J0 + LN, ldbd, Bd + J0, ldbd, LN,
                                                             (int)rows, nrhs, -1.0, 1.0, s)))
           break;
-        if ((rc = launch_trsolve<double>(tile, xch, ++epoch, s))) break;
+        if ((rc = solve_tile())) break;
       }
       if (!l_dev) {
         OOC_CUDA_TRY(cudaEventRecord(evf[slot], s));

@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(Cfg<T>::BS * 4, sizeof(T) == 8 ? 2 : 1)
         D[k + c * (BS + 1)] = (k <= c && c < mi) ? U[k + (i64)c * ldu] : T(0);
       }
     }
-    unsigned long long* out = xch + (fwd ? 0 : dir_words);
+    unsigned long long* out = xch + (fwd || nsw == 1 ? 0 : dir_words);
     auto fetch = [&](int j, int buf) {  // block j of this sweep's solution into xs[buf]
       i64 sj;
       int mj, l2;
@@ -350,8 +350,8 @@ int launch_r(const TriSolve<T>& a, int nblk, int ngrp, void* exchange, unsigned 
 
 }  // namespace
 
-size_t trsolve_bytes(i64 n, int r, int elem_size) {
-  return TS_CTL + (size_t)2 * (size_t)n * (size_t)r * (elem_size == 4 ? 8 : 16);
+size_t trsolve_bytes(i64 n, int r, int elem_size, int sweeps) {
+  return TS_CTL + (size_t)sweeps * (size_t)n * (size_t)r * (elem_size == 4 ? 8 : 16);
 }
 
 template <typename T>

@@ -22,9 +22,9 @@ struct TriSolve {
   int sweeps;  // 1: L y = b, 2: L^T x = b, 3: both
 };
 
-// Exchange buffer of a solve (n, r): zeroed once when allocated; epoch is a number > 0 that no
+// Exchange buffer of a solve (n, r) whose launches make both sweeps or one each: zeroed once when allocated; epoch is a number > 0 that no
 // earlier launch on the buffer since then has used.
-size_t trsolve_bytes(i64 n, int r, int elem_size);
+size_t trsolve_bytes(i64 n, int r, int elem_size, int sweeps = 2);
 template <typename T>
 int launch_trsolve(const TriSolve<T>& a, void* exchange, unsigned epoch, cudaStream_t s);
 // The buffer's error word (an int, 0 while every wait has ended), for the host to read after
