@@ -2146,6 +2146,17 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
     const size_t pb = bf16x3_work_bytes((int)(n - std::min(nb, P.nb2)), nb);
     if ((rc = F->work.ensure(pb)) || (rc = F->work2.ensure(pb))) return rc;
   }
+  bool planes = F->planes;
+  if (prec == OOC_PREC_FP32) {
+    // the updates' buffer once for all of them: a growth later would free memory, and wait for the device, inside
+    // the look-ahead
+    const int w = P.tail0 == 0 ? P.nb2 : nb;
+    auto digits = [](i64 m, int K) { return digit32_bytes(m, std::min(K, DIGIT32_CHUNK)); };
+    auto copies = [](i64 m, int K) { return (size_t)((m + 3) / 4 * 4) * K * sizeof(float); };
+    planes = planes && F->work.ensure(syrk32_largest(n, nb, w, digits)) == OOC_OK;
+    const bool aligned = (uintptr_t)A % 16 == 0 && lda % 4 == 0 && nb % 4 == 0 && w % 4 == 0;
+    if (!planes && !aligned && (rc = F->work.ensure(syrk32_largest(n, nb, w, copies)))) return rc;
+  }
   OOC_CUDA_TRY(cudaFuncSetAttribute(k_diag_f32, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DG_SMEM));
   OOC_CUDA_TRY(cudaFuncSetAttribute(k_diag_s256, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DS_SMEM));
   cudaEvent_t evA, evP;  // A: next panel's columns updated (s0 -> s1); P: diagonal tile done (s1 -> s0)
@@ -2213,12 +2224,12 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
       Syrk32Way way = Syrk32Way::kNone;                             // of the updates below
       if (grouped && J0 + LN < G1) {  // the rest of the tile
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, (int)((G1 - J0 - LN + 127) / 128), 1,
-                      0, nullptr, F->planes);
+                      0, nullptr, planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
       } else if (grouped) {  // everything right of the tile, the next panel first
         float* Xg = A + G1 + G0 * lda;
-        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, 0, bjn, 1, 0, &way, F->planes);
+        rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, 0, bjn, 1, 0, &way, planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
         rc = syrk_f32(prec, Xg, lda, C, lda, (int)m, (int)(G1 - G0), F->status, s0, F->work, bjn, -1, 0, kChainSMs,
@@ -2234,12 +2245,12 @@ int factor_f32(ooc_factor* F, int prec, cudaStream_t s0, cudaStream_t s1, int64_
         }
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, bjn, -1, 0, kChainSMs);
       } else if (split) {
-        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 1, 0, &way, F->planes);
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, bjn, 1, 0, &way, planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
         rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, bjn, -1, 0, kChainSMs, &way);
       } else {
-        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, -1, 1, 0, nullptr, F->planes);
+        rc = syrk_f32(prec, Pn, lda, C, lda, (int)m, LN, F->status, s0, F->work, 0, -1, 1, 0, nullptr, planes);
         if (rc) return rc;
         OOC_CUDA_TRY(cudaEventRecord(evA, s0));
       }

@@ -27,6 +27,19 @@ int syrk32_choose(Buf& work, bool digits_serve, size_t digit_bytes, bool aligned
   return rc;
 }
 
+// Bytes of the largest preparation in a factorization of order n with tiles of nb columns in panels of w <= nb:
+// bytes(rows, columns) for the updates inside the first tile by its first panel, and right of it by all of it.
+template <typename Bytes>
+size_t syrk32_largest(int64_t n, int nb, int w, Bytes bytes) {
+  size_t b = 0;
+  if (w < nb && n > w) b = bytes(n - w, w);
+  if (n > nb) {
+    const size_t whole = bytes(n - nb, nb);
+    b = whole > b ? whole : b;
+  }
+  return b;
+}
+
 // Panel width of an out-of-core FP32 factorization (0: not even nb columns fit): the widest multiple of nb with 3 n W
 // floats within the budget.  *planes: an update's digit planes (plane_bytes(rows, columns), at most `chunk`
 // columns at a time) fit beside them.  Up to a quarter of the width is given for them: the update by

@@ -26,6 +26,11 @@ struct Buf {
 int main() {
   const size_t digits = 4096, copy = 2048;
   auto planes_of = [](int64_t rows, int k) { return (size_t)rows * k * 8; };
+  auto chunked = [](int64_t rows, int k) { return (size_t)((rows + 127) / 128) * 128 * (size_t)(k < 512 ? k : 512) * 8; };
+  for (int64_t n : {1, 100, 511, 512, 513, 1000, 6001})
+    for (int nb : {64, 256, 384, 512})
+      for (int w = nb % 256 ? 64 : 128; w <= nb; w *= 2)
+        printf("m %lld %d %d: %zu\n", (long long)n, nb, w, syrk32_largest(n, nb, w, chunked));
   for (int64_t n : {100, 1000, 6000})
     for (int nb : {64, 100, 512})
       for (size_t budget = 0; budget <= (size_t)12 * n * 8 * nb; budget += (size_t)n * nb) {
@@ -96,3 +101,24 @@ def test_out_of_core_width_and_planes_stay_within_the_budget(table):
             continue
         fits = [w for w in range(nb, widest + 1, nb) if 4 * w >= 3 * widest and 12 * n * w + 8 * n * min(w, 512) <= budget]
         assert (W, planes) == ((max(fits), 1) if fits else (widest, 0)), (n, nb, budget)
+
+
+def test_the_first_reservation_holds_every_update(table):
+    """Panels of w columns inside tiles of nb: the rest of a tile takes each panel, everything right of it the whole tile."""
+    rows = {k[1:]: v[0] for k, v in table.items() if k[0] == "m"}
+    assert len(rows) > 40
+    for (n, nb, w), reserved in rows.items():
+        most = 0
+        for j in range(0, n, w):
+            end, tile = min(j + w, n), min(j // nb * nb + nb, n)
+            if end < n:
+                k = end - j if end < tile else tile - j // nb * nb
+                most = max(most, -(-(n - end) // 128) * 128 * min(k, 512) * 8)
+        assert most <= reserved, (n, nb, w)
+        assert reserved <= -(-n // 128) * 128 * min(nb, 512) * 8
+
+
+def test_the_buffer_is_reserved_before_the_look_ahead():
+    text = open(os.path.join(CSRC, "mixed.cu")).read()
+    body = text[text.index("int factor_f32(ooc_factor* F") : text.index("int factor_f32_lb(")]
+    assert 0 < body.index("F->work.ensure(syrk32_largest(") < body.index("for (int j = 0; j < bb; j++)")
