@@ -10,8 +10,11 @@
 // the others as packets: 64-bit words of 32 data bits and a 32-bit tag (the launch's epoch), so
 // the arrival of the data is its own flag and one L2 round trip passes it on.
 // Bound by that chain: 2.2 us per 128 rows in FP32 (0.69 ms for both sweeps at n = 20000, where
-// the launches per panel took 1.7 ms), 5.7 us per 64 rows in FP64, most of it the FP64 pipe of one
-// SM (1.47 ms at n = 8192 with four right-hand sides); the factor streams from HBM beside it.
+// the launches per panel took 1.7 ms), 3.1 us per 64 rows in FP64, two thirds of it the FP64 pipe of one SM
+// (0.58 ms for both sweeps at n = 6000, 0.67 by launches per panel of 512 columns and 0.73 with L^T's
+// sums by shuffles, an addition chain per block and the words of a number polled one after the other); the
+// factor streams from HBM beside it.  Several right-hand sides in FP64 are bound by the FP64 pipe: 16 at
+// n = 30000 take 37 ms (40.7 by launches per panel).
 // Sums are block by block in a fixed order, so results do not depend on scheduling.
 //
 // Every wait is bounded: one that runs out raises the buffer's error word, which ends the
@@ -51,9 +54,11 @@ __device__ __forceinline__ unsigned long long pack(uint32_t bits, unsigned tag) 
 __device__ __forceinline__ void send(unsigned long long* x, i64 at, float v, unsigned tag) {
   st_packet(x + at, pack(__float_as_uint(v), tag));
 }
+// The two words of a double go and come together (each has its tag, so they may still arrive apart).
 __device__ __forceinline__ void send(unsigned long long* x, i64 at, double v, unsigned tag) {
-  st_packet(x + 2 * at, pack((uint32_t)__double2loint(v), tag));
-  st_packet(x + 2 * at + 1, pack((uint32_t)__double2hiint(v), tag));
+  asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};\n" ::"l"(x + 2 * at), "l"(pack((uint32_t)__double2loint(v), tag)),
+               "l"(pack((uint32_t)__double2hiint(v), tag))
+               : "memory");
 }
 // One word, waiting (bounded) for its tag; 0 when the wait ends without it.
 __device__ __forceinline__ uint32_t take(const unsigned long long* p, unsigned tag, int* ctl) {
@@ -69,8 +74,14 @@ __device__ __forceinline__ float receive(const unsigned long long* x, i64 at, un
   return __uint_as_float(take(x + at, tag, ctl));
 }
 __device__ __forceinline__ double receive(const unsigned long long* x, i64 at, unsigned tag, int* ctl, double) {
-  const uint32_t lo = take(x + 2 * at, tag, ctl), hi = take(x + 2 * at + 1, tag, ctl);
-  return __hiloint2double((int)hi, (int)lo);
+  for (unsigned i = 0; i < TS_POLLS; i++) {
+    unsigned long long lo, hi;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];\n" : "=l"(lo), "=l"(hi) : "l"(x + 2 * at) : "memory");
+    if ((unsigned)(lo >> 32) == tag && (unsigned)(hi >> 32) == tag) return __hiloint2double((int)(uint32_t)hi, (int)(uint32_t)lo);
+    if ((i & 63) == 63 && *(volatile int*)(ctl + 1)) return 0.0;
+  }
+  atomicExch(ctl + 1, 1);
+  return 0.0;
 }
 
 // Rows of block b: start, count, and its diagonal inverse (ld).
@@ -127,7 +138,7 @@ __device__ __forceinline__ int warp_transpose_sum(T (&v)[V], int lane) {
 }
 
 template <typename T, int R>
-__global__ void __launch_bounds__(Cfg<T>::BS * 4, sizeof(T) == 8 ? 2 : 1)
+__global__ void __launch_bounds__(Cfg<T>::BS * 4)
     k_trsolve(const __grid_constant__ TriSolve<T> a, int nblk, int ngrp, unsigned long long* __restrict__ xch, int* ctl,
               unsigned tag) {
   constexpr int BS = Cfg<T>::BS, NT = BS * 4, KS = BS / 4, NW = NT / 32, CPW = BS / NW, RPL = BS / 32;
@@ -332,6 +343,138 @@ __global__ void __launch_bounds__(Cfg<T>::BS * 4, sizeof(T) == 8 ? 2 : 1)
   }
 }
 
+// FP64, one right-hand side per task.  A block step is 64 x 64 products with L and with the inverse on one SM's
+// FP64 pipe (1.75 FMAs per clock, a warp-wide instruction every 64 clocks of a sub-partition), so the chain has nothing
+// in it but the FMAs of the last block and of the inverse, and eight additions: the other blocks' sums are put
+// together while the last block is waited for, L^T's elements go through shared memory to the thread (row of the
+// result, slice of 16 columns) that sums them, the next block's loads are in flight meanwhile, and a half of the
+// inverse's triangle is cut so that each sub-partition has 24 of its FMAs.
+__global__ void __launch_bounds__(256, 2)
+    k_trsolve_f64(const __grid_constant__ TriSolve<double> a, int nblk, unsigned long long* __restrict__ xch, int* ctl,
+                  unsigned tag) {
+  constexpr int BS = 64, KS = 16, LD = BS + 1;
+  constexpr int FOLD = 4;  // blocks summed before they join the row's sum
+  __shared__ double Lt[BS * LD];  // L^T of a block, Lt[column * LD + row]
+  __shared__ double xs[2][BS], red[4 * BS], ys[BS];
+  __shared__ int s_ticket;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int half = warp >> 2, slice = warp & 3, row = lane + 32 * half;
+  const int nsw = a.sweeps == 3 ? 2 : 1;
+  const int total = nsw * nblk * a.r;
+  const i64 dir_words = 2 * (i64)a.n * a.r;
+  for (;;) {
+    __syncthreads();
+    if (t == 0) s_ticket = atomicAdd(ctl, 1);
+    __syncthreads();
+    const int tk = s_ticket;
+    if (tk >= total || *(volatile int*)(ctl + 1)) {
+      // the last CTA to stop leaves the counter at zero for the next launch
+      if (t == 0 && atomicAdd(ctl + 2, 1) == (int)gridDim.x - 1) {
+        ctl[0] = 0;
+        ctl[2] = 0;
+      }
+      return;
+    }
+    const int q = tk % a.r, u = tk / a.r;  // (right-hand sides side by side: L comes from L2 for all but one)
+    const bool fwd = a.sweeps != 2 && u < nblk;
+    const int i = fwd ? u : (nsw * nblk - 1 - u);
+    i64 si;
+    int mi, ldu;
+    const double* U;
+    block_of(a, i, &si, &mi, &U, &ldu);
+    unsigned long long* out = xch + (fwd || nsw == 1 ? 0 : dir_words);
+    double* Bq = a.B + (i64)q * a.ldb;
+    // the thread's elements of the inverse: forward columns k <= row of U^T, backward k >= row of U
+    const bool whole = fwd == (half == 1);  // 16 columns, else 8 of the 32 that the triangle leaves
+    const int kd = whole ? KS * slice : (fwd ? 8 * slice : 32 + 8 * slice);
+    double dr[KS];
+#pragma unroll
+    for (int k = 0; k < KS; k++) {
+      const int kk = kd + k;
+      dr[k] = 0.0;
+      if ((k < 8 || whole) && row < mi && kk < mi && (fwd ? kk <= row : kk >= row))
+        dr[k] = fwd ? U[kk + (i64)row * ldu] : U[row + (i64)kk * ldu];
+    }
+    // block j of L as it lies in memory: forward the thread's own elements, backward rows lane and lane + 32 of
+    // eight columns
+    double nx[KS];
+    auto load = [&](int j) {
+      i64 sj;
+      int mj, l2;
+      const double* u2;
+      block_of(a, j, &sj, &mj, &u2, &l2);
+      if (fwd) {
+        const double* p = a.L + si + (row < mi ? row : 0) + (sj + KS * slice) * a.ldl;
+#pragma unroll
+        for (int k = 0; k < KS; k++) nx[k] = row < mi && KS * slice + k < mj ? p[k * a.ldl] : 0.0;
+      } else {
+        const double* p = a.L + sj + (si + 8 * warp) * a.ldl;
+#pragma unroll
+        for (int k = 0; k < KS; k++) {
+          const int c = k >> 1, r = lane + 32 * (k & 1);
+          nx[k] = r < mj && 8 * warp + c < mi ? p[r + c * a.ldl] : 0.0;
+        }
+      }
+    };
+    const int steps = fwd ? i : nblk - 1 - i;
+    if (steps > 0) load(fwd ? 0 : nblk - 1);
+    // b (forward) or y (backward), off the chain; it meets the sums once, at the end, so that they are rounded to
+    // their own size
+    double rhs = 0.0, acc = 0.0, p = 0.0;
+    if (t < mi) rhs = fwd || nsw == 1 ? Bq[si + t] : receive(xch, (i64)q * a.n + si + t, tag, ctl, 0.0);
+    for (int st = 0; st < steps; st++) {
+      const int j = fwd ? st : nblk - 1 - st;
+      double l[KS];
+      if (fwd) {
+#pragma unroll
+        for (int k = 0; k < KS; k++) l[k] = nx[k];
+      } else {
+        // (the last block's elements were read before the barrier that followed)
+#pragma unroll
+        for (int k = 0; k < KS; k++) Lt[(8 * warp + (k >> 1)) * LD + lane + 32 * (k & 1)] = nx[k];
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < KS; k++) l[k] = Lt[row * LD + KS * slice + k];
+      }
+      if ((st & (FOLD - 1)) == 0 || st + 1 == steps) {
+        acc += p;
+        p = 0.0;
+      }
+      if (st + 1 < steps) load(fwd ? j + 1 : j - 1);
+      if (t < BS) {
+        i64 sj;
+        int mj, l2;
+        const double* u2;
+        block_of(a, j, &sj, &mj, &u2, &l2);
+        xs[st & 1][t] = t < mj ? receive(out, (i64)q * a.n + sj + t, tag, ctl, 0.0) : 0.0;
+      }
+      __syncthreads();
+      const double* x = xs[st & 1] + KS * slice;
+#pragma unroll
+      for (int k = 0; k < KS; k++) p = fma(l[k], x[k], p);
+    }
+    red[slice * BS + row] = acc + p;
+    __syncthreads();
+    if (t < BS) ys[t] = t < mi ? rhs - ((red[t] + red[BS + t]) + (red[2 * BS + t] + red[3 * BS + t])) : 0.0;
+    __syncthreads();
+    p = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) p = fma(dr[k], ys[kd + k], p);
+    if (whole) {
+#pragma unroll
+      for (int k = 8; k < KS; k++) p = fma(dr[k], ys[kd + k], p);
+    }
+    // (red was last read before the barrier above)
+    red[slice * BS + row] = p;
+    __syncthreads();
+    if (t < mi) {
+      const double x = (red[t] + red[BS + t]) + (red[2 * BS + t] + red[3 * BS + t]);
+      send(out, (i64)q * a.n + si + t, x, tag);
+      if (!fwd || nsw == 1) Bq[si + t] = x;
+    }
+  }
+}
+
 template <typename T, int R>
 int launch_r(const TriSolve<T>& a, int nblk, int ngrp, void* exchange, unsigned epoch, cudaStream_t s) {
   constexpr int BS = Cfg<T>::BS;
@@ -341,8 +484,7 @@ int launch_r(const TriSolve<T>& a, int nblk, int ngrp, void* exchange, unsigned 
   OOC_CUDA_TRY(cudaGetDevice(&dev));
   OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int tasks = nblk * ngrp;  // tasks of one sweep
-  // FP64: two CTAs per SM, one's products beside the other's round trips
-  k_trsolve<T, R><<<std::max(1, std::min(tasks, (sizeof(T) == 8 ? 2 : 1) * nsm)), BS * 4, smem, s>>>(
+  k_trsolve<T, R><<<std::max(1, std::min(tasks, nsm)), BS * 4, smem, s>>>(
       a, nblk, ngrp, (unsigned long long*)((char*)exchange + TS_CTL), (int*)exchange, epoch);
   OOC_CUDA_TRY(cudaGetLastError());
   return OOC_OK;
@@ -384,12 +526,16 @@ int launch_trsolve(const TriSolve<T>& a, void* exchange, unsigned epoch, cudaStr
   //                      n = 30000 r = 8 6238 3542 2381 2676, r = 16 11591 6503 4005 3703
   const int r = b.r;
   if (nblk * r * 2 > 0x3fffffff) return OOC_ERR_INTERNAL;
+  int dev = 0, nsm = 0;
+  OOC_CUDA_TRY(cudaGetDevice(&dev));
+  OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   if constexpr (sizeof(T) == 8) {
-    return launch_r<T, 1>(b, (int)nblk, r, exchange, epoch, s);
+    // two CTAs per SM, one's products beside the other's round trips
+    k_trsolve_f64<<<(unsigned)std::min<i64>(nblk * r, 2 * nsm), 256, 0, s>>>(
+        b, (int)nblk, (unsigned long long*)((char*)exchange + TS_CTL), (int*)exchange, epoch);
+    OOC_CUDA_TRY(cudaGetLastError());
+    return OOC_OK;
   } else {
-    int dev = 0, nsm = 0;
-    OOC_CUDA_TRY(cudaGetDevice(&dev));
-    OOC_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     auto groups = [&](int R) { return (r + R - 1) / R; };
     if (r == 1 || nblk * r <= nsm) return launch_r<T, 1>(b, (int)nblk, r, exchange, epoch, s);
     if (r == 2 || 4 * nblk * groups(2) <= 5 * nsm) return launch_r<T, 2>(b, (int)nblk, groups(2), exchange, epoch, s);
