@@ -189,7 +189,7 @@ class Result:
 
 def _int_table(values, count: int, dtype):
     """`values` (anything that int() takes, one by one) as an array of `count` integers, zeros after the last.  Lists and
-    arrays of integers are converted at once: 4000 systems took 1.2 ms as Python integers one by one."""
+    arrays of integers are converted at once (4000 of each of three tables took 1.2 ms as Python integers one by one)."""
     import numpy as np
 
     v = None
@@ -353,19 +353,25 @@ class Handle:
         import numpy as np
 
         count = len(ns)
-        n_arr, ao, bo = (_int_table(v, count, t) for v, t in ((ns, np.int32), (a_off, np.int64), (b_off, np.int64)))
-        info = np.zeros(max(count, 1), dtype=np.int32)
+        tables = (ns, ctypes.c_int), (a_off, ctypes.c_int64), (b_off, ctypes.c_int64)
+        if count <= 32:  # (a few systems: 2 to 30 us as Python integers, 17 to 36 as arrays)
+            args = [(t * count)(*[int(x) for x in v]) for v, t in tables]
+            info = (ctypes.c_int * count)()
+            args.append(info)
+        else:
+            arrays = [_int_table(v, count, np.dtype(t)) for v, t in tables]
+            info = np.zeros(count, dtype=np.int32)
+            args = [v.ctypes.data_as(ctypes.POINTER(t)) for v, t in zip(arrays + [info], [t for _, t in tables] + [ctypes.c_int])]
         tbl = None
         if blk_table is not None:
             tbl = (ctypes.c_int * 16)(*[int(x) for x in blk_table])
         sec = ctypes.c_double(0)
         self._after_torch(A, B)
         fn = load().ooc_batched_dposv if prec == "fp64" else load().ooc_batched_sposv
-        i32, i64 = ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int64)
-        _check(fn(self._h, count, n_arr.ctypes.data_as(i32), ao.ctypes.data_as(i64), bo.ctypes.data_as(i64), _ptr(A), _ptr(B),
-                  info.ctypes.data_as(i32), tbl, ctypes.c_int(ctas_per_sm), ctypes.byref(sec)),
+        n_arr, ao, bo, infos = args
+        _check(fn(self._h, count, n_arr, ao, bo, _ptr(A), _ptr(B), infos, tbl, ctypes.c_int(ctas_per_sm), ctypes.byref(sec)),
                "ooc_batched_posv")
-        return info[:count].tolist(), sec.value
+        return list(info) if count <= 32 else info.tolist(), sec.value
 
     def fp64_peak(self, ms: float = 200.0) -> float:
         r = ctypes.c_double()
