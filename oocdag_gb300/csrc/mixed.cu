@@ -1731,7 +1731,8 @@ __global__ void k_take_shift(const int* __restrict__ t_of, int* __restrict__ shi
 //   n = 4096   r = 16        1.42 / 0.76     1.30 / 0.58    r = 2  0.54 / 0.52  0.43 / 0.35  r = 1  0.39 / 0.51  0.26 / 0.32
 //   n = 3072                                                r = 2  0.40 / 0.42  0.33 / 0.28
 //   n = 2048   r = 5         0.72 / 0.41     0.64 / 0.29    r = 3  0.35 / 0.34  0.26 / 0.22  r = 2  0.32 / 0.33  0.25 / 0.24
-// One right-hand side has too few FMAs for the planes to pay.
+// One right-hand side has too few FMAs for the planes to pay; two to four where the planes are made again for every
+// residual: refinement at n = 50000, ms for r = 2, 4, 8 72, 75, 249 and 77, 78, 84.
 // The one shift per row suits solutions whose columns are of a kind.  Columns graded differently leave X 2^-shift
 // uneven in some column and run (fp64_tc.cu), which raises `wide`: the caller forms such a residual by symv_lower.
 bool symm_by_digits(i64 n, int r) { return r >= 2 && n >= (r == 2 ? 3072 : 2048); }
@@ -1745,7 +1746,7 @@ struct SymmDigits {
   int* status;    // of the products; the word after it: X was too uneven for them
   DigitCheck chk; // of X
 };
-// OOC_ERR_NOMEM without room for the planes.
+// OOC_ERR_NOMEM without room for the planes, or for enough of them to pay.
 int symm_digits_begin(SymmDigits* D, DevBuf& buf, int n, int r, cudaStream_t s) {
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
   D->sa = up(digit_plane_bytes(n, DIGIT_K));
@@ -1757,6 +1758,7 @@ int symm_digits_begin(SymmDigits* D, DevBuf& buf, int n, int r, cudaStream_t s) 
   D->kept = (D->sa + D->sx) * nrun <= SYMM_KEEP;
   if (D->kept) rc = buf.ensure((D->sa + D->sx) * nrun + rest);
   if (rc) D->kept = false;
+  if (!D->kept && r <= 4) return OOC_ERR_NOMEM;
   D->runs = D->kept ? nrun : (int)std::max<size_t>(1, std::min<size_t>(nrun, SYMM_CHUNK / (D->sa + D->sx)));
   if (rc && buf.ensure((D->sa + D->sx) * D->runs + rest)) return OOC_ERR_NOMEM;
   D->pa = (char*)buf.p;
@@ -3420,47 +3422,51 @@ extern "C" int ooc_dsyrk_ln(ooc_handle* h, int prec, int n, int k, const double*
   if (n == 0 || k == 0) return OOC_OK;
   cudaSetDevice(ooc_device(h));
   cudaStream_t s = ooc_compute_stream(h);
-  int* status = nullptr;
-  if (cudaMalloc(&status, sizeof(int)) != cudaSuccess) { cudaGetLastError(); return OOC_ERR_NOMEM; }
-  cudaMemsetAsync(status, 0, sizeof(int), s);
-  DevBuf work;
+  DevBuf work, small;
   int rc;
+  int word[2] = {0, 0};  // status, operand too uneven for digits
+  bool read = false;     // word holds the call's final status
   const int group = std::min(k, DIGIT_RUNS * DIGIT_K);
   const size_t slot = (digit_plane_bytes(n, std::min(k, DIGIT_K)) + 255) / 256 * 256;
-  const size_t planes = slot * ((group + DIGIT_K - 1) / DIGIT_K), notes = digit_check_bytes(n, group), cols = digit_cols_bytes(k);
-  if (prec == OOC_PREC_FP64 && n > 64 && k >= 16 && !work.ensure(planes + notes + cols + 256)) {
-    // digit products on the tensor cores (from one block and half a stage on: fp64_tc.cu); the columns from
-    // the first group on in which the caller's rows are too uneven for them on the FP64 pipe
+  const size_t planes = slot * ((group + DIGIT_K - 1) / DIGIT_K), notes = digit_check_bytes(n, group);
+  const size_t cols = (digit_cols_bytes(k) + 255) / 256 * 256;
+  // From 2^18 products on: us per call by FP64 MMAs and by digits, n = 65, k = 16 65, 72; 128, 64 76, 76; 256, 32 65, 74; 256,
+  // 128 93, 86; 400, 100 120, 87; 1000, 16 81, 75; 4096, 16 353, 148.  (Half of a small call is its allocation: one either way.)
+  const bool digits = prec == OOC_PREC_FP64 && n > 64 && k >= 16 && (double)n * n * k >= 262144.0 &&
+                      work.ensure(256 + cols + notes + planes) == OOC_OK;
+  if (!digits && small.ensure(256)) return OOC_ERR_NOMEM;
+  int* status = (int*)(digits ? work.p : small.p);
+  cudaMemsetAsync(status, 0, digits ? 256 + cols : 2 * sizeof(int), s);
+  if (digits) {
+    // digit products on the tensor cores (fp64_tc.cu); the columns from the first group on in which the
+    // caller's rows are too uneven for them on the FP64 pipe
     const int nb = (n + 63) / 64 * 64;  // one tile
-    char* base = (char*)work.p;
-    int* flag = (int*)(base + planes + notes + cols);
-    int wide = 0;
-    cudaMemsetAsync(base + planes + notes, 0, cols + 256, s);
+    char* base = (char*)work.p + 256;   // columns' notes, rows' notes, planes
     rc = OOC_OK;
-    for (int k0 = 0; k0 < k && !rc && !wide; k0 += DIGIT_RUNS * DIGIT_K) {
+    for (int k0 = 0; k0 < k && !rc && !word[1]; k0 += DIGIT_RUNS * DIGIT_K) {
       const double* Ak = A + (i64)k0 * lda;
-      DigitRuns D{Ak, lda, nb, nb, 0, n, std::min(DIGIT_RUNS * DIGIT_K, k - k0), base, slot, {}};
-      D.chk = DigitCheck{(uint32_t*)(base + planes), (uint32_t*)(base + planes + notes + digit_cols_bytes(k0)), flag};
+      DigitRuns D{Ak, lda, nb, nb, 0, n, std::min(DIGIT_RUNS * DIGIT_K, k - k0), base + cols + notes, slot, {}};
+      D.chk = DigitCheck{(uint32_t*)(base + cols), (uint32_t*)(base + digit_cols_bytes(k0)), status + 1};
       rc = launch_digits(D, status, s);
       if (!rc) rc = launch_digit_check(D, D, s);
       if (!rc) rc = launch_digit_update(D, TileMap{C, ldc, 0, 1, nb}, 0, n, status, s);
-      if (!rc) rc = read_int(flag, &wide, s);
-      if (!rc && wide) rc = launch_gemm_nt(Ak, lda, Ak, lda, C, ldc, n, n, k - k0, 1, -1.0, status, s);
+      if (!rc && cudaMemcpyAsync(word, status, sizeof(word), cudaMemcpyDeviceToHost, s) != cudaSuccess) rc = OOC_ERR_CUDA;
+      if (!rc && cudaStreamSynchronize(s) != cudaSuccess) rc = OOC_ERR_CUDA;
+      read = !word[1];
+      if (!rc && word[1]) rc = launch_gemm_nt(Ak, lda, Ak, lda, C, ldc, n, n, k - k0, 1, -1.0, status, s);
     }
   } else if (prec == OOC_PREC_FP64) {
     rc = launch_gemm_nt(A, lda, A, lda, C, ldc, n, n, k, 1, -1.0, status, s);
   } else {
     rc = syrk_lowprec(prec, A, lda, C, ldc, n, k, status, s, work);
   }
-  int st = 0;
-  if (!rc) rc = read_int(status, &st, s);
+  if (!rc && !read) rc = read_int(status, word, s);
   if (!rc) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { ooc_set_last_error(e, "ooc_dsyrk_ln", __FILE__, __LINE__); rc = OOC_ERR_CUDA; }
   }
-  cudaFree(status);
   if (rc) return rc;
-  return st == 0 ? OOC_OK : OOC_ERR_TIMEOUT;
+  return word[0] == 0 ? OOC_OK : OOC_ERR_TIMEOUT;
 }
 
 // ---------------------------------------------------------------------------------
