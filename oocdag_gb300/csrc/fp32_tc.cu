@@ -51,7 +51,8 @@ struct Op32 {
 // CTA: 32 rows x one run; thread (row, stage of 32 columns).
 __global__ void __launch_bounds__(256) k_digits32(const Op32 o, uint8_t* __restrict__ planes, int* __restrict__ exps,
                                                   const int* status) {
-  if (status && *(volatile const int*)status) return;
+  // (one answer for the CTA: the next diagonal tile beside this kernel may set it)
+  if (__syncthreads_or(status ? *(volatile const int*)status : 0)) return;
   __shared__ int smax[FRUN][32];
   const int rl = threadIdx.x & 31, cg = threadIdx.x >> 5;
   const int row = blockIdx.x * 32 + rl, run = blockIdx.y;
@@ -135,7 +136,7 @@ __device__ __noinline__ float plain_sum(const Op32& A, int run, int r, int c) {
 __global__ void __launch_bounds__(F_THREADS, 1)
     k_digit32(const __grid_constant__ Op32 X, float* __restrict__ C, i64 ldc, int T, int bj_lo, int bj_hi, i64 nblk,
               int* status) {
-  if (*(volatile int*)status) return;
+  if (__syncthreads_or(*(volatile int*)status)) return;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + F_STAGES * F_STAGE);

@@ -321,7 +321,9 @@ __global__ void __launch_bounds__(D_THREADS, 1)
   asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
   const uint32_t tmem = *tmem_slot;
   pdl_wait();  // (the set-up above touches no other kernel's data)
-  if (*(volatile int*)status || (X.unless && *(volatile const int*)X.unless)) nblk = 0;
+  // (one answer for all roles: a kernel beside this one may set the status)
+  const int skip = *(volatile int*)status | (X.unless ? *(volatile const int*)X.unless : 0);
+  if (__syncthreads_or(skip)) nblk = 0;
   auto run_stages = [&](int run) {
     return MODE == UPDATE ? X.nst[run] : run + 1 < X.nrun ? DIGIT_K / DK : (X.K - run * DIGIT_K + DK - 1) / DK;
   };

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     k_syrk_bf16x3(const __grid_constant__ CUtensorMap map_hi, const __grid_constant__ CUtensorMap map_lo,
                   TC* __restrict__ C, i64 ldc, int m, int Kp, int T, int bj_lo, int bj_hi, i64 nblk,
                   int* status) {
-  if (*(volatile int*)status) return;
+  if (__syncthreads_or(*(volatile int*)status)) return;  // (one answer for the CTA: a kernel beside this one may set it)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);  // TMA -> MMA, per stage
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(THREADS2, 1)
                    const __grid_constant__ CUtensorMap map_c, int m, int Kp, int T, int bj_lo, int bj_hi, i64 nblk,
                    unsigned long long* __restrict__ tickets, int* status) {
   static_assert(sizeof(TC) == 4, "the reduction epilogue adds into FP32 C");
-  if (*(volatile int*)status) return;
+  if (__syncthreads_or(*(volatile int*)status)) return;  // (one answer for the CTA: a kernel beside this one may set it)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + STAGES2 * STAGE2_BYTES);
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(THREADS2, 1)
                     const __grid_constant__ CUtensorMap map_bhi, const __grid_constant__ CUtensorMap map_blo,
                     const __grid_constant__ CUtensorMap map_c, int m, int Kp, int T, int bj_lo, int bj_hi, i64 nblk,
                     unsigned long long* __restrict__ tickets, int* status) {
-  if (*(volatile int*)status) return;
+  if (__syncthreads_or(*(volatile int*)status)) return;  // (one answer for the CTA: a kernel beside this one may set it)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + STAGES_T * STAGE_T_BYTES);
@@ -920,7 +920,7 @@ __global__ void __launch_bounds__(THREADS2, 1)
                    const __grid_constant__ CUtensorMap map_xhi, const __grid_constant__ CUtensorMap map_xlo,
                    float* __restrict__ P, i64 ldp, __nv_bfloat16* __restrict__ shi, __nv_bfloat16* __restrict__ slo,
                    i64 lds, int Kp, int m, int ncb, i64 nblk, unsigned long long* __restrict__ tickets, int* status) {
-  if (*(volatile int*)status) return;
+  if (__syncthreads_or(*(volatile int*)status)) return;  // (one answer for the CTA: a kernel beside this one may set it)
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + STAGES2 * STAGE2_BYTES);

@@ -156,10 +156,10 @@ __global__ void __launch_bounds__(Cfg<T>::BS * 4)
   const i64 dir_words = (i64)a.n * a.r * Cfg<T>::WORDS;
   for (;;) {
     __syncthreads();
-    if (t == 0) s_ticket = atomicAdd(ctl, 1);
+    if (t == 0) s_ticket = *(volatile int*)(ctl + 1) ? total : atomicAdd(ctl, 1);  // (a wait ran out: stop)
     __syncthreads();
     const int tk = s_ticket;
-    if (tk >= total || *(volatile int*)(ctl + 1)) {
+    if (tk >= total) {
       // the last CTA to stop leaves the counter at zero for the next launch
       if (t == 0 && atomicAdd(ctl + 2, 1) == (int)gridDim.x - 1) {
         ctl[0] = 0;
@@ -364,10 +364,10 @@ __global__ void __launch_bounds__(256, 2)
   const i64 dir_words = 2 * (i64)a.n * a.r;
   for (;;) {
     __syncthreads();
-    if (t == 0) s_ticket = atomicAdd(ctl, 1);
+    if (t == 0) s_ticket = *(volatile int*)(ctl + 1) ? total : atomicAdd(ctl, 1);  // (a wait ran out: stop)
     __syncthreads();
     const int tk = s_ticket;
-    if (tk >= total || *(volatile int*)(ctl + 1)) {
+    if (tk >= total) {
       // the last CTA to stop leaves the counter at zero for the next launch
       if (t == 0 && atomicAdd(ctl + 2, 1) == (int)gridDim.x - 1) {
         ctl[0] = 0;

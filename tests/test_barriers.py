@@ -32,6 +32,24 @@ def test_no_barrier_behind_a_condition_of_its_expression(path):
     assert _conditional_barriers(open(path).read()) == []
 
 
+def test_kernels_of_several_roles_read_the_status_word_once_for_the_block():
+    """A kernel whose warps wait for one another on mbarriers must not have some of them leave, or see no work, because the
+    status word was raised (by the diagonal tile on another stream) between two of its threads' reads."""
+    kernels = 0
+    for path in glob.glob(os.path.join(CSRC, "*.cu")):
+        for body in open(path).read().split("__global__")[1:]:
+            if "tcgen05.alloc" not in body:
+                continue
+            kernels += 1
+            lines = [line for line in body.split("// ---- teardown")[0].split("\n") if re.search(r"\*\(volatile (const )?int\*\)status", line)]
+            assert lines
+            for line in lines:
+                assert "__syncthreads_or(" in line or re.match(r"\s*const int skip = ", line), (path, line)
+            if any("const int skip" in line for line in lines):
+                assert "if (__syncthreads_or(skip))" in body
+    assert kernels >= 6
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n", [130, 161, 300])
 def test_zero_subnormal_and_normal_rows_in_one_warp(handle, n):
