@@ -61,7 +61,7 @@ def fp64_update_roofline(tflops, fp64_peak, nb):
                 "peak": fp64_peak, "unit": "TFLOP/s", "frac": tflops / fp64_peak if tflops else None} | pipe
     path = os.path.join(ROOT, "MEASURED_PEAKS.json")
     peak = json.load(open(path)).get("bf16_tflops") if os.path.exists(path) else None
-    return {"bound": "tensor", "kernel": "k_digit_update (tcgen05, exact products of BF16 digits)", "achieved": tflops,
+    return {"bound": "tensor", "kernel": "k_digit_update (tcgen05, products of BF16 digits)", "achieved": tflops,
             "peak": peak / DIGIT_PRODUCTS if peak else None, "unit": "TFLOP/s",
             "frac": tflops * DIGIT_PRODUCTS / peak if tflops and peak else None,
             "peak_source": f"MEASURED_PEAKS.json bf16_tflops / {DIGIT_PRODUCTS} products"} | pipe
@@ -746,7 +746,7 @@ def run_mixed(args):
     upd_roof = {"kernel": "k_syrk2t_bf16x3 (long-K catch-ups: N=256 tcgen05 MMAs, C transposed in TMEM, four-stage "
                           "K=32 operand ring) + k_syrk2_bf16x3<float> (in-block K=256 updates): persistent split-BF16 "
                           "trailing updates, 256x128 blocks, FP32 C updated by TMA reductions"
-                if args.prec == "bf16x3" else "k_digit32 (tcgen05, exact products of BF16 digits of FP32 panels)",
+                if args.prec == "bf16x3" else "k_digit32 (tcgen05, products of BF16 digits of FP32 panels)",
                 "bound": "tensor",
                 "achieved": upd_flops / (upd_ms / 1e3) / 1e12 if upd_ms else None,
                 "peak": bf16_peak, "unit": "TFLOP/s",

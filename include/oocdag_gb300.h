@@ -184,7 +184,7 @@ int ooc_panel_plan(int64_t n, int nb, int64_t memBlock, int nx, int* out, int ca
  * products for OOC_PREC_BF16X3 (nb a multiple of 128).                               */
 enum {
   OOC_PREC_FP64 = 0,  /* FP64 updates (the plain path)                             */
-  OOC_PREC_FP32 = 1,  /* FP32 operands, sums exact or in FP32                       */
+  OOC_PREC_FP32 = 1,  /* FP32 operands, sums of digit products or in FP32           */
   OOC_PREC_BF16X3 = 2 /* hi/lo BF16 splits, 3 tensor-core products, FP32 accumulate */
 };
 

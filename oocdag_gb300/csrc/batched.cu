@@ -312,7 +312,7 @@ __device__ void solve_back_f32(const float* __restrict__ L, int n, float* bs) {
 // ---- FP64 ----------------------------------------------------------------------------
 // One matrix by a CTA of NT threads, in steps of blk columns (8, 16 or 32; KS = K / 16 of a step's
 // products).  The FP64 pipe does ~1.75 FMAs per clock per SM and was all of the time (57 % of its
-// peak), so the n^3 / 6 of the trailing updates go to the tensor cores as exact digit products (the
+// peak), so the n^3 / 6 of the trailing updates go to the tensor cores as digit products (the
 // method: fp64_tc.cu):
 //   1. four warps factor the diagonal block (two 16-column blocks of potrf_panel), from the second
 //      step on inside the previous step's trailing update, while the other warps update the rest;
@@ -325,7 +325,7 @@ __device__ void solve_back_f32(const float* __restrict__ L, int n, float* bs) {
 // mma.sync, not tcgen05: a step's operands are at most 480 rows by 32 columns, written by the CTA's own
 // threads, and its results are wanted in registers at once; 16 x 8 blocks keep the triangle's
 // waste small at these orders.
-// 1200 matrices of 16..512: 5.7 ms against 26.7 ms with FP64 FMAs (7.4 with every class in steps of 32 columns and
+// 1200 matrices of 16..512: 5.3 ms against 26.7 ms with FP64 FMAs (7.4 with every class in steps of 32 columns and
 // no class beside another's tail).
 __device__ __forceinline__ void bar_group() { asm volatile("bar.sync 1, 128;\n" ::: "memory"); }  // warps 0..3
 constexpr int DP = 33;          // column pitch of the diagonal block

@@ -1,4 +1,4 @@
-// FP32 trailing updates on the tensor cores: exact digit products, as for
+// FP32 trailing updates on the tensor cores: digit products, as for
 // FP64 (fp64_tc.cu, where the method is described), with four balanced base-256 digits.
 //
 // With |x(i, k)| < 2^e(i) over a run of at most 256 columns, x(i, k) ~ 2^(e(i) - 31) X with X of 32 bits:

@@ -1,4 +1,4 @@
-// FP32 products on the tensor cores by exact digit products (fp32_tc.cu).
+// FP32 products on the tensor cores by digit products (fp32_tc.cu).
 #pragma once
 
 #include "common.cuh"

@@ -3,7 +3,7 @@
 // GB300 executes FP64 at about 1/1800 of its dense BF16 tensor rate: the measured
 // FP64 DMMA rate is ~1.05 TFLOP/s per GPU (about two FP64 FMAs per clock per SM).  At
 // that rate every FP64 tile operation is bound by the FP64 pipe, not by HBM or shared
-// memory.  The large contractions therefore go to the BF16 tensor cores as exact digit products
+// memory.  The large contractions therefore go to the BF16 tensor cores as digit products
 // (fp64_tc.cu); here are the chain's kernels and the contraction for what digits do not take
 // (tile widths that 64 does not divide, small tile calls, no room for the planes):
 //   * the contraction (gemm / syrk, oocquark.cpp:130,176,222 use cuBLAS there) runs on

@@ -1,5 +1,5 @@
-// FP64 trailing updates on the tensor cores: C -= X X^T in FP64 from exact products of
-// integer digits (the error-free splitting of Ozaki, Ogita, Oishi and Rump, 2012).
+// FP64 trailing updates on the tensor cores: C -= X X^T in FP64 from products of
+// integer digits (the splitting of Ozaki, Ogita, Oishi and Rump, 2012).
 //
 // The FP64 pipe of this part does ~1.7 FMAs per clock per SM (1.05 TFLOP/s in all), the
 // BF16 tensor pipe ~1900 times as much.  So a run of at most 128 columns of X is rewritten

@@ -1,4 +1,4 @@
-// FP64 updates on the tensor cores by exact digit products (fp64_tc.cu).
+// FP64 updates on the tensor cores by digit products (fp64_tc.cu).
 #pragma once
 
 #include <cstdint>

@@ -8,7 +8,7 @@
 //                    256 columns, held in shared memory; k_diag_f32 for wider ones);
 //   column solve   : the panel times the tile's inverse, in FP32 (k_colsolve_f32) or as
 //                    three split-BF16 tensor-core products (k_trsm2_bf16x3, tc_bf16x3.cu);
-//   trailing update: OOC_PREC_FP32 - exact products of BF16 digits (fp32_tc.cu; k_syrk_f32 on
+//   trailing update: OOC_PREC_FP32 - products of BF16 digits (fp32_tc.cu; k_syrk_f32 on
 //                    the FP32 pipe for a few columns or without room for the digits);
 //                    OOC_PREC_BF16X3 - hi/lo BF16 planes of the panel, three tensor-core
 //                    products (hi*hi + hi*lo + lo*hi) accumulated in FP32 in TMEM and added
@@ -1363,7 +1363,7 @@ int syrk_lowprec(int prec, const double* X, i64 ldx, double* C, i64 ldc, int m, 
   return OOC_ERR_UNSUPPORTED;
 }
 
-// FP32 products as exact digit products (fp32_tc.cu): from K = 16 and half a block on.
+// FP32 products as digit products (fp32_tc.cu): from K = 16 and half a block on.
 constexpr int DIGIT32_MIN_K = 16, DIGIT32_CHUNK = 512;
 
 // The same for the FP32 working matrix of a reduced-precision factor: C (FP32) -= X X^T
