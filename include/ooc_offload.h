@@ -14,7 +14,7 @@
  *     digit products on the tensor cores or DMMA, device potrf, blocked column solve); no
  *     cuBLAS/cuSOLVER.  A product's error is bounded like that of an FP64 sum, by a multiple of
  *     2^-53 sum |a| |b|: the tensor cores take operands whose rows are even in size (at most
- *     2^-43 sum |a| |b|, and less than an FP64 sum's error for uniform or normal values), DMMA the others.
+ *     2^-41 sum |a| |b|, and less than an FP64 sum's error for uniform or normal values), DMMA the others.
  * MKL_INT is the LP64 int.  All functions have C linkage (the reference's were C++ except
  * offload_init_/offload_destroy_).  Errors: the BLAS-style calls return void as in the
  * reference; ooc_offload_last_error() reports the last failure (0 = none).

@@ -30,8 +30,9 @@
 // k_uneven counts.  If both rows have 5/8 of the columns that matter (not all zero in either operand) there, at
 // least a quarter of these have a product of at least 2^(e(i) + e(j) - 10), so the loss, 2^-55 of 2^(e(i) + e(j)) per
 // column, stays below 2^-43 of sum |a| |b| whatever the values; for uniform and normal ones it is below what an FP64
-// sum rounds off.  A last run of at most 32 columns is too short to count: its rows have to be within a
-// factor of 2 of the run before it, whose sum then covers its loss.  Where a row fails, the FP64 pipe takes the product.
+// sum rounds off.  A last run of at most 32 columns is too short to count: after a run with 64 columns that matter its
+// rows have to be within a factor of 2 of that run's, whose sum is then at least 16 2^(e(i) + e(j) - 10) and its loss below 2^-42 of
+// it.  Where a row fails, the FP64 pipe takes the product.
 // 2^-5 and 5/8: of 128 normally distributed elements 80 % or more are that large; a row that is mostly zeros, or a
 // few large elements, fails.
 
@@ -196,20 +197,27 @@ __global__ void __launch_bounds__(128) k_uneven(const __grid_constant__ UnevenAr
   auto words = [&](int q) { return reinterpret_cast<const uint4*>(a.large[z])[(i64)q * a.pad[z] + row]; };
   const uint4 l = words(run);
   if (!(l.x | l.y | l.z | l.w)) return;  // a row of zeros
+  // columns of run q that are not all zero in either operand, and how many of them `w` marks
+  auto count = [&](int q, const uint4& w, int* marked) {
+    const uint32_t lw[W] = {w.x, w.y, w.z, w.w};
+    int n = 0;
+    *marked = 0;
+#pragma unroll
+    for (int i = 0; i < W; i++) {
+      const uint32_t both = a.cols[0][q * W + i] & a.cols[1][q * W + i];
+      n += __popc(both);
+      *marked += __popc(lw[i] & both);
+    }
+    return n;
+  };
+  int c;
   bool ok;
-  if (run > 0 && a.K - run * DIGIT_K <= SHORT_RUN) {
-    const uint4 b = words(run - 1);
+  const uint4 b = run > 0 ? words(run - 1) : make_uint4(0, 0, 0, 0);
+  if (run > 0 && a.K - run * DIGIT_K <= SHORT_RUN && count(run - 1, b, &c) >= DIGIT_K / 2) {
     ok = (b.x | b.y | b.z | b.w) && a.last_exps[z][row] <= a.exps[z][(run - 1) * a.step[z] + row] + 1;
     ok = ok || a.last_exps[z][row] == EXP_NONFINITE;
   } else {
-    const uint32_t lw[W] = {l.x, l.y, l.z, l.w};
-    int n = 0, c = 0;
-#pragma unroll
-    for (int q = 0; q < W; q++) {
-      const uint32_t both = a.cols[0][run * W + q] & a.cols[1][run * W + q];
-      n += __popc(both);
-      c += __popc(lw[q] & both);
-    }
+    const int n = count(run, l, &c);
     ok = 8 * c >= 5 * n;
   }
   if (!ok) *a.wide = 1;

@@ -45,6 +45,13 @@ def _operands(kind, m, n, k, rng):
         A[:, -2:] = [0.0, 2.0**40]
         B[:, -2:] = [1.0, 2.0**-60]
         A[:, :-2] *= 2.0**-40
+    elif kind == "tail after zeros":  # a last run whose predecessor has eight columns, one of them 2^5 times the others
+        A[:, : k - k % 128 - 8 if k > 128 else 0] = 0.0
+        B[:, : k - k % 128 - 8 if k > 128 else 0] = 0.0
+        A, B = A * 2.0**-5, B * 2.0**-5
+        if k > 128:
+            A[:, k - k % 128 - 8] = 1.0
+            B[:, k - k % 128 - 7] = 1.0
     elif kind == "subnormal":
         A, B = A * 2.0**-1040, B * 2.0**1000
     elif kind == "zero rows":
@@ -53,7 +60,7 @@ def _operands(kind, m, n, k, rng):
     return A, B
 
 
-KINDS = ["uniform", "normal", "alternating", "graded", "mildly graded", "few large", "sparse", "one bad row", "tail", "subnormal", "zero rows"]
+KINDS = ["uniform", "normal", "alternating", "graded", "mildly graded", "few large", "sparse", "one bad row", "tail", "tail after zeros", "subnormal", "zero rows"]
 SHAPES = [(128, 128, 128), (72, 130, 257), (150, 100, 160), (129, 140, 130), (64, 65, 517), (300, 8, 1040)]
 
 
