@@ -147,13 +147,17 @@ __device__ __forceinline__ void digit_rows(const DigitArgs& a, int run) {
   if (st == 0 && ch == 0) exps[row] = bmax >= EXP_NONFINITE ? EXP_NONFINITE : e;
   if constexpr (CHECK) {
     uint32_t large = 0, some = 0;
+    int least = bmax;
 #pragma unroll
     for (int k = 0; k < KT; k++)
       if (v[k] << 1) {
         some |= 1u << (KT * ch + k);
-        if (true_exponent(v[k]) + (SHIFT ? sft[SHIFT ? k : 0] : 0) > bmax - WIDE_BITS) large |= 1u << (KT * ch + k);
+        const int ex = true_exponent(v[k]) + (SHIFT ? sft[SHIFT ? k : 0] : 0);
+        if (ex > bmax - WIDE_BITS) large |= 1u << (KT * ch + k);
+        least = min(least, ex);
       }
     if (bmax >= EXP_NONFINITE) large = ~0u;  // (plain sums: nothing to lose)
+    else if (bmax - least >= a.chk.least) *a.chk.wide = 1;
     large |= __shfl_xor_sync(0xffffffffu, large, 1);
     large |= __shfl_xor_sync(0xffffffffu, large, 2);
     if (ch == 0) a.chk.large[((i64)run * (gridDim.x * 32) + row) * (DIGIT_K / DK) + st] = large;

@@ -16,6 +16,7 @@ struct DigitCheck {
   uint32_t* large = nullptr;
   uint32_t* cols = nullptr;
   int* wide = nullptr;
+  int least = 1 << 20;  // launch_digits itself raises it at an element below 2^-least of its row's scale in a run
 };
 
 // Runs of at most DIGIT_K columns of a column of tiles: element (r, k), r = org .. org + rows - 1,

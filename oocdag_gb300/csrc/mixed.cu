@@ -1734,7 +1734,10 @@ __global__ void k_take_shift(const int* __restrict__ t_of, int* __restrict__ shi
 // One right-hand side has too few FMAs for the planes to pay; two to four where the planes are made again for every
 // residual: refinement at n = 50000, ms for r = 2, 4, 8 72, 75, 249 and 77, 78, 84.
 // The one shift per row suits solutions whose columns are of a kind.  Columns graded differently leave X 2^-shift
-// uneven in some column and run (fp64_tc.cu), which raises `wide`: the caller forms such a residual by symv_lower.
+// uneven in some column and run (fp64_tc.cu), or single elements of it below 2^-SYMM_LEAST of the others (a component
+// rounded to nothing would never converge; a normally distributed X of 10^6 elements has one in 1 of 200
+// cases), which raises `wide`: the caller forms such a residual by symv_lower.
+constexpr int SYMM_LEAST = 30;
 bool symm_by_digits(i64 n, int r) { return r >= 2 && n >= (r == 2 ? 3072 : 2048); }
 constexpr size_t SYMM_KEEP = 16ull << 30, SYMM_CHUNK = 512ull << 20;
 struct SymmDigits {
@@ -1788,6 +1791,7 @@ int symm_digits(const SymmDigits& D, const double* A, i64 lda, const double* X, 
     DigitRuns Dx{X + c0, 1, ldx, 1, 0, r, K, D.px, D.sx, {}, D.shift, -1, 0, c0};
     Dx.chk = D.chk;
     Dx.chk.cols += digit_cols_bytes((int)c0) / sizeof(uint32_t);
+    Dx.chk.least = SYMM_LEAST;
     int rc = launch_digits(Da, D.status, s);
     if (!rc) rc = launch_digits(Dx, D.status, s);
     if (!rc) rc = launch_digit_check(Dx, Dx, s);

@@ -49,3 +49,29 @@ def test_each_half_to_its_own_size(handle, kind, n, r):
         for p in (0, 1):
             scale = X[q, p::2].abs().max().item()
             assert (out - X)[q, p::2].abs().max().item() <= TOL * scale, (q, p)
+
+
+@pytest.mark.parametrize("n,r", [(2048, 3), (3072, 2), (4097, 16)])
+def test_a_quarter_of_the_rows(handle, n, r):
+    """The same with four separate systems, one of them 2^-60 the size of the others in every other column: most elements of a
+    run are of a kind, and the small ones would round to 0 beside them."""
+    import torch
+
+    g = torch.Generator().manual_seed(n * r)
+    A = torch.rand(n, n, generator=g, dtype=torch.float64) * 2 - 1
+    A = torch.tril(A) + torch.tril(A, -1).T
+    k = torch.arange(n)
+    A *= (k[:, None] - k[None, :]) % 4 == 0
+    A.diagonal().copy_(torch.full((n,), 2.0 * n**0.5, dtype=torch.float64))
+    A = A.cuda()
+    X = torch.randint(1, 1 << 20, (r, n), generator=g).double().cuda()
+    X[::2, 1::4] *= 2.0**-60
+    B = (X @ A).contiguous()
+    out = torch.empty_like(B)
+    with handle.factor(A.clone(), n, n, 256, "fp32") as F:
+        assert F.info == 0
+        F.refine(A, n, B, n, out, n, r, 0.0, 6)
+    for q in range(r):
+        for p in range(4):
+            scale = X[q, p::4].abs().max().item()
+            assert (out - X)[q, p::4].abs().max().item() <= TOL * scale, (q, p)
