@@ -43,10 +43,9 @@ def test_kernels_of_several_roles_read_the_status_word_once_for_the_block():
             kernels += 1
             lines = [line for line in body.split("// ---- teardown")[0].split("\n") if re.search(r"\*\(volatile (const )?int\*\)status", line)]
             assert lines
-            for line in lines:
-                assert "__syncthreads_or(" in line or re.match(r"\s*const int skip = ", line), (path, line)
-            if any("const int skip" in line for line in lines):
-                assert "if (__syncthreads_or(skip))" in body
+            for line in lines:  # directly in the block-wide OR, or through a variable
+                name = re.match(r"\s*const int (\w+) = ", line)
+                assert "__syncthreads_or(" in line or (name and f"__syncthreads_or({name.group(1)})" in body), (path, line)
     assert kernels >= 6
 
 

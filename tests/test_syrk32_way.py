@@ -81,16 +81,6 @@ def test_every_choice(table):
         assert (rc, way, held) == want, (limit, serve, aligned)
 
 
-def test_later_ranges_take_the_prepared_way():
-    """Every syrk_f32 call without preparation on an FP32 panel passes the way of the call that prepared it."""
-    text = open(os.path.join(CSRC, "mixed.cu")).read()
-    body = text[text.index("int factor_f32(ooc_factor* F") : text.index("int factor_f32_lb(")]
-    for branch in ("} else if (grouped) {", "} else if (split) {"):
-        part = body[body.index(branch) + len(branch) :]
-        part = part[: part.index("} else")]
-        assert part.count("syrk_f32(") == 2 and part.count("&way") == 2
-
-
 def test_out_of_core_width_and_planes_stay_within_the_budget(table):
     rows = {k[1:]: v for k, v in table.items() if k[0] == "w"}
     assert len(rows) > 500 and {p for _, p in rows.values()} == {0, 1}
@@ -116,9 +106,3 @@ def test_the_first_reservation_holds_every_update(table):
                 most = max(most, -(-(n - end) // 128) * 128 * min(k, 512) * 8)
         assert most <= reserved, (n, nb, w)
         assert reserved <= -(-n // 128) * 128 * min(nb, 512) * 8
-
-
-def test_the_buffer_is_reserved_before_the_look_ahead():
-    text = open(os.path.join(CSRC, "mixed.cu")).read()
-    body = text[text.index("int factor_f32(ooc_factor* F") : text.index("int factor_f32_lb(")]
-    assert 0 < body.index("F->work.ensure(syrk32_largest(") < body.index("for (int j = 0; j < bb; j++)")
